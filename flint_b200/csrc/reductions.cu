@@ -827,63 +827,489 @@ __global__ void __launch_bounds__(kSortThreads)
     }
 }
 
-// offsets[v] = number of sorted tokens below v, for v = 0..vocab (binary search).
-__global__ void __launch_bounds__(256)
-    fb_token_offsets(unsigned* __restrict__ offsets, const uint16_t* __restrict__ sorted_tokens,
-                     size_t rows, unsigned vocab) {
-    const unsigned v = blockIdx.x * 256 + threadIdx.x;
-    if (v > vocab) {
+// ---- embedding backward: two launches --------------------------------------------------
+//
+// The bytes are dwte's 4 * vocab * width written and dx read twice; what the path spent its
+// time on was a chain of nine small launches and, on tokens distributed like text, one CTA
+// that walked the most frequent word's rows one memory latency at a time. So the first
+// launch does everything that does not need the sorted order, with the sort itself on one
+// CTA beside it: that CTA sorts and lists the words in use while the others write dwte's
+// zeros (most of the bytes; the rows in use are written again later) and the position
+// table. The second launch adds up the listed words.
+// 8 x 1,024 tokens x 768, words as frequent as in text: 678 us -> 53 us (prepare 32.6: 188 MB,
+// 5.8 TB/s; words 18.9); uniform tokens 175 us before.
+
+constexpr int kPrepareThreads = 512;
+constexpr int kPrepareWarps = kPrepareThreads / 32;
+// Keys per lane of the one-CTA sort: 32 registers hold 16,384 keys. More rows (or row
+// numbers that do not fit 16 bits) take the multi-launch sort, whose cost then counts less.
+constexpr int kSortSteps = 32;
+constexpr size_t kOneCtaRows = size_t{kPrepareThreads} * kSortSteps;
+constexpr size_t kZeroQuads = size_t{kPrepareThreads} * 8;  // float4s a zeroing CTA writes
+
+// Runs of one token's rows by length: a warp adds a short run whole, a warp per 128 columns
+// a middling one, a CTA per 128 columns a long one.
+constexpr unsigned kMiddleRun = 9;
+constexpr unsigned kLongRun = 96;
+
+// The sorted positions at which runs begin. Short runs from the front of heads[rows], long
+// ones from its back; middling ones (at most rows / 9) in middle[rows / 2].
+struct RunLists {
+    unsigned* heads;
+    unsigned* middle;
+    unsigned* counts;   // short, middling, long
+};
+
+struct PrepareParams {
+    float4* dwte;
+    float4* dwpe;
+    float4* partial;          // position partial sums: cols sums, then cols errors
+    const float4* dx;
+    const uint16_t* tokens;
+    uint16_t* sorted_tokens;
+    unsigned* sorted_rows;
+    RunLists lists;
+    unsigned rows, sequences;
+    unsigned sort_blocks, position_blocks;  // 0 or 1; 0 when launch_partials does the table
+    size_t word_quads, position_quads;
+    bool accumulate_wpe;
+};
+
+// Lists sorted position i if a run begins there. The order in a list is whatever the atomics
+// make it; every run is added up on its own, so no result depends on it.
+template <typename Token>
+__device__ __forceinline__ void list_head(const RunLists& lists, unsigned* counts, size_t i,
+                                          size_t rows, Token token_at) {
+    const unsigned token = token_at(i);
+    if (i > 0 && token_at(i - 1) == token) {
         return;
     }
-    size_t lo = 0;
-    size_t hi = rows;
-    while (lo < hi) {
-        const size_t mid = lo + (hi - lo) / 2;
-        if (sorted_tokens[mid] < v) {
-            lo = mid + 1;
-        } else {
-            hi = mid;
-        }
+    auto reaches = [&](unsigned n) { return i + n <= rows && token_at(i + n - 1) == token; };
+    const unsigned value = static_cast<unsigned>(i);
+    if (!reaches(kMiddleRun)) {
+        lists.heads[atomicAdd(&counts[0], 1u)] = value;
+    } else if (!reaches(kLongRun)) {
+        lists.middle[atomicAdd(&counts[1], 1u)] = value;
+    } else {
+        lists.heads[rows - 1 - atomicAdd(&counts[2], 1u)] = value;
     }
-    offsets[v] = static_cast<unsigned>(lo);
 }
 
-// One CTA per word-table row v; each thread owns float4 columns q, q+128, ...
-// and adds token v's rows of dx in ascending row order with a compensated sum.
-constexpr int kWordThreads = 128;
+__global__ void __launch_bounds__(256)
+    fb_list_heads(const RunLists lists, const uint16_t* __restrict__ sorted_tokens, size_t rows) {
+    const size_t i = size_t{blockIdx.x} * 256 + threadIdx.x;
+    if (i < rows) {
+        list_head(lists, lists.counts, i, rows,
+                  [&](size_t k) -> unsigned { return sorted_tokens[k]; });
+    }
+}
 
-__global__ void __launch_bounds__(kWordThreads)
-    fb_word_gradient(float4* __restrict__ dwte, const float4* __restrict__ dx,
-                     const unsigned* __restrict__ sorted_rows,
-                     const unsigned* __restrict__ offsets, unsigned quads, bool accumulate) {
-    const size_t v = blockIdx.x;
-    const unsigned begin = offsets[v];
-    const unsigned end = offsets[v + 1];
-    if (begin == end && accumulate) {
+// Stable sort of rows <= kOneCtaRows (token, row) pairs packed as token << 16 | row. Warp w
+// owns keys [w * share, (w + 1) * share), 32 at a time in order: the order within a digit is
+// (warp, step, lane), i.e. the input's.
+__device__ void sort_tokens(const PrepareParams& p, unsigned* keys, unsigned (*next)[kDigits],
+                            unsigned* warp_totals) {
+    const int lane = threadIdx.x % 32;
+    const int warp = threadIdx.x / 32;
+    const int steps = static_cast<int>((p.rows + kPrepareThreads - 1) / kPrepareThreads);
+    const unsigned first = static_cast<unsigned>(warp * steps * 32 + lane);
+    unsigned held[kSortSteps];
+#pragma unroll
+    for (int step = 0; step < kSortSteps; ++step) {
+        const unsigned i = first + step * 32;
+        held[step] = 0;
+        if (step < steps && i < p.rows) {
+            held[step] = (static_cast<unsigned>(p.tokens[i]) << 16) | i;
+        }
+    }
+    for (int pass = 0; pass < 2; ++pass) {
+        const int shift = 16 + 8 * pass;
+        for (int i = threadIdx.x; i < kPrepareWarps * kDigits; i += kPrepareThreads) {
+            (&next[0][0])[i] = 0;
+        }
+        __syncthreads();
+        if (pass == 1) {
+#pragma unroll
+            for (int step = 0; step < kSortSteps; ++step) {
+                const unsigned i = first + step * 32;
+                if (step < steps && i < p.rows) {
+                    held[step] = keys[i];
+                }
+            }
+        }
+#pragma unroll
+        for (int step = 0; step < kSortSteps; ++step) {
+            if (step < steps && first + step * 32 < p.rows) {
+                atomicAdd(&next[warp][(held[step] >> shift) & (kDigits - 1)], 1u);
+            }
+        }
+        __syncthreads();
+        // Thread d: digit d's total, its exclusive prefix over the digits, then each warp's start.
+        unsigned total = 0;
+        unsigned inclusive = 0;
+        if (threadIdx.x < kDigits) {
+            for (int w = 0; w < kPrepareWarps; ++w) {
+                total += next[w][threadIdx.x];
+            }
+            inclusive = total;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const unsigned o = __shfl_up_sync(fb::kFullMask, inclusive, off);
+                inclusive += lane >= off ? o : 0;
+            }
+            if (lane == 31) {
+                warp_totals[warp] = inclusive;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < kDigits) {
+            unsigned position = inclusive - total;
+            for (int w = 0; w < warp; ++w) {
+                position += warp_totals[w];
+            }
+            for (int w = 0; w < kPrepareWarps; ++w) {
+                const unsigned c = next[w][threadIdx.x];
+                next[w][threadIdx.x] = position;
+                position += c;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int step = 0; step < kSortSteps; ++step) {
+            if (step < steps) {
+                const bool live = first + step * 32 < p.rows;
+                const unsigned digit = live ? (held[step] >> shift) & (kDigits - 1) : kNoDigit;
+                const unsigned peers = __match_any_sync(fb::kFullMask, digit);
+                if (live) {
+                    const unsigned at = next[warp][digit] + __popc(peers & ((1u << lane) - 1u));
+                    keys[at] = held[step];
+                }
+                __syncwarp();
+                if (live && rank_leader(peers, lane)) {
+                    next[warp][digit] += __popc(peers);
+                }
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < 3) {
+        warp_totals[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    for (unsigned i = threadIdx.x; i < p.rows; i += kPrepareThreads) {
+        p.sorted_tokens[i] = static_cast<uint16_t>(keys[i] >> 16);
+        p.sorted_rows[i] = keys[i] & 0xffffu;
+        list_head(p.lists, warp_totals, i, p.rows,
+                  [&](size_t k) -> unsigned { return keys[k] >> 16; });
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        p.lists.counts[threadIdx.x] = warp_totals[threadIdx.x];
+    }
+}
+
+__device__ __forceinline__ void comp_add4(Comp (&a)[4], const float4& v) {
+    fb::comp_add(a[0], v.x);
+    fb::comp_add(a[1], v.y);
+    fb::comp_add(a[2], v.z);
+    fb::comp_add(a[3], v.w);
+}
+
+__device__ __forceinline__ float4 add4(const float4& a, const float4& b) {
+    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z),
+                       __fadd_rn(a.w, b.w));
+}
+
+// The column-sum scheme for a single chunk (at most 256 sequences), four columns a thread:
+// a stream's rows are a row stride apart, so the first rows of all eight streams are asked
+// for together. The second pass over one chunk merges it with nothing, which leaves value
+// and bits as they are: it is done here.
+__device__ void position_columns(const PrepareParams& p, size_t quad) {
+    float4 head[kLaneRows];
+#pragma unroll
+    for (int y = 0; y < kLaneRows; ++y) {
+        head[y] = y < static_cast<int>(p.sequences) ? p.dx[y * p.position_quads + quad]
+                                                    : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    Comp total[4];
+#pragma unroll
+    for (int y = 0; y < kLaneRows; ++y) {
+        Comp acc[4];
+        if (y < static_cast<int>(p.sequences)) {
+            comp_add4(acc, head[y]);
+        }
+#pragma unroll 4
+        for (unsigned r = y + kLaneRows; r < p.sequences; r += kLaneRows) {
+            comp_add4(acc, p.dx[r * p.position_quads + quad]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (y == 0) {
+                total[j] = acc[j];
+            } else {
+                fb::comp_merge(total[j], acc[j].s, acc[j].e);
+            }
+        }
+    }
+    p.partial[quad] = make_float4(total[0].s, total[1].s, total[2].s, total[3].s);
+    p.partial[p.position_quads + quad] =
+        make_float4(total[0].e, total[1].e, total[2].e, total[3].e);
+    Comp last[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        fb::comp_merge(last[j], total[j].s, total[j].e);
+    }
+    float4 r = make_float4(fb::comp_value(last[0]), fb::comp_value(last[1]),
+                           fb::comp_value(last[2]), fb::comp_value(last[3]));
+    if (p.accumulate_wpe) {
+        r = add4(p.dwpe[quad], r);
+    }
+    p.dwpe[quad] = r;
+}
+
+__global__ void __launch_bounds__(kPrepareThreads, 2)
+    fb_embedding_prepare(const __grid_constant__ PrepareParams p) {
+    extern __shared__ unsigned sort_keys[];   // [rows], sorting CTA only
+    __shared__ unsigned next[kPrepareWarps][kDigits];
+    __shared__ unsigned warp_totals[kDigits / 32];
+    fb::dependency_wait();
+    fb::dependency_release();
+    unsigned block = blockIdx.x;
+    if (block < p.sort_blocks) {
+        sort_tokens(p, sort_keys, next, warp_totals);
         return;
     }
-    for (unsigned q = threadIdx.x; q < quads; q += kWordThreads) {
-        float4* out = dwte + v * quads + q;
-        if (begin == end) {
-            *out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    block -= p.sort_blocks;
+    if (block < p.position_blocks) {
+        const size_t quad = size_t{block} * kPrepareThreads + threadIdx.x;
+        if (quad < p.position_quads) {
+            position_columns(p, quad);
+        }
+        return;
+    }
+    block -= p.position_blocks;
+    const size_t base = size_t{block} * kZeroQuads + threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const size_t at = base + size_t(i) * kPrepareThreads;
+        if (at < p.word_quads) {
+            __stcs(p.dwte + at, make_float4(0.0f, 0.0f, 0.0f, 0.0f));  // dx stays in L2
+        }
+    }
+}
+
+// The words in use, a slice of 128 columns at a time: each run's rows of dx are added in
+// ascending row order with a compensated sum. That order is a chain of additions, so what
+// bounds a run is how many of its rows are on their way at once. Long runs (a handful of
+// words, first) take a CTA: all its threads fetch rows into a ring in shared memory, 96
+// ahead, and a thread per column adds them. Middling runs take a warp, which asks for
+// sixteen rows at a time; short ones a warp for all their columns. The last blocks fill
+// `offsets`.
+constexpr int kWordThreads = 256;
+constexpr int kWordWarps = kWordThreads / 32;
+constexpr int kWordStages = 4;
+constexpr int kStageRows = 32;
+constexpr int kSliceColumns = 128;
+constexpr int kWordSmem = kWordStages * kStageRows * kSliceColumns * 4;
+
+struct WordParams {
+    float4* dwte;
+    const float4* dx;
+    const uint16_t* sorted_tokens;
+    const unsigned* sorted_rows;
+    RunLists lists;
+    unsigned* offsets;
+    unsigned rows, vocab, quads, slices, word_blocks;
+    bool accumulate;
+};
+
+// One long run's slice, by the whole CTA. Row numbers are read a stage before the copies
+// that need them, so that no stage waits for one load after another.
+__device__ void add_long_run(const WordParams& p, size_t head, unsigned slice, float* ring) {
+    const unsigned token = p.sorted_tokens[head];
+    const int lane = threadIdx.x % 32;
+    const int warp = threadIdx.x / 32;
+    const unsigned quad = slice * 32 + lane;
+    const unsigned column = slice * kSliceColumns + threadIdx.x;
+    const uint32_t ring_at = shared_address(ring);
+    // A stage's 32 sorted positions, one a lane: the token there (none past the end) and its row.
+    unsigned at_token = 0;
+    unsigned at_row = 0;
+    auto look_up = [&](int stage) {
+        const size_t k = head + size_t(stage) * kStageRows + lane;
+        at_token = k < p.rows ? p.sorted_tokens[k] : 0x10000u;
+        at_row = k < p.rows ? p.sorted_rows[k] : 0;
+    };
+    // Warp w fetches rows w, w + 8, ... of a stage; returns how many of the stage's rows belong
+    // to the run (sorted: they come first), and looks the next stage up.
+    auto fetch = [&](int stage) {
+        const int count = __popc(__ballot_sync(fb::kFullMask, at_token == token));
+#pragma unroll
+        for (int j = 0; j < kStageRows / kWordWarps; ++j) {
+            const int row = warp + j * kWordWarps;
+            const unsigned from = __shfl_sync(fb::kFullMask, at_row, row);
+            if (quad < p.quads && row < count) {
+                const uint32_t dst =
+                    ring_at + ((stage % kWordStages) * kStageRows + row) * (kSliceColumns * 4) + lane * 16;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                             "l"(p.dx + size_t{from} * p.quads + quad)
+                             : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        look_up(stage + 1);
+        return count;
+    };
+    int counts[kWordStages];
+    look_up(0);
+#pragma unroll
+    for (int stage = 0; stage < kWordStages - 1; ++stage) {
+        counts[stage] = fetch(stage);
+    }
+    Comp acc;
+    for (int stage = 0;; stage += kWordStages) {
+        bool done = false;
+#pragma unroll
+        for (int i = 0; i < kWordStages && !done; ++i) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kWordStages - 2) : "memory");
+            __syncthreads();   // the stage has landed, and everyone is done with the one before it
+            counts[(i + kWordStages - 1) % kWordStages] = fetch(stage + i + kWordStages - 1);
+            const int count = counts[i];
+            if (threadIdx.x < kSliceColumns) {
+                const float* from = ring + i * kStageRows * kSliceColumns + threadIdx.x;
+                if (count == kStageRows) {
+                    float v[kStageRows];
+#pragma unroll
+                    for (int row = 0; row < kStageRows; ++row) {
+                        v[row] = from[row * kSliceColumns];
+                    }
+#pragma unroll
+                    for (int row = 0; row < kStageRows; ++row) {
+                        fb::comp_add(acc, v[row]);
+                    }
+                } else {
+                    for (int row = 0; row < count; ++row) {
+                        fb::comp_add(acc, from[row * kSliceColumns]);
+                    }
+                }
+            }
+            done = count < kStageRows;
+        }
+        if (done) {
+            break;
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();       // the ring is free for the next run
+    if (threadIdx.x < kSliceColumns && column < p.quads * 4) {
+        float* out = reinterpret_cast<float*>(p.dwte) + size_t{token} * p.quads * 4 + column;
+        const float r = fb::comp_value(acc);
+        *out = p.accumulate ? __fadd_rn(*out, r) : r;
+    }
+}
+
+// kSlices slices of a run from `slice` on, by a warp, kRows rows at a time.
+template <int kSlices, int kRows>
+__device__ __forceinline__ void add_slices(const WordParams& p, size_t head, unsigned token,
+                                           unsigned slice) {
+    const int lane = threadIdx.x % 32;
+    Comp acc[kSlices][4];
+    for (size_t base = head;; base += 32) {
+        const size_t k = base + lane;
+        const unsigned at_token = k < p.rows ? p.sorted_tokens[k] : 0x10000u;
+        const unsigned row = k < p.rows ? p.sorted_rows[k] : 0;
+        // Sorted: the run's lanes come first.
+        const int count = __popc(__ballot_sync(fb::kFullMask, at_token == token));
+        for (int part = 0; part < count; part += kRows) {
+            float4 d[kSlices][kRows];
+#pragma unroll
+            for (int j = 0; j < kRows; ++j) {
+                // Past the run's end the last row is read again, and not added.
+                const size_t r = __shfl_sync(fb::kFullMask, row, min(part + j, count - 1));
+#pragma unroll
+                for (int i = 0; i < kSlices; ++i) {
+                    const unsigned quad = (slice + i) * 32 + lane;
+                    d[i][j] = p.dx[r * p.quads + (quad < p.quads ? quad : 0)];
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < kRows; ++j) {
+                if (part + j < count) {
+#pragma unroll
+                    for (int i = 0; i < kSlices; ++i) {
+                        comp_add4(acc[i], d[i][j]);
+                    }
+                }
+            }
+        }
+        if (count < 32) {
+            break;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kSlices; ++i) {
+        const unsigned quad = (slice + i) * 32 + lane;
+        if (quad >= p.quads) {
             continue;
         }
-        Comp acc[4];
-        for (unsigned k = begin; k < end; ++k) {
-            const float4 d = dx[size_t{sorted_rows[k]} * quads + q];
-            fb::comp_add(acc[0], d.x);
-            fb::comp_add(acc[1], d.y);
-            fb::comp_add(acc[2], d.z);
-            fb::comp_add(acc[3], d.w);
+        float4* out = p.dwte + size_t{token} * p.quads + quad;
+        const float4 r = make_float4(fb::comp_value(acc[i][0]), fb::comp_value(acc[i][1]),
+                                     fb::comp_value(acc[i][2]), fb::comp_value(acc[i][3]));
+        *out = p.accumulate ? add4(*out, r) : r;
+    }
+}
+
+__global__ void __launch_bounds__(kWordThreads)
+    fb_word_gradient(const __grid_constant__ WordParams p) {
+    extern __shared__ float word_ring[];
+    fb::dependency_wait();
+    fb::dependency_release();
+    if (blockIdx.x >= p.word_blocks) {
+        // offsets[v] = number of sorted tokens below v, for v = 0..vocab (binary search).
+        const unsigned v = (blockIdx.x - p.word_blocks) * kWordThreads + threadIdx.x;
+        if (v > p.vocab) {
+            return;
         }
-        float4 r = make_float4(fb::comp_value(acc[0]), fb::comp_value(acc[1]),
-                               fb::comp_value(acc[2]), fb::comp_value(acc[3]));
-        if (accumulate) {
-            const float4 old = *out;
-            r = make_float4(__fadd_rn(old.x, r.x), __fadd_rn(old.y, r.y), __fadd_rn(old.z, r.z),
-                            __fadd_rn(old.w, r.w));
+        unsigned lo = 0;
+        unsigned hi = p.rows;
+        while (lo < hi) {
+            const unsigned mid = lo + (hi - lo) / 2;
+            if (p.sorted_tokens[mid] < v) {
+                lo = mid + 1;
+            } else {
+                hi = mid;
+            }
         }
-        *out = r;
+        p.offsets[v] = lo;
+        return;
+    }
+    const size_t longs = size_t{p.lists.counts[2]} * p.slices;
+    for (size_t task = blockIdx.x; task < longs; task += p.word_blocks) {
+        const size_t head = p.lists.heads[p.rows - 1 - task / p.slices];
+        if (p.sorted_tokens[head] < p.vocab) {
+            add_long_run(p, head, static_cast<unsigned>(task % p.slices), word_ring);
+        }
+    }
+    // The others from the last block backwards: the first ones may still hold a long run.
+    const size_t first = size_t{p.word_blocks - 1 - blockIdx.x} * kWordWarps + threadIdx.x / 32;
+    const size_t stride = size_t{p.word_blocks} * kWordWarps;
+    const size_t middles = size_t{p.lists.counts[1]} * p.slices;
+    const size_t tasks = middles + p.lists.counts[0];
+    for (size_t task = first; task < tasks; task += stride) {
+        const bool middle = task < middles;
+        const size_t head = middle ? p.lists.middle[task / p.slices] : p.lists.heads[task - middles];
+        const unsigned token = p.sorted_tokens[head];
+        if (token >= p.vocab) {
+            continue;
+        }
+        if (middle) {
+            add_slices<1, 16>(p, head, token, static_cast<unsigned>(task % p.slices));
+        } else {
+            for (unsigned slice = 0; slice < p.slices; slice += 6) {
+                add_slices<6, 2>(p, head, token, slice);
+            }
+        }
     }
 }
 
@@ -1069,21 +1495,11 @@ cudaError_t launch_layernorm_backward(void* dx, void* dgamma, void* dbeta, const
     return e;
 }
 
-cudaError_t launch_embedding_backward(void* dwte, void* dwpe, const void* dx, const void* tokens,
-                                      size_t sequences, size_t length, size_t vocab, size_t width,
-                                      bool accumulate_wte, bool accumulate_wpe, void* workspace,
-                                      cudaStream_t stream) {
-    const size_t rows = sequences * length;
-    const EmbeddingLayout l = embedding_layout(sequences, length, vocab, width);
-    auto* base = static_cast<unsigned char*>(workspace);
-    auto* sorted_tokens = reinterpret_cast<uint16_t*>(base + l.sorted_tokens);
-    auto* sorted_rows = reinterpret_cast<unsigned*>(base + l.sorted_rows);
-    auto* offsets = reinterpret_cast<unsigned*>(base + l.offsets);
-    auto* pass_tokens = reinterpret_cast<uint16_t*>(base + l.pass_tokens);
-    auto* pass_rows = reinterpret_cast<unsigned*>(base + l.pass_rows);
-    auto* counts = reinterpret_cast<unsigned*>(base + l.counts);
-    const auto* in_tokens = static_cast<const uint16_t*>(tokens);
-
+namespace {
+// The sort for more rows than one CTA holds.
+cudaError_t sort_by_launches(uint16_t* sorted_tokens, unsigned* sorted_rows, uint16_t* pass_tokens,
+                             unsigned* pass_rows, unsigned* counts, const uint16_t* in_tokens,
+                             size_t rows, cudaStream_t stream) {
     const unsigned tiles = static_cast<unsigned>((rows + kSortTileRows - 1) / kSortTileRows);
     const size_t entries = size_t{tiles} * kDigits;
     for (int pass = 0; pass < 2; ++pass) {
@@ -1109,17 +1525,103 @@ cudaError_t launch_embedding_backward(void* dwte, void* dwpe, const void* dx, co
             return e;
         }
     }
-    fb_token_offsets<<<static_cast<unsigned>((vocab + 1 + 255) / 256), 256, 0, stream>>>(
-        offsets, sorted_tokens, rows, static_cast<unsigned>(vocab));
-    cudaError_t e = fb::after_launch();
+    // The first pass's arrays and the counters have served: they carry the lists of runs.
+    const cudaError_t e = cudaMemsetAsync(counts, 0, 12, stream);
     if (e != cudaSuccess) {
         return e;
     }
-    fb_word_gradient<<<static_cast<unsigned>(vocab), kWordThreads, 0, stream>>>(
-        static_cast<float4*>(dwte), static_cast<const float4*>(dx), sorted_rows, offsets,
-        static_cast<unsigned>(width / 4), accumulate_wte);
-    e = fb::after_launch();
+    fb_list_heads<<<static_cast<unsigned>((rows + 255) / 256), 256, 0, stream>>>(
+        RunLists{pass_rows, reinterpret_cast<unsigned*>(pass_tokens), counts}, sorted_tokens, rows);
+    return fb::after_launch();
+}
+}  // namespace
+
+cudaError_t launch_embedding_backward(void* dwte, void* dwpe, const void* dx, const void* tokens,
+                                      size_t sequences, size_t length, size_t vocab, size_t width,
+                                      bool accumulate_wte, bool accumulate_wpe, void* workspace,
+                                      cudaStream_t stream) {
+    const size_t rows = sequences * length;
+    const EmbeddingLayout l = embedding_layout(sequences, length, vocab, width);
+    auto* base = static_cast<unsigned char*>(workspace);
+    auto* sorted_tokens = reinterpret_cast<uint16_t*>(base + l.sorted_tokens);
+    auto* sorted_rows = reinterpret_cast<unsigned*>(base + l.sorted_rows);
+    auto* offsets = reinterpret_cast<unsigned*>(base + l.offsets);
+    auto* pass_tokens = reinterpret_cast<uint16_t*>(base + l.pass_tokens);
+    auto* pass_rows = reinterpret_cast<unsigned*>(base + l.pass_rows);
+    auto* counts = reinterpret_cast<unsigned*>(base + l.counts);
+    const auto* in_tokens = static_cast<const uint16_t*>(tokens);
+
+    const bool one_cta = rows <= kOneCtaRows;
+    if (!one_cta) {
+        const cudaError_t e = sort_by_launches(sorted_tokens, sorted_rows, pass_tokens, pass_rows,
+                                               counts, in_tokens, rows, stream);
+        if (e != cudaSuccess) {
+            return e;
+        }
+    }
+    const unsigned quads = static_cast<unsigned>(width / 4);
+    const bool table_here = sequences <= kChunkRows;   // one chunk of the column-sum scheme
+    PrepareParams p{};
+    p.dwte = static_cast<float4*>(dwte);
+    p.dwpe = static_cast<float4*>(dwpe);
+    p.partial = reinterpret_cast<float4*>(base);
+    p.dx = static_cast<const float4*>(dx);
+    p.tokens = in_tokens;
+    p.sorted_tokens = sorted_tokens;
+    p.sorted_rows = sorted_rows;
+    p.lists = RunLists{pass_rows, reinterpret_cast<unsigned*>(pass_tokens), counts};
+    p.rows = static_cast<unsigned>(rows);
+    p.sequences = static_cast<unsigned>(sequences);
+    p.sort_blocks = one_cta ? 1 : 0;
+    p.position_quads = length * quads;
+    p.position_blocks = table_here ? static_cast<unsigned>((p.position_quads + kPrepareThreads - 1) /
+                                                           kPrepareThreads)
+                                   : 0;
+    p.word_quads = accumulate_wte ? 0 : vocab * quads;
+    p.accumulate_wpe = accumulate_wpe;
+    const unsigned zero_blocks = static_cast<unsigned>((p.word_quads + kZeroQuads - 1) / kZeroQuads);
+    const unsigned blocks = p.sort_blocks + p.position_blocks + zero_blocks;
+    cudaError_t e = cudaSuccess;
+    if (blocks > 0) {
+        const int smem = one_cta ? static_cast<int>(align16(rows * 4)) : 0;
+        static std::atomic<bool> configured[64] = {};
+        e = fb::allow_shared_memory(fb_embedding_prepare, static_cast<int>(kOneCtaRows) * 4, configured);
+        if (e == cudaSuccess) {
+            e = fb::launch_dependent(fb_embedding_prepare, dim3(blocks), dim3(kPrepareThreads),
+                                     static_cast<size_t>(smem), stream, p);
+        }
+        if (e != cudaSuccess) {
+            return e;
+        }
+    }
+    int sms = 0;
+    e = fb::sm_count(&sms);
     if (e != cudaSuccess) {
+        return e;
+    }
+    static std::atomic<bool> words_configured[64] = {};
+    e = fb::allow_shared_memory(fb_word_gradient, kWordSmem, words_configured);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    WordParams q{};
+    q.dwte = p.dwte;
+    q.dx = p.dx;
+    q.sorted_tokens = sorted_tokens;
+    q.sorted_rows = sorted_rows;
+    q.lists = p.lists;
+    q.offsets = offsets;
+    q.rows = p.rows;
+    q.vocab = static_cast<unsigned>(vocab);
+    q.quads = quads;
+    q.slices = (quads + 31) / 32;
+    // Two CTAs per SM (64 KB of shared memory and 88 registers a thread each).
+    q.word_blocks = static_cast<unsigned>(2 * sms);
+    q.accumulate = accumulate_wte;
+    const unsigned offset_blocks = static_cast<unsigned>((vocab + kWordThreads) / kWordThreads);
+    e = fb::launch_dependent(fb_word_gradient, dim3(q.word_blocks + offset_blocks), dim3(kWordThreads),
+                             kWordSmem, stream, q);
+    if (e != cudaSuccess || table_here) {
         return e;
     }
     // The position table: dx viewed as sequences x (length * width), FP32.

@@ -376,6 +376,31 @@ def test_embedding_backward_matches_the_oracle_at_gpt2_size(flint):
     assert same_bits(dwte, want_wte)
     assert same_bits(dwpe, want_wpe)
 
+@pytest.mark.parametrize("shape", [(300, 8, 300, 16), (17, 1000, 5000, 136), (16, 1024, 1000, 768),
+                                   (1, 1, 1, 8), (2, 95, 40, 200), (256, 8, 20, 1032)])
+def test_embedding_backward_on_skewed_tokens_matches_the_oracle(flint, shape):
+    """Runs of every length class (a warp, a warp per slice, a CTA), tokens past the vocabulary,
+    rows that the one-CTA sort holds exactly (16,384) and more (17,000), and a position table of
+    more sequences than one chunk: bit for bit, writing and accumulating."""
+    seqs, length, vocab, width = shape
+    rows = seqs * length
+    rng = np.random.default_rng(rows + width)
+    tokens = np.minimum(np.exp(rng.random(rows) * np.log(2 * vocab + 1)).astype(np.int64) - 1, 65535)
+    tokens = tokens.astype(np.uint16)
+    dx = crafted(rng, (rows, width), 3).astype(np.float32)
+    old_wte = rng.standard_normal((vocab, width)).astype(np.float32)
+    old_wpe = rng.standard_normal((length, width)).astype(np.float32)
+    ws = workspace(flint.embedding_backward_workspace(seqs, length, vocab, width))
+    for accumulate in (False, True):
+        dwte, dwpe = torch.from_numpy(old_wte.copy()).to(DEV), torch.from_numpy(old_wpe.copy()).to(DEV)
+        flint.embedding_backward(dwte, dwpe, torch.from_numpy(dx).to(DEV), tokens16(tokens), seqs, length,
+                                 vocab, width, accumulate, accumulate, ws)
+        torch.cuda.synchronize()
+        want_wte, want_wpe, *_ = oracle.embedding_backward(
+            dx, tokens, seqs, length, vocab, old_wte if accumulate else None, old_wpe if accumulate else None)
+        assert same_bits(dwte, want_wte)
+        assert same_bits(dwpe, want_wpe)
+
 
 def test_cross_entropy_with_extreme_and_non_finite_logits(flint):
     """The exponential's clamp and NaN handling: logits spanning FP16's range, -inf entries
