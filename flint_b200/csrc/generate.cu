@@ -8,12 +8,15 @@
 //   prefill   the prompt's rows go through the library's tensor-core GEMMs and the
 //             fused causal attention kernel, exactly as in the training forward pass,
 //             and their keys and values are copied into the cache
-//   decode    one new token per sequence. The step is bound by HBM traffic: every
-//             weight is read once per step (2 bytes each in FP16, 1 in int8) and the
-//             cache of every layer once; the linear layers for up to eight sequences
-//             run on a streaming kernel (a warp per one or two output features, 16-byte
-//             weight loads past L1, the eight rows' activations through L1, FP32
-//             accumulation), more sequences use the tensor-core GEMMs.
+//   decode    one new token per sequence, five kernels per layer. At this size no single
+//             kernel is long enough to be bound by HBM; a step is a chain of dependent
+//             kernels, so what counts is how little each does after the one before it has
+//             finished. Every kernel is launched to start early (programmatic dependent
+//             launch), fetches what does not depend on the step into registers (its weights,
+//             the cache's older keys and values), and only then waits for its predecessor.
+//             Products run on mma.sync with the sequences as the 16 rows of A and eight
+//             output features as the columns of B, so up to 16 sequences cost one MMA per
+//             16 weights of a feature.
 //             Positions live in device memory, so a step's launches do not change from
 //             token to token and are captured once into a CUDA graph.
 //
@@ -36,13 +39,12 @@
 #include "flint/flint_b200.h"
 #include "gemm.h"
 #include "gpt2.h"
+#include "sm100.cuh"
 
 namespace {
 
 constexpr flint_status kInvalid = FLINT_ERROR_INVALID_ARGUMENT;
 constexpr int kHeadWidth = 64;
-constexpr int kSkinnyRows = 8;       // sequences the streaming linear kernel serves at once
-constexpr int kLinearWarps = 4;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kEps = 1e-5f;
 
@@ -104,43 +106,18 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// ---- the streaming linear layer for up to eight rows ---------------------------------------------
+// ---- linear layers of a decode step -----------------------------------------------------------
 //
-// y[b, n] = act(sum_k x[b, k] w[n, k] (* scale[n]) + bias[n]) for eight rows b. A warp owns F
-// output features (1 for narrow outputs, so that enough warps exist to keep HBM busy; 2
-// otherwise, halving the activations' L1 traffic per weight byte). In one step a lane takes
-// 16 bytes of each feature's weights (8 FP16 or 16 int8 values: a warp reads 512 contiguous
-// bytes of a weight row) and the matching activations of all eight rows, which come through
-// L1: the eight rows are at most 48 KB and every warp of the SM reads the same ones. The
-// weights are touched once, so they are loaded past L1. FP32 accumulation; the lanes' sums
-// are added by a butterfly at the end.
+// y[b, n] = act(sum_k x[b, k] w[n, k] (* scale[n]) + bias[n]) for one row b per sequence.
+// A dot product does not care in which order k is taken, so a lane's share of an MMA is
+// chosen to be contiguous: lane (g, t) = (lane / 4, lane % 4) loads 16 bytes of feature g's
+// weights and the matching activations of rows g and g + 8, and each group of four values
+// becomes the four k positions that lane holds in one m16n8k16. Weights need no shuffling,
+// no shared memory and no conversion (int8 becomes FP16 exactly: all 256 values are FP16
+// integers), and come straight into registers before the kernel waits for its predecessor.
 
-template <typename W>
-struct WeightVector;
-
-template <>
-struct WeightVector<__half> {
-    static constexpr int kValues = 8;
-    static __device__ __forceinline__ void unpack(const uint4& raw, float (&v)[8]) {
-        fb::unpack8(v, raw);
-    }
-};
-
-template <>
-struct WeightVector<int8_t> {
-    static constexpr int kValues = 16;
-    static __device__ __forceinline__ void unpack(const uint4& raw, float (&v)[16]) {
-        const unsigned words[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int word = static_cast<int>(words[i]);
-            v[4 * i] = static_cast<float>(static_cast<int8_t>(word));
-            v[4 * i + 1] = static_cast<float>(static_cast<int8_t>(word >> 8));
-            v[4 * i + 2] = static_cast<float>(static_cast<int8_t>(word >> 16));
-            v[4 * i + 3] = static_cast<float>(word >> 24);
-        }
-    }
-};
+constexpr int kWarps = 8;
+constexpr int kThreads = 32 * kWarps;
 
 // 16 bytes that will not be read again: bypass L1.
 __device__ __forceinline__ uint4 load_streaming(const void* p) {
@@ -151,122 +128,439 @@ __device__ __forceinline__ uint4 load_streaming(const void* p) {
     return v;
 }
 
-// S warps share a feature group: S = 1 gives every warp of the CTA its own F features; S = 4
-// gives the CTA's four warps a quarter of k each for the same F features (their sums meet
-// in shared memory and are added in warp order), which multiplies the warps, and the bytes
-// in flight, for narrow outputs whose few features would otherwise leave most SMs idle.
-template <typename W, Act A, int F, int S>
-__global__ void __launch_bounds__(32 * kLinearWarps)
-    fb_decode_linear(void* __restrict__ out, const W* __restrict__ w,
-                     const float* __restrict__ scale, const float* __restrict__ bias,
-                     const __half* __restrict__ x, const float* __restrict__ residual, int n,
-                     int k, int out_stride) {
-    constexpr int kValues = WeightVector<W>::kValues;
-    constexpr int kRows = kSkinnyRows;
-    constexpr int kGroups = kLinearWarps / S;          // feature groups per CTA
-    static_assert(S == 1 || S == kLinearWarps, "a feature group is one warp or the whole CTA");
-    __shared__ float meet[S == 1 ? 1 : kLinearWarps][F][kRows];
+__device__ __forceinline__ void mma_16x8x16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2,
+                                            unsigned a3, unsigned b0, unsigned b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+        "{%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Four int8 values as two FP16 pairs: the byte with its sign bit flipped is v + 128, under
+// 0x64 the FP16 number 1024 + (v + 128), from which 1152 is subtracted exactly.
+__device__ __forceinline__ void int8_to_half(unsigned word, unsigned& lo, unsigned& hi) {
+    const unsigned biased = word ^ 0x80808080u;
+    const __half2 offset = __half2half2(__ushort_as_half(0x6480));  // 1152
+    unsigned l = __byte_perm(biased, 0x64646464u, 0x4140);
+    unsigned h = __byte_perm(biased, 0x64646464u, 0x4342);
+    const __half2 l2 = __hsub2(*reinterpret_cast<const __half2*>(&l), offset);
+    const __half2 h2 = __hsub2(*reinterpret_cast<const __half2*>(&h), offset);
+    lo = *reinterpret_cast<const unsigned*>(&l2);
+    hi = *reinterpret_cast<const unsigned*>(&h2);
+}
+
+// A lane's 16 weight bytes of one step: kStepK values of k per warp and step, kValues of them
+// this lane's, in kPieces groups of eight activations.
+template <typename W>
+struct Step;
+template <>
+struct Step<__half> {
+    static constexpr int kStepK = 32, kValues = 8, kPieces = 1;
+    static __device__ __forceinline__ void weights(const uint4& raw, int i, unsigned& b0,
+                                                   unsigned& b1) {
+        b0 = i == 0 ? raw.x : raw.z;
+        b1 = i == 0 ? raw.y : raw.w;
+    }
+};
+template <>
+struct Step<int8_t> {
+    static constexpr int kStepK = 64, kValues = 16, kPieces = 2;
+    static __device__ __forceinline__ void weights(const uint4& raw, int i, unsigned& b0,
+                                                   unsigned& b1) {
+        const unsigned word = i == 0 ? raw.x : i == 1 ? raw.y : i == 2 ? raw.z : raw.w;
+        int8_to_half(word, b0, b1);
+    }
+};
+
+// One step of NT feature tiles: `low(m, piece)` and `high(m, piece)` give this lane's eight
+// activations of rows 16 m + g and 16 m + g + 8.
+template <typename W, int MB, int NT, typename Low, typename High>
+__device__ __forceinline__ void multiply(float (&acc)[MB][NT][4], const uint4 (&raw)[NT], Low low,
+                                         High high) {
+#pragma unroll
+    for (int piece = 0; piece < Step<W>::kPieces; ++piece) {
+#pragma unroll
+        for (int m = 0; m < MB; ++m) {
+            const uint4 xa = low(m, piece);
+            const uint4 xb = high(m, piece);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                unsigned b0, b1;
+                Step<W>::weights(raw[nt], 2 * piece, b0, b1);
+                mma_16x8x16(acc[m][nt], xa.x, xb.x, xa.y, xb.y, b0, b1);
+                Step<W>::weights(raw[nt], 2 * piece + 1, b0, b1);
+                mma_16x8x16(acc[m][nt], xa.z, xb.z, xa.w, xb.w, b0, b1);
+            }
+        }
+    }
+}
+
+// LayerNorm of `rows` FP32 rows into FP16 rows of k + 8 values in shared memory (the 16 bytes
+// between rows keep eight rows' 16-byte reads off each other's banks): a warp per row, the
+// row in registers, mean first and then the centred squares. QN float4s a lane.
+template <int QN>
+__device__ __forceinline__ void normalise_rows(__half* h, const float* x, const float* gain,
+                                               const float* shift, int rows, int k) {
+    const int lane = threadIdx.x % 32;
+    for (int row = threadIdx.x / 32; row < rows; row += kWarps) {
+        const float4* src = reinterpret_cast<const float4*>(x + static_cast<size_t>(row) * k);
+        float4 v[QN];
+        float sum = 0.0f;
+#pragma unroll
+        for (int i = 0; i < QN; ++i) {
+            const int q = lane + 32 * i;
+            v[i] = 4 * q < k ? src[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int i = 0; i < QN; ++i) {
+            sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+        }
+        const float mean = fb::warp_sum_rn(sum) / static_cast<float>(k);
+        float squares = 0.0f;
+#pragma unroll
+        for (int i = 0; i < QN; ++i) {
+            if (4 * (lane + 32 * i) < k) {
+                v[i].x -= mean;
+                v[i].y -= mean;
+                v[i].z -= mean;
+                v[i].w -= mean;
+                squares += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+            }
+        }
+        const float variance = fb::warp_sum_rn(squares) / static_cast<float>(k);
+        const float rstd = 1.0f / sqrtf(variance + kEps);
+#pragma unroll
+        for (int i = 0; i < QN; ++i) {
+            const int q = lane + 32 * i;
+            if (4 * q < k) {
+                const float4 g = reinterpret_cast<const float4*>(gain)[q];
+                const float4 b = reinterpret_cast<const float4*>(shift)[q];
+                uint2 packed;
+                packed.x = fb::pack2(v[i].x * rstd * g.x + b.x, v[i].y * rstd * g.y + b.y);
+                packed.y = fb::pack2(v[i].z * rstd * g.z + b.z, v[i].w * rstd * g.w + b.w);
+                reinterpret_cast<uint2*>(h + static_cast<size_t>(row) * (k + 8))[q] = packed;
+            }
+        }
+    }
+}
+
+struct LinearArgs {
+    void* out;
+    const void* w;
+    const float* scale;     // int8: one per feature
+    const float* bias;
+    const void* x;          // FP16 rows, or FP32 rows to normalise first
+    const float* gain;
+    const float* shift;
+    const float* residual;
+    int rows, n, k;
+};
+
+// Shared memory of a kernel that normalises: gain, shift and the FP16 rows.
+__host__ __device__ constexpr int norm_bytes(int rows, int k) { return 8 * k + rows * (k + 8) * 2; }
+
+// Shared memory of a linear kernel: the above, then the warps' sums (of 64 rows they do not
+// fit beside 64 wide rows; they then take the rows' place once those have been used).
+__host__ __device__ constexpr int sums_bytes(int mb, int nt) { return kWarps * 16 * mb * 8 * nt * 4; }
+__host__ __device__ constexpr int linear_bytes(bool norm, int mb, int nt, int rows, int k) {
+    const int first = norm ? norm_bytes(rows, k) : 0;
+    return mb < 4 ? first + sums_bytes(mb, nt)
+                  : (first > sums_bytes(mb, nt) ? first : sums_bytes(mb, nt));
+}
+
+// A CTA owns 8 NT features, its warps a share of k each; the warps' sums meet in shared
+// memory and are added in warp order. kSteps: the steps a warp's share can have.
+template <typename W, Act A, bool kNorm, int MB, int NT, int kSteps, int QN>
+__global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p) {
+    using S = Step<W>;
+    constexpr int kColumns = 8 * NT;
+    extern __shared__ __align__(16) unsigned char decode_smem[];
+    using Sums = float[16 * MB][kColumns];
+    Sums* sums = reinterpret_cast<Sums*>(decode_smem +
+                                         (kNorm && MB < 4 ? norm_bytes(p.rows, p.k) : 0));
+    fb::dependency_release();
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
-    const int first = (blockIdx.x * kGroups + (S == 1 ? warp : 0)) * F;
-    if (S == 1 && first >= n) {
-        return;
-    }
-    // This warp's share of k, in whole lane-steps.
-    const int steps = (k + 32 * kValues - 1) / (32 * kValues);
-    const int share = (steps + S - 1) / S;
-    const int k_begin = (S == 1 ? 0 : warp * share) * 32 * kValues;
-    const int k_end = min(k, (S == 1 ? steps : (warp + 1) * share) * 32 * kValues);
-    float acc[F][kRows];
+    const int g = lane / 4;
+    const int t = lane % 4;
+    const int first = blockIdx.x * kColumns;
+    const int steps = p.k / S::kStepK;
+    const int share = (steps + kWarps - 1) / kWarps;
+    const int begin = warp * share;
+    const int mine = min(share, steps - begin);   // may be none
+    uint4 raw[kSteps][NT];
 #pragma unroll
-    for (int f = 0; f < F; ++f) {
+    for (int j = 0; j < kSteps; ++j) {
 #pragma unroll
-        for (int b = 0; b < kRows; ++b) {
-            acc[f][b] = 0.0f;
+        for (int nt = 0; nt < NT; ++nt) {
+            raw[j][nt] = make_uint4(0u, 0u, 0u, 0u);
+            if (j < mine) {
+                raw[j][nt] = load_streaming(static_cast<const W*>(p.w) +
+                                            static_cast<size_t>(first + 8 * nt + g) * p.k +
+                                            (begin + j) * S::kStepK + t * S::kValues);
+            }
         }
     }
-#pragma unroll 2
-    for (int k0 = k_begin + lane * kValues; k0 < k_end; k0 += 32 * kValues) {
-        uint4 raw[F];
-#pragma unroll
-        for (int f = 0; f < F; ++f) {
-            const int feature = min(first + f, n - 1);
-            raw[f] = load_streaming(w + static_cast<size_t>(feature) * k + k0);
+    const int feature = first + static_cast<int>(threadIdx.x) % kColumns;
+    const float scale = p.scale != nullptr ? p.scale[feature] : 1.0f;
+    const float bias = p.bias[feature];
+    float* gain = reinterpret_cast<float*>(decode_smem);
+    float* shift = gain + p.k;
+    __half* rows = reinterpret_cast<__half*>(shift + p.k);
+    if constexpr (kNorm) {
+        for (int i = threadIdx.x; i < p.k / 4; i += kThreads) {
+            reinterpret_cast<float4*>(gain)[i] = reinterpret_cast<const float4*>(p.gain)[i];
+            reinterpret_cast<float4*>(shift)[i] = reinterpret_cast<const float4*>(p.shift)[i];
         }
-        float wv[F][kValues];
+        __syncthreads();
+    }
+    // Nothing above depends on the step's kernels.
+    fb::dependency_wait();
+    const size_t out_at = static_cast<size_t>(threadIdx.x / kColumns) * p.n + feature;
+    float residual = 0.0f;
+    if (A == Act::kResidual && static_cast<int>(threadIdx.x) / kColumns < p.rows) {
+        residual = p.residual[out_at];
+    }
+    const __half* x = static_cast<const __half*>(p.x);
+    int stride = p.k;
+    if constexpr (kNorm) {
+        normalise_rows<QN>(rows, static_cast<const float*>(p.x), gain, shift, p.rows, p.k);
+        __syncthreads();
+        x = rows;
+        stride = p.k + 8;
+    }
+    float acc[MB][NT][4] = {};
 #pragma unroll
-        for (int f = 0; f < F; ++f) {
-            WeightVector<W>::unpack(raw[f], wv[f]);
+    for (int j = 0; j < kSteps; ++j) {
+        if (j < mine) {
+            const __half* at = x + (begin + j) * S::kStepK + t * S::kValues;
+            auto row_values = [&](int row, int piece) {
+                return row < p.rows ? *reinterpret_cast<const uint4*>(
+                                          at + static_cast<size_t>(row) * stride + 8 * piece)
+                                    : make_uint4(0u, 0u, 0u, 0u);
+            };
+            multiply<W, MB, NT>(
+                acc, raw[j], [&](int m, int piece) { return row_values(16 * m + g, piece); },
+                [&](int m, int piece) { return row_values(16 * m + g + 8, piece); });
         }
+    }
+    if (kNorm && MB == 4) {
+        __syncthreads();   // the rows' place is free
+    }
 #pragma unroll
-        for (int b = 0; b < kRows; ++b) {
-            const uint4* row = reinterpret_cast<const uint4*>(x + static_cast<size_t>(b) * k + k0);
+    for (int m = 0; m < MB; ++m) {
 #pragma unroll
-            for (int piece = 0; piece < kValues / 8; ++piece) {
-                float xv[8];
-                fb::unpack8(xv, __ldg(row + piece));
+        for (int nt = 0; nt < NT; ++nt) {
+            sums[warp][16 * m + g][8 * nt + 2 * t] = acc[m][nt][0];
+            sums[warp][16 * m + g][8 * nt + 2 * t + 1] = acc[m][nt][1];
+            sums[warp][16 * m + g + 8][8 * nt + 2 * t] = acc[m][nt][2];
+            sums[warp][16 * m + g + 8][8 * nt + 2 * t + 1] = acc[m][nt][3];
+        }
+    }
+    __syncthreads();
+    // kThreads is a multiple of kColumns: a thread keeps its feature from row to row.
+    for (int row = threadIdx.x / kColumns; row < p.rows; row += kThreads / kColumns) {
+        float v = sums[0][row][threadIdx.x % kColumns];
 #pragma unroll
-                for (int f = 0; f < F; ++f) {
+        for (int other = 1; other < kWarps; ++other) {
+            v += sums[other][row][threadIdx.x % kColumns];
+        }
+        if (sizeof(W) == 1) {
+            v *= scale;
+        }
+        v += bias;
+        const size_t at = static_cast<size_t>(row) * p.n + feature;
+        if constexpr (A == Act::kResidual) {
+            static_cast<float*>(p.out)[at] = (at == out_at ? residual : p.residual[at]) + v;
+        } else if constexpr (A == Act::kGelu) {
+            static_cast<__half*>(p.out)[at] = __float2half_rn(gelu_tanh(v));
+        } else {
+            static_cast<__half*>(p.out)[at] = __float2half_rn(v);
+        }
+    }
+}
+
+// ---- final LayerNorm, output layer and greedy choice ---------------------------------------------
+//
+// The one kernel of a step whose weights are many (77 MB in FP16): two CTAs per SM stream
+// them, a warp per eight features, the next twelve steps' weights on their way while twelve
+// are used. Every lane remembers the largest logit it saw; a sequence's best candidates meet
+// in a 64-bit maximum of (ordered logit, inverted index), and the last CTA writes the tokens,
+// advances the position and leaves the scratch as it found it.
+
+struct HeadArgs {
+    float* logits;
+    const void* w;
+    const float* scale;
+    const float* x;
+    const float* gain;
+    const float* shift;
+    unsigned long long* best;
+    unsigned* ticket;
+    uint16_t* next;
+    int* position;
+    int rows, n, k, vocab, advance;
+};
+
+__device__ __forceinline__ unsigned long long candidate(float value, int index) {
+    const unsigned bits = __float_as_uint(value + 0.0f);   // -0 counts as +0
+    const unsigned ordered = (bits & 0x80000000u) != 0 ? ~bits : bits | 0x80000000u;
+    return (static_cast<unsigned long long>(ordered) << 32) | (0xffffffffu - static_cast<unsigned>(index));
+}
+
+template <typename W, int MB, int QN>
+__global__ void __launch_bounds__(kThreads, 2) fb_decode_head(const HeadArgs p) {
+    using S = Step<W>;
+    constexpr int kAhead = 12 / S::kPieces;   // steps per batch of loads
+    extern __shared__ __align__(16) unsigned char decode_smem[];
+    __shared__ unsigned long long chosen[kWarps][16 * MB];
+    __shared__ bool last_cta;
+    fb::dependency_release();
+    const int warp = threadIdx.x / 32;
+    const int lane = threadIdx.x % 32;
+    const int g = lane / 4;
+    const int t = lane % 4;
+    const int steps = p.k / S::kStepK;
+    const int batches = (steps + kAhead - 1) / kAhead;
+    const int tiles = (p.n + 7) / 8;
+    const int stride_tiles = gridDim.x * kWarps;
+    auto load = [&](uint4 (&raw)[kAhead], int tile, int batch) {
+        const W* row = static_cast<const W*>(p.w) +
+                       static_cast<size_t>(min(8 * tile + g, p.n - 1)) * p.k + t * S::kValues;
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        acc[f][b] = fmaf(wv[f][8 * piece + j], xv[j], acc[f][b]);
+        for (int j = 0; j < kAhead; ++j) {
+            const int step = batch * kAhead + j;
+            raw[j] = make_uint4(0u, 0u, 0u, 0u);
+            if (tile < tiles && step < steps) {
+                raw[j] = load_streaming(row + step * S::kStepK);
+            }
+        }
+    };
+    int tile = blockIdx.x * kWarps + warp;
+    int batch = 0;
+    uint4 raw[kAhead];
+    load(raw, tile, batch);
+    float* gain = reinterpret_cast<float*>(decode_smem);
+    float* shift = gain + p.k;
+    __half* rows = reinterpret_cast<__half*>(shift + p.k);
+    for (int i = threadIdx.x; i < p.k / 4; i += kThreads) {
+        reinterpret_cast<float4*>(gain)[i] = reinterpret_cast<const float4*>(p.gain)[i];
+        reinterpret_cast<float4*>(shift)[i] = reinterpret_cast<const float4*>(p.shift)[i];
+    }
+    __syncthreads();
+    fb::dependency_wait();
+    normalise_rows<QN>(rows, p.x, gain, shift, p.rows, p.k);
+    __syncthreads();
+    float best_value[MB][2];
+    int best_index[MB][2];
+#pragma unroll
+    for (int m = 0; m < MB; ++m) {
+        best_value[m][0] = best_value[m][1] = -INFINITY;
+        best_index[m][0] = best_index[m][1] = 0;
+    }
+    float acc[MB][1][4] = {};
+    while (tile < tiles) {
+        const bool done = batch + 1 == batches;
+        const int next_tile = done ? tile + stride_tiles : tile;
+        const int next_batch = done ? 0 : batch + 1;
+        uint4 ahead[kAhead];
+        load(ahead, next_tile, next_batch);
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            const int step = batch * kAhead + j;
+            if (step < steps) {
+                const __half* at = rows + step * S::kStepK + t * S::kValues;
+                auto row_values = [&](int row, int piece) {
+                    return row < p.rows ? *reinterpret_cast<const uint4*>(at + row * (p.k + 8) + 8 * piece)
+                                        : make_uint4(0u, 0u, 0u, 0u);
+                };
+                const uint4 one[1] = {raw[j]};
+                multiply<W, MB, 1>(
+                    acc, one, [&](int m, int piece) { return row_values(16 * m + g, piece); },
+                    [&](int m, int piece) { return row_values(16 * m + g + 8, piece); });
+            }
+        }
+        if (done) {
+            const int column = 8 * tile + 2 * t;    // n is a multiple of 8
+            float s0 = 1.0f;
+            float s1 = 1.0f;
+            if (sizeof(W) == 1) {
+                s0 = p.scale[column];
+                s1 = p.scale[column + 1];
+            }
+#pragma unroll
+            for (int m = 0; m < MB; ++m) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int row = 16 * m + 8 * half + g;
+                    const float v0 = acc[m][0][2 * half] * s0;
+                    const float v1 = acc[m][0][2 * half + 1] * s1;
+                    if (row < p.rows) {
+                        *reinterpret_cast<float2*>(p.logits + static_cast<size_t>(row) * p.n + column) =
+                            make_float2(v0, v1);
                     }
+                    if (column < p.vocab && v0 > best_value[m][half]) {
+                        best_value[m][half] = v0;
+                        best_index[m][half] = column;
+                    }
+                    if (column + 1 < p.vocab && v1 > best_value[m][half]) {
+                        best_value[m][half] = v1;
+                        best_index[m][half] = column + 1;
+                    }
+                    acc[m][0][2 * half] = 0.0f;
+                    acc[m][0][2 * half + 1] = 0.0f;
                 }
             }
         }
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            raw[j] = ahead[j];
+        }
+        tile = next_tile;
+        batch = next_batch;
     }
+    // The lowest index of the largest logit: over the row's four lanes, the warps, the CTAs.
 #pragma unroll
-    for (int f = 0; f < F; ++f) {
+    for (int m = 0; m < MB; ++m) {
 #pragma unroll
-        for (int b = 0; b < kRows; ++b) {
-            acc[f][b] = fb::warp_sum_rn(acc[f][b]);
-        }
-    }
-    // Lane (f, b) holds output (b, first + f).
-    const int f = lane / kRows;
-    const int b = lane % kRows;
-    float v = 0.0f;
+        for (int half = 0; half < 2; ++half) {
+            unsigned long long key = candidate(best_value[m][half], best_index[m][half]);
 #pragma unroll
-    for (int ff = 0; ff < F; ++ff) {
-#pragma unroll
-        for (int bb = 0; bb < kRows; ++bb) {
-            v = (ff == f && bb == b) ? acc[ff][bb] : v;
-        }
-    }
-    if constexpr (S > 1) {
-        if (lane < F * kRows) {
-            meet[warp][f][b] = v;
-        }
-        __syncthreads();
-        if (warp != 0) {
-            return;
-        }
-        if (lane < F * kRows) {
-            v = meet[0][f][b];
-#pragma unroll
-            for (int other = 1; other < S; ++other) {
-                v += meet[other][f][b];
+            for (int off = 1; off < 4; off <<= 1) {
+                const unsigned long long other = __shfl_xor_sync(fb::kFullMask, key, off);
+                key = other > key ? other : key;
+            }
+            if (t == 0) {
+                chosen[warp][16 * m + 8 * half + g] = key;
             }
         }
     }
-    if (lane < F * kRows && first + f < n) {
-        const int feature = first + f;
-        if (scale != nullptr) {
-            v *= scale[feature];
+    __syncthreads();
+    for (int row = threadIdx.x; row < p.rows; row += kThreads) {
+        unsigned long long key = chosen[0][row];
+        for (int w2 = 1; w2 < kWarps; ++w2) {
+            key = chosen[w2][row] > key ? chosen[w2][row] : key;
         }
-        if (bias != nullptr) {
-            v += bias[feature];
-        }
-        const size_t at = static_cast<size_t>(b) * out_stride + feature;
-        if constexpr (A == Act::kResidual) {
-            static_cast<float*>(out)[at] = residual[at] + v;
-        } else if constexpr (A == Act::kLogits) {
-            static_cast<float*>(out)[at] = v;
-        } else if constexpr (A == Act::kGelu) {
-            static_cast<__half*>(out)[at] = __float2half_rn(gelu_tanh(v));
-        } else {
-            static_cast<__half*>(out)[at] = __float2half_rn(v);
-        }
+        atomicMax(&p.best[row], key);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last_cta = atomicAdd(p.ticket, 1u) + 1 == gridDim.x;
+    }
+    __syncthreads();
+    if (!last_cta) {
+        return;
+    }
+    __threadfence();
+    for (int row = threadIdx.x; row < p.rows; row += kThreads) {
+        const unsigned long long key = atomicExch(&p.best[row], 0ull);
+        p.next[row] = static_cast<uint16_t>(0xffffffffu - static_cast<unsigned>(key));
+    }
+    if (threadIdx.x == 0) {
+        *p.ticket = 0;
+        *p.position += p.advance;
     }
 }
 
@@ -286,17 +580,16 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Copies the keys and values of `count` consecutive positions per sequence from packed qkv
-// rows [sequences * count, 3 width] into the cache, starting at cache position *position
-// (decode: count 1) or `first` when position is null (prefill).
+// Prefill: copies the keys and values of `count` consecutive positions per sequence from
+// packed qkv rows [sequences * count, 3 width] into the cache, starting at position `first`.
 __global__ void __launch_bounds__(256)
     fb_cache_store(__half* __restrict__ cache_k, __half* __restrict__ cache_v,
-                   const __half* __restrict__ qkv, const int* __restrict__ position, int first,
-                   int count, int heads, int max_length) {
+                   const __half* __restrict__ qkv, int first, int count, int heads,
+                   int max_length) {
     const int width = heads * kHeadWidth;
     const int row = blockIdx.x;            // sequence * count + offset
     const int sequence = row / count;
-    const int t = (position != nullptr ? *position : first) + row % count;
+    const int t = first + row % count;
     const uint4* src = reinterpret_cast<const uint4*>(qkv + static_cast<size_t>(row) * 3 * width);
     const int pieces = width / 8;          // 16-byte pieces per K (or V) row
     for (int i = threadIdx.x; i < 2 * pieces; i += blockDim.x) {
@@ -310,121 +603,218 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// One query per (sequence, head) against the cache's positions 0 .. *position. The new
-// token's own key and value come straight from its qkv row; the CTA also stores them in the
-// cache for the steps to come (no other CTA reads that position during this launch).
-constexpr int kDecodeThreads = 512;
+// One query per (sequence, head) against the cache's positions 0 .. *position, by a cluster
+// of CTAs that share the older positions out evenly. Eight lanes hold a position (16 bytes
+// of its key and value each), 32 positions per CTA and round; up to 256 positions per CTA
+// are in registers before the kernel waits for the new token's qkv row. Each group of eight
+// lanes keeps its own running maximum, sum and weighted values; they are merged over the
+// warp, the CTA and, through distributed shared memory, the cluster. The leading CTA takes
+// the new token's own key and value from the row and stores them in the cache for the steps
+// to come (no other CTA reads that position during this launch).
+constexpr int kRounds = 8;
+constexpr int kMostSplits = 8;
 
-__global__ void __launch_bounds__(kDecodeThreads)
+// (m, l, acc) of two disjoint sets of positions, m possibly -inf for an empty one.
+__device__ __forceinline__ float merge_weight(float m, float top) {
+    return m == -INFINITY ? 0.0f : exp2f(m - top);
+}
+
+__global__ void __launch_bounds__(kThreads)
     fb_decode_attention(__half* __restrict__ out, const __half* __restrict__ qkv,
                         __half* __restrict__ cache_k, __half* __restrict__ cache_v,
-                        const int* __restrict__ position, int heads, int max_length, float scale) {
-    extern __shared__ float scores[];      // [max_length]
-    constexpr int kGroups = kDecodeThreads / 8;
-    __shared__ float q[kHeadWidth];
-    __shared__ float red[kDecodeThreads / 32];
-    __shared__ float partial[kGroups][kHeadWidth];
-    const int head = blockIdx.x % heads;
-    const int sequence = blockIdx.x / heads;
+                        const int* __restrict__ position, int heads, int max_length, int splits,
+                        float scale) {
+    __shared__ float partial[kWarps][kHeadWidth];
+    __shared__ float partial_m[kWarps];
+    __shared__ float partial_l[kWarps];
+    __shared__ float meet[kMostSplits][kHeadWidth + 2];
+    fb::dependency_release();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    const int rank = static_cast<int>(sm100::cluster_cta_rank());
+    const int pair = blockIdx.x / splits;
+    const int head = pair % heads;
+    const int sequence = pair / heads;
     const int width = heads * kHeadWidth;
-    const int newest = *position;
-    const int length = newest + 1;
     const int tid = threadIdx.x;
     const int lane = tid % 32;
     const int warp = tid / 32;
-    const __half* row_q = qkv + static_cast<size_t>(sequence) * 3 * width + head * kHeadWidth;
-    const __half* new_k = row_q + width;
-    const __half* new_v = row_q + 2 * width;
-    __half* keys = cache_k + (static_cast<size_t>(sequence) * heads + head) * max_length * kHeadWidth;
-    __half* values = cache_v + (static_cast<size_t>(sequence) * heads + head) * max_length * kHeadWidth;
-    if (tid < kHeadWidth) {
-        q[tid] = __half2float(row_q[tid]) * scale * kLog2e;
-    } else if (tid < kHeadWidth + 8) {
-        const int piece = tid - kHeadWidth;
-        reinterpret_cast<uint4*>(keys + static_cast<size_t>(newest) * kHeadWidth)[piece] =
-            reinterpret_cast<const uint4*>(new_k)[piece];
-    } else if (tid < kHeadWidth + 16) {
-        const int piece = tid - kHeadWidth - 8;
-        reinterpret_cast<uint4*>(values + static_cast<size_t>(newest) * kHeadWidth)[piece] =
-            reinterpret_cast<const uint4*>(new_v)[piece];
-    }
-    __syncthreads();
-    float top = -INFINITY;
-    for (int t = tid; t < length; t += kDecodeThreads) {
-        const uint4* row = reinterpret_cast<const uint4*>(
-            t == newest ? new_k : keys + static_cast<size_t>(t) * kHeadWidth);
-        uint4 raw[8];
+    const int eighth = lane % 8;
+    const int group = warp * 4 + lane / 8;
+    // The position and every older row were written before this step's first kernel began.
+    const int newest = *position;
+    const int share = (newest + splits - 1) / splits;
+    const int begin = rank * share;
+    const int end = min(newest, begin + share);
+    const size_t base = (static_cast<size_t>(sequence) * heads + head) * max_length * kHeadWidth;
+    const uint4* keys = reinterpret_cast<const uint4*>(cache_k + base) + eighth;
+    const uint4* values = reinterpret_cast<const uint4*>(cache_v + base) + eighth;
+    uint4 k[kRounds];
+    uint4 v[kRounds];
+    auto fetch = [&](int from) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            raw[i] = load_streaming(row + i);
-        }
-        float s = 0.0f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            float v[8];
-            fb::unpack8(v, raw[i]);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                s = fmaf(v[j], q[8 * i + j], s);
+        for (int i = 0; i < kRounds; ++i) {
+            const int at = from + group + 32 * i;
+            k[i] = v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (at < end) {
+                k[i] = load_streaming(keys + static_cast<size_t>(at) * (kHeadWidth / 8));
+                v[i] = load_streaming(values + static_cast<size_t>(at) * (kHeadWidth / 8));
             }
         }
-        scores[t] = s;
-        top = fmaxf(top, s);
-    }
-    top = fb::warp_max(top);
-    if (lane == 0) {
-        red[warp] = top;
-    }
-    __syncthreads();
-    top = red[0];
-#pragma unroll
-    for (int i = 1; i < kDecodeThreads / 32; ++i) {
-        top = fmaxf(top, red[i]);
-    }
-    __syncthreads();
-    float sum = 0.0f;
-    for (int t = tid; t < length; t += kDecodeThreads) {
-        const float p = exp2f(scores[t] - top);
-        scores[t] = p;
-        sum += p;
-    }
-    sum = fb::warp_sum_rn(sum);
-    if (lane == 0) {
-        red[warp] = sum;
-    }
-    __syncthreads();
-    sum = red[0];
-#pragma unroll
-    for (int i = 1; i < kDecodeThreads / 32; ++i) {
-        sum += red[i];
-    }
-    // Thread (group, piece): positions group, group + 64, ...; eight output columns.
-    const int piece = tid % 8;
-    const int group = tid / 8;
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll 8
-    for (int t = group; t < length; t += kGroups) {
-        const __half* row = t == newest ? new_v : values + static_cast<size_t>(t) * kHeadWidth;
-        const uint4 raw = load_streaming(reinterpret_cast<const uint4*>(row) + piece);
-        float v[8];
-        fb::unpack8(v, raw);
-        const float p = scores[t];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            acc[j] = fmaf(p, v[j], acc[j]);
-        }
-    }
+    };
+    fetch(begin);
+    fb::dependency_wait();
+    const uint4* row = reinterpret_cast<const uint4*>(qkv + static_cast<size_t>(sequence) * 3 * width +
+                                                      head * kHeadWidth) + eighth;
+    float q[8];
+    fb::unpack8(q, *row);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        partial[group][piece * 8 + j] = acc[j];
+        q[j] = q[j] * scale * kLog2e;
+    }
+    auto score_of = [&](const uint4& raw) {
+        float kv[8];
+        fb::unpack8(kv, raw);
+        float s = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            s = fmaf(kv[j], q[j], s);
+        }
+        s += __shfl_xor_sync(fb::kFullMask, s, 1);
+        s += __shfl_xor_sync(fb::kFullMask, s, 2);
+        return s + __shfl_xor_sync(fb::kFullMask, s, 4);
+    };
+    float m = -INFINITY;
+    float l = 0.0f;
+    float acc[8] = {};
+    auto add_value = [&](float p, const uint4& raw) {
+        float vv[8];
+        fb::unpack8(vv, raw);
+        l += p;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            acc[j] = fmaf(p, vv[j], acc[j]);
+        }
+    };
+    for (int from = begin; from < end; from += 32 * kRounds) {
+        if (from != begin) {
+            fetch(from);
+        }
+        float s[kRounds];
+        float top = m;
+#pragma unroll
+        for (int i = 0; i < kRounds; ++i) {
+            s[i] = score_of(k[i]);
+            if (from + group + 32 * i < end) {
+                top = fmaxf(top, s[i]);
+            }
+        }
+        const float keep = merge_weight(m, top);
+        l *= keep;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            acc[j] *= keep;
+        }
+        m = top;
+#pragma unroll
+        for (int i = 0; i < kRounds; ++i) {
+            if (from + group + 32 * i < end) {
+                add_value(s[i] == -INFINITY ? 0.0f : exp2f(s[i] - m), v[i]);
+            }
+        }
+    }
+    if (rank == 0 && warp == 0) {
+        const uint4 new_k = row[width / 8];
+        const uint4 new_v = row[2 * (width / 8)];
+        const float s = score_of(new_k);
+        if (lane < 8) {
+            const float top = fmaxf(m, s);
+            const float keep = merge_weight(m, top);
+            l *= keep;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                acc[j] *= keep;
+            }
+            m = top;
+            add_value(s == -INFINITY ? 0.0f : exp2f(s - m), new_v);
+            reinterpret_cast<uint4*>(cache_k + base + static_cast<size_t>(newest) * kHeadWidth)[eighth] = new_k;
+            reinterpret_cast<uint4*>(cache_v + base + static_cast<size_t>(newest) * kHeadWidth)[eighth] = new_v;
+        }
+    }
+    // The warp's four groups.
+#pragma unroll
+    for (int off = 8; off < 32; off <<= 1) {
+        const float other_m = __shfl_xor_sync(fb::kFullMask, m, off);
+        const float top = fmaxf(m, other_m);
+        const float mine = merge_weight(m, top);
+        const float theirs = merge_weight(other_m, top);
+        l = l * mine + __shfl_xor_sync(fb::kFullMask, l, off) * theirs;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            acc[j] = acc[j] * mine + __shfl_xor_sync(fb::kFullMask, acc[j], off) * theirs;
+        }
+        m = top;
+    }
+    if (lane < 8) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            partial[warp][8 * lane + j] = acc[j];
+        }
+        if (lane == 0) {
+            partial_m[warp] = m;
+            partial_l[warp] = l;
+        }
     }
     __syncthreads();
+    float total = 0.0f;
+    float sum = 0.0f;
+    float top = -INFINITY;
     if (tid < kHeadWidth) {
-        float total = 0.0f;
-#pragma unroll 8
-        for (int g2 = 0; g2 < kGroups; ++g2) {
-            total += partial[g2][tid];
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            top = fmaxf(top, partial_m[w]);
         }
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const float weight = merge_weight(partial_m[w], top);
+            sum += weight * partial_l[w];
+            total += weight * partial[w][tid];
+        }
+    }
+    // Every CTA of the cluster has begun: the leading one's shared memory may be written.
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (splits > 1) {
+        if (tid < kHeadWidth) {
+            auto put = [&](int at, float value) {
+                const uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(&meet[rank][at]));
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(sm100::map_to_cta(local, 0)),
+                             "f"(value)
+                             : "memory");
+            };
+            put(tid, total);
+            if (tid == 0) {
+                put(kHeadWidth, top);
+                put(kHeadWidth + 1, sum);
+            }
+        }
+        sm100::cluster_sync_all();
+        if (rank != 0) {
+            return;
+        }
+        if (tid < kHeadWidth) {
+            top = -INFINITY;
+            for (int r = 0; r < splits; ++r) {
+                top = fmaxf(top, meet[r][kHeadWidth]);
+            }
+            total = 0.0f;
+            sum = 0.0f;
+            for (int r = 0; r < splits; ++r) {
+                const float weight = merge_weight(meet[r][kHeadWidth], top);
+                sum += weight * meet[r][kHeadWidth + 1];
+                total += weight * meet[r][tid];
+            }
+        }
+    }
+    if (tid < kHeadWidth) {
         out[static_cast<size_t>(sequence) * width + head * kHeadWidth + tid] =
             __float2half_rn(total / sum);
     }
@@ -439,49 +829,6 @@ __global__ void __launch_bounds__(256)
         out[static_cast<size_t>(b) * width + c] = src[c];
     }
 }
-
-// Greedy choice: the lowest index of the largest logit below `vocab`.
-__global__ void __launch_bounds__(256)
-    fb_argmax_rows(uint16_t* __restrict__ next, const float* __restrict__ logits, int vocab,
-                   int stride) {
-    __shared__ float best_value[8];
-    __shared__ int best_index[8];
-    const float* row = logits + static_cast<size_t>(blockIdx.x) * stride;
-    float value = -INFINITY;
-    int index = 0;
-    for (int c = threadIdx.x; c < vocab; c += 256) {
-        const float v = row[c];
-        if (v > value) {
-            value = v;
-            index = c;
-        }
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const float ov = __shfl_xor_sync(fb::kFullMask, value, off);
-        const int oi = __shfl_xor_sync(fb::kFullMask, index, off);
-        if (ov > value || (ov == value && oi < index)) {
-            value = ov;
-            index = oi;
-        }
-    }
-    if (threadIdx.x % 32 == 0) {
-        best_value[threadIdx.x / 32] = value;
-        best_index[threadIdx.x / 32] = index;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w2 = 1; w2 < 8; ++w2) {
-            if (best_value[w2] > value || (best_value[w2] == value && best_index[w2] < index)) {
-                value = best_value[w2];
-                index = best_index[w2];
-            }
-        }
-        next[blockIdx.x] = static_cast<uint16_t>(index);
-    }
-}
-
-__global__ void fb_advance_position(int* position, int by) { *position += by; }
 
 }  // namespace
 
@@ -501,6 +848,8 @@ struct flint_b200_generator {
     __half *h = nullptr, *qkv = nullptr, *attn = nullptr, *act = nullptr, *pre = nullptr;
     float *mean = nullptr, *rstd = nullptr, *lse = nullptr, *logits = nullptr;
     uint16_t* next = nullptr;
+    unsigned long long* best = nullptr;  // greedy choice in progress, per sequence
+    unsigned* ticket = nullptr;
     __half* dequantized = nullptr;     // int8: FP16 scratch for one matrix
     std::vector<void*> owned;
     cudaGraphExec_t step_graph = nullptr;
@@ -552,36 +901,103 @@ flint_status quantize(flint_b200_generator& g, Matrix& m, cudaStream_t stream) {
     return FLINT_OK;
 }
 
-template <typename W, Act A, int F, int S>
-flint_status launch_skinny(void* out, const W* w, const float* scale, const float* bias,
-                           const __half* x, const float* residual, size_t n, size_t k,
-                           size_t out_stride, cudaStream_t stream) {
-    const size_t per_cta = static_cast<size_t>(kLinearWarps / S) * F;
-    const unsigned grid = static_cast<unsigned>((n + per_cta - 1) / per_cta);
-    fb_decode_linear<W, A, F, S><<<grid, 32 * kLinearWarps, 0, stream>>>(
-        out, w, scale, bias, x, residual, static_cast<int>(n), static_cast<int>(k),
-        static_cast<int>(out_stride));
-    FB_CUDA(fb::after_launch());
+// A decode kernel's launch: dependent on the one before it, in clusters of `cluster` CTAs.
+template <typename... Params, typename... Args>
+cudaError_t launch_cluster(void (*kernel)(Params...), unsigned grid, unsigned cluster,
+                           cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(kThreads);
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = cluster;
+    attributes[0].val.clusterDim.y = 1;
+    attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = fb::dependent_launch_enabled() ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+    const cudaError_t last = fb::after_launch();
+    return e != cudaSuccess ? e : last;
+}
+
+template <typename W, Act A, bool kNorm, int MB, int NT, int kSteps, int QN>
+flint_status launch_linear(const LinearArgs& args, cudaStream_t stream) {
+    auto kernel = fb_decode_linear<W, A, kNorm, MB, NT, kSteps, QN>;
+    const int smem = linear_bytes(kNorm, MB, NT, args.rows, args.k);
+    static std::atomic<bool> configured[64] = {};
+    FB_CUDA(fb::allow_shared_memory(kernel, linear_bytes(kNorm, MB, NT, 16 * MB, 128 * QN), configured));
+    FB_CUDA(fb::launch_dependent(kernel, dim3(static_cast<unsigned>(args.n / (8 * NT))), dim3(kThreads),
+                                 static_cast<size_t>(smem), stream, args));
     return FLINT_OK;
 }
 
-// Eight rows at `x` (spare rows of the caller's buffers are scratch when fewer are live).
-template <Act A>
-flint_status skinny(const flint_b200_generator& g, const Matrix& m, void* out, const __half* x,
-                    const float* residual, size_t out_stride, cudaStream_t stream) {
-    // Narrow outputs: two features per CTA with k split over its four warps (as many CTAs as
-    // a wide output has). Wide outputs: two features per warp.
-    const bool narrow = m.n <= 1024;
-    if (g.int8) {
-        return narrow ? launch_skinny<int8_t, A, 2, kLinearWarps>(out, m.q, m.scale, m.bias, x, residual,
-                                                                  m.n, m.k, out_stride, stream)
-                      : launch_skinny<int8_t, A, 2, 1>(out, m.q, m.scale, m.bias, x, residual, m.n, m.k,
-                                                       out_stride, stream);
+// The step counts and register rows follow from k: the layers' k is the width (at most 768,
+// or at most 1,536) or, behind the GELU, four times that. A normalising kernel takes 16
+// features per CTA (its CTAs each normalise every row, so there should not be many), the
+// others 8 (so that 768 of them spread over 96 CTAs).
+template <typename W, Act A, int MB>
+flint_status linear_for(const LinearArgs& args, cudaStream_t stream) {
+    constexpr bool kNorm = A != Act::kResidual;
+    constexpr int kPer = Step<W>::kPieces;   // int8 takes twice the k per step
+    if constexpr (kNorm) {
+        return args.k <= 768 ? launch_linear<W, A, true, MB, 2, (3 + kPer - 1) / kPer, 6>(args, stream)
+                             : launch_linear<W, A, true, MB, 2, 6 / kPer, 12>(args, stream);
+    } else {
+        if (args.k <= 768) {
+            return launch_linear<W, A, false, MB, 1, (3 + kPer - 1) / kPer, 1>(args, stream);
+        }
+        if (args.k <= 3072) {
+            return launch_linear<W, A, false, MB, 1, 12 / kPer, 1>(args, stream);
+        }
+        return launch_linear<W, A, false, MB, 1, 24 / kPer, 1>(args, stream);
     }
-    return narrow ? launch_skinny<__half, A, 2, kLinearWarps>(out, m.half, nullptr, m.bias, x, residual,
-                                                              m.n, m.k, out_stride, stream)
-                  : launch_skinny<__half, A, 2, 1>(out, m.half, nullptr, m.bias, x, residual, m.n, m.k,
-                                                   out_stride, stream);
+}
+
+// One decode linear layer. kNone and kGelu normalise x (FP32 rows) first.
+template <Act A>
+flint_status decode_linear(const flint_b200_generator& g, const Matrix& m, void* out, const void* x,
+                           const float* gain, const float* shift, const float* residual,
+                           cudaStream_t stream) {
+    const LinearArgs args{out,  g.int8 ? static_cast<const void*>(m.q) : m.half,
+                          m.scale, m.bias, x, gain, shift, residual,
+                          static_cast<int>(g.sequences), static_cast<int>(m.n), static_cast<int>(m.k)};
+    if (g.int8) {
+        return g.sequences <= 16   ? linear_for<int8_t, A, 1>(args, stream)
+               : g.sequences <= 32 ? linear_for<int8_t, A, 2>(args, stream)
+                                   : linear_for<int8_t, A, 4>(args, stream);
+    }
+    return g.sequences <= 16   ? linear_for<__half, A, 1>(args, stream)
+           : g.sequences <= 32 ? linear_for<__half, A, 2>(args, stream)
+                               : linear_for<__half, A, 4>(args, stream);
+}
+
+template <typename W, int MB, int QN>
+flint_status launch_head(const HeadArgs& args, cudaStream_t stream) {
+    auto kernel = fb_decode_head<W, MB, QN>;
+    static std::atomic<bool> configured[64] = {};
+    FB_CUDA(fb::allow_shared_memory(kernel, norm_bytes(16 * MB, 128 * QN), configured));
+    int sms = 0;
+    FB_CUDA(fb::sm_count(&sms));
+    const int tiles = (args.n + 8 * kWarps - 1) / (8 * kWarps);
+    FB_CUDA(fb::launch_dependent(kernel, dim3(static_cast<unsigned>(std::min(2 * sms, tiles))),
+                                 dim3(kThreads), static_cast<size_t>(norm_bytes(args.rows, args.k)),
+                                 stream, args));
+    return FLINT_OK;
+}
+
+template <typename W>
+flint_status head_for(const HeadArgs& args, cudaStream_t stream) {
+    const bool narrow = args.k <= 768;
+    if (args.rows <= 16) {
+        return narrow ? launch_head<W, 1, 6>(args, stream) : launch_head<W, 1, 12>(args, stream);
+    }
+    if (args.rows <= 32) {
+        return narrow ? launch_head<W, 2, 6>(args, stream) : launch_head<W, 2, 12>(args, stream);
+    }
+    return narrow ? launch_head<W, 4, 6>(args, stream) : launch_head<W, 4, 12>(args, stream);
 }
 
 // The FP16 weights the tensor-core GEMMs read: the model's copy, or the int8 weights
@@ -598,27 +1014,11 @@ flint_status dense_weights(const flint_b200_generator& g, const Matrix& m, const
     return FLINT_OK;
 }
 
-// y = act(x w^T + bias) for `rows` rows. kNone/kGelu: FP16 out; kResidual: FP32 out =
-// residual + (x w^T + bias). (The output layer always takes the streaming kernel.)
+// y = act(x w^T + bias) for a prompt's rows. kNone/kGelu: FP16 out; kResidual: FP32 out =
+// residual + (x w^T + bias).
 template <Act A>
 flint_status linear(const flint_b200_generator& g, const Matrix& m, void* out, const __half* x,
-                    const float* residual, size_t rows, bool decode, cudaStream_t stream) {
-    static_assert(A != Act::kLogits, "the output layer does not come through here");
-    if (decode && rows <= kSkinnyRows) {
-        return skinny<A>(g, m, out, x, residual, m.n, stream);
-    }
-    if (decode && g.int8) {
-        // More than eight sequences on int8 weights: groups of eight through the streaming
-        // kernel (the weights are re-read per group; the tensor cores take FP16 only).
-        for (size_t first = 0; first < rows; first += kSkinnyRows) {
-            const size_t stride = m.n;
-            const size_t bytes = A == Act::kResidual ? 4 : 2;
-            FB_TRY(skinny<A>(g, m, static_cast<char*>(out) + first * stride * bytes,
-                             x + first * m.k, residual == nullptr ? nullptr : residual + first * m.n,
-                             stride, stream));
-        }
-        return FLINT_OK;
-    }
+                    const float* residual, size_t rows, cudaStream_t stream) {
     const __half* w = nullptr;
     FB_TRY(dense_weights(g, m, &w, stream));
     if constexpr (A == Act::kNone) {
@@ -639,82 +1039,84 @@ flint_status layernorm(const flint_b200_generator& g, const float* gain, const f
     return flint_layernorm_forward(g.h, g.mean, g.rstd, x, gain, bias, rows, g.width, kEps, stream);
 }
 
-// The transformer over `rows` = sequences * count rows. decode: count == 1 and attention
-// runs against the cache; otherwise the fused causal kernel runs over the prompt.
-flint_status run_blocks(flint_b200_generator& g, size_t count, bool decode, cudaStream_t stream) {
+float attention_scale() { return 1.0f / std::sqrt(static_cast<float>(kHeadWidth)); }
+
+// The transformer over a prompt of `count` positions per sequence. The stream of rows starts
+// and ends in x_a: every block moves it to x_b and back.
+flint_status run_prompt(flint_b200_generator& g, size_t count, cudaStream_t stream) {
     const size_t rows = g.sequences * count;
-    float* x = g.x_a;
-    float* other = g.x_b;
-    const float scale = 1.0f / std::sqrt(static_cast<float>(kHeadWidth));
     for (size_t i = 0; i < g.layers; ++i) {
         const Layer& l = g.blocks[i];
-        FB_TRY(layernorm(g, l.ln1_w, l.ln1_b, x, rows, stream));
-        FB_TRY(linear<Act::kNone>(g, l.attn, g.qkv, g.h, nullptr, rows, decode, stream));
-        if (decode) {
-            // (The kernel also stores the new token's key and value in the cache.)
-            const int smem = static_cast<int>(g.max_length * sizeof(float));
-            fb_decode_attention<<<static_cast<unsigned>(g.sequences * g.heads), kDecodeThreads, smem,
-                                  stream>>>(
-                g.attn, g.qkv, g.keys(i), g.values(i), g.position, static_cast<int>(g.heads),
-                static_cast<int>(g.max_length), scale);
-            FB_CUDA(fb::after_launch());
-        } else {
-            fb_cache_store<<<static_cast<unsigned>(rows), 256, 0, stream>>>(
-                g.keys(i), g.values(i), g.qkv, nullptr, static_cast<int>(g.host_position),
-                static_cast<int>(count), static_cast<int>(g.heads), static_cast<int>(g.max_length));
-            FB_CUDA(fb::after_launch());
-            const size_t w3 = 3 * g.width;
-            auto view = [&](const void* base, size_t first, size_t row_width) {
-                return fb::AttentionView{static_cast<const __half*>(base) + first,
-                                         static_cast<long long>(row_width), kHeadWidth,
-                                         static_cast<long long>(count * row_width)};
-            };
-            FB_CUDA(fb::attention_forward(view(g.attn, 0, g.width), g.lse, view(g.qkv, 0, w3),
-                                          view(g.qkv, g.width, w3), view(g.qkv, 2 * g.width, w3),
-                                          fb::AttentionShape{g.sequences, g.heads, count}, scale,
-                                          stream));
-        }
-        FB_TRY(linear<Act::kResidual>(g, l.proj, other, g.attn, x, rows, decode, stream));
-        std::swap(x, other);
-        FB_TRY(layernorm(g, l.ln2_w, l.ln2_b, x, rows, stream));
-        FB_TRY(linear<Act::kGelu>(g, l.fc, g.act, g.h, nullptr, rows, decode, stream));
-        FB_TRY(linear<Act::kResidual>(g, l.fcproj, other, g.act, x, rows, decode, stream));
-        std::swap(x, other);
-    }
-    if (x != g.x_a) {
-        // An even number of swaps per block keeps the stream in x_a; this is a safeguard.
-        FB_CUDA(cudaMemcpyAsync(g.x_a, x, rows * g.width * 4, cudaMemcpyDeviceToDevice, stream));
+        FB_TRY(layernorm(g, l.ln1_w, l.ln1_b, g.x_a, rows, stream));
+        FB_TRY(linear<Act::kNone>(g, l.attn, g.qkv, g.h, nullptr, rows, stream));
+        fb_cache_store<<<static_cast<unsigned>(rows), 256, 0, stream>>>(
+            g.keys(i), g.values(i), g.qkv, static_cast<int>(g.host_position),
+            static_cast<int>(count), static_cast<int>(g.heads), static_cast<int>(g.max_length));
+        FB_CUDA(fb::after_launch());
+        const size_t w3 = 3 * g.width;
+        auto view = [&](const void* base, size_t first, size_t row_width) {
+            return fb::AttentionView{static_cast<const __half*>(base) + first,
+                                     static_cast<long long>(row_width), kHeadWidth,
+                                     static_cast<long long>(count * row_width)};
+        };
+        FB_CUDA(fb::attention_forward(view(g.attn, 0, g.width), g.lse, view(g.qkv, 0, w3),
+                                      view(g.qkv, g.width, w3), view(g.qkv, 2 * g.width, w3),
+                                      fb::AttentionShape{g.sequences, g.heads, count},
+                                      attention_scale(), stream));
+        FB_TRY(linear<Act::kResidual>(g, l.proj, g.x_b, g.attn, g.x_a, rows, stream));
+        FB_TRY(layernorm(g, l.ln2_w, l.ln2_b, g.x_b, rows, stream));
+        FB_TRY(linear<Act::kGelu>(g, l.fc, g.act, g.h, nullptr, rows, stream));
+        FB_TRY(linear<Act::kResidual>(g, l.fcproj, g.x_a, g.act, g.x_b, rows, stream));
     }
     return FLINT_OK;
 }
 
-// Final LayerNorm + output layer over the `sequences` rows at `x`, then the greedy choice.
-flint_status run_head(flint_b200_generator& g, const float* x, void* next_tokens,
-                      cudaStream_t stream) {
-    FB_TRY(layernorm(g, g.lnf_w, g.lnf_b, x, g.sequences, stream));
-    // Groups of eight rows through the streaming kernel: FP32 logits straight from the sums.
-    for (size_t first = 0; first < g.sequences; first += kSkinnyRows) {
-        FB_TRY(skinny<Act::kLogits>(g, g.head, g.logits + first * g.padded_vocab, g.h + first * g.width,
-                                    nullptr, g.padded_vocab, stream));
+// The transformer over one new position per sequence.
+flint_status run_token(flint_b200_generator& g, cudaStream_t stream) {
+    // As many CTAs per (sequence, head) as fill the GPU, up to a cluster of eight.
+    int sms = 0;
+    FB_CUDA(fb::sm_count(&sms));
+    const size_t pairs = g.sequences * g.heads;
+    unsigned splits = 1;
+    while (splits < kMostSplits && pairs * splits < static_cast<size_t>(sms)) {
+        splits *= 2;
     }
-    uint16_t* next = next_tokens != nullptr ? static_cast<uint16_t*>(next_tokens) : g.next;
-    fb_argmax_rows<<<static_cast<unsigned>(g.sequences), 256, 0, stream>>>(
-        next, g.logits, static_cast<int>(g.vocab), static_cast<int>(g.padded_vocab));
-    FB_CUDA(fb::after_launch());
+    for (size_t i = 0; i < g.layers; ++i) {
+        const Layer& l = g.blocks[i];
+        FB_TRY(decode_linear<Act::kNone>(g, l.attn, g.qkv, g.x_a, l.ln1_w, l.ln1_b, nullptr, stream));
+        FB_CUDA(launch_cluster(fb_decode_attention, static_cast<unsigned>(pairs) * splits, splits, stream,
+                               g.attn, g.qkv, g.keys(i), g.values(i), g.position,
+                               static_cast<int>(g.heads), static_cast<int>(g.max_length),
+                               static_cast<int>(splits), attention_scale()));
+        FB_TRY(decode_linear<Act::kResidual>(g, l.proj, g.x_b, g.attn, nullptr, nullptr, g.x_a, stream));
+        FB_TRY(decode_linear<Act::kGelu>(g, l.fc, g.act, g.x_b, l.ln2_w, l.ln2_b, nullptr, stream));
+        FB_TRY(decode_linear<Act::kResidual>(g, l.fcproj, g.x_a, g.act, nullptr, nullptr, g.x_b, stream));
+    }
     return FLINT_OK;
+}
+
+// Final LayerNorm, output layer and greedy choice over the `sequences` rows at `x`; the
+// position moves on by `advance`.
+flint_status run_head(flint_b200_generator& g, const float* x, void* next_tokens, int advance,
+                      cudaStream_t stream) {
+    const HeadArgs args{g.logits, g.int8 ? static_cast<const void*>(g.head.q) : g.head.half,
+                        g.head.scale, x, g.lnf_w, g.lnf_b, g.best, g.ticket,
+                        next_tokens != nullptr ? static_cast<uint16_t*>(next_tokens) : g.next,
+                        g.position, static_cast<int>(g.sequences), static_cast<int>(g.head.n),
+                        static_cast<int>(g.head.k), static_cast<int>(g.vocab), advance};
+    return g.int8 ? head_for<int8_t>(args, stream) : head_for<__half>(args, stream);
 }
 
 flint_status enqueue_step(flint_b200_generator& g, const void* tokens, void* next_tokens,
                           cudaStream_t stream) {
+    // Launched the ordinary way: it begins when everything before the step has finished, and
+    // so do the step's other kernels, which read weights and older cache rows ahead of time.
     fb_decode_embed<<<static_cast<unsigned>(g.sequences), 256, 0, stream>>>(
         g.x_a, static_cast<const uint16_t*>(tokens), g.wte, g.wpe, g.position,
         static_cast<int>(g.width), static_cast<int>(g.padded_vocab));
     FB_CUDA(fb::after_launch());
-    FB_TRY(run_blocks(g, 1, true, stream));
-    FB_TRY(run_head(g, g.x_a, next_tokens, stream));
-    fb_advance_position<<<1, 1, 0, stream>>>(g.position, 1);
-    FB_CUDA(fb::after_launch());
-    return FLINT_OK;
+    FB_TRY(run_token(g, stream));
+    return run_head(g, g.x_a, next_tokens, 1, stream);
 }
 
 flint_status build(flint_b200_generator& g, cudaStream_t stream) {
@@ -743,16 +1145,14 @@ flint_status build(flint_b200_generator& g, cudaStream_t stream) {
         l.fcproj = matrix_of(w.fcproj_w, w.fcproj_b);
         g.blocks.push_back(l);
     }
-    // The streaming kernel always computes groups of eight rows: every buffer holds whole groups.
-    const size_t groups = (g.sequences + kSkinnyRows - 1) / kSkinnyRows * kSkinnyRows;
-    const size_t rows = std::max<size_t>(g.sequences * g.max_length, groups);
+    const size_t rows = g.sequences * g.max_length;
     const size_t w = g.width;
     FB_TRY(allocate(g, &g.position, 4));
     FB_CUDA(cudaMemsetAsync(g.position, 0, 16, stream));
     FB_TRY(allocate(g, &g.cache, 2 * g.layers * g.cache_stride()));
     FB_TRY(allocate(g, &g.x_a, rows * w));
     FB_TRY(allocate(g, &g.x_b, rows * w));
-    FB_TRY(allocate(g, &g.last, groups * w));
+    FB_TRY(allocate(g, &g.last, g.sequences * w));
     FB_TRY(allocate(g, &g.h, rows * w));
     FB_TRY(allocate(g, &g.qkv, rows * 3 * w));
     FB_TRY(allocate(g, &g.attn, rows * w));
@@ -761,15 +1161,12 @@ flint_status build(flint_b200_generator& g, cudaStream_t stream) {
     FB_TRY(allocate(g, &g.mean, rows));
     FB_TRY(allocate(g, &g.rstd, rows));
     FB_TRY(allocate(g, &g.lse, g.sequences * g.heads * g.max_length));
-    FB_TRY(allocate(g, &g.logits, groups * g.padded_vocab));
-    FB_TRY(allocate(g, &g.next, groups));
-    FB_CUDA(cudaMemsetAsync(g.last, 0, groups * w * 4, stream));
-    // Spare rows of the small buffers are read by the streaming kernel: keep them finite.
-    FB_CUDA(cudaMemsetAsync(g.h, 0, rows * w * 2, stream));
-    FB_CUDA(cudaMemsetAsync(g.attn, 0, rows * w * 2, stream));
-    FB_CUDA(cudaMemsetAsync(g.act, 0, rows * 4 * w * 2, stream));
-    FB_CUDA(cudaMemsetAsync(g.x_a, 0, rows * w * 4, stream));
-    FB_CUDA(cudaMemsetAsync(g.x_b, 0, rows * w * 4, stream));
+    FB_TRY(allocate(g, &g.logits, g.sequences * g.padded_vocab));
+    FB_TRY(allocate(g, &g.next, g.sequences));
+    FB_TRY(allocate(g, &g.best, g.sequences));
+    FB_TRY(allocate(g, &g.ticket, 1));
+    FB_CUDA(cudaMemsetAsync(g.best, 0, g.sequences * sizeof(*g.best), stream));
+    FB_CUDA(cudaMemsetAsync(g.ticket, 0, sizeof(*g.ticket), stream));
     if (g.int8) {
         // Holds one matrix at a time: the largest of the output layer and the MLP's.
         FB_TRY(allocate(g, &g.dequantized, std::max(g.padded_vocab * w, 4 * w * w)));
@@ -863,13 +1260,11 @@ flint_status flint_b200_generator_prefill(flint_b200_generator* generator, const
     FB_CUDA(cudaMemsetAsync(g.position, 0, 4, stream));
     FB_TRY(flint_embedding_forward(g.x_a, tokens, g.wte, g.wpe, g.sequences, length, g.padded_vocab,
                                    g.width, stream));
-    FB_TRY(run_blocks(g, length, false, stream));
+    FB_TRY(run_prompt(g, length, stream));
     fb_take_last_rows<<<static_cast<unsigned>(g.sequences), 256, 0, stream>>>(
         g.last, g.x_a, static_cast<int>(length), static_cast<int>(g.width));
     FB_CUDA(fb::after_launch());
-    FB_TRY(run_head(g, g.last, nullptr, stream));
-    fb_advance_position<<<1, 1, 0, stream>>>(g.position, static_cast<int>(length));
-    FB_CUDA(fb::after_launch());
+    FB_TRY(run_head(g, g.last, nullptr, static_cast<int>(length), stream));
     g.host_position = length;
     return FLINT_OK;
 }
@@ -953,8 +1348,6 @@ flint_status flint_b200_generator_bytes_per_step(const flint_b200_generator* gen
             weights += m->n * m->k * element;
         }
     }
-    // The output layer is streamed once per group of eight sequences.
-    weights += g.head.n * g.head.k * element * ((g.sequences + kSkinnyRows - 1) / kSkinnyRows - 1);
     if (weight_bytes != nullptr) {
         *weight_bytes = weights;
     }

@@ -210,8 +210,8 @@ FLINT_API flint_status flint_b200_generator_step(flint_b200_generator* generator
 FLINT_API flint_status flint_b200_generator_logits(const flint_b200_generator* generator,
                                                    const void** logits, size_t* position);
 
-/* Bytes the next decode step must read from HBM: the weights (each matrix once;
- * the output layer once per group of eight sequences) and the cache. */
+/* Bytes the next decode step must read from HBM: the weights (each matrix once)
+ * and the cache. */
 FLINT_API flint_status flint_b200_generator_bytes_per_step(const flint_b200_generator* generator,
                                                            size_t* weight_bytes,
                                                            size_t* cache_bytes);
