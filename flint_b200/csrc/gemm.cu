@@ -765,7 +765,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
     } else if (warp == 1) {
         // ---- MMA issuer ----
-        if (lane == 0) {
+        // The whole warp runs the loop, so that its state stays warp-uniform; one elected
+        // lane issues (with the loop inside `lane == 0`, every MMA paid moves into uniform
+        // registers: a k-block of a 64-column tile took 0.27 us instead of 0.24).
+        {
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
@@ -791,20 +794,23 @@ __global__ void __launch_bounds__(kThreads, 1)
                     sm100::tc_fence_after_sync();
                     const uint32_t a_addr = smem_base + stage * R::kStage;
                     const uint32_t b_addr = a_addr + R::kStageA;
+                    const uint64_t a_desc = kAMn ? sm100::smem_desc_sw128(a_addr, 8192, 1024)
+                                                 : sm100::smem_desc_sw128(a_addr, 16, 1024);
+                    const uint64_t b_desc = kBMn ? sm100::smem_desc_sw128(b_addr, 8192, 1024)
+                                                 : sm100::smem_desc_sw128(b_addr, 16, 1024);
+                    if (sm100::elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < kBK / 16; ++ks) {
-                        // K-major: 16 halves = 32 bytes along the swizzled row.
-                        // MN-major: 16 k-rows of 128 bytes.
-                        const uint64_t a_desc =
-                            kAMn ? sm100::smem_desc_sw128(a_addr + ks * 2048, 8192, 1024)
-                                 : sm100::smem_desc_sw128(a_addr + ks * 32, 16, 1024);
-                        const uint64_t b_desc =
-                            kBMn ? sm100::smem_desc_sw128(b_addr + ks * 2048, 8192, 1024)
-                                 : sm100::smem_desc_sw128(b_addr + ks * 32, 16, 1024);
-                        sm100::mma_f16_ss(d_tmem, a_desc, b_desc, kIdesc, accumulate);
-                        accumulate = 1;
+                        for (int ks = 0; ks < kBK / 16; ++ks) {
+                            if (ks == 0) {
+                                sm100::mma_f16_ss_at<-1>(d_tmem, a_desc, 0, b_desc, 0, kIdesc, accumulate);
+                            } else {
+                                sm100::mma_f16_ss_at<1>(d_tmem, a_desc, ks * (kAMn ? 128 : 2), b_desc,
+                                                        ks * (kBMn ? 128 : 2), kIdesc);
+                            }
+                        }
+                        sm100::mma_commit(empty_bar(stage));
                     }
-                    sm100::mma_commit(empty_bar(stage));
+                    accumulate = 1;
                     if (++stage == R::kStages) {
                         stage = 0;
                         phase ^= 1u;
@@ -813,7 +819,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (!ok) {
                     break;
                 }
-                sm100::mma_commit(acc_full_bar(acc));
+                if (sm100::elect_one()) {
+                    sm100::mma_commit(acc_full_bar(acc));
+                }
                 acc ^= 1;
                 if (acc == 0) {
                     acc_phase ^= 1u;
@@ -1089,7 +1097,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
         }
     } else if (warp == 1) {
         // ---- MMA issuer (leader only) ----
-        if (leader && lane == 0) {
+        if (leader) {
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
@@ -1115,18 +1123,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
                     sm100::tc_fence_after_sync();
                     const uint32_t a_addr = smem_base + stage * kPairStage;
                     const uint32_t b_addr = a_addr + kPairStageA;
+                    const uint64_t a_desc = kAMn ? sm100::smem_desc_sw128(a_addr, 8192, 1024)
+                                                 : sm100::smem_desc_sw128(a_addr, 16, 1024);
+                    const uint64_t b_desc = kBMn ? sm100::smem_desc_sw128(b_addr, 8192, 1024)
+                                                 : sm100::smem_desc_sw128(b_addr, 16, 1024);
+                    if (sm100::elect_one()) {
 #pragma unroll
-                    for (int ks = 0; ks < kBK / 16; ++ks) {
-                        const uint64_t a_desc =
-                            kAMn ? sm100::smem_desc_sw128(a_addr + ks * 2048, 8192, 1024)
-                                 : sm100::smem_desc_sw128(a_addr + ks * 32, 16, 1024);
-                        const uint64_t b_desc =
-                            kBMn ? sm100::smem_desc_sw128(b_addr + ks * 2048, 8192, 1024)
-                                 : sm100::smem_desc_sw128(b_addr + ks * 32, 16, 1024);
-                        sm100::mma_f16_ss_pair(d_tmem, a_desc, b_desc, kIdesc, accumulate);
-                        accumulate = 1;
+                        for (int ks = 0; ks < kBK / 16; ++ks) {
+                            sm100::mma_f16_ss_pair(d_tmem, a_desc + ks * (kAMn ? 128 : 2),
+                                                   b_desc + ks * (kBMn ? 128 : 2), kIdesc,
+                                                   ks == 0 ? accumulate : 1u);
+                        }
+                        sm100::mma_commit_pair(empty_bar(stage), 3);
                     }
-                    sm100::mma_commit_pair(empty_bar(stage), 3);
+                    accumulate = 1;
                     if (++stage == kPairStages) {
                         stage = 0;
                         phase ^= 1u;
@@ -1135,7 +1145,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
                 if (!ok) {
                     break;
                 }
-                sm100::mma_commit_pair(acc_full_bar(acc), 3);
+                if (sm100::elect_one()) {
+                    sm100::mma_commit_pair(acc_full_bar(acc), 3);
+                }
                 acc ^= 1;
                 if (acc == 0) {
                     acc_phase ^= 1u;
@@ -1438,7 +1450,132 @@ bool use_simt() {
     return cached == 1;
 }
 
-int pick_bn(size_t n) { return n > 128 ? 256 : (n > 64 ? 128 : 64); }
+bool pair_disabled() {
+    static int cached = -1;
+    if (cached < 0) {
+        const char* v = std::getenv("FLINT_B200_GEMM");
+        cached = (v != nullptr && std::strcmp(v, "single") == 0) ? 1 : 0;
+    }
+    return cached == 1;
+}
+
+// ---- which tile a problem gets ---------------------------------------------------------------
+//
+// The pair kernel's 256 x 256 tiles move the fewest bytes per FLOP and win wherever they fill
+// the GPU more than twice. Below that a problem is a few rounds of tiles at most, and its
+// time is what one SM spends: the k loop of a tile, which costs about the same per 64 of k
+// for every width up to 128 (0.24-0.26 us; 0.28 for a pair, 0.34 for 128 x 256), and the
+// epilogue, which grows with the tile's columns. So small problems take the narrowest tile
+// that still fits one round. Measured in a chain of launches, pair -> chosen: bias+residual
+// 1,000 x 768 x 768 12.3 -> 6.2 us, x 3,072 22.6 -> 14.8; NN 1,000 x 768 x 3,072 18.2 -> 14.3,
+// 2,048 x 768 x 3,072 18.4 -> 16.5; bias 1,000 x 2,304 x 768 9.3 -> 7.4; TN 3,072 x 768 x 1,000
+// 12.4 -> 9.8; bias+GELU 500 x 3,072 x 768 11.6 -> 9.5. The estimate below reproduces the
+// measured times of 64 to 8,192 rows (widths 768 to 3,072) to about 15 %.
+
+enum class Tile { k64, k128, k256, kPair };
+
+int tile_columns(Tile t) { return t == Tile::k64 ? 64 : t == Tile::k128 ? 128 : 256; }
+
+// Microseconds that all tiles have alike, and per 32-column chunk of an epilogue warp: when
+// it is the last thing a launch does, and when it runs beside the next tile's k loop (the
+// pair kernel stores asynchronously and reads the accumulators a chunk ahead).
+constexpr double kTileFixed = 2.7;
+struct ChunkTime {
+    double last, steady_pair, steady_single;
+};
+constexpr ChunkTime chunk_time(Epilogue e) {
+    switch (e) {
+    case Epilogue::kNone:
+    case Epilogue::kScale:
+        return {0.4, 0.5, 0.6};
+    case Epilogue::kBias:
+        return {0.7, 0.9, 1.2};
+    case Epilogue::kTnStore:
+    case Epilogue::kTnPartial:
+        return {1.1, 1.3, 1.5};
+    case Epilogue::kBiasResidual:
+        return {1.4, 2.3, 2.6};
+    case Epilogue::kDGelu:
+        return {1.5, 1.7, 2.7};
+    default:
+        return {1.4, 1.4, 2.6};
+    }
+}
+
+double tile_time(Tile t, Layout l, Epilogue e, long long tiles, size_t k, int sms) {
+    constexpr double kBlock[2][4] = {{0.24, 0.26, 0.34, 0.28}, {0.28, 0.34, 0.37, 0.33}};
+    const double loop = kBlock[l == Layout::kTN][static_cast<int>(t)] * static_cast<double>((k + kBK - 1) / kBK);
+    const long long slots = t == Tile::kPair ? std::max(1, sms / 2) : sms;
+    const double more = static_cast<double>((tiles + slots - 1) / slots - 1);
+    const int chunks = tile_columns(t) / 64;   // per epilogue warp
+    const ChunkTime c = chunk_time(e);
+    return kTileFixed + loop + chunks * c.last + more * std::max(1.2 * loop, chunks * (t == Tile::kPair ? c.steady_pair : c.steady_single));
+}
+
+long long tile_count(Tile t, size_t m, size_t n) {
+    const size_t rows = t == Tile::kPair ? 256 : kBM;
+    const size_t columns = tile_columns(t);
+    return static_cast<long long>((m + rows - 1) / rows) * static_cast<long long>((n + columns - 1) / columns);
+}
+
+// Whether a shape can use a tile at all: no tile whose second half would be empty.
+bool tile_fits(Tile t, size_t m, size_t n) {
+    switch (t) {
+    case Tile::k64:
+        return true;
+    case Tile::k128:
+        return n > 64;
+    case Tile::k256:
+        return n > 128;
+    default:
+        return !pair_disabled() && m > 128 && n > 128;
+    }
+}
+
+// How often TN may split k with tile `t`: into pieces of at least 1,024, and not at all where
+// whole tiles keep three quarters of the CTAs (or pairs) busy.
+int most_splits(Tile t, size_t m, size_t n, size_t k, int sms) {
+    const long long tiles = tile_count(t, m, n);
+    const long long slots = t == Tile::kPair ? std::max(1, sms / 2) : sms;
+    const long long waves = (tiles + slots - 1) / slots;
+    if (4 * tiles >= 3 * waves * slots) {
+        return 1;
+    }
+    return static_cast<int>(std::min<size_t>(16, std::max<size_t>(1, k / 1024)));
+}
+
+// The tile for `batches` problems of one shape; *splits (TN, or null) is how often k is split,
+// whose partial sums cost a second launch that reads and adds them.
+Tile pick_tile(Layout l, Epilogue e, size_t m, size_t n, size_t k, long long batches, int sms,
+               int* splits) {
+    constexpr Tile kTiles[] = {Tile::kPair, Tile::k256, Tile::k128, Tile::k64};
+    Tile chosen = Tile::k64;
+    double best = 0.0;
+    for (Tile t : kTiles) {
+        if (!tile_fits(t, m, n)) {
+            continue;
+        }
+        const int most = splits != nullptr ? most_splits(t, m, n, k, sms) : 1;
+        for (int s = 1; s <= most; ++s) {
+            double time = tile_time(t, l, e, tile_count(t, m, n) * batches * s, (k + s - 1) / s, sms);
+            if (s > 1) {
+                time += 1.0 + static_cast<double>(s + 1) * static_cast<double>(m) * static_cast<double>(n) * 4.0 / 16e6;
+            }
+            // A wider tile, or fewer splits, are given up for a gain of a twentieth, no less.
+            if (best == 0.0 || time < 0.95 * best) {
+                best = time;
+                chosen = t;
+                if (splits != nullptr) {
+                    *splits = s;
+                }
+            }
+        }
+        if (t == Tile::kPair && tile_count(t, m, n) * batches > static_cast<long long>(sms)) {
+            break;  // more than two rounds of pairs
+        }
+    }
+    return chosen;
+}
 
 template <Layout L, Epilogue E, int BN>
 cudaError_t launch_tc(GemmParams& p, const void* x, const void* w, int sms, cudaStream_t stream) {
@@ -1476,21 +1613,6 @@ cudaError_t launch_tc(GemmParams& p, const void* x, const void* w, int sms, cuda
     }
     const unsigned grid = static_cast<unsigned>(std::min<long long>(p.tiles_total, sms));
     return fb::launch_dependent(kernel, dim3(grid), dim3(kThreads), R::kSmemBytes, stream, p);
-}
-
-bool pair_disabled() {
-    static int cached = -1;
-    if (cached < 0) {
-        const char* v = std::getenv("FLINT_B200_GEMM");
-        cached = (v != nullptr && std::strcmp(v, "single") == 0) ? 1 : 0;
-    }
-    return cached == 1;
-}
-
-// The CTA-pair kernel pays off once both CTAs of a pair have rows to work on
-// and the tile is full width.
-bool use_pair(const GemmParams& p) {
-    return !pair_disabled() && p.m > 128 && p.n > 128;
 }
 
 template <Layout L, Epilogue E>
@@ -1562,13 +1684,19 @@ cudaError_t launch_any(GemmParams& p, const void* x, const void* w, cudaStream_t
                                                      static_cast<const __half*>(w));
         return fb::after_launch();
     }
-    if (use_pair(p)) {
-        return launch_pair<L, E>(p, x, w, sms, stream);
+    Tile tile;
+    if (L == Layout::kTN && p.batched == 0) {
+        int splits = 1;   // as gemm_tn has set them already
+        tile = pick_tile(L, E, p.m, p.n, p.k, 1, sms, &splits);
+    } else {
+        tile = pick_tile(L, E, p.m, p.n, p.k, p.batches, sms, nullptr);
     }
-    switch (pick_bn(static_cast<size_t>(p.n))) {
-    case 256:
+    switch (tile) {
+    case Tile::kPair:
+        return launch_pair<L, E>(p, x, w, sms, stream);
+    case Tile::k256:
         return launch_tc<L, E, 256>(p, x, w, sms, stream);
-    case 128:
+    case Tile::k128:
         return launch_tc<L, E, 128>(p, x, w, sms, stream);
     default:
         return launch_tc<L, E, 64>(p, x, w, sms, stream);
@@ -1595,29 +1723,9 @@ GemmParams base_params(void* y, size_t m, size_t n, size_t k, size_t batches, bo
 // ---- internal launchers (declared in gemm.h) --------------------------------------------
 
 TnSplit tn_split(size_t m, size_t n, size_t k, int sms) {
-    // Tiles and the CTAs (or CTA pairs) that run at once, for the kernel this shape gets.
-    const bool pair = !pair_disabled() && m > 128 && n > 128;
-    const long long tiles =
-        pair ? static_cast<long long>((m + 255) / 256) * static_cast<long long>((n + 255) / 256)
-             : static_cast<long long>((m + kBM - 1) / kBM) *
-                   static_cast<long long>((n + pick_bn(n) - 1) / pick_bn(n));
-    const long long slots = pair ? std::max(1, sms / 2) : sms;
-    const int most = static_cast<int>(std::min<size_t>(16, std::max<size_t>(1, k / 1024)));
+    // (kTnPartial's and kTnStore's chunks cost the same, so both see one choice.)
     int want = 1;
-    double best = 0.0;
-    for (int s = 1; s <= most; ++s) {
-        const long long blocks = tiles * s;
-        const long long waves = (blocks + slots - 1) / slots;
-        const double fill = static_cast<double>(blocks) / static_cast<double>(waves * slots);
-        if (fill > best) {
-            best = fill;
-            want = s;
-        }
-        if (fill >= 0.75) {
-            want = s;
-            break;
-        }
-    }
+    pick_tile(Layout::kTN, Epilogue::kTnStore, m, n, k, 1, sms, &want);
     const size_t per = (k + want - 1) / want;
     TnSplit r;
     r.len = static_cast<int>((per + kBK - 1) / kBK * kBK);

@@ -405,3 +405,33 @@ def test_gelu_derivative_is_within_one_ulp_and_correctly_rounded_where_that_is_d
     assert safe.sum() > 0.95 * safe.numel()
     wrong = safe & (oracle.half_ordered(y) != oracle.half_ordered(exact))
     assert not wrong.any(), int(wrong.sum())
+
+
+@pytest.mark.parametrize("m, n, k", [(129, 136, 64), (1000, 768, 328), (250, 2304, 72), (2056, 768, 512),
+                                     (500, 3072, 768), (64, 3080, 1032)])
+def test_small_problems_agree_between_layouts_and_epilogues(flint, m, n, k):
+    """Small problems take tiles of 64 to 256 columns by an estimate of their time, so the forms
+    of one product can run on different kernels: NT, NN, TN (unsplit) and the biased forms (bias
+    -0) must still round the same sums, ragged edges included."""
+    x, w = inputs((m, k), (n, k), m + n)
+    xd, wd = x.to(DEV), w.to(DEV)
+    zero = torch.full((n,), -0.0, device=DEV)
+    nt, nn, biased, pre, act = (torch.full((m, n), 7.0, dtype=torch.half, device=DEV) for _ in range(5))
+    flint.gemm_nt(nt, xd, wd, m, n, k)
+    flint.gemm_nn(nn, xd, wd.t().contiguous(), m, n, k)
+    flint.gemm_nt_bias(biased, xd, wd, zero, m, n, k)
+    flint.gemm_nt_bias_gelu(act, pre, xd, wd, zero, m, n, k)
+    batched = torch.full((2, m, n), 7.0, dtype=torch.half, device=DEV) if m <= 1024 else None
+    if batched is not None:
+        flint.gemm_nt_batched(batched, torch.stack([xd, xd]), torch.stack([wd, wd]), 2, m, n, k)
+    added = torch.full((m, n), 7.0, device=DEV)
+    flint.gemm_nt_bias_residual(added, xd, wd, zero, torch.zeros(m, n, device=DEV), m, n, k)
+    if m % 8 == 0 and flint.gemm_tn_workspace(m, n, k) == 0:
+        tn = torch.full((m, n), 7.0, device=DEV)
+        flint.gemm_tn(tn, xd.t().contiguous(), wd.t().contiguous(), m, n, k)
+        assert torch.equal(tn, added)
+    no_fault(flint)
+    assert rel_error(nt, oracle.gemm_nt(x, w)) <= 2e-3
+    assert torch.equal(nn, nt) and torch.equal(pre, nt) and torch.equal(biased, nt)
+    assert torch.equal(added.half(), nt)
+    assert batched is None or (torch.equal(batched[0], nt) and torch.equal(batched[1], nt))
