@@ -32,7 +32,6 @@ using fb::Comp;
 
 constexpr size_t kChunkRows = 256;
 constexpr int kLaneRows = 8;    // interleaved row streams per chunk
-constexpr int kTilePieces = 32; // 8-column pieces per CTA tile
 constexpr size_t kMaxCols = size_t{65535} * 256;            // 16,776,960
 constexpr size_t kMaxBiasRows = size_t{0x7fffffff} * 256;   // 549,755,813,632
 constexpr size_t kMaxRows8 = size_t{0x7fffffff} * 8;
@@ -43,9 +42,13 @@ constexpr size_t column_sum_workspace(size_t rows, size_t cols) {
 
 enum class Source { kHalf, kHalfTimesXhat, kFloat };
 
-// First pass. CTA (chunk, tile) with 32 x 9 threads: warps 0-7 add (thread
-// (px, ly) owns the 8 columns of piece tile*32+px and the row stream ly), warp 8
-// fetches.
+// First pass. CTA (chunk, tile of 64 columns): warp ly adds row stream ly, a lane two columns,
+// and a ninth warp fetches.
+//
+// A chunk's adding is a chain of 32 rows per stream, seven (with a product eleven) dependent
+// FP32 operations each. A small matrix needs that chain short, so a lane has one column pair
+// only; a large one needs bytes in flight, which many narrow CTAs give as well. In the place of 256
+// columns and eight a lane: 300 x 768 with a product 8.8 -> 5.7 us, 8,192 x 768 FP16 9.0 -> 6.4 us.
 //
 // The chunk's rows reach the CTA through shared memory: lane l of the fetching
 // warp issues one bulk asynchronous copy per row segment (32 rows per stage, a
@@ -54,6 +57,11 @@ enum class Source { kHalf, kHalfTimesXhat, kFloat };
 // strictly in row order. (A thread that loaded its own rows would add each one as
 // it arrived, paying one memory latency per row.) The additions run on packed
 // FP32 pairs: columns (0,1), (2,3), (4,5), (6,7) of the piece.
+constexpr int kTilePieces = 8;
+constexpr int kTileColumns = kTilePieces * 8;
+constexpr int kAddThreads = 32 * kLaneRows;            // a warp per stream; and a fetching warp
+constexpr unsigned kTilesY = 32768;                    // tiles per grid layer
+
 template <Source kSource>
 struct Staging {
     static constexpr int kMainBytes = kSource == Source::kFloat ? 32 : 16;  // per piece and row
@@ -61,12 +69,13 @@ struct Staging {
     static constexpr int kRows = 32;                                        // rows per stage
     static constexpr int kMainStage = kRows * kTilePieces * kMainBytes;
     static constexpr int kStage = kMainStage + kRows * kTilePieces * kXBytes;
-    static constexpr int kStages = kSource == Source::kHalf ? 4 : 2;
+    // All of a chunk's 256 rows at once (FP16), or half of them.
+    static constexpr int kStages = kSource == Source::kHalf ? 8 : 4;
     static constexpr int kBytes = kStages * kStage + 128;
 };
 // After the last stage the ring's memory holds the eight streams' sums for the merge.
 static_assert(Staging<Source::kHalf>::kStages * Staging<Source::kHalf>::kStage >=
-                  2 * kLaneRows * kTilePieces * 8 * 4,
+                  2 * kLaneRows * kTileColumns * 4,
               "the merge buffers must fit in the ring");
 
 __device__ int g_reduction_error = 0;
@@ -110,14 +119,14 @@ struct ColumnMaps {
 // instead of seven); the eight streams, the chunks and the lanes are still merged with
 // compensated adds in the same fixed order. This is not the reference's pinned
 // arithmetic (the public entry points never use it); the model built on the fused
-// attention kernels does, where it makes these kernels bandwidth-bound. In that variant
-// the FP16-times-xhat kernel (LayerNorm's dgamma) also sums the FP16 values themselves
-// (dbeta) from the same staged rows, with the operations the plain FP16 kernel would
-// use, and writes those partial sums as a second block right behind the first one.
-template <Source kSource, bool kPlain>
-__global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
-    fb_column_partials(const __grid_constant__ ColumnMaps maps, float4* __restrict__ partial,
-                       const void* __restrict__ src, const float4* __restrict__ x,
+// attention kernels does, where it makes these kernels bandwidth-bound.
+// The FP16-times-xhat kernel (LayerNorm's dgamma) also sums the FP16 values themselves
+// (dbeta) from the same staged rows, with the operations the FP16 kernel would use, and
+// writes those partial sums to `second` (unless kAlso is false).
+template <Source kSource, bool kPlain, bool kAlso>
+__global__ void __launch_bounds__(kAddThreads + 32)
+    fb_column_partials(const __grid_constant__ ColumnMaps maps, float* __restrict__ partial,
+                       float* __restrict__ second, const void* __restrict__ src, const float4* __restrict__ x,
                        const float* __restrict__ mean, const float* __restrict__ rstd, size_t rows,
                        int pieces) {
     using S = Staging<kSource>;
@@ -126,10 +135,12 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
     __shared__ float sh_rstd[kSource == Source::kHalfTimesXhat ? kChunkRows : 1];
     __shared__ alignas(8) unsigned long long barriers[2 * S::kStages];
     __shared__ int abort_flag;
-    const int px = threadIdx.x;
-    const int ly = threadIdx.y;  // 0-7 add, 8 fetches
-    const int first_piece = blockIdx.y * kTilePieces;
-    const int piece = first_piece + px;
+    const int lane = threadIdx.x % 32;   // adding: columns 2 lane, 2 lane + 1 of the tile
+    const int ly = threadIdx.x / 32;     // 0-7: the row stream; 8: fetching
+    const int first_piece = (blockIdx.z * kTilesY + blockIdx.y) * kTilePieces;
+    if (first_piece >= pieces) {
+        return;
+    }
     const int width = min(kTilePieces, pieces - first_piece);  // pieces this tile holds
     const size_t first = size_t{blockIdx.x} * kChunkRows;
     const int chunk_rows = static_cast<int>(rows - first < kChunkRows ? rows - first : kChunkRows);
@@ -139,7 +150,7 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
     auto full_bar = [&](int slot) { return bar0 + 8u * slot; };
     auto empty_bar = [&](int slot) { return bar0 + 8u * (S::kStages + slot); };
 
-    if (ly == 0 && px == 0) {
+    if (threadIdx.x == 0) {
         abort_flag = 0;
         for (int i = 0; i < S::kStages; ++i) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full_bar(i)) : "memory");
@@ -151,12 +162,11 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     fb::dependency_wait();
-    if (ly == 0 && px == 0) {
+    if (threadIdx.x == 0) {
         fb::dependency_release();
     }
     if constexpr (kSource == Source::kHalfTimesXhat) {
-        const int t = ly * kTilePieces + px;
-        if (t < chunk_rows) {
+        for (int t = threadIdx.x; t < chunk_rows; t += kAddThreads + 32) {
             sh_mean[t] = mean[first + t];
             sh_rstd[t] = rstd[first + t];
         }
@@ -165,9 +175,10 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
     volatile int* abort = &abort_flag;
     bool ok = true;
     int issued = 0;  // fetching warp: stages whose copies have been started
-    fb::Comp2 acc[4];
-    constexpr bool kAlsoPlainSums = kPlain && kSource == Source::kHalfTimesXhat;
-    fb::F2 also[4] = {0, 0, 0, 0};
+    fb::Comp2 acc;
+    // LayerNorm's two parameter gradients come from one reading of dy.
+    constexpr bool kAlsoSums = kAlso && kSource == Source::kHalfTimesXhat;
+    fb::Comp2 also;
 
     if (ly == kLaneRows) {
         // ---- fetching warp: lane l copies row l of each stage (and its x segment) ----
@@ -186,7 +197,7 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
             if (maps.use != 0) {
                 // One tensor load per operand: the box is always delivered whole (zeros
                 // past the matrix's edges, which the adding warps never read).
-                if (px == 0) {
+                if (lane == 0) {
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                                      full_bar(slot)),
                                  "r"(static_cast<uint32_t>(S::kStage))
@@ -211,17 +222,17 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
                 }
                 continue;
             }
-            if (px == 0) {
+            if (lane == 0) {
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                                  full_bar(slot)),
                              "r"(static_cast<uint32_t>(here) * (main_bytes + x_bytes))
                              : "memory");
             }
-            if (px < here) {
+            if (lane < here) {
                 const size_t at =
-                    (first + static_cast<size_t>(k) * S::kRows + px) * pieces + first_piece;
+                    (first + static_cast<size_t>(k) * S::kRows + lane) * pieces + first_piece;
                 const uint32_t dst =
-                    staging + slot * S::kStage + px * (kTilePieces * S::kMainBytes);
+                    staging + slot * S::kStage + lane * (kTilePieces * S::kMainBytes);
                 asm volatile(
                     "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                     ::"r"(dst), "l"(static_cast<const unsigned char*>(src) + at * S::kMainBytes),
@@ -229,7 +240,7 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
                     : "memory");
                 if constexpr (S::kXBytes != 0) {
                     const uint32_t xdst = staging + slot * S::kStage + S::kMainStage +
-                                          px * (kTilePieces * S::kXBytes);
+                                          lane * (kTilePieces * S::kXBytes);
                     asm volatile(
                         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                         ::"r"(xdst),
@@ -241,14 +252,8 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
         }
     } else {
         // ---- adding warps ----
-        auto load16 = [](uint4& q, uint32_t at) {
-            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w)
-                         : "r"(at));
-        };
-        auto pair_of = [](uint32_t lo, uint32_t hi) {
-            return static_cast<fb::F2>(lo) | (static_cast<fb::F2>(hi) << 32);
-        };
+        const int at_main = lane * (S::kMainBytes / 4);   // two columns' bytes
+        const int at_x = S::kMainStage + lane * (S::kXBytes / 4);
         for (int k = 0; k < stages_total; ++k) {
             const int slot = k % S::kStages;
             if (!staged_wait(full_bar(slot), static_cast<uint32_t>(k / S::kStages) & 1u, abort)) {
@@ -257,77 +262,58 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
             }
             const int here = min(S::kRows, chunk_rows - k * S::kRows);
             const uint32_t stage = staging + slot * S::kStage;
-            if (px < width) {
+            if (lane < 4 * width) {
 #pragma unroll
                 for (int j = 0; j < S::kRows / kLaneRows; ++j) {
                     const int row = ly + kLaneRows * j;  // row inside the stage
                     if (row >= here) {
                         break;
                     }
-                    fb::F2 v[4];
-                    const uint32_t at =
-                        stage + row * (kTilePieces * S::kMainBytes) + px * S::kMainBytes;
-                    uint4 a;
-                    load16(a, at);
+                    fb::F2 v;
+                    const uint32_t at = stage + row * (kTilePieces * S::kMainBytes) + at_main;
                     if constexpr (kSource == Source::kFloat) {
-                        uint4 b;
-                        load16(b, at + 16);
-                        v[0] = pair_of(a.x, a.y);
-                        v[1] = pair_of(a.z, a.w);
-                        v[2] = pair_of(b.x, b.y);
-                        v[3] = pair_of(b.z, b.w);
+                        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(at));
                     } else {
-                        float f[8];
-                        fb::unpack8(f, a);
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            v[c] = fb::f2_pack(f[2 * c], f[2 * c + 1]);
-                        }
+                        unsigned bits;
+                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(bits) : "r"(at));
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&bits));
+                        v = fb::f2_pack(f.x, f.y);
                     }
                     if constexpr (kSource == Source::kHalfTimesXhat) {
-                        uint4 x0;
-                        uint4 x1;
-                        const uint32_t xat = stage + S::kMainStage +
-                                             row * (kTilePieces * S::kXBytes) + px * S::kXBytes;
-                        load16(x0, xat);
-                        load16(x1, xat + 16);
-                        const fb::F2 xs[4] = {pair_of(x0.x, x0.y), pair_of(x0.z, x0.w),
-                                              pair_of(x1.x, x1.y), pair_of(x1.z, x1.w)};
+                        fb::F2 xs;
+                        asm volatile("ld.shared.b64 %0, [%1];"
+                                     : "=l"(xs)
+                                     : "r"(stage + row * (kTilePieces * S::kXBytes) + at_x));
                         const float m = sh_mean[k * S::kRows + row];
                         const float rs = sh_rstd[k * S::kRows + row];
-                        const fb::F2 m2 = fb::f2_pack(m, m);
-                        const fb::F2 rs2 = fb::f2_pack(rs, rs);
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            const fb::F2 xhat = fb::f2_mul(fb::f2_sub(xs[c], m2), rs2);
-                            if constexpr (kPlain) {
-                                acc[c].s = fb::f2_fma(v[c], xhat, acc[c].s);
-                                also[c] = fb::f2_add(also[c], v[c]);
-                            } else {
-                                fb::comp_add_product2(acc[c], v[c], xhat);
-                            }
+                        const fb::F2 xhat =
+                            fb::f2_mul(fb::f2_sub(xs, fb::f2_pack(m, m)), fb::f2_pack(rs, rs));
+                        if constexpr (kPlain) {
+                            acc.s = fb::f2_fma(v, xhat, acc.s);
+                        } else {
+                            fb::comp_add_product2(acc, v, xhat);
                         }
+                        if constexpr (kAlsoSums && kPlain) {
+                            also.s = fb::f2_add(also.s, v);
+                        } else if constexpr (kAlsoSums) {
+                            fb::comp_add2(also, v);
+                        }
+                    } else if constexpr (kPlain) {
+                        acc.s = fb::f2_add(acc.s, v);
                     } else {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            if constexpr (kPlain) {
-                                acc[c].s = fb::f2_add(acc[c].s, v[c]);
-                            } else {
-                                fb::comp_add2(acc[c], v[c]);
-                            }
-                        }
+                        fb::comp_add2(acc, v);
                     }
                 }
             }
-            // This warp is done with the slot; the fetching warp refills it once all eight are.
+            // This stream is done with the slot; the fetching warp refills it once all eight are.
             __syncwarp();
-            if (px == 0) {
+            if (lane == 0) {
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty_bar(slot))
                              : "memory");
             }
         }
     }
-    if (!ok && px == 0) {
+    if (!ok && lane == 0) {
         atomicExch(&g_reduction_error, 1);
     }
     __syncthreads();
@@ -337,7 +323,7 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
         // leaves, the fetching warp waits, again with a limit, for the copies it started
         // into the ring: shared memory must not be handed to another CTA with a copy
         // still on its way.
-        if (ly == kLaneRows && px == 0) {
+        if (ly == kLaneRows && lane == 0) {
             for (int k = max(0, issued - S::kStages); k < issued; ++k) {
                 int unused = 0;
                 staged_wait(full_bar(k % S::kStages), static_cast<uint32_t>(k / S::kStages) & 1u,
@@ -347,51 +333,36 @@ __global__ void __launch_bounds__(kTilePieces * (kLaneRows + 1))
         return;
     }
     // Every stage has been consumed: the ring's memory now carries the eight streams'
-    // (sum, error) pairs to stream 0, which merges them in stream order.
+    // (sum, error) pairs to a thread per column, which merges them in stream order.
     float* sh_s = reinterpret_cast<float*>(staging_raw + (staging - shared_address(staging_raw)));
-    float* sh_e = sh_s + kLaneRows * kTilePieces * 8;
-    const size_t block_quads = size_t{gridDim.x} * pieces * 4;  // float4s in one block of partials
+    float* sh_e = sh_s + kLaneRows * kTileColumns;
 #pragma unroll
-    for (int set = 0; set < (kAlsoPlainSums ? 2 : 1); ++set) {
+    for (int set = 0; set < (kAlsoSums ? 2 : 1); ++set) {
         if (set == 1) {
-            __syncthreads();  // stream 0 has read the first set
+            __syncthreads();  // the first set has been read
         }
         if (ly < kLaneRows) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                float lo, hi;
-                fb::f2_unpack(set == 0 ? acc[c].s : also[c], lo, hi);
-                sh_s[(ly * kTilePieces + px) * 8 + 2 * c] = lo;
-                sh_s[(ly * kTilePieces + px) * 8 + 2 * c + 1] = hi;
-                fb::f2_unpack(set == 0 ? acc[c].e : fb::F2{0}, lo, hi);
-                sh_e[(ly * kTilePieces + px) * 8 + 2 * c] = lo;
-                sh_e[(ly * kTilePieces + px) * 8 + 2 * c + 1] = hi;
-            }
+            const int at = ly * kTileColumns + 2 * lane;
+            fb::f2_unpack(set == 0 ? acc.s : also.s, sh_s[at], sh_s[at + 1]);
+            fb::f2_unpack(set == 0 ? acc.e : also.e, sh_e[at], sh_e[at + 1]);
         }
         __syncthreads();
-        if (ly != 0 || piece >= pieces) {
+        const int column = threadIdx.x;
+        if (column >= width * 8) {
             continue;
         }
-        Comp total[8];
+        Comp total;
+        total.s = sh_s[column];
+        total.e = sh_e[column];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            total[j].s = sh_s[px * 8 + j];
-            total[j].e = sh_e[px * 8 + j];
-        }
         for (int other = 1; other < kLaneRows; ++other) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                fb::comp_merge(total[j], sh_s[(other * kTilePieces + px) * 8 + j],
-                               sh_e[(other * kTilePieces + px) * 8 + j]);
-            }
+            fb::comp_merge(total, sh_s[other * kTileColumns + column],
+                           sh_e[other * kTileColumns + column]);
         }
         // Chunk c occupies rows 2c (sums) and 2c+1 (errors) of a [2*chunks, cols] FP32 matrix.
-        float4* out = partial + set * block_quads + size_t{blockIdx.x} * pieces * 4 + size_t(piece) * 2;
-        out[0] = make_float4(total[0].s, total[1].s, total[2].s, total[3].s);
-        out[1] = make_float4(total[4].s, total[5].s, total[6].s, total[7].s);
-        out += size_t(pieces) * 2;
-        out[0] = make_float4(total[0].e, total[1].e, total[2].e, total[3].e);
-        out[1] = make_float4(total[4].e, total[5].e, total[6].e, total[7].e);
+        float* out = (set == 0 ? partial : second) + size_t{blockIdx.x} * pieces * 16 + first_piece * 8 + column;
+        out[0] = total.s;
+        out[size_t(pieces) * 8] = total.e;
     }
 }
 
@@ -477,9 +448,10 @@ __global__ void __launch_bounds__(32 * kFinishWarps)
     }
 }
 
-template <Source kSource, bool kPlain = false>
+template <Source kSource, bool kPlain = false, bool kAlso = true>
 cudaError_t launch_partials(void* workspace, const void* src, const void* x, const void* mean,
-                            const void* rstd, size_t rows, size_t cols, cudaStream_t stream) {
+                            const void* rstd, size_t rows, size_t cols, cudaStream_t stream,
+                            void* second = nullptr) {
     const unsigned chunks = static_cast<unsigned>((rows + kChunkRows - 1) / kChunkRows);
     const int pieces = static_cast<int>(cols / 8);
     const unsigned tiles = static_cast<unsigned>((pieces + kTilePieces - 1) / kTilePieces);
@@ -491,7 +463,7 @@ cudaError_t launch_partials(void* workspace, const void* src, const void* x, con
         return e;
     }
     if (device >= 64 || !configured[device].load(std::memory_order_relaxed)) {
-        e = cudaFuncSetAttribute(fb_column_partials<kSource, kPlain>,
+        e = cudaFuncSetAttribute(fb_column_partials<kSource, kPlain, kAlso>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kDynamic);
         if (e != cudaSuccess) {
             return e;
@@ -513,9 +485,10 @@ cudaError_t launch_partials(void* workspace, const void* src, const void* x, con
             return e;
         }
     }
-    return fb::launch_dependent(fb_column_partials<kSource, kPlain>, dim3(chunks, tiles),
-                                dim3(kTilePieces, kLaneRows + 1), kDynamic, stream, maps,
-                                static_cast<float4*>(workspace), src, static_cast<const float4*>(x),
+    return fb::launch_dependent(fb_column_partials<kSource, kPlain, kAlso>, dim3(chunks, std::min(tiles, kTilesY), (tiles + kTilesY - 1) / kTilesY),
+                                dim3(kAddThreads + 32), kDynamic, stream, maps,
+                                static_cast<float*>(workspace), static_cast<float*>(second), src,
+                                static_cast<const float4*>(x),
                                 static_cast<const float*>(mean), static_cast<const float*>(rstd),
                                 rows, pieces);
 }
@@ -1429,40 +1402,43 @@ cudaError_t launch_layernorm_backward(void* dx, void* dgamma, void* dbeta, const
                                       bool accumulate_dx, bool accumulate_params, void* workspace,
                                       cudaStream_t stream, void* dx_half, bool plain,
                                       ColumnFinishList* later) {
+    // One pass over dy serves both parameter gradients: dgamma's partial sums fill the
+    // workspace, dbeta's follow them (plain: the caller provides twice the public workspace
+    // size), or else lie where dx will be written afterwards. Where dx holds something that
+    // is added to, or has less room (a single row), dbeta takes a pass of its own, before
+    // dgamma's partial sums reuse the workspace (stream order).
+    const size_t partial_bytes = column_sum_workspace(rows, cols);
+    void* second = static_cast<unsigned char*>(workspace) + partial_bytes;
+    const bool apart = !plain && (accumulate_dx || rows * cols * 4 < partial_bytes);
     cudaError_t e = cudaSuccess;
-    if (plain) {
-        // One pass over dy serves both parameter gradients: dgamma's partial sums fill the
-        // first block of the workspace, dbeta's the second (the caller provides twice the
-        // public workspace size for this variant).
-        e = launch_partials<Source::kHalfTimesXhat, true>(workspace, dy, x, mean, rstd, rows, cols,
-                                                          stream);
-        if (e != cudaSuccess) {
-            return e;
-        }
-        e = finish_or_defer(dgamma, workspace, rows, cols, accumulate_params, stream, later);
-        if (e != cudaSuccess) {
-            return e;
-        }
-        e = finish_or_defer(dbeta,
-                            static_cast<unsigned char*>(workspace) + column_sum_workspace(rows, cols),
-                            rows, cols, accumulate_params, stream, later);
-        if (e != cudaSuccess) {
-            return e;
-        }
-    } else {
-        // dbeta first; its second pass is done with the workspace before dgamma's
-        // partial sums reuse it (stream order).
-        e = launch_bias_gradient(dbeta, dy, rows, cols, accumulate_params, workspace, stream,
-                                 false);
-        if (e != cudaSuccess) {
-            return e;
-        }
-        e = launch_partials<Source::kHalfTimesXhat>(workspace, dy, x, mean, rstd, rows, cols,
-                                                    stream);
-        if (e != cudaSuccess) {
-            return e;
-        }
-        e = launch_finish(dgamma, workspace, rows, cols, accumulate_params, stream);
+    if (apart) {
+        e = launch_bias_gradient(dbeta, dy, rows, cols, accumulate_params, workspace, stream, false);
+        second = nullptr;
+    } else if (!plain) {
+        second = dx;
+    }
+    if (e == cudaSuccess) {
+        e = plain ? launch_partials<Source::kHalfTimesXhat, true>(workspace, dy, x, mean, rstd, rows,
+                                                                  cols, stream, second)
+            : apart ? launch_partials<Source::kHalfTimesXhat, false, false>(
+                          workspace, dy, x, mean, rstd, rows, cols, stream)
+                    : launch_partials<Source::kHalfTimesXhat>(workspace, dy, x, mean, rstd, rows, cols,
+                                                              stream, second);
+    }
+    if (e != cudaSuccess) {
+        return e;
+    }
+    if (!plain) {
+        later = nullptr;   // (dx is written below: the sums in it do not keep)
+    }
+    ColumnFinishList here;
+    ColumnFinishList* list = later != nullptr ? later : &here;
+    if (!list->add(dgamma, workspace, cols, accumulate_params) ||
+        (second != nullptr && !list->add(dbeta, second, cols, accumulate_params))) {
+        return cudaErrorInvalidValue;
+    }
+    if (later == nullptr) {
+        e = launch_column_finishes(here, rows, stream);
         if (e != cudaSuccess) {
             return e;
         }
