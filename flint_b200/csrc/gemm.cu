@@ -53,7 +53,7 @@ __device__ int g_gemm_error = 0;
 struct GemmParams {
     CUtensorMap map_a;
     CUtensorMap map_b;
-    CUtensorMap map_y;    // FP16 outputs of the pair kernel leave through TMA stores
+    CUtensorMap map_y;    // FP16 outputs leave through TMA stores
     CUtensorMap map_pre;  // bias+GELU: the pre-activation output
     int tma_out;          // the two maps above are valid
     void* y;
@@ -365,6 +365,14 @@ __device__ __forceinline__ void store_chunk_async(const CUtensorMap* map, uint32
         : "memory");
 }
 
+__device__ __forceinline__ void store_chunk_async(const CUtensorMap* map, uint32_t slot, int col,
+                                                  int row, int batch) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+        ::"l"(reinterpret_cast<uint64_t>(map)), "r"(slot), "r"(col), "r"(row), "r"(batch)
+        : "memory");
+}
+
 // Moves the warp's staged FP16 chunk (4 slots per row) to `out` (row-major, ld = n).
 __device__ __forceinline__ void flush_half_chunk(uint32_t stage, __half* out_chunk, size_t n,
                                                  int rows_left, int valid, int lane) {
@@ -561,6 +569,9 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, uint32_t stage,
                 if constexpr (E == Epilogue::kBiasGelu) {
                     store_chunk_async(&p.map_pre, stage, col, static_cast<int>(row0));
                     store_chunk_async(&p.map_y, stage + 2048u, col, static_cast<int>(row0));
+                } else if (p.batched) {
+                    store_chunk_async(&p.map_y, stage, col, static_cast<int>(row0),
+                                      static_cast<int>(split));
                 } else {
                     store_chunk_async(&p.map_y, stage, col, static_cast<int>(row0));
                 }
@@ -902,6 +913,10 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (acc == 0) {
                 acc_phase ^= 1u;
             }
+        }
+        // Asynchronous output stores must have landed before the kernel is over.
+        if (p.tma_out != 0 && lane == 0) {
+            store_wait_all();
         }
     }
 
@@ -1441,6 +1456,41 @@ cudaError_t make_map(CUtensorMap* map, const void* base, size_t inner, size_t ou
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// FP16 outputs leave through TMA stores when the rows are 16-byte multiples (the tensor map's
+// requirement; the same rule as the coalesced path). Batches are a third dimension, so that
+// a ragged last tile is clipped at its own batch's edge.
+template <Epilogue E>
+cudaError_t make_store_maps(GemmParams& p) {
+    constexpr bool kHalfOut = E == Epilogue::kNone || E == Epilogue::kBias ||
+                              E == Epilogue::kBiasGelu || E == Epilogue::kDGelu ||
+                              E == Epilogue::kScale;
+    p.tma_out = 0;
+    if (!kHalfOut || p.n % 8 != 0) {
+        return cudaSuccess;
+    }
+    EncodeTiled encode = nullptr;
+    cudaError_t e = encode_fn(&encode);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(p.n), static_cast<cuuint64_t>(p.m),
+                                static_cast<cuuint64_t>(p.batches)};
+    const cuuint64_t strides[2] = {dims[0] * 2, dims[0] * dims[1] * 2};
+    const cuuint32_t box[3] = {32, 32, 1};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    auto make = [&](CUtensorMap* map, void* base) {
+        return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.batched ? 3 : 2, base, dims, strides,
+                      box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (!make(&p.map_y, p.y) || (E == Epilogue::kBiasGelu && !make(&p.map_pre, p.aux_out))) {
+        return cudaErrorInvalidValue;
+    }
+    p.tma_out = 1;
+    return cudaSuccess;
+}
+
 bool use_simt() {
     static int cached = -1;
     if (cached < 0) {
@@ -1600,6 +1650,10 @@ cudaError_t launch_tc(GemmParams& p, const void* x, const void* w, int sms, cuda
     if (e != cudaSuccess) {
         return e;
     }
+    e = make_store_maps<E>(p);
+    if (e != cudaSuccess) {
+        return e;
+    }
     p.tiles_m = (p.m + kBM - 1) / kBM;
     p.tiles_n = (p.n + BN - 1) / BN;
     const long long z = L == Layout::kTN && !batched ? p.splits : p.batches;
@@ -1637,21 +1691,9 @@ cudaError_t launch_pair(GemmParams& p, const void* x, const void* w, int sms, cu
     if (e != cudaSuccess) {
         return e;
     }
-    // FP16 outputs of unbatched calls leave through TMA stores when the rows are 16-byte
-    // multiples (the tensor map's requirement; the same rule as the coalesced path).
-    constexpr bool kHalfOut = E == Epilogue::kNone || E == Epilogue::kBias ||
-                              E == Epilogue::kBiasGelu || E == Epilogue::kDGelu ||
-                              E == Epilogue::kScale;
-    p.tma_out = 0;
-    if (kHalfOut && L != Layout::kTN && !batched && p.n % 8 == 0) {
-        e = fb::encode_rows_map(&p.map_y, p.y, p.m, p.n, 2, 32, 32, 64);
-        if (e == cudaSuccess && E == Epilogue::kBiasGelu) {
-            e = fb::encode_rows_map(&p.map_pre, p.aux_out, p.m, p.n, 2, 32, 32, 64);
-        }
-        if (e != cudaSuccess) {
-            return e;
-        }
-        p.tma_out = 1;
+    e = make_store_maps<E>(p);
+    if (e != cudaSuccess) {
+        return e;
     }
     p.tiles_m = (p.m + 255) / 256;
     p.tiles_n = (p.n + kPairBN - 1) / kPairBN;

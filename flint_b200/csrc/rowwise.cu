@@ -233,6 +233,8 @@ template <int kChunks>
 __global__ void __launch_bounds__(kThreads)
     fb_causal_softmax_forward(uint4* __restrict__ p, const uint4* __restrict__ s, size_t rows,
                               int length) {
+    fb::dependency_wait();
+    fb::dependency_release();
     const size_t row = size_t{blockIdx.x} * kWarpsPerBlock + threadIdx.x / 32;
     if (row >= rows) {
         return;
@@ -329,6 +331,8 @@ template <int kChunks>
 __global__ void __launch_bounds__(kThreads)
     fb_causal_softmax_backward(uint4* ds, const uint4* __restrict__ p, const uint4* dp,
                                size_t rows, int length, float scale) {
+    fb::dependency_wait();
+    fb::dependency_release();
     const size_t row = size_t{blockIdx.x} * kWarpsPerBlock + threadIdx.x / 32;
     if (row >= rows) {
         return;
@@ -1084,15 +1088,10 @@ flint_status flint_causal_softmax_forward(void* p, const void* s, size_t batches
     auto* pq = static_cast<uint4*>(p);
     const auto* sq = static_cast<const uint4*>(s);
     const int len = static_cast<int>(length);
-    if (length <= 256) {
-        fb_causal_softmax_forward<1><<<blocks, kThreads, 0, stream>>>(pq, sq, rows, len);
-    } else if (length <= 512) {
-        fb_causal_softmax_forward<2><<<blocks, kThreads, 0, stream>>>(pq, sq, rows, len);
-    } else {
-        fb_causal_softmax_forward<kMaxChunksPerLane><<<blocks, kThreads, 0, stream>>>(pq, sq, rows,
-                                                                                      len);
-    }
-    FB_CUDA(fb::after_launch());
+    auto* kernel = length <= 256   ? fb_causal_softmax_forward<1>
+                   : length <= 512 ? fb_causal_softmax_forward<2>
+                                   : fb_causal_softmax_forward<kMaxChunksPerLane>;
+    FB_CUDA(fb::launch_dependent(kernel, dim3(blocks), dim3(kThreads), 0, stream, pq, sq, rows, len));
     return FLINT_OK;
 }
 
@@ -1117,17 +1116,11 @@ flint_status flint_causal_softmax_backward(void* ds, const void* p, const void* 
     const auto* pq = static_cast<const uint4*>(p);
     const auto* dpq = static_cast<const uint4*>(dp);
     const int len = static_cast<int>(length);
-    if (length <= 256) {
-        fb_causal_softmax_backward<1><<<blocks, kThreads, 0, stream>>>(dsq, pq, dpq, rows, len,
-                                                                       scale);
-    } else if (length <= 512) {
-        fb_causal_softmax_backward<2><<<blocks, kThreads, 0, stream>>>(dsq, pq, dpq, rows, len,
-                                                                       scale);
-    } else {
-        fb_causal_softmax_backward<kMaxChunksPerLane><<<blocks, kThreads, 0, stream>>>(
-            dsq, pq, dpq, rows, len, scale);
-    }
-    FB_CUDA(fb::after_launch());
+    auto* kernel = length <= 256   ? fb_causal_softmax_backward<1>
+                   : length <= 512 ? fb_causal_softmax_backward<2>
+                                   : fb_causal_softmax_backward<kMaxChunksPerLane>;
+    FB_CUDA(fb::launch_dependent(kernel, dim3(blocks), dim3(kThreads), 0, stream, dsq, pq, dpq, rows,
+                                 len, scale));
     return FLINT_OK;
 }
 
