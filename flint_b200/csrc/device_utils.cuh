@@ -30,6 +30,15 @@ __device__ __forceinline__ void dependency_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// A pointer as it is after dependency_wait(): loads through it cannot be moved above the wait.
+// (Behind `const __restrict__` a compiler may take memory for unchanging while the kernel
+// runs; a dependent launch runs while the kernel before it still writes.)
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* p) {
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
+
 struct Comp {
     float s = 0.0f;  // rounded sum
     float e = 0.0f;  // sum of the rounding errors

@@ -39,7 +39,6 @@
 #include "flint/flint_b200.h"
 #include "gemm.h"
 #include "gpt2.h"
-#include "sm100.cuh"
 
 namespace {
 
@@ -128,6 +127,23 @@ __device__ __forceinline__ uint4 load_streaming(const void* p) {
     return v;
 }
 
+// 16 bytes that an earlier kernel of the step wrote while this one was already resident:
+// volatile, so after the wait it stands behind, and from L2.
+__device__ __forceinline__ uint4 load_fresh(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+
+__device__ __forceinline__ float load_fresh_float(const float* p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void mma_16x8x16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2,
                                             unsigned a3, unsigned b0, unsigned b1) {
     asm volatile(
@@ -173,17 +189,16 @@ struct Step<int8_t> {
     }
 };
 
-// One step of NT feature tiles: `low(m, piece)` and `high(m, piece)` give this lane's eight
-// activations of rows 16 m + g and 16 m + g + 8.
-template <typename W, int MB, int NT, typename Low, typename High>
-__device__ __forceinline__ void multiply(float (&acc)[MB][NT][4], const uint4 (&raw)[NT], Low low,
-                                         High high) {
+// One step of NT feature tiles: x(block, piece) gives this lane's eight activations of row
+// 8 * block + g. RB: blocks of eight rows (1, or an even number).
+template <typename W, int RB, int NT, typename X>
+__device__ __forceinline__ void multiply(float (&acc)[(RB + 1) / 2][NT][4], const uint4 (&raw)[NT], X x) {
 #pragma unroll
     for (int piece = 0; piece < Step<W>::kPieces; ++piece) {
 #pragma unroll
-        for (int m = 0; m < MB; ++m) {
-            const uint4 xa = low(m, piece);
-            const uint4 xb = high(m, piece);
+        for (int m = 0; m < (RB + 1) / 2; ++m) {
+            const uint4 xa = x(2 * m, piece);
+            const uint4 xb = RB > 1 ? x(2 * m + 1, piece) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 unsigned b0, b1;
@@ -198,38 +213,54 @@ __device__ __forceinline__ void multiply(float (&acc)[MB][NT][4], const uint4 (&
 
 // LayerNorm of `rows` FP32 rows into FP16 rows of k + 8 values in shared memory (the 16 bytes
 // between rows keep eight rows' 16-byte reads off each other's banks): a warp per row, the
-// row in registers, mean first and then the centred squares. QN float4s a lane.
+// row in registers, QN float4s a lane. Each lane takes its own values' mean and centred
+// squares; one butterfly merges both (Chan, Golub and LeVeque's update for equal counts: k is
+// a multiple of 128, so every lane has k / 32 values).
 template <int QN>
 __device__ __forceinline__ void normalise_rows(__half* h, const float* x, const float* gain,
                                                const float* shift, int rows, int k) {
     const int lane = threadIdx.x % 32;
+    const float inverse = 32.0f / static_cast<float>(k);   // of a lane's count
     for (int row = threadIdx.x / 32; row < rows; row += kWarps) {
         const float4* src = reinterpret_cast<const float4*>(x + static_cast<size_t>(row) * k);
         float4 v[QN];
-        float sum = 0.0f;
 #pragma unroll
         for (int i = 0; i < QN; ++i) {
             const int q = lane + 32 * i;
-            v[i] = 4 * q < k ? src[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (4 * q < k) {
+                const uint4 raw = load_fresh(src + q);
+                v[i] = make_float4(__uint_as_float(raw.x), __uint_as_float(raw.y),
+                                   __uint_as_float(raw.z), __uint_as_float(raw.w));
+            }
         }
+        float4 sum = v[0];
 #pragma unroll
-        for (int i = 0; i < QN; ++i) {
-            sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+        for (int i = 1; i < QN; ++i) {
+            sum = make_float4(sum.x + v[i].x, sum.y + v[i].y, sum.z + v[i].z, sum.w + v[i].w);
         }
-        const float mean = fb::warp_sum_rn(sum) / static_cast<float>(k);
-        float squares = 0.0f;
+        float mean = ((sum.x + sum.y) + (sum.z + sum.w)) * inverse;
+        float4 squares = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
         for (int i = 0; i < QN; ++i) {
             if (4 * (lane + 32 * i) < k) {
-                v[i].x -= mean;
-                v[i].y -= mean;
-                v[i].z -= mean;
-                v[i].w -= mean;
-                squares += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+                const float4 d = make_float4(v[i].x - mean, v[i].y - mean, v[i].z - mean, v[i].w - mean);
+                squares = make_float4(fmaf(d.x, d.x, squares.x), fmaf(d.y, d.y, squares.y),
+                                      fmaf(d.z, d.z, squares.z), fmaf(d.w, d.w, squares.w));
             }
         }
-        const float variance = fb::warp_sum_rn(squares) / static_cast<float>(k);
-        const float rstd = 1.0f / sqrtf(variance + kEps);
+        float centred = (squares.x + squares.y) + (squares.z + squares.w);
+        float half_count = static_cast<float>(k) / 64.0f;   // half of what each side has
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const float other = __shfl_xor_sync(fb::kFullMask, mean, off);
+            const float theirs = __shfl_xor_sync(fb::kFullMask, centred, off);
+            const float apart = other - mean;
+            mean = 0.5f * (mean + other);
+            centred = (centred + theirs) + apart * apart * half_count;
+            half_count *= 2.0f;
+        }
+        const float rstd = rsqrtf(centred * (1.0f / static_cast<float>(k)) + kEps);
 #pragma unroll
         for (int i = 0; i < QN; ++i) {
             const int q = lane + 32 * i;
@@ -237,8 +268,8 @@ __device__ __forceinline__ void normalise_rows(__half* h, const float* x, const 
                 const float4 g = reinterpret_cast<const float4*>(gain)[q];
                 const float4 b = reinterpret_cast<const float4*>(shift)[q];
                 uint2 packed;
-                packed.x = fb::pack2(v[i].x * rstd * g.x + b.x, v[i].y * rstd * g.y + b.y);
-                packed.y = fb::pack2(v[i].z * rstd * g.z + b.z, v[i].w * rstd * g.w + b.w);
+                packed.x = fb::pack2((v[i].x - mean) * rstd * g.x + b.x, (v[i].y - mean) * rstd * g.y + b.y);
+                packed.y = fb::pack2((v[i].z - mean) * rstd * g.z + b.z, (v[i].w - mean) * rstd * g.w + b.w);
                 reinterpret_cast<uint2*>(h + static_cast<size_t>(row) * (k + 8))[q] = packed;
             }
         }
@@ -262,23 +293,23 @@ __host__ __device__ constexpr int norm_bytes(int rows, int k) { return 8 * k + r
 
 // Shared memory of a linear kernel: the above, then the warps' sums (of 64 rows they do not
 // fit beside 64 wide rows; they then take the rows' place once those have been used).
-__host__ __device__ constexpr int sums_bytes(int mb, int nt) { return kWarps * 16 * mb * 8 * nt * 4; }
-__host__ __device__ constexpr int linear_bytes(bool norm, int mb, int nt, int rows, int k) {
+__host__ __device__ constexpr int sums_bytes(int rb, int nt) { return kWarps * 8 * rb * 8 * nt * 4; }
+__host__ __device__ constexpr int linear_bytes(bool norm, int rb, int nt, int rows, int k) {
     const int first = norm ? norm_bytes(rows, k) : 0;
-    return mb < 4 ? first + sums_bytes(mb, nt)
-                  : (first > sums_bytes(mb, nt) ? first : sums_bytes(mb, nt));
+    return rb < 8 ? first + sums_bytes(rb, nt)
+                  : (first > sums_bytes(rb, nt) ? first : sums_bytes(rb, nt));
 }
 
 // A CTA owns 8 NT features, its warps a share of k each; the warps' sums meet in shared
 // memory and are added in warp order. kSteps: the steps a warp's share can have.
-template <typename W, Act A, bool kNorm, int MB, int NT, int kSteps, int QN>
+template <typename W, Act A, bool kNorm, int RB, int NT, int kSteps, int QN>
 __global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p) {
     using S = Step<W>;
     constexpr int kColumns = 8 * NT;
     extern __shared__ __align__(16) unsigned char decode_smem[];
-    using Sums = float[16 * MB][kColumns];
+    using Sums = float[8 * RB][kColumns];
     Sums* sums = reinterpret_cast<Sums*>(decode_smem +
-                                         (kNorm && MB < 4 ? norm_bytes(p.rows, p.k) : 0));
+                                         (kNorm && RB < 8 ? norm_bytes(p.rows, p.k) : 0));
     fb::dependency_release();
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
@@ -320,7 +351,7 @@ __global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p)
     const size_t out_at = static_cast<size_t>(threadIdx.x / kColumns) * p.n + feature;
     float residual = 0.0f;
     if (A == Act::kResidual && static_cast<int>(threadIdx.x) / kColumns < p.rows) {
-        residual = p.residual[out_at];
+        residual = load_fresh_float(p.residual + out_at);
     }
     const __half* x = static_cast<const __half*>(p.x);
     int stride = p.k;
@@ -330,32 +361,53 @@ __global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p)
         x = rows;
         stride = p.k + 8;
     }
-    float acc[MB][NT][4] = {};
+    // Activations of a chunk of steps are all asked for before the first product needs one, and
+    // two sets of accumulators take turns, so that neither loads nor MMAs form one long chain.
+    constexpr int MB = (RB + 1) / 2;
+    constexpr int kSets = MB == 1 ? 2 : 1;
+    constexpr int kRoom = RB == 1 ? 12 : RB == 2 ? 6 : 2;          // steps' worth of registers
+    constexpr int kChunk = kSteps * S::kPieces <= kRoom ? kSteps : (kRoom + S::kPieces - 1) / S::kPieces;
+    float acc[kSets][MB][NT][4] = {};
 #pragma unroll
-    for (int j = 0; j < kSteps; ++j) {
-        if (j < mine) {
-            const __half* at = x + (begin + j) * S::kStepK + t * S::kValues;
-            auto row_values = [&](int row, int piece) {
-                return row < p.rows ? *reinterpret_cast<const uint4*>(
-                                          at + static_cast<size_t>(row) * stride + 8 * piece)
-                                    : make_uint4(0u, 0u, 0u, 0u);
-            };
-            multiply<W, MB, NT>(
-                acc, raw[j], [&](int m, int piece) { return row_values(16 * m + g, piece); },
-                [&](int m, int piece) { return row_values(16 * m + g + 8, piece); });
+    for (int from = 0; from < kSteps; from += kChunk) {
+        uint4 values[kChunk][RB][S::kPieces];
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) {
+#pragma unroll
+            for (int block = 0; block < RB; ++block) {
+#pragma unroll
+                for (int piece = 0; piece < S::kPieces; ++piece) {
+                    const int row = 8 * block + g;
+                    values[j][block][piece] = make_uint4(0u, 0u, 0u, 0u);
+                    if (from + j < mine && row < p.rows) {
+                        const __half* at = x + static_cast<size_t>(row) * stride +
+                                           (begin + from + j) * S::kStepK + t * S::kValues + 8 * piece;
+                        values[j][block][piece] =
+                            kNorm ? *reinterpret_cast<const uint4*>(at) : load_fresh(at);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) {
+            if (from + j < kSteps && from + j < mine) {
+                multiply<W, RB, NT>(acc[j % kSets], raw[from + j < kSteps ? from + j : 0],
+                                    [&](int block, int piece) { return values[j][block][piece]; });
+            }
         }
     }
-    if (kNorm && MB == 4) {
+    if (kNorm && RB == 8) {
         __syncthreads();   // the rows' place is free
     }
 #pragma unroll
     for (int m = 0; m < MB; ++m) {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-            sums[warp][16 * m + g][8 * nt + 2 * t] = acc[m][nt][0];
-            sums[warp][16 * m + g][8 * nt + 2 * t + 1] = acc[m][nt][1];
-            sums[warp][16 * m + g + 8][8 * nt + 2 * t] = acc[m][nt][2];
-            sums[warp][16 * m + g + 8][8 * nt + 2 * t + 1] = acc[m][nt][3];
+#pragma unroll
+            for (int i = 0; i < (RB == 1 ? 2 : 4); ++i) {
+                const float v = acc[0][m][nt][i] + (kSets == 2 ? acc[kSets - 1][m][nt][i] : 0.0f);
+                sums[warp][16 * m + 8 * (i / 2) + g][8 * nt + 2 * t + i % 2] = v;
+            }
         }
     }
     __syncthreads();
@@ -372,7 +424,7 @@ __global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p)
         v += bias;
         const size_t at = static_cast<size_t>(row) * p.n + feature;
         if constexpr (A == Act::kResidual) {
-            static_cast<float*>(p.out)[at] = (at == out_at ? residual : p.residual[at]) + v;
+            static_cast<float*>(p.out)[at] = (at == out_at ? residual : load_fresh_float(p.residual + at)) + v;
         } else if constexpr (A == Act::kGelu) {
             static_cast<__half*>(p.out)[at] = __float2half_rn(gelu_tanh(v));
         } else {
@@ -409,12 +461,14 @@ __device__ __forceinline__ unsigned long long candidate(float value, int index) 
     return (static_cast<unsigned long long>(ordered) << 32) | (0xffffffffu - static_cast<unsigned>(index));
 }
 
-template <typename W, int MB, int QN>
+template <typename W, int RB, int QN>
 __global__ void __launch_bounds__(kThreads, 2) fb_decode_head(const HeadArgs p) {
     using S = Step<W>;
+    constexpr int MB = (RB + 1) / 2;
+    constexpr int kHalves = RB == 1 ? 1 : 2;
     constexpr int kAhead = 12 / S::kPieces;   // steps per batch of loads
     extern __shared__ __align__(16) unsigned char decode_smem[];
-    __shared__ unsigned long long chosen[kWarps][16 * MB];
+    __shared__ unsigned long long chosen[kWarps][8 * RB];
     __shared__ bool last_cta;
     fb::dependency_release();
     const int warp = threadIdx.x / 32;
@@ -471,14 +525,12 @@ __global__ void __launch_bounds__(kThreads, 2) fb_decode_head(const HeadArgs p) 
             const int step = batch * kAhead + j;
             if (step < steps) {
                 const __half* at = rows + step * S::kStepK + t * S::kValues;
-                auto row_values = [&](int row, int piece) {
+                const uint4 one[1] = {raw[j]};
+                multiply<W, RB, 1>(acc, one, [&](int block, int piece) {
+                    const int row = 8 * block + g;
                     return row < p.rows ? *reinterpret_cast<const uint4*>(at + row * (p.k + 8) + 8 * piece)
                                         : make_uint4(0u, 0u, 0u, 0u);
-                };
-                const uint4 one[1] = {raw[j]};
-                multiply<W, MB, 1>(
-                    acc, one, [&](int m, int piece) { return row_values(16 * m + g, piece); },
-                    [&](int m, int piece) { return row_values(16 * m + g + 8, piece); });
+                });
             }
         }
         if (done) {
@@ -492,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 2) fb_decode_head(const HeadArgs p) 
 #pragma unroll
             for (int m = 0; m < MB; ++m) {
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
+                for (int half = 0; half < kHalves; ++half) {
                     const int row = 16 * m + 8 * half + g;
                     const float v0 = acc[m][0][2 * half] * s0;
                     const float v1 = acc[m][0][2 * half + 1] * s1;
@@ -524,7 +576,7 @@ __global__ void __launch_bounds__(kThreads, 2) fb_decode_head(const HeadArgs p) 
 #pragma unroll
     for (int m = 0; m < MB; ++m) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
+        for (int half = 0; half < kHalves; ++half) {
             unsigned long long key = candidate(best_value[m][half], best_index[m][half]);
 #pragma unroll
             for (int off = 1; off < 4; off <<= 1) {
@@ -603,70 +655,77 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// One query per (sequence, head) against the cache's positions 0 .. *position, by a cluster
-// of CTAs that share the older positions out evenly. Eight lanes hold a position (16 bytes
-// of its key and value each), 32 positions per CTA and round; up to 256 positions per CTA
-// are in registers before the kernel waits for the new token's qkv row. Each group of eight
+// One query per (sequence, head) against the cache's positions 0 .. *position, a CTA each.
+// Eight lanes hold a position (16 bytes of its key and value each), so a round of the CTA is
+// 64 positions. Before it waits for the new token's qkv row, a thread copies its share of up
+// to 512 older positions into its own slots of shared memory (which cost the neighbouring
+// kernels no registers); further positions come four rounds at a time. Each group of eight
 // lanes keeps its own running maximum, sum and weighted values; they are merged over the
-// warp, the CTA and, through distributed shared memory, the cluster. The leading CTA takes
-// the new token's own key and value from the row and stores them in the cache for the steps
-// to come (no other CTA reads that position during this launch).
-constexpr int kRounds = 8;
-constexpr int kMostSplits = 8;
+// warp and then the CTA. The new token's own key and value come from its row, and are stored
+// in the cache for the steps to come (nothing else reads that position during this launch).
+// (A cluster of up to eight CTAs per head was tried: its two barriers cost 1,900 clocks, more
+// than eight times the positions do.)
+constexpr int kAttentionThreads = 512;
+constexpr int kAttentionWarps = kAttentionThreads / 32;
+constexpr int kRoundPositions = kAttentionThreads / 8;
+constexpr int kBatch = 4;              // rounds whose scores are worked on together
+constexpr int kStaged = 512;           // positions in shared memory
 
-// (m, l, acc) of two disjoint sets of positions, m possibly -inf for an empty one.
+constexpr int attention_bytes(int staged) { return staged * 2 * kHeadWidth * 2; }
+
+// The weight of a set of positions whose largest score is m (-inf: no positions).
 __device__ __forceinline__ float merge_weight(float m, float top) {
     return m == -INFINITY ? 0.0f : exp2f(m - top);
 }
 
-__global__ void __launch_bounds__(kThreads)
-    fb_decode_attention(__half* __restrict__ out, const __half* __restrict__ qkv,
-                        __half* __restrict__ cache_k, __half* __restrict__ cache_v,
-                        const int* __restrict__ position, int heads, int max_length, int splits,
-                        float scale) {
-    __shared__ float partial[kWarps][kHeadWidth];
-    __shared__ float partial_m[kWarps];
-    __shared__ float partial_l[kWarps];
-    __shared__ float meet[kMostSplits][kHeadWidth + 2];
+__global__ void __launch_bounds__(kAttentionThreads)
+    fb_decode_attention(__half* out, const __half* qkv, __half* cache_k, __half* cache_v,
+                        const int* position, int heads, int max_length,
+                        int staged_rounds, float scale) {
+    extern __shared__ __align__(16) unsigned char attention_smem[];
+    __shared__ float partial[kAttentionWarps][kHeadWidth];
+    __shared__ float partial_m[kAttentionWarps];
+    __shared__ float partial_l[kAttentionWarps];
     fb::dependency_release();
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    const int rank = static_cast<int>(sm100::cluster_cta_rank());
-    const int pair = blockIdx.x / splits;
-    const int head = pair % heads;
-    const int sequence = pair / heads;
+    const int head = blockIdx.x % heads;
+    const int sequence = blockIdx.x / heads;
     const int width = heads * kHeadWidth;
     const int tid = threadIdx.x;
     const int lane = tid % 32;
     const int warp = tid / 32;
     const int eighth = lane % 8;
-    const int group = warp * 4 + lane / 8;
+    const int group = tid / 8;
     // The position and every older row were written before this step's first kernel began.
     const int newest = *position;
-    const int share = (newest + splits - 1) / splits;
-    const int begin = rank * share;
-    const int end = min(newest, begin + share);
     const size_t base = (static_cast<size_t>(sequence) * heads + head) * max_length * kHeadWidth;
     const uint4* keys = reinterpret_cast<const uint4*>(cache_k + base) + eighth;
     const uint4* values = reinterpret_cast<const uint4*>(cache_v + base) + eighth;
-    uint4 k[kRounds];
-    uint4 v[kRounds];
-    auto fetch = [&](int from) {
-#pragma unroll
-        for (int i = 0; i < kRounds; ++i) {
-            const int at = from + group + 32 * i;
-            k[i] = v[i] = make_uint4(0u, 0u, 0u, 0u);
-            if (at < end) {
-                k[i] = load_streaming(keys + static_cast<size_t>(at) * (kHeadWidth / 8));
-                v[i] = load_streaming(values + static_cast<size_t>(at) * (kHeadWidth / 8));
-            }
+    uint4* slots = reinterpret_cast<uint4*>(attention_smem) + tid;   // [round][K, V][thread]
+    const uint32_t slots_at = static_cast<uint32_t>(__cvta_generic_to_shared(slots));
+    for (int i = 0; i < staged_rounds && i * kRoundPositions < newest; ++i) {
+        const int at = group + kRoundPositions * i;
+        if (at < newest) {
+            const uint32_t dst = slots_at + i * (2 * kAttentionThreads * 16);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                         "l"(keys + static_cast<size_t>(at) * (kHeadWidth / 8))
+                         : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + kAttentionThreads * 16),
+                         "l"(values + static_cast<size_t>(at) * (kHeadWidth / 8))
+                         : "memory");
         }
-    };
-    fetch(begin);
+    }
     fb::dependency_wait();
     const uint4* row = reinterpret_cast<const uint4*>(qkv + static_cast<size_t>(sequence) * 3 * width +
                                                       head * kHeadWidth) + eighth;
+    const uint4 raw_q = load_fresh(row);
+    uint4 new_k = make_uint4(0u, 0u, 0u, 0u);
+    uint4 new_v = new_k;
+    if (warp == 0) {
+        new_k = load_fresh(row + width / 8);
+        new_v = load_fresh(row + 2 * (width / 8));
+    }
     float q[8];
-    fb::unpack8(q, *row);
+    fb::unpack8(q, raw_q);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         q[j] = q[j] * scale * kLog2e;
@@ -675,10 +734,13 @@ __global__ void __launch_bounds__(kThreads)
         float kv[8];
         fb::unpack8(kv, raw);
         float s = 0.0f;
+        float s2 = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < 8; j += 2) {
             s = fmaf(kv[j], q[j], s);
+            s2 = fmaf(kv[j + 1], q[j + 1], s2);
         }
+        s += s2;
         s += __shfl_xor_sync(fb::kFullMask, s, 1);
         s += __shfl_xor_sync(fb::kFullMask, s, 2);
         return s + __shfl_xor_sync(fb::kFullMask, s, 4);
@@ -686,7 +748,17 @@ __global__ void __launch_bounds__(kThreads)
     float m = -INFINITY;
     float l = 0.0f;
     float acc[8] = {};
-    auto add_value = [&](float p, const uint4& raw) {
+    auto rescale = [&](float top) {
+        const float keep = merge_weight(m, top);
+        l *= keep;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            acc[j] *= keep;
+        }
+        m = top;
+    };
+    auto add_value = [&](float s, const uint4& raw) {
+        const float p = s == -INFINITY ? 0.0f : exp2f(s - m);
         float vv[8];
         fb::unpack8(vv, raw);
         l += p;
@@ -695,47 +767,49 @@ __global__ void __launch_bounds__(kThreads)
             acc[j] = fmaf(p, vv[j], acc[j]);
         }
     };
-    for (int from = begin; from < end; from += 32 * kRounds) {
-        if (from != begin) {
-            fetch(from);
-        }
-        float s[kRounds];
-        float top = m;
+    asm volatile("cp.async.wait_all;" ::: "memory");   // (a thread reads its own slots only)
+    for (int from = 0; from * kRoundPositions < newest; from += kBatch) {
+        uint4 k[kBatch];
+        uint4 v[kBatch];
 #pragma unroll
-        for (int i = 0; i < kRounds; ++i) {
-            s[i] = score_of(k[i]);
-            if (from + group + 32 * i < end) {
-                top = fmaxf(top, s[i]);
+        for (int i = 0; i < kBatch; ++i) {
+            const int at = group + kRoundPositions * (from + i);
+            k[i] = v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (from + i < staged_rounds) {
+                if (at < newest) {
+                    k[i] = slots[(from + i) * (2 * kAttentionThreads)];
+                    v[i] = slots[(from + i) * (2 * kAttentionThreads) + kAttentionThreads];
+                }
+            } else if (at < newest) {
+                k[i] = load_streaming(keys + static_cast<size_t>(at) * (kHeadWidth / 8));
+                v[i] = load_streaming(values + static_cast<size_t>(at) * (kHeadWidth / 8));
             }
         }
-        const float keep = merge_weight(m, top);
-        l *= keep;
+        float s[kBatch];
+        float top = m;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            acc[j] *= keep;
+        for (int i = 0; i < kBatch; ++i) {
+            s[i] = -INFINITY;
+            if ((from + i) * kRoundPositions < newest) {   // the same for the whole CTA
+                s[i] = score_of(k[i]);
+                if (group + kRoundPositions * (from + i) < newest) {
+                    top = fmaxf(top, s[i]);
+                }
+            }
         }
-        m = top;
+        rescale(top);
 #pragma unroll
-        for (int i = 0; i < kRounds; ++i) {
-            if (from + group + 32 * i < end) {
-                add_value(s[i] == -INFINITY ? 0.0f : exp2f(s[i] - m), v[i]);
+        for (int i = 0; i < kBatch; ++i) {
+            if (group + kRoundPositions * (from + i) < newest) {
+                add_value(s[i], v[i]);
             }
         }
     }
-    if (rank == 0 && warp == 0) {
-        const uint4 new_k = row[width / 8];
-        const uint4 new_v = row[2 * (width / 8)];
+    if (warp == 0) {
         const float s = score_of(new_k);
         if (lane < 8) {
-            const float top = fmaxf(m, s);
-            const float keep = merge_weight(m, top);
-            l *= keep;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                acc[j] *= keep;
-            }
-            m = top;
-            add_value(s == -INFINITY ? 0.0f : exp2f(s - m), new_v);
+            rescale(fmaxf(m, s));
+            add_value(s, new_v);
             reinterpret_cast<uint4*>(cache_k + base + static_cast<size_t>(newest) * kHeadWidth)[eighth] = new_k;
             reinterpret_cast<uint4*>(cache_v + base + static_cast<size_t>(newest) * kHeadWidth)[eighth] = new_v;
         }
@@ -765,56 +839,20 @@ __global__ void __launch_bounds__(kThreads)
         }
     }
     __syncthreads();
-    float total = 0.0f;
-    float sum = 0.0f;
-    float top = -INFINITY;
     if (tid < kHeadWidth) {
+        float top = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
+        for (int w = 0; w < kAttentionWarps; ++w) {
             top = fmaxf(top, partial_m[w]);
         }
+        float sum = 0.0f;
+        float total = 0.0f;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
+        for (int w = 0; w < kAttentionWarps; ++w) {
             const float weight = merge_weight(partial_m[w], top);
             sum += weight * partial_l[w];
             total += weight * partial[w][tid];
         }
-    }
-    // Every CTA of the cluster has begun: the leading one's shared memory may be written.
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (splits > 1) {
-        if (tid < kHeadWidth) {
-            auto put = [&](int at, float value) {
-                const uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(&meet[rank][at]));
-                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(sm100::map_to_cta(local, 0)),
-                             "f"(value)
-                             : "memory");
-            };
-            put(tid, total);
-            if (tid == 0) {
-                put(kHeadWidth, top);
-                put(kHeadWidth + 1, sum);
-            }
-        }
-        sm100::cluster_sync_all();
-        if (rank != 0) {
-            return;
-        }
-        if (tid < kHeadWidth) {
-            top = -INFINITY;
-            for (int r = 0; r < splits; ++r) {
-                top = fmaxf(top, meet[r][kHeadWidth]);
-            }
-            total = 0.0f;
-            sum = 0.0f;
-            for (int r = 0; r < splits; ++r) {
-                const float weight = merge_weight(meet[r][kHeadWidth], top);
-                sum += weight * meet[r][kHeadWidth + 1];
-                total += weight * meet[r][tid];
-            }
-        }
-    }
-    if (tid < kHeadWidth) {
         out[static_cast<size_t>(sequence) * width + head * kHeadWidth + tid] =
             __float2half_rn(total / sum);
     }
@@ -901,34 +939,12 @@ flint_status quantize(flint_b200_generator& g, Matrix& m, cudaStream_t stream) {
     return FLINT_OK;
 }
 
-// A decode kernel's launch: dependent on the one before it, in clusters of `cluster` CTAs.
-template <typename... Params, typename... Args>
-cudaError_t launch_cluster(void (*kernel)(Params...), unsigned grid, unsigned cluster,
-                           cudaStream_t stream, Args&&... args) {
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(grid);
-    config.blockDim = dim3(kThreads);
-    config.stream = stream;
-    cudaLaunchAttribute attributes[2];
-    attributes[0].id = cudaLaunchAttributeClusterDimension;
-    attributes[0].val.clusterDim.x = cluster;
-    attributes[0].val.clusterDim.y = 1;
-    attributes[0].val.clusterDim.z = 1;
-    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attributes[1].val.programmaticStreamSerializationAllowed = 1;
-    config.attrs = attributes;
-    config.numAttrs = fb::dependent_launch_enabled() ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
-    const cudaError_t last = fb::after_launch();
-    return e != cudaSuccess ? e : last;
-}
-
-template <typename W, Act A, bool kNorm, int MB, int NT, int kSteps, int QN>
+template <typename W, Act A, bool kNorm, int RB, int NT, int kSteps, int QN>
 flint_status launch_linear(const LinearArgs& args, cudaStream_t stream) {
-    auto kernel = fb_decode_linear<W, A, kNorm, MB, NT, kSteps, QN>;
-    const int smem = linear_bytes(kNorm, MB, NT, args.rows, args.k);
+    auto kernel = fb_decode_linear<W, A, kNorm, RB, NT, kSteps, QN>;
+    const int smem = linear_bytes(kNorm, RB, NT, args.rows, args.k);
     static std::atomic<bool> configured[64] = {};
-    FB_CUDA(fb::allow_shared_memory(kernel, linear_bytes(kNorm, MB, NT, 16 * MB, 128 * QN), configured));
+    FB_CUDA(fb::allow_shared_memory(kernel, linear_bytes(kNorm, RB, NT, 8 * RB, 128 * QN), configured));
     FB_CUDA(fb::launch_dependent(kernel, dim3(static_cast<unsigned>(args.n / (8 * NT))), dim3(kThreads),
                                  static_cast<size_t>(smem), stream, args));
     return FLINT_OK;
@@ -938,22 +954,30 @@ flint_status launch_linear(const LinearArgs& args, cudaStream_t stream) {
 // or at most 1,536) or, behind the GELU, four times that. A normalising kernel takes 16
 // features per CTA (its CTAs each normalise every row, so there should not be many), the
 // others 8 (so that 768 of them spread over 96 CTAs).
-template <typename W, Act A, int MB>
+template <typename W, Act A, int RB>
 flint_status linear_for(const LinearArgs& args, cudaStream_t stream) {
     constexpr bool kNorm = A != Act::kResidual;
     constexpr int kPer = Step<W>::kPieces;   // int8 takes twice the k per step
     if constexpr (kNorm) {
-        return args.k <= 768 ? launch_linear<W, A, true, MB, 2, (3 + kPer - 1) / kPer, 6>(args, stream)
-                             : launch_linear<W, A, true, MB, 2, 6 / kPer, 12>(args, stream);
+        return args.k <= 768 ? launch_linear<W, A, true, RB, 2, (3 + kPer - 1) / kPer, 6>(args, stream)
+                             : launch_linear<W, A, true, RB, 2, 6 / kPer, 12>(args, stream);
     } else {
         if (args.k <= 768) {
-            return launch_linear<W, A, false, MB, 1, (3 + kPer - 1) / kPer, 1>(args, stream);
+            return launch_linear<W, A, false, RB, 1, (3 + kPer - 1) / kPer, 1>(args, stream);
         }
         if (args.k <= 3072) {
-            return launch_linear<W, A, false, MB, 1, 12 / kPer, 1>(args, stream);
+            return launch_linear<W, A, false, RB, 1, 12 / kPer, 1>(args, stream);
         }
-        return launch_linear<W, A, false, MB, 1, 24 / kPer, 1>(args, stream);
+        return launch_linear<W, A, false, RB, 1, 24 / kPer, 1>(args, stream);
     }
+}
+
+template <typename W, Act A>
+flint_status linear_rows(const LinearArgs& args, cudaStream_t stream) {
+    return args.rows <= 8    ? linear_for<W, A, 1>(args, stream)
+           : args.rows <= 16 ? linear_for<W, A, 2>(args, stream)
+           : args.rows <= 32 ? linear_for<W, A, 4>(args, stream)
+                             : linear_for<W, A, 8>(args, stream);
 }
 
 // One decode linear layer. kNone and kGelu normalise x (FP32 rows) first.
@@ -964,21 +988,14 @@ flint_status decode_linear(const flint_b200_generator& g, const Matrix& m, void*
     const LinearArgs args{out,  g.int8 ? static_cast<const void*>(m.q) : m.half,
                           m.scale, m.bias, x, gain, shift, residual,
                           static_cast<int>(g.sequences), static_cast<int>(m.n), static_cast<int>(m.k)};
-    if (g.int8) {
-        return g.sequences <= 16   ? linear_for<int8_t, A, 1>(args, stream)
-               : g.sequences <= 32 ? linear_for<int8_t, A, 2>(args, stream)
-                                   : linear_for<int8_t, A, 4>(args, stream);
-    }
-    return g.sequences <= 16   ? linear_for<__half, A, 1>(args, stream)
-           : g.sequences <= 32 ? linear_for<__half, A, 2>(args, stream)
-                               : linear_for<__half, A, 4>(args, stream);
+    return g.int8 ? linear_rows<int8_t, A>(args, stream) : linear_rows<__half, A>(args, stream);
 }
 
-template <typename W, int MB, int QN>
+template <typename W, int RB, int QN>
 flint_status launch_head(const HeadArgs& args, cudaStream_t stream) {
-    auto kernel = fb_decode_head<W, MB, QN>;
+    auto kernel = fb_decode_head<W, RB, QN>;
     static std::atomic<bool> configured[64] = {};
-    FB_CUDA(fb::allow_shared_memory(kernel, norm_bytes(16 * MB, 128 * QN), configured));
+    FB_CUDA(fb::allow_shared_memory(kernel, norm_bytes(8 * RB, 128 * QN), configured));
     int sms = 0;
     FB_CUDA(fb::sm_count(&sms));
     const int tiles = (args.n + 8 * kWarps - 1) / (8 * kWarps);
@@ -988,16 +1005,17 @@ flint_status launch_head(const HeadArgs& args, cudaStream_t stream) {
     return FLINT_OK;
 }
 
+template <typename W, int RB>
+flint_status head_width(const HeadArgs& args, cudaStream_t stream) {
+    return args.k <= 768 ? launch_head<W, RB, 6>(args, stream) : launch_head<W, RB, 12>(args, stream);
+}
+
 template <typename W>
 flint_status head_for(const HeadArgs& args, cudaStream_t stream) {
-    const bool narrow = args.k <= 768;
-    if (args.rows <= 16) {
-        return narrow ? launch_head<W, 1, 6>(args, stream) : launch_head<W, 1, 12>(args, stream);
-    }
-    if (args.rows <= 32) {
-        return narrow ? launch_head<W, 2, 6>(args, stream) : launch_head<W, 2, 12>(args, stream);
-    }
-    return narrow ? launch_head<W, 4, 6>(args, stream) : launch_head<W, 4, 12>(args, stream);
+    return args.rows <= 8    ? head_width<W, 1>(args, stream)
+           : args.rows <= 16 ? head_width<W, 2>(args, stream)
+           : args.rows <= 32 ? head_width<W, 4>(args, stream)
+                             : head_width<W, 8>(args, stream);
 }
 
 // The FP16 weights the tensor-core GEMMs read: the model's copy, or the int8 weights
@@ -1073,21 +1091,17 @@ flint_status run_prompt(flint_b200_generator& g, size_t count, cudaStream_t stre
 
 // The transformer over one new position per sequence.
 flint_status run_token(flint_b200_generator& g, cudaStream_t stream) {
-    // As many CTAs per (sequence, head) as fill the GPU, up to a cluster of eight.
-    int sms = 0;
-    FB_CUDA(fb::sm_count(&sms));
-    const size_t pairs = g.sequences * g.heads;
-    unsigned splits = 1;
-    while (splits < kMostSplits && pairs * splits < static_cast<size_t>(sms)) {
-        splits *= 2;
-    }
+    static std::atomic<bool> configured[64] = {};
+    FB_CUDA(fb::allow_shared_memory(fb_decode_attention, attention_bytes(kStaged), configured));
+    const size_t staged = std::min<size_t>(kStaged, (g.max_length + 63) / 64 * 64);
     for (size_t i = 0; i < g.layers; ++i) {
         const Layer& l = g.blocks[i];
         FB_TRY(decode_linear<Act::kNone>(g, l.attn, g.qkv, g.x_a, l.ln1_w, l.ln1_b, nullptr, stream));
-        FB_CUDA(launch_cluster(fb_decode_attention, static_cast<unsigned>(pairs) * splits, splits, stream,
-                               g.attn, g.qkv, g.keys(i), g.values(i), g.position,
-                               static_cast<int>(g.heads), static_cast<int>(g.max_length),
-                               static_cast<int>(splits), attention_scale()));
+        FB_CUDA(fb::launch_dependent(
+            fb_decode_attention, dim3(static_cast<unsigned>(g.sequences * g.heads)),
+            dim3(kAttentionThreads), static_cast<size_t>(attention_bytes(static_cast<int>(staged))),
+            stream, g.attn, g.qkv, g.keys(i), g.values(i), g.position, static_cast<int>(g.heads),
+            static_cast<int>(g.max_length), static_cast<int>(staged / 64), attention_scale()));
         FB_TRY(decode_linear<Act::kResidual>(g, l.proj, g.x_b, g.attn, nullptr, nullptr, g.x_a, stream));
         FB_TRY(decode_linear<Act::kGelu>(g, l.fc, g.act, g.x_b, l.ln2_w, l.ln2_b, nullptr, stream));
         FB_TRY(decode_linear<Act::kResidual>(g, l.fcproj, g.x_a, g.act, nullptr, nullptr, g.x_b, stream));

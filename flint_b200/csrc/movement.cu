@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(kThreads)
                   unsigned first_word, unsigned rows_per_block) {
     fb::dependency_wait();
     fb::dependency_release();
+    x = fb::after_wait(x);
     const unsigned span = heads * words_per_head;  // words moved per row
     const bool short_length = length < (size_t{1} << 31);
     const unsigned length32 = static_cast<unsigned>(length);
@@ -212,6 +213,9 @@ __global__ void __launch_bounds__(kThreads)
                          size_t rows, size_t length, unsigned quads) {
     fb::dependency_wait();
     fb::dependency_release();
+    tokens = fb::after_wait(tokens);
+    wte = fb::after_wait(wte);
+    wpe = fb::after_wait(wpe);
     const unsigned lane = threadIdx.x % 32;
     const unsigned warp = threadIdx.x / 32;
     for (size_t row = size_t{blockIdx.x} * (kThreads / 32) + warp; row < rows;

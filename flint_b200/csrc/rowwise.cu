@@ -235,6 +235,7 @@ __global__ void __launch_bounds__(kThreads)
                               int length) {
     fb::dependency_wait();
     fb::dependency_release();
+    s = fb::after_wait(s);
     const size_t row = size_t{blockIdx.x} * kWarpsPerBlock + threadIdx.x / 32;
     if (row >= rows) {
         return;
@@ -333,6 +334,8 @@ __global__ void __launch_bounds__(kThreads)
                                size_t rows, int length, float scale) {
     fb::dependency_wait();
     fb::dependency_release();
+    p = fb::after_wait(p);
+    dp = fb::after_wait(dp);
     const size_t row = size_t{blockIdx.x} * kWarpsPerBlock + threadIdx.x / 32;
     if (row >= rows) {
         return;

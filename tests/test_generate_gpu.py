@@ -79,18 +79,18 @@ def test_prefill_and_teacher_forced_steps_match_the_full_model(flint, sequences,
 @pytest.mark.parametrize("int8", [False, True], ids=["fp16", "int8"])
 @pytest.mark.parametrize("sequences, heads, prompt", [(1, 2, 600), (20, 4, 8), (40, 4, 584), (2, 24, 24)])
 def test_decode_kernels_at_their_edges_match_the_full_model(flint, sequences, heads, prompt, int8):
-    """One sequence spread over a cluster of eight; 17 to 32 and 33 to 64 rows of the linear
-    kernels; more positions per CTA than one round of attention holds; the widest model."""
+    """More positions than attention stages in shared memory; 17 to 32 and 33 to 64 rows of the
+    linear kernels; the widest model; captured steps, whose kernels are resident several deep."""
     cfg = dict(n_layer=1, n_head=heads, n_embd=64 * heads, block_size=640, vocab_size=200, padded_vocab_size=208)
     params = weights(cfg)
     g = torch.Generator().manual_seed(5)
-    tokens = torch.randint(0, 200, (sequences, prompt + 3), generator=g)
+    tokens = torch.randint(0, 200, (sequences, prompt + 8), generator=g)
     want = oracle.gpt2_decode_logits(cfg, params, tokens, int8=int8)
     model = model_for(flint, cfg, params)
     try:
         with Generator(flint, model, sequences, 640, int8) as gen:
             gen.prefill(u16(tokens[:, :prompt]))
-            for t in range(prompt, prompt + 3):
+            for t in range(prompt, prompt + 8):
                 chosen = gen.step(u16(tokens[:, t]), graph=t > prompt).cpu().to(torch.int64) & 0xFFFF
                 got = gen.logits().cpu()
                 assert rel_l2(got, want[:, t]) <= 5e-3, t
