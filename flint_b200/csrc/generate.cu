@@ -226,10 +226,9 @@ __device__ __forceinline__ void normalise_rows(__half* h, const float* x, const 
         float4 v[QN];
 #pragma unroll
         for (int i = 0; i < QN; ++i) {
-            const int q = lane + 32 * i;
             v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (4 * q < k) {
-                const uint4 raw = load_fresh(src + q);
+            if (128 * i < k) {
+                const uint4 raw = load_fresh(src + lane + 32 * i);
                 v[i] = make_float4(__uint_as_float(raw.x), __uint_as_float(raw.y),
                                    __uint_as_float(raw.z), __uint_as_float(raw.w));
             }
@@ -243,7 +242,7 @@ __device__ __forceinline__ void normalise_rows(__half* h, const float* x, const 
         float4 squares = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
         for (int i = 0; i < QN; ++i) {
-            if (4 * (lane + 32 * i) < k) {
+            if (128 * i < k) {
                 const float4 d = make_float4(v[i].x - mean, v[i].y - mean, v[i].z - mean, v[i].w - mean);
                 squares = make_float4(fmaf(d.x, d.x, squares.x), fmaf(d.y, d.y, squares.y),
                                       fmaf(d.z, d.z, squares.z), fmaf(d.w, d.w, squares.w));
@@ -264,7 +263,7 @@ __device__ __forceinline__ void normalise_rows(__half* h, const float* x, const 
 #pragma unroll
         for (int i = 0; i < QN; ++i) {
             const int q = lane + 32 * i;
-            if (4 * q < k) {
+            if (128 * i < k) {
                 const float4 g = reinterpret_cast<const float4*>(gain)[q];
                 const float4 b = reinterpret_cast<const float4*>(shift)[q];
                 uint2 packed;
@@ -310,7 +309,6 @@ __global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p)
     using Sums = float[8 * RB][kColumns];
     Sums* sums = reinterpret_cast<Sums*>(decode_smem +
                                          (kNorm && RB < 8 ? norm_bytes(p.rows, p.k) : 0));
-    fb::dependency_release();
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
     const int g = lane / 4;
@@ -348,6 +346,7 @@ __global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p)
     }
     // Nothing above depends on the step's kernels.
     fb::dependency_wait();
+    fb::dependency_release();
     const size_t out_at = static_cast<size_t>(threadIdx.x / kColumns) * p.n + feature;
     float residual = 0.0f;
     if (A == Act::kResidual && static_cast<int>(threadIdx.x) / kColumns < p.rows) {
@@ -370,21 +369,24 @@ __global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p)
     float acc[kSets][MB][NT][4] = {};
 #pragma unroll
     for (int from = 0; from < kSteps; from += kChunk) {
+        if (from >= mine) {
+            break;
+        }
         uint4 values[kChunk][RB][S::kPieces];
 #pragma unroll
         for (int j = 0; j < kChunk; ++j) {
+            const int step = min(from + j, mine - 1);
 #pragma unroll
             for (int block = 0; block < RB; ++block) {
+                // (Rows past the last one repeat it: an MMA's rows do not meet, and theirs go
+                // nowhere. A load without a condition costs no branch.)
+                const int row = min(8 * block + g, p.rows - 1);
+                const __half* at = x + static_cast<size_t>(row) * stride + (begin + step) * S::kStepK +
+                                   t * S::kValues;
 #pragma unroll
                 for (int piece = 0; piece < S::kPieces; ++piece) {
-                    const int row = 8 * block + g;
-                    values[j][block][piece] = make_uint4(0u, 0u, 0u, 0u);
-                    if (from + j < mine && row < p.rows) {
-                        const __half* at = x + static_cast<size_t>(row) * stride +
-                                           (begin + from + j) * S::kStepK + t * S::kValues + 8 * piece;
-                        values[j][block][piece] =
-                            kNorm ? *reinterpret_cast<const uint4*>(at) : load_fresh(at);
-                    }
+                    values[j][block][piece] = kNorm ? *reinterpret_cast<const uint4*>(at + 8 * piece)
+                                                    : load_fresh(at + 8 * piece);
                 }
             }
         }
@@ -470,7 +472,6 @@ __global__ void __launch_bounds__(kThreads, 2) fb_decode_head(const HeadArgs p) 
     extern __shared__ __align__(16) unsigned char decode_smem[];
     __shared__ unsigned long long chosen[kWarps][8 * RB];
     __shared__ bool last_cta;
-    fb::dependency_release();
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
     const int g = lane / 4;
@@ -504,6 +505,7 @@ __global__ void __launch_bounds__(kThreads, 2) fb_decode_head(const HeadArgs p) 
     }
     __syncthreads();
     fb::dependency_wait();
+    fb::dependency_release();
     normalise_rows<QN>(rows, p.x, gain, shift, p.rows, p.k);
     __syncthreads();
     float best_value[MB][2];
@@ -527,9 +529,8 @@ __global__ void __launch_bounds__(kThreads, 2) fb_decode_head(const HeadArgs p) 
                 const __half* at = rows + step * S::kStepK + t * S::kValues;
                 const uint4 one[1] = {raw[j]};
                 multiply<W, RB, 1>(acc, one, [&](int block, int piece) {
-                    const int row = 8 * block + g;
-                    return row < p.rows ? *reinterpret_cast<const uint4*>(at + row * (p.k + 8) + 8 * piece)
-                                        : make_uint4(0u, 0u, 0u, 0u);
+                    return *reinterpret_cast<const uint4*>(at + min(8 * block + g, p.rows - 1) * (p.k + 8) +
+                                                           8 * piece);
                 });
             }
         }
@@ -655,178 +656,209 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// One query per (sequence, head) against the cache's positions 0 .. *position, a CTA each.
-// Eight lanes hold a position (16 bytes of its key and value each), so a round of the CTA is
-// 64 positions. Before it waits for the new token's qkv row, a thread copies its share of up
-// to 512 older positions into its own slots of shared memory (which cost the neighbouring
-// kernels no registers); further positions come four rounds at a time. Each group of eight
-// lanes keeps its own running maximum, sum and weighted values; they are merged over the
-// warp and then the CTA. The new token's own key and value come from its row, and are stored
-// in the cache for the steps to come (nothing else reads that position during this launch).
+// One query per (sequence, head) against the cache's positions 0 .. *position, a CTA each. A
+// warp takes 16 positions at a time, the CTA 256.
+//   scores   K times q on mma.sync: the 16 positions are A's rows, q is column 0 of B (the
+//            other seven are zeros). As in the linear layers a lane's 16 contiguous bytes of
+//            a key are the k positions it holds; lane 4g gets positions g and g + 8. (With
+//            FP32 FMAs on unpacked halves the conversions alone made this kernel issue-bound:
+//            1,800 clocks per 256 positions.)
+//   values   in FP32: eight lanes per position, 16 bytes each, probabilities as FP32 numbers
+//            passed round by shuffles.
+// A warp keeps one running maximum. Before it waits for the new token's qkv row, a thread
+// copies its share of up to 512 older positions into its own slots of shared memory (which
+// cost the neighbouring kernels no registers). The warps' (maximum, sum, weighted values)
+// meet at the end. The new token's own key and value come from its row, and are stored in the
+// cache for the steps to come (nothing else reads that position during this launch).
 // (A cluster of up to eight CTAs per head was tried: its two barriers cost 1,900 clocks, more
 // than eight times the positions do.)
 constexpr int kAttentionThreads = 512;
 constexpr int kAttentionWarps = kAttentionThreads / 32;
-constexpr int kRoundPositions = kAttentionThreads / 8;
-constexpr int kBatch = 4;              // rounds whose scores are worked on together
-constexpr int kStaged = 512;           // positions in shared memory
+constexpr int kBatchPositions = 16 * kAttentionWarps;
+constexpr int kMostStaged = 2;         // batches in shared memory
 
-constexpr int attention_bytes(int staged) { return staged * 2 * kHeadWidth * 2; }
+constexpr int attention_bytes(int batches) { return batches * kBatchPositions * 2 * kHeadWidth * 2; }
 
 // The weight of a set of positions whose largest score is m (-inf: no positions).
 __device__ __forceinline__ float merge_weight(float m, float top) {
     return m == -INFINITY ? 0.0f : exp2f(m - top);
 }
 
+// A thread's share of 16 positions: of positions g and g + 8, pieces t and t + 4 of the key
+// (i = 0..3: position half i / 2, piece half i % 2); of positions 4 i + lane / 8, piece
+// lane % 8 of the value.
+__device__ __forceinline__ int key_position(int lane, int i) { return lane / 4 + 8 * (i / 2); }
+__device__ __forceinline__ int key_piece(int lane, int i) { return lane % 4 + 4 * (i % 2); }
+
 __global__ void __launch_bounds__(kAttentionThreads)
     fb_decode_attention(__half* out, const __half* qkv, __half* cache_k, __half* cache_v,
-                        const int* position, int heads, int max_length,
-                        int staged_rounds, float scale) {
+                        const int* position, int heads, int max_length, int staged, float scale) {
     extern __shared__ __align__(16) unsigned char attention_smem[];
     __shared__ float partial[kAttentionWarps][kHeadWidth];
     __shared__ float partial_m[kAttentionWarps];
     __shared__ float partial_l[kAttentionWarps];
-    fb::dependency_release();
+    static_assert(kAttentionWarps == 16, "half a warp holds the warps' maxima");
     const int head = blockIdx.x % heads;
     const int sequence = blockIdx.x / heads;
     const int width = heads * kHeadWidth;
     const int tid = threadIdx.x;
     const int lane = tid % 32;
     const int warp = tid / 32;
-    const int eighth = lane % 8;
-    const int group = tid / 8;
     // The position and every older row were written before this step's first kernel began.
     const int newest = *position;
     const size_t base = (static_cast<size_t>(sequence) * heads + head) * max_length * kHeadWidth;
-    const uint4* keys = reinterpret_cast<const uint4*>(cache_k + base) + eighth;
-    const uint4* values = reinterpret_cast<const uint4*>(cache_v + base) + eighth;
-    uint4* slots = reinterpret_cast<uint4*>(attention_smem) + tid;   // [round][K, V][thread]
+    const uint4* keys = reinterpret_cast<const uint4*>(cache_k + base);
+    const uint4* values = reinterpret_cast<const uint4*>(cache_v + base);
+    uint4* slots = reinterpret_cast<uint4*>(attention_smem) + tid;   // [batch][K 0-3, V 0-3][thread]
     const uint32_t slots_at = static_cast<uint32_t>(__cvta_generic_to_shared(slots));
-    for (int i = 0; i < staged_rounds && i * kRoundPositions < newest; ++i) {
-        const int at = group + kRoundPositions * i;
-        if (at < newest) {
-            const uint32_t dst = slots_at + i * (2 * kAttentionThreads * 16);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
-                         "l"(keys + static_cast<size_t>(at) * (kHeadWidth / 8))
-                         : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + kAttentionThreads * 16),
-                         "l"(values + static_cast<size_t>(at) * (kHeadWidth / 8))
-                         : "memory");
+    for (int batch = 0; batch < staged; ++batch) {
+        const int first = batch * kBatchPositions + 16 * warp;
+        if (first >= newest) {
+            break;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k_at = first + key_position(lane, i);
+            const int v_at = first + 4 * i + lane / 8;
+            const uint32_t dst = slots_at + (batch * 8 + i) * (kAttentionThreads * 16);
+            if (k_at < newest) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst),
+                             "l"(keys + static_cast<size_t>(k_at) * (kHeadWidth / 8) + key_piece(lane, i))
+                             : "memory");
+            }
+            if (v_at < newest) {
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                 dst + 4 * kAttentionThreads * 16),
+                             "l"(values + static_cast<size_t>(v_at) * (kHeadWidth / 8) + lane % 8)
+                             : "memory");
+            }
         }
     }
     fb::dependency_wait();
+    fb::dependency_release();
     const uint4* row = reinterpret_cast<const uint4*>(qkv + static_cast<size_t>(sequence) * 3 * width +
-                                                      head * kHeadWidth) + eighth;
-    const uint4 raw_q = load_fresh(row);
-    uint4 new_k = make_uint4(0u, 0u, 0u, 0u);
-    uint4 new_v = new_k;
+                                                      head * kHeadWidth);
+    // B's column 0 (lanes 0-3): this lane's pieces of q.
+    uint4 q0 = load_fresh(row + lane % 4);
+    uint4 q1 = load_fresh(row + lane % 4 + 4);
+    uint4 new_q = make_uint4(0u, 0u, 0u, 0u);
+    uint4 new_k = new_q;
+    uint4 new_v = new_q;
     if (warp == 0) {
-        new_k = load_fresh(row + width / 8);
-        new_v = load_fresh(row + 2 * (width / 8));
+        new_q = load_fresh(row + lane % 8);
+        new_k = load_fresh(row + width / 8 + lane % 8);
+        new_v = load_fresh(row + 2 * (width / 8) + lane % 8);
     }
-    float q[8];
-    fb::unpack8(q, raw_q);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        q[j] = q[j] * scale * kLog2e;
+    if (lane >= 4) {
+        q0 = q1 = make_uint4(0u, 0u, 0u, 0u);
     }
-    auto score_of = [&](const uint4& raw) {
-        float kv[8];
-        fb::unpack8(kv, raw);
-        float s = 0.0f;
-        float s2 = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-            s = fmaf(kv[j], q[j], s);
-            s2 = fmaf(kv[j + 1], q[j + 1], s2);
-        }
-        s += s2;
-        s += __shfl_xor_sync(fb::kFullMask, s, 1);
-        s += __shfl_xor_sync(fb::kFullMask, s, 2);
-        return s + __shfl_xor_sync(fb::kFullMask, s, 4);
-    };
+    const float to_base2 = scale * kLog2e;
     float m = -INFINITY;
-    float l = 0.0f;
-    float acc[8] = {};
-    auto rescale = [&](float top) {
+    float l = 0.0f;          // lanes 4g: over their own positions
+    float acc[8] = {};       // this lane's positions, columns 8 (lane % 8) ...
+    asm volatile("cp.async.wait_all;" ::: "memory");   // (a thread reads its own slots only)
+    for (int batch = 0; batch * kBatchPositions + 16 * warp < newest; ++batch) {
+        const int first = batch * kBatchPositions + 16 * warp;
+        uint4 k[4];
+        uint4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k_at = first + key_position(lane, i);
+            const int v_at = first + 4 * i + lane / 8;
+            k[i] = v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (batch < staged) {
+                const uint4* slot = slots + (batch * 8 + i) * kAttentionThreads;
+                if (k_at < newest) {
+                    k[i] = slot[0];
+                }
+                if (v_at < newest) {
+                    v[i] = slot[4 * kAttentionThreads];
+                }
+            } else {
+                if (k_at < newest) {
+                    k[i] = load_streaming(keys + static_cast<size_t>(k_at) * (kHeadWidth / 8) +
+                                          key_piece(lane, i));
+                }
+                if (v_at < newest) {
+                    v[i] = load_streaming(values + static_cast<size_t>(v_at) * (kHeadWidth / 8) + lane % 8);
+                }
+            }
+        }
+        float even[4] = {};
+        float odd[4] = {};
+        mma_16x8x16(even, k[0].x, k[2].x, k[0].y, k[2].y, q0.x, q0.y);
+        mma_16x8x16(odd, k[1].x, k[3].x, k[1].y, k[3].y, q1.x, q1.y);
+        mma_16x8x16(even, k[0].z, k[2].z, k[0].w, k[2].w, q0.z, q0.w);
+        mma_16x8x16(odd, k[1].z, k[3].z, k[1].w, k[3].w, q1.z, q1.w);
+        // Positions g and g + 8, in lanes 4g (column 0).
+        const bool holds = lane % 4 == 0;
+        float s0 = holds && first + lane / 4 < newest ? (even[0] + odd[0]) * to_base2 : -INFINITY;
+        float s1 = holds && first + lane / 4 + 8 < newest ? (even[2] + odd[2]) * to_base2 : -INFINITY;
+        float top = fmaxf(s0, s1);
+        top = fmaxf(top, __shfl_xor_sync(fb::kFullMask, top, 4));
+        top = fmaxf(top, __shfl_xor_sync(fb::kFullMask, top, 8));
+        top = fmaxf(top, __shfl_xor_sync(fb::kFullMask, top, 16));
+        top = fmaxf(m, __shfl_sync(fb::kFullMask, top, 0));
         const float keep = merge_weight(m, top);
-        l *= keep;
+        m = top;
+        s0 = s0 == -INFINITY ? 0.0f : exp2f(s0 - m);
+        s1 = s1 == -INFINITY ? 0.0f : exp2f(s1 - m);
+        l = l * keep + (s0 + s1);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             acc[j] *= keep;
         }
-        m = top;
-    };
-    auto add_value = [&](float s, const uint4& raw) {
-        const float p = s == -INFINITY ? 0.0f : exp2f(s - m);
-        float vv[8];
-        fb::unpack8(vv, raw);
-        l += p;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            acc[j] = fmaf(p, vv[j], acc[j]);
-        }
-    };
-    asm volatile("cp.async.wait_all;" ::: "memory");   // (a thread reads its own slots only)
-    for (int from = 0; from * kRoundPositions < newest; from += kBatch) {
-        uint4 k[kBatch];
-        uint4 v[kBatch];
+        for (int i = 0; i < 4; ++i) {
+            // Position 4 i + lane / 8: half i / 2, g = 4 (i % 2) + lane / 8, in lane 4 g.
+            const float p = __shfl_sync(fb::kFullMask, i < 2 ? s0 : s1, 16 * (i % 2) + lane / 8 * 4);
+            float vv[8];
+            fb::unpack8(vv, v[i]);
 #pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-            const int at = group + kRoundPositions * (from + i);
-            k[i] = v[i] = make_uint4(0u, 0u, 0u, 0u);
-            if (from + i < staged_rounds) {
-                if (at < newest) {
-                    k[i] = slots[(from + i) * (2 * kAttentionThreads)];
-                    v[i] = slots[(from + i) * (2 * kAttentionThreads) + kAttentionThreads];
-                }
-            } else if (at < newest) {
-                k[i] = load_streaming(keys + static_cast<size_t>(at) * (kHeadWidth / 8));
-                v[i] = load_streaming(values + static_cast<size_t>(at) * (kHeadWidth / 8));
-            }
-        }
-        float s[kBatch];
-        float top = m;
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-            s[i] = -INFINITY;
-            if ((from + i) * kRoundPositions < newest) {   // the same for the whole CTA
-                s[i] = score_of(k[i]);
-                if (group + kRoundPositions * (from + i) < newest) {
-                    top = fmaxf(top, s[i]);
-                }
-            }
-        }
-        rescale(top);
-#pragma unroll
-        for (int i = 0; i < kBatch; ++i) {
-            if (group + kRoundPositions * (from + i) < newest) {
-                add_value(s[i], v[i]);
+            for (int j = 0; j < 8; ++j) {
+                acc[j] = fmaf(p, vv[j], acc[j]);
             }
         }
     }
     if (warp == 0) {
-        const float s = score_of(new_k);
-        if (lane < 8) {
-            rescale(fmaxf(m, s));
-            add_value(s, new_v);
-            reinterpret_cast<uint4*>(cache_k + base + static_cast<size_t>(newest) * kHeadWidth)[eighth] = new_k;
-            reinterpret_cast<uint4*>(cache_v + base + static_cast<size_t>(newest) * kHeadWidth)[eighth] = new_v;
-        }
-    }
-    // The warp's four groups.
-#pragma unroll
-    for (int off = 8; off < 32; off <<= 1) {
-        const float other_m = __shfl_xor_sync(fb::kFullMask, m, off);
-        const float top = fmaxf(m, other_m);
-        const float mine = merge_weight(m, top);
-        const float theirs = merge_weight(other_m, top);
-        l = l * mine + __shfl_xor_sync(fb::kFullMask, l, off) * theirs;
+        float qv[8];
+        float kv[8];
+        float vv[8];
+        fb::unpack8(qv, new_q);
+        fb::unpack8(kv, new_k);
+        fb::unpack8(vv, new_v);
+        float s = 0.0f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            acc[j] = acc[j] * mine + __shfl_xor_sync(fb::kFullMask, acc[j], off) * theirs;
+            s = fmaf(kv[j], qv[j], s);
         }
+        s += __shfl_xor_sync(fb::kFullMask, s, 1);
+        s += __shfl_xor_sync(fb::kFullMask, s, 2);
+        s += __shfl_xor_sync(fb::kFullMask, s, 4);
+        s *= to_base2;
+        const float top = fmaxf(m, s);
+        const float keep = merge_weight(m, top);
+        const float p = s == -INFINITY ? 0.0f : exp2f(s - top);
         m = top;
+        l = l * keep + (lane == 0 ? p : 0.0f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            acc[j] = acc[j] * keep + (lane < 8 ? p * vv[j] : 0.0f);
+        }
+        if (lane < 8) {
+            reinterpret_cast<uint4*>(cache_k + base + static_cast<size_t>(newest) * kHeadWidth)[lane] = new_k;
+            reinterpret_cast<uint4*>(cache_v + base + static_cast<size_t>(newest) * kHeadWidth)[lane] = new_v;
+        }
+    }
+    // The warp: l over lanes 4g, the values over lanes with the same columns.
+    l += __shfl_xor_sync(fb::kFullMask, l, 4);
+#pragma unroll
+    for (int off = 8; off < 32; off <<= 1) {
+        l += __shfl_xor_sync(fb::kFullMask, l, off);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            acc[j] += __shfl_xor_sync(fb::kFullMask, acc[j], off);
+        }
     }
     if (lane < 8) {
 #pragma unroll
@@ -840,21 +872,28 @@ __global__ void __launch_bounds__(kAttentionThreads)
     }
     __syncthreads();
     if (tid < kHeadWidth) {
-        float top = -INFINITY;
+        // Lane w (and w + 16) weighs warp w's share; the weights go round by shuffles.
+        const float mine = partial_m[lane % 16];
+        float top = mine;
 #pragma unroll
-        for (int w = 0; w < kAttentionWarps; ++w) {
-            top = fmaxf(top, partial_m[w]);
+        for (int off = 1; off < 16; off <<= 1) {
+            top = fmaxf(top, __shfl_xor_sync(fb::kFullMask, top, off));
         }
-        float sum = 0.0f;
-        float total = 0.0f;
+        const float weight = merge_weight(mine, top);
+        float sum = weight * partial_l[lane % 16];
 #pragma unroll
-        for (int w = 0; w < kAttentionWarps; ++w) {
-            const float weight = merge_weight(partial_m[w], top);
-            sum += weight * partial_l[w];
-            total += weight * partial[w][tid];
+        for (int off = 1; off < 16; off <<= 1) {
+            sum += __shfl_xor_sync(fb::kFullMask, sum, off);
+        }
+        float even = 0.0f;
+        float odd = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kAttentionWarps; w += 2) {
+            even = fmaf(__shfl_sync(fb::kFullMask, weight, w), partial[w][tid], even);
+            odd = fmaf(__shfl_sync(fb::kFullMask, weight, w + 1), partial[w + 1][tid], odd);
         }
         out[static_cast<size_t>(sequence) * width + head * kHeadWidth + tid] =
-            __float2half_rn(total / sum);
+            __float2half_rn((even + odd) / sum);
     }
 }
 
@@ -1091,17 +1130,23 @@ flint_status run_prompt(flint_b200_generator& g, size_t count, cudaStream_t stre
 
 // The transformer over one new position per sequence.
 flint_status run_token(flint_b200_generator& g, cudaStream_t stream) {
+    // Shared memory for as many positions as there can be, within what one CTA per SM may have,
+    // or two where there are more CTAs than SMs.
+    int sms = 0;
+    FB_CUDA(fb::sm_count(&sms));
+    const size_t pairs = g.sequences * g.heads;
+    const size_t batches = std::min<size_t>(pairs <= static_cast<size_t>(sms) ? kMostStaged : 1,
+                                            (g.max_length + kBatchPositions - 1) / kBatchPositions);
     static std::atomic<bool> configured[64] = {};
-    FB_CUDA(fb::allow_shared_memory(fb_decode_attention, attention_bytes(kStaged), configured));
-    const size_t staged = std::min<size_t>(kStaged, (g.max_length + 63) / 64 * 64);
+    FB_CUDA(fb::allow_shared_memory(fb_decode_attention, attention_bytes(kMostStaged), configured));
     for (size_t i = 0; i < g.layers; ++i) {
         const Layer& l = g.blocks[i];
         FB_TRY(decode_linear<Act::kNone>(g, l.attn, g.qkv, g.x_a, l.ln1_w, l.ln1_b, nullptr, stream));
         FB_CUDA(fb::launch_dependent(
-            fb_decode_attention, dim3(static_cast<unsigned>(g.sequences * g.heads)),
-            dim3(kAttentionThreads), static_cast<size_t>(attention_bytes(static_cast<int>(staged))),
+            fb_decode_attention, dim3(static_cast<unsigned>(pairs)), dim3(kAttentionThreads),
+            static_cast<size_t>(attention_bytes(static_cast<int>(batches))),
             stream, g.attn, g.qkv, g.keys(i), g.values(i), g.position, static_cast<int>(g.heads),
-            static_cast<int>(g.max_length), static_cast<int>(staged / 64), attention_scale()));
+            static_cast<int>(g.max_length), static_cast<int>(batches), attention_scale()));
         FB_TRY(decode_linear<Act::kResidual>(g, l.proj, g.x_b, g.attn, nullptr, nullptr, g.x_a, stream));
         FB_TRY(decode_linear<Act::kGelu>(g, l.fc, g.act, g.x_b, l.ln2_w, l.ln2_b, nullptr, stream));
         FB_TRY(decode_linear<Act::kResidual>(g, l.fcproj, g.x_a, g.act, nullptr, nullptr, g.x_b, stream));
