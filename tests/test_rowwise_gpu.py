@@ -238,6 +238,45 @@ def test_layernorm_backward_matches_the_oracle_bit_for_bit(flint, shape):
     assert same_bits(dbeta, want[2])
 
 
+@pytest.mark.parametrize("shape", [(1, 72), (2, 8), (257, 520), (300, 1600)])
+@pytest.mark.parametrize("accumulate_dx", [False, True])
+def test_layernorm_parameter_sums_wherever_they_lie(flint, shape, accumulate_dx):
+    """dbeta's partial sums lie where dx is written afterwards, or (dx added to, or a single row)
+    take a pass of their own: the same bits, and the workspace ends with dgamma's either way."""
+    rows, cols = shape
+    rng = np.random.default_rng(rows * 7 + cols)
+    x = crafted(rng, shape, 3).astype(np.float32)
+    dy = crafted(rng, shape, 3).astype(np.float16)
+    gamma = (1 + 0.02 * rng.standard_normal(cols)).astype(np.float32)
+    mean = x.astype(np.float64).mean(1).astype(np.float32)
+    rstd = (1 / np.sqrt(x.astype(np.float64).var(1) + 1e-5)).astype(np.float32)
+    old = rng.standard_normal(shape).astype(np.float32)
+    to = lambda a: torch.from_numpy(a.copy()).to(DEV)
+    dx, dgamma, dbeta = to(old), torch.zeros(cols, device=DEV), torch.zeros(cols, device=DEV)
+    ws = workspace(flint.layernorm_backward_workspace(rows, cols))
+    flint.layernorm_backward(dx, dgamma, dbeta, to(dy), to(x), to(mean), to(rstd), to(gamma), rows, cols,
+                             accumulate_dx, False, ws)
+    torch.cuda.synchronize()
+    want = oracle.layernorm_backward(dy, x, mean, rstd, gamma)
+    want_dx = (old + want[0]).astype(np.float32) if accumulate_dx else want[0]
+    assert same_bits(dx, want_dx)
+    assert same_bits(dgamma, want[1])
+    assert same_bits(dbeta, want[2])
+
+
+@pytest.mark.parametrize("shape", [(3, 32768 * 64 + 8), (255, 72), (512, 64)])
+def test_bias_gradient_at_the_edges_of_its_grid(flint, shape):
+    """More 64-column tiles than one layer of the grid holds; ragged tiles and chunks."""
+    rows, cols = shape
+    rng = np.random.default_rng(cols)
+    dy = crafted(rng, shape).astype(np.float16)
+    out = torch.zeros(cols, device=DEV)
+    flint.bias_gradient(out, torch.from_numpy(dy).to(DEV), rows, cols, False,
+                        workspace(flint.bias_gradient_workspace(rows, cols)))
+    torch.cuda.synchronize()
+    assert same_bits(out, oracle.bias_gradient(dy))
+
+
 # ---- causal softmax ---------------------------------------------------------------------------
 
 
