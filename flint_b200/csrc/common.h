@@ -108,11 +108,10 @@ cudaError_t allow_shared_memory(Kernel kernel, int bytes, std::atomic<bool> (&do
 cudaError_t sm_count(int* sms);
 
 // Tensor map over a row-major matrix [rows, cols] of 2- or 4-byte elements (zero
-// fill outside; swizzle_bytes 0 or 64), for boxes of box_cols x box_rows. The row
+// fill outside, no swizzle), for boxes of box_cols x box_rows. The row
 // pitch must be a multiple of 16 bytes and both extents below 2^32.
 cudaError_t encode_rows_map(void* map, const void* base, size_t rows, size_t cols,
-                            int element_bytes, unsigned box_cols, unsigned box_rows,
-                            int swizzle_bytes = 0);
+                            int element_bytes, unsigned box_cols, unsigned box_rows);
 
 // LayerNorm forward whose row sums use plain FP32 adds (see rowwise.cu); returns false, having
 // launched nothing, for shapes it does not cover.

@@ -47,7 +47,7 @@ constexpr int kHeadWidth = 64;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kEps = 1e-5f;
 
-enum class Act { kNone, kGelu, kResidual, kLogits };
+enum class Act { kNone, kGelu, kResidual };
 
 struct Matrix {
     const __half* half = nullptr;   // [n, k] FP16 (the model's compute copy)
