@@ -30,13 +30,39 @@ __device__ __forceinline__ void dependency_release() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// A pointer as it is after dependency_wait(): loads through it cannot be moved above the wait.
-// (Behind `const __restrict__` a compiler may take memory for unchanging while the kernel
-// runs; a dependent launch runs while the kernel before it still writes.)
+// A pointer to global memory as it is after dependency_wait(): loads through it cannot be
+// moved above the wait. Behind `const __restrict__` (and in __ldg) a compiler may take memory
+// for unchanging while the kernel runs, and a dependent launch runs while the kernel before it
+// still writes: every such parameter of a kernel that waits goes through here first.
 template <typename T>
 __device__ __forceinline__ T* after_wait(T* p) {
-    asm volatile("" : "+l"(p)::"memory");
-    return p;
+    unsigned long long at = __cvta_generic_to_global(p);
+    asm volatile("" : "+l"(at)::"memory");
+    return static_cast<T*>(__cvta_global_to_generic(at));
+}
+
+// A load through an after_wait() pointer from memory that this kernel does not write. To the
+// compiler it is a function of the address alone: it stays behind the wait, which the address
+// comes from, and may still be moved past this kernel's own stores. (Not __ldg: that asks for
+// memory that nothing writes while the kernel runs.)
+__device__ __forceinline__ uint4 load_input(const uint4* p) {
+    uint4 v;
+    asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+        : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
+__device__ __forceinline__ float4 load_input(const float4* p) {
+    float4 v;
+    asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+        : "l"(__cvta_generic_to_global(p)));
+    return v;
+}
+__device__ __forceinline__ unsigned short load_input(const unsigned short* p) {
+    unsigned short v;
+    asm("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(__cvta_generic_to_global(p)));
+    return v;
 }
 
 struct Comp {
@@ -192,6 +218,14 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
 __device__ __forceinline__ void load8(float (&v)[8], const float4* p) {
     const float4 a = p[0];
     const float4 b = p[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+// The same through load_input.
+__device__ __forceinline__ void load8_input(float (&v)[8], const float4* p) {
+    const float4 a = load_input(p);
+    const float4 b = load_input(p + 1);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }

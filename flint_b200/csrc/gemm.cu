@@ -447,7 +447,7 @@ template <Epilogue E>
 __device__ __forceinline__ float load_bias_lane(const GemmParams& p, int col, int lane) {
     if constexpr (E == Epilogue::kBias || E == Epilogue::kBiasGelu ||
                   E == Epilogue::kBiasResidual) {
-        return col + lane < p.n ? __ldg(p.bias + col + lane) : 0.0f;
+        return col + lane < p.n ? p.bias[col + lane] : 0.0f;
     } else {
         return 0.0f;
     }
@@ -1391,6 +1391,7 @@ __global__ void __launch_bounds__(256)
                       int splits, int accumulate) {
     fb::dependency_wait();
     fb::dependency_release();
+    partials = fb::after_wait(partials);
     for (size_t i = size_t{blockIdx.x} * 256 + threadIdx.x; i < quads;
          i += size_t{gridDim.x} * 256) {
         float4 s = partials[i];

@@ -165,6 +165,10 @@ __global__ void __launch_bounds__(kAddThreads + 32)
     if (threadIdx.x == 0) {
         fb::dependency_release();
     }
+    src = fb::after_wait(src);
+    x = fb::after_wait(x);
+    mean = fb::after_wait(mean);
+    rstd = fb::after_wait(rstd);
     if constexpr (kSource == Source::kHalfTimesXhat) {
         for (int t = threadIdx.x; t < chunk_rows; t += kAddThreads + 32) {
             sh_mean[t] = mean[first + t];
@@ -416,6 +420,7 @@ __global__ void __launch_bounds__(32 * kFinishWarps)
                      int quads, bool accumulate) {
     fb::dependency_wait();
     fb::dependency_release();
+    partial = fb::after_wait(partial);
     const int quad = blockIdx.x * kFinishWarps + threadIdx.x / 32;
     if (quad < quads) {
         finish_quad(out, partial, chunks, quads, quad, accumulate);
@@ -443,7 +448,7 @@ __global__ void __launch_bounds__(32 * kFinishWarps)
     const int quad =
         (static_cast<int>(blockIdx.x) - jobs.first_block[j]) * kFinishWarps + threadIdx.x / 32;
     if (quad < jobs.quads[j]) {
-        finish_quad(jobs.out[j], jobs.partial[j], chunks, jobs.quads[j], quad,
+        finish_quad(jobs.out[j], fb::after_wait(jobs.partial[j]), chunks, jobs.quads[j], quad,
                     ((jobs.accumulate >> j) & 1u) != 0);
     }
 }
@@ -519,6 +524,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
                              size_t rows, int pieces, bool accumulate, uint4* __restrict__ dx_half) {
     fb::dependency_wait();
     fb::dependency_release();
+    dy = fb::after_wait(dy);
+    x = fb::after_wait(x);
+    mean = fb::after_wait(mean);
+    rstd = fb::after_wait(rstd);
+    gamma = fb::after_wait(gamma);
     const size_t row = size_t{blockIdx.x} * kWarpsPerBlock + threadIdx.x / 32;
     if (row >= rows) {
         return;
@@ -586,9 +596,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
             float d[8];
             float xs[8];
             float gs[8];
-            fb::unpack8(d, dyr[i]);
-            fb::load8(xs, xr + 2 * i);
-            fb::load8(gs, gamma + 2 * i);
+            fb::unpack8(d, fb::load_input(dyr + i));
+            fb::load8_input(xs, xr + 2 * i);
+            fb::load8_input(gs, gamma + 2 * i);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float g = __fmul_rn(d[j], gs[j]);
@@ -602,9 +612,9 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
             float d[8];
             float xs[8];
             float gs[8];
-            fb::unpack8(d, dyr[i]);
-            fb::load8(xs, xr + 2 * i);
-            fb::load8(gs, gamma + 2 * i);
+            fb::unpack8(d, fb::load_input(dyr + i));
+            fb::load8_input(xs, xr + 2 * i);
+            fb::load8_input(gs, gamma + 2 * i);
             float o[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {

@@ -46,6 +46,9 @@ __global__ void __launch_bounds__(kThreads)
                               size_t rows, int cols, float eps) {
     fb::dependency_wait();
     fb::dependency_release();
+    x = fb::after_wait(x);
+    gamma = fb::after_wait(gamma);
+    beta = fb::after_wait(beta);
     const size_t row = size_t{blockIdx.x} * kWarpsPerBlock + threadIdx.x / 32;
     if (row >= rows) {
         return;
@@ -117,18 +120,22 @@ __global__ void __launch_bounds__(kThreads)
     const float4* g4 = reinterpret_cast<const float4*>(gamma);
     const float4* b4 = reinterpret_cast<const float4*>(beta);
     uint2* yr = reinterpret_cast<uint2*>(y + row * cols);
+    float4 g = fb::load_input(g4 + min(lane, groups - 1));
+    float4 b = fb::load_input(b4 + min(lane, groups - 1));
 #pragma unroll
     for (int j = 0; j < kQuads; ++j) {
         const int i = lane + 32 * j;
+        const float4 g_next = fb::load_input(g4 + min(i + 32, groups - 1));
+        const float4 b_next = fb::load_input(b4 + min(i + 32, groups - 1));
         if (i < groups) {
-            const float4 g = g4[i];
-            const float4 b = b4[i];
             const float o0 = fmaf(__fmul_rn(__fsub_rn(v[j].x, m), r), g.x, b.x);
             const float o1 = fmaf(__fmul_rn(__fsub_rn(v[j].y, m), r), g.y, b.y);
             const float o2 = fmaf(__fmul_rn(__fsub_rn(v[j].z, m), r), g.z, b.z);
             const float o3 = fmaf(__fmul_rn(__fsub_rn(v[j].w, m), r), g.w, b.w);
             yr[i] = make_uint2(fb::pack2(o0, o1), fb::pack2(o2, o3));
         }
+        g = g_next;
+        b = b_next;
     }
     if (lane == 0) {
         mean[row] = m;
@@ -558,6 +565,8 @@ __global__ void __launch_bounds__(kCeThreads, 1)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     fb::dependency_wait();
+    logits = fb::after_wait(logits);
+    targets = fb::after_wait(targets);
     if (threadIdx.x == 0) {
         fb::dependency_release();
         if (blockIdx.x < rows) {
@@ -675,7 +684,7 @@ __global__ void __launch_bounds__(kCeThreads, 1)
         const fb::F2 inv2 = fb::f2_pack(inv, inv);
         const fb::F2 scale2 = fb::f2_pack(scale, scale);
 
-        const int target = targets[row];
+        const int target = fb::load_input(targets + row);
         const int target_chunk = target / 8;
         const int target_slot = target % 8;
         for (int i = threadIdx.x; i < chunks; i += kCeThreads) {
@@ -803,12 +812,17 @@ __global__ void __launch_bounds__(kThreadsT, 1)
     const int tid = static_cast<int>(threadIdx.x);
     const size_t first = blockIdx.x;
     const size_t stride = gridDim.x;
-    const __half* logit_values = reinterpret_cast<const __half*>(logits);
 
     fb::dependency_wait();
     if (threadIdx.x == 0) {
         fb::dependency_release();
     }
+    logits = fb::after_wait(logits);
+    targets = fb::after_wait(targets);
+    auto logit_value = [&](size_t row, int column) {
+        const auto* values = reinterpret_cast<const unsigned short*>(logits);
+        return __half2float(__ushort_as_half(fb::load_input(values + row * cols + column)));
+    };
     if (first >= rows) {
         return;
     }
@@ -845,14 +859,13 @@ __global__ void __launch_bounds__(kThreadsT, 1)
 #pragma unroll
     for (int j = 0; j < kHeld; ++j) {
         const int i = tid + j * kThreadsT;
-        held[j] = i < vocab_chunks ? __ldg(logits + first * chunks + i) : make_uint4(0u, 0u, 0u, 0u);
+        held[j] = i < vocab_chunks ? fb::load_input(logits + first * chunks + i) : make_uint4(0u, 0u, 0u, 0u);
     }
     float mx_cur = held_max();
     ce_block_max_total<kThreadsT / 32>(mx_cur, Comp{}, scratch);
     // A row's target and the target's logit are fetched a step before they are needed.
-    int target_cur = targets[first];
-    float target_logit_cur =
-        target_cur < vocab ? __half2float(logit_values[first * cols + target_cur]) : 0.0f;
+    int target_cur = fb::load_input(targets + first);
+    float target_logit_cur = target_cur < vocab ? logit_value(first, target_cur) : 0.0f;
 
     // Of the row whose gradient is due: maximum, sum, target and the target's logit.
     float mx_prev = 0.0f, sum_prev = 1.0f, target_logit_prev = 0.0f;
@@ -870,7 +883,7 @@ __global__ void __launch_bounds__(kThreadsT, 1)
         if (tid == 0 && s + 2 < steps) {
             prefetch_row(row_cur + 2 * stride);
         }
-        const int target_next = more ? targets[row_cur + stride] : 0;
+        const int target_next = more ? fb::load_input(targets + (row_cur + stride)) : 0;
         const float inv = __fdiv_rn(1.0f, sum_prev);
         const fb::F2 inv2 = fb::f2_pack(inv, inv);
         const int target_chunk = target_prev / 8;
@@ -936,7 +949,7 @@ __global__ void __launch_bounds__(kThreadsT, 1)
                 }
             }
             if (more) {
-                held[j] = __ldg(next_in + i);
+                held[j] = fb::load_input(next_in + i);
             }
         }
         if (grad) {
@@ -966,9 +979,7 @@ __global__ void __launch_bounds__(kThreadsT, 1)
             }
         }
         const float target_logit_next =
-            more && target_next < vocab
-                ? __half2float(logit_values[(row_cur + stride) * cols + target_next])
-                : 0.0f;
+            more && target_next < vocab ? logit_value(row_cur + stride, target_next) : 0.0f;
         float mx_next = more ? held_max() : -INFINITY;
         const float sum_cur = ce_block_max_total<kThreadsT / 32>(mx_next, mine, scratch);
         mx_prev = mx_cur;

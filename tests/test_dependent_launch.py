@@ -1,0 +1,77 @@
+"""What the source of kernels that may start early has to keep to, checked on the CPU.
+
+A kernel launched with fb::launch_dependent runs while the kernel before it still writes. The
+language lets a compiler move a load of memory that it takes for unchanging (a `const
+__restrict__` kernel parameter, or __ldg) above fb::dependency_wait(); whether one does shows in
+no test that happens to pass. So the source is held to the rule that makes such a load
+impossible: these parameters are replaced by fb::after_wait() of themselves behind the wait.
+"""
+
+import re
+from pathlib import Path
+
+import pytest
+
+SOURCES = sorted((Path(__file__).parent.parent / "flint_b200" / "csrc").glob("*.cu"))
+
+
+def kernels(text):
+    """(name, parameters, body) of every __global__ function."""
+    text = re.sub(r"//[^\n]*", "", text)
+    for head in re.finditer(r"__global__", text):
+        opening = re.compile(r"(\w+)\s*\(").search
+        at = head.end()
+        while True:
+            found = opening(text, at)
+            depth, end = 1, found.end()
+            while depth:
+                depth += {"(": 1, ")": -1}.get(text[end], 0)
+                end += 1
+            if found.group(1) in ("__launch_bounds__", "__cluster_dims__"):
+                at = end
+                continue
+            break
+        parameters = text[found.end():end - 1]
+        begin = text.index("{", end)
+        depth, stop = 1, begin + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[stop], 0)
+            stop += 1
+        yield found.group(1), parameters, text[begin:stop]
+
+
+def waiting_kernels():
+    for path in SOURCES:
+        for name, parameters, body in kernels(path.read_text()):
+            if "dependency_wait()" in body:
+                yield pytest.param(parameters, body, id=f"{path.stem}:{name}")
+
+
+def test_the_scan_finds_the_kernels():
+    names = {p.id.split(":")[1] for p in waiting_kernels()}
+    assert {"fb_layernorm_forward_regs", "fb_softmax_cross_entropy_rolling", "fb_column_partials",
+            "fb_layernorm_backward_dx", "fb_gemm_tn_reduce", "fb_column_finish", "fb_heads_move",
+            "fb_decode_linear", "fb_attention_forward", "fb_embedding_prepare"} <= names
+
+
+@pytest.mark.parametrize("parameters, body", list(waiting_kernels()))
+def test_inputs_are_read_behind_the_wait(parameters, body):
+    behind = body[body.index("dependency_wait()"):]
+    for parameter in parameters.split(","):
+        declared = re.search(r"\bconst\b.*\*\s*__restrict__\s+(\w+)\s*$", parameter.strip(), re.S)
+        if declared:
+            name = declared.group(1)
+            assert re.search(rf"\b{name} = fb::after_wait\({name}\);", behind), name
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.stem)
+def test_no_loads_that_ask_for_unchanging_memory(path):
+    text = re.sub(r"//[^\n]*", "", path.read_text())
+    assert "__ldg(" not in text
+
+
+@pytest.mark.parametrize("parameters, body", list(waiting_kernels()))
+def test_a_kernel_releases_the_next_one_behind_its_own_wait(parameters, body):
+    # So that whatever a kernel depends on is over before the one after the next can begin.
+    assert "dependency_release()" in body
+    assert body.index("dependency_wait()") < body.index("dependency_release()")
