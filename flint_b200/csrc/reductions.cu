@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <type_traits>
 
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -42,42 +43,38 @@ constexpr size_t column_sum_workspace(size_t rows, size_t cols) {
 
 enum class Source { kHalf, kHalfTimesXhat, kFloat };
 
-// First pass. CTA (chunk, tile of 64 columns): warp ly adds row stream ly, a lane two columns,
-// and a ninth warp fetches.
+// First pass. CTA (chunk, tile of 64 kPairs columns): warp ly adds row stream ly, a lane the
+// column pairs 64 i + 2 lane of the tile, and a ninth warp fetches.
 //
 // A chunk's adding is a chain of 32 rows per stream, seven (with a product eleven) dependent
-// FP32 operations each. A small matrix needs that chain short, so a lane has one column pair
-// only; a large one needs bytes in flight, which many narrow CTAs give as well. In the place of 256
-// columns and eight a lane: 300 x 768 with a product 8.8 -> 5.7 us, 8,192 x 768 FP16 9.0 -> 6.4 us.
+// FP32 operations each. A small matrix needs many CTAs with that chain alone, 64 columns each
+// (in the place of 256: 300 x 768 with a product 8.8 -> 5.7 us, 8,192 x 768 FP16 9.0 -> 6.4 us). Once
+// there are more than three CTAs per SM the chains of two column pairs a lane hide each other
+// better than more CTAs do, and the CTAs pass in fewer rounds: see wide_tiles().
 //
-// The chunk's rows reach the CTA through shared memory: lane l of the fetching
-// warp issues one bulk asynchronous copy per row segment (32 rows per stage, a
-// ring of stages, each completing on its own mbarrier), so whole stages are in
-// flight per CTA while every adding thread still takes its stream's rows
-// strictly in row order. (A thread that loaded its own rows would add each one as
-// it arrived, paying one memory latency per row.) The additions run on packed
-// FP32 pairs: columns (0,1), (2,3), (4,5), (6,7) of the piece.
-constexpr int kTilePieces = 8;
-constexpr int kTileColumns = kTilePieces * 8;
+// The chunk's rows reach the CTA through shared memory, 32 to a stage: one TMA tensor load
+// per operand, or (where the row count does not fit a tensor map) a bulk copy per row segment
+// by the fetching warp's lanes. The next stages load while this one is added, so the memory
+// has many bytes in flight although every stream takes its rows strictly in order. (A thread
+// that loaded its own rows would add each one as it arrived, paying one memory latency per
+// row.) The additions run on packed FP32 pairs, a lane's two neighbouring columns.
+constexpr int kPairPieces = 8;                         // pieces that a warp's column pairs cover
 constexpr int kAddThreads = 32 * kLaneRows;            // a warp per stream; and a fetching warp
 constexpr unsigned kTilesY = 32768;                    // tiles per grid layer
 
-template <Source kSource>
+template <Source kSource, int kPairs>
 struct Staging {
+    static constexpr int kTilePieces = kPairPieces * kPairs;
+    static constexpr int kTileColumns = kTilePieces * 8;
     static constexpr int kMainBytes = kSource == Source::kFloat ? 32 : 16;  // per piece and row
     static constexpr int kXBytes = kSource == Source::kHalfTimesXhat ? 32 : 0;
     static constexpr int kRows = 32;                                        // rows per stage
     static constexpr int kMainStage = kRows * kTilePieces * kMainBytes;
     static constexpr int kStage = kMainStage + kRows * kTilePieces * kXBytes;
-    // All of a chunk's 256 rows at once (FP16), or half of them.
-    static constexpr int kStages = kSource == Source::kHalf ? 8 : 4;
+    // All of a chunk's 256 rows at once (FP16, 64 columns), or half of them.
+    static constexpr int kStages = kSource == Source::kHalf && kPairs == 1 ? 8 : 4;
     static constexpr int kBytes = kStages * kStage + 128;
 };
-// After the last stage the ring's memory holds the eight streams' sums for the merge.
-static_assert(Staging<Source::kHalf>::kStages * Staging<Source::kHalf>::kStage >=
-                  2 * kLaneRows * kTileColumns * 4,
-              "the merge buffers must fit in the ring");
-
 __device__ int g_reduction_error = 0;
 
 __device__ __forceinline__ uint32_t shared_address(const void* p) {
@@ -123,19 +120,25 @@ struct ColumnMaps {
 // The FP16-times-xhat kernel (LayerNorm's dgamma) also sums the FP16 values themselves
 // (dbeta) from the same staged rows, with the operations the FP16 kernel would use, and
 // writes those partial sums to `second` (unless kAlso is false).
-template <Source kSource, bool kPlain, bool kAlso>
+template <Source kSource, bool kPlain, bool kAlso, int kPairs>
 __global__ void __launch_bounds__(kAddThreads + 32)
     fb_column_partials(const __grid_constant__ ColumnMaps maps, float* __restrict__ partial,
                        float* __restrict__ second, const void* __restrict__ src, const float4* __restrict__ x,
                        const float* __restrict__ mean, const float* __restrict__ rstd, size_t rows,
                        int pieces) {
-    using S = Staging<kSource>;
+    using S = Staging<kSource, kPairs>;
+    constexpr int kTilePieces = S::kTilePieces;
+    constexpr int kTileColumns = S::kTileColumns;
+    // After the last stage the ring's memory holds the eight streams' sums for the merge.
+    static_assert(S::kStages * S::kStage >= 2 * kLaneRows * kTileColumns * 4 &&
+                      kTileColumns <= kAddThreads,
+                  "the merge buffers must fit in the ring, and a thread merge a column");
     extern __shared__ unsigned char staging_raw[];
     __shared__ float sh_mean[kSource == Source::kHalfTimesXhat ? kChunkRows : 1];
     __shared__ float sh_rstd[kSource == Source::kHalfTimesXhat ? kChunkRows : 1];
     __shared__ alignas(8) unsigned long long barriers[2 * S::kStages];
     __shared__ int abort_flag;
-    const int lane = threadIdx.x % 32;   // adding: columns 2 lane, 2 lane + 1 of the tile
+    const int lane = threadIdx.x % 32;
     const int ly = threadIdx.x / 32;     // 0-7: the row stream; 8: fetching
     const int first_piece = (blockIdx.z * kTilesY + blockIdx.y) * kTilePieces;
     if (first_piece >= pieces) {
@@ -179,10 +182,10 @@ __global__ void __launch_bounds__(kAddThreads + 32)
     volatile int* abort = &abort_flag;
     bool ok = true;
     int issued = 0;  // fetching warp: stages whose copies have been started
-    fb::Comp2 acc;
+    fb::Comp2 sums[kPairs];
     // LayerNorm's two parameter gradients come from one reading of dy.
     constexpr bool kAlsoSums = kAlso && kSource == Source::kHalfTimesXhat;
-    fb::Comp2 also;
+    fb::Comp2 also_sums[kPairs];
 
     if (ly == kLaneRows) {
         // ---- fetching warp: lane l copies row l of each stage (and its x segment) ----
@@ -266,48 +269,61 @@ __global__ void __launch_bounds__(kAddThreads + 32)
             }
             const int here = min(S::kRows, chunk_rows - k * S::kRows);
             const uint32_t stage = staging + slot * S::kStage;
-            if (lane < 4 * width) {
+            // The first `pairs` of this lane's column pairs, whose rows are added in step.
+            auto add_rows = [&](auto pairs) {
 #pragma unroll
                 for (int j = 0; j < S::kRows / kLaneRows; ++j) {
                     const int row = ly + kLaneRows * j;  // row inside the stage
                     if (row >= here) {
                         break;
                     }
-                    fb::F2 v;
-                    const uint32_t at = stage + row * (kTilePieces * S::kMainBytes) + at_main;
-                    if constexpr (kSource == Source::kFloat) {
-                        asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(at));
-                    } else {
-                        unsigned bits;
-                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(bits) : "r"(at));
-                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&bits));
-                        v = fb::f2_pack(f.x, f.y);
-                    }
-                    if constexpr (kSource == Source::kHalfTimesXhat) {
-                        fb::F2 xs;
-                        asm volatile("ld.shared.b64 %0, [%1];"
-                                     : "=l"(xs)
-                                     : "r"(stage + row * (kTilePieces * S::kXBytes) + at_x));
-                        const float m = sh_mean[k * S::kRows + row];
-                        const float rs = sh_rstd[k * S::kRows + row];
-                        const fb::F2 xhat =
-                            fb::f2_mul(fb::f2_sub(xs, fb::f2_pack(m, m)), fb::f2_pack(rs, rs));
-                        if constexpr (kPlain) {
-                            acc.s = fb::f2_fma(v, xhat, acc.s);
+#pragma unroll
+                    for (int i = 0; i < pairs.value; ++i) {
+                        fb::Comp2& acc = sums[i];
+                        [[maybe_unused]] fb::Comp2& also = also_sums[i];
+                        fb::F2 v;
+                        const uint32_t at = stage + row * (kTilePieces * S::kMainBytes) + at_main +
+                                            i * (kPairPieces * S::kMainBytes);
+                        if constexpr (kSource == Source::kFloat) {
+                            asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(at));
                         } else {
-                            fb::comp_add_product2(acc, v, xhat);
+                            unsigned bits;
+                            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(bits) : "r"(at));
+                            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&bits));
+                            v = fb::f2_pack(f.x, f.y);
                         }
-                        if constexpr (kAlsoSums && kPlain) {
-                            also.s = fb::f2_add(also.s, v);
-                        } else if constexpr (kAlsoSums) {
-                            fb::comp_add2(also, v);
+                        if constexpr (kSource == Source::kHalfTimesXhat) {
+                            fb::F2 xs;
+                            asm volatile("ld.shared.b64 %0, [%1];"
+                                         : "=l"(xs)
+                                         : "r"(stage + row * (kTilePieces * S::kXBytes) + at_x +
+                                               i * (kPairPieces * S::kXBytes)));
+                            const float m = sh_mean[k * S::kRows + row];
+                            const float rs = sh_rstd[k * S::kRows + row];
+                            const fb::F2 xhat =
+                                fb::f2_mul(fb::f2_sub(xs, fb::f2_pack(m, m)), fb::f2_pack(rs, rs));
+                            if constexpr (kPlain) {
+                                acc.s = fb::f2_fma(v, xhat, acc.s);
+                            } else {
+                                fb::comp_add_product2(acc, v, xhat);
+                            }
+                            if constexpr (kAlsoSums && kPlain) {
+                                also.s = fb::f2_add(also.s, v);
+                            } else if constexpr (kAlsoSums) {
+                                fb::comp_add2(also, v);
+                            }
+                        } else if constexpr (kPlain) {
+                            acc.s = fb::f2_add(acc.s, v);
+                        } else {
+                            fb::comp_add2(acc, v);
                         }
-                    } else if constexpr (kPlain) {
-                        acc.s = fb::f2_add(acc.s, v);
-                    } else {
-                        fb::comp_add2(acc, v);
                     }
                 }
+            };
+            if (lane + 32 * (kPairs - 1) < 4 * width) {
+                add_rows(std::integral_constant<int, kPairs>{});
+            } else if (kPairs == 2 && lane < 4 * width) {
+                add_rows(std::integral_constant<int, 1>{});
             }
             // This stream is done with the slot; the fetching warp refills it once all eight are.
             __syncwarp();
@@ -346,9 +362,13 @@ __global__ void __launch_bounds__(kAddThreads + 32)
             __syncthreads();  // the first set has been read
         }
         if (ly < kLaneRows) {
-            const int at = ly * kTileColumns + 2 * lane;
-            fb::f2_unpack(set == 0 ? acc.s : also.s, sh_s[at], sh_s[at + 1]);
-            fb::f2_unpack(set == 0 ? acc.e : also.e, sh_e[at], sh_e[at + 1]);
+#pragma unroll
+            for (int i = 0; i < kPairs; ++i) {
+                const int at = ly * kTileColumns + 64 * i + 2 * lane;
+                const fb::Comp2& from = set == 0 ? sums[i] : also_sums[i];
+                fb::f2_unpack(from.s, sh_s[at], sh_s[at + 1]);
+                fb::f2_unpack(from.e, sh_e[at], sh_e[at + 1]);
+            }
         }
         __syncthreads();
         const int column = threadIdx.x;
@@ -453,14 +473,15 @@ __global__ void __launch_bounds__(32 * kFinishWarps)
     }
 }
 
-template <Source kSource, bool kPlain = false, bool kAlso = true>
-cudaError_t launch_partials(void* workspace, const void* src, const void* x, const void* mean,
-                            const void* rstd, size_t rows, size_t cols, cudaStream_t stream,
-                            void* second = nullptr) {
+template <Source kSource, bool kPlain, bool kAlso, int kPairs>
+cudaError_t launch_partials_of(void* workspace, const void* src, const void* x, const void* mean,
+                               const void* rstd, size_t rows, size_t cols, cudaStream_t stream,
+                               void* second) {
+    constexpr int kTilePieces = Staging<kSource, kPairs>::kTilePieces;
     const unsigned chunks = static_cast<unsigned>((rows + kChunkRows - 1) / kChunkRows);
     const int pieces = static_cast<int>(cols / 8);
     const unsigned tiles = static_cast<unsigned>((pieces + kTilePieces - 1) / kTilePieces);
-    constexpr int kDynamic = Staging<kSource>::kBytes;
+    constexpr int kDynamic = Staging<kSource, kPairs>::kBytes;
     static std::atomic<bool> configured[64] = {};  // per instantiation and device
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
@@ -468,7 +489,7 @@ cudaError_t launch_partials(void* workspace, const void* src, const void* x, con
         return e;
     }
     if (device >= 64 || !configured[device].load(std::memory_order_relaxed)) {
-        e = cudaFuncSetAttribute(fb_column_partials<kSource, kPlain, kAlso>,
+        e = cudaFuncSetAttribute(fb_column_partials<kSource, kPlain, kAlso, kPairs>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kDynamic);
         if (e != cudaSuccess) {
             return e;
@@ -480,7 +501,7 @@ cudaError_t launch_partials(void* workspace, const void* src, const void* x, con
     ColumnMaps maps;
     maps.use = rows < (size_t{1} << 31) ? 1 : 0;
     if (maps.use != 0) {
-        using S = Staging<kSource>;
+        using S = Staging<kSource, kPairs>;
         e = fb::encode_rows_map(&maps.main, src, rows, cols, S::kMainBytes / 8, kTilePieces * 8,
                                 S::kRows);
         if (e == cudaSuccess && S::kXBytes != 0) {
@@ -490,12 +511,45 @@ cudaError_t launch_partials(void* workspace, const void* src, const void* x, con
             return e;
         }
     }
-    return fb::launch_dependent(fb_column_partials<kSource, kPlain, kAlso>, dim3(chunks, std::min(tiles, kTilesY), (tiles + kTilesY - 1) / kTilesY),
+    return fb::launch_dependent(fb_column_partials<kSource, kPlain, kAlso, kPairs>,
+                                dim3(chunks, std::min(tiles, kTilesY), (tiles + kTilesY - 1) / kTilesY),
                                 dim3(kAddThreads + 32), kDynamic, stream, maps,
                                 static_cast<float*>(workspace), static_cast<float*>(second), src,
                                 static_cast<const float4*>(x),
                                 static_cast<const float*>(mean), static_cast<const float*>(rstd),
                                 rows, pieces);
+}
+
+// Whether FP16 sums take 128 columns per CTA: where 64 would make more than three CTAs per SM.
+// Bias gradient, 64 -> 128 columns: 8,192 x 2,304 (1,152 CTAs) 14.0 -> 12.4 us, x 1,600 (800)
+// 11.4 -> 10.3, x 3,072 17.7 -> 16.1, 4,096 x 2,304 (576) 8.9 -> 8.1, 2,048 x 4,096 (512)
+// 8.8 -> 8.0; but 4,096 x 1,600 (400) 7.5 -> 8.0, 8,192 x 768 (384) 7.6 -> 8.1, 1,024 x 768 (48)
+// 5.8 -> 6.8. 256 columns lie between or behind (8,192 x 2,304 12.1 us, x 3,072 16.5). LayerNorm's
+// sums, 12 bytes per element to stage, are slower in wide tiles (8,192 x 768 backward 25 -> 31 us).
+cudaError_t wide_tiles(size_t rows, size_t cols, bool* wide) {
+    int sms = 0;
+    const cudaError_t e = fb::sm_count(&sms);
+    *wide = (rows + kChunkRows - 1) / kChunkRows * ((cols + 63) / 64) > 3 * static_cast<size_t>(sms);
+    return e;
+}
+
+template <Source kSource, bool kPlain = false, bool kAlso = true>
+cudaError_t launch_partials(void* workspace, const void* src, const void* x, const void* mean,
+                            const void* rstd, size_t rows, size_t cols, cudaStream_t stream,
+                            void* second = nullptr) {
+    if constexpr (kSource == Source::kHalf) {
+        bool wide = false;
+        const cudaError_t e = wide_tiles(rows, cols, &wide);
+        if (e != cudaSuccess) {
+            return e;
+        }
+        if (wide) {
+            return launch_partials_of<kSource, kPlain, kAlso, 2>(workspace, src, x, mean, rstd, rows, cols,
+                                                                 stream, second);
+        }
+    }
+    return launch_partials_of<kSource, kPlain, kAlso, 1>(workspace, src, x, mean, rstd, rows, cols, stream,
+                                                         second);
 }
 
 cudaError_t launch_finish(void* out, const void* workspace, size_t rows, size_t cols,

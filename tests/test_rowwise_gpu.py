@@ -264,9 +264,11 @@ def test_layernorm_parameter_sums_wherever_they_lie(flint, shape, accumulate_dx)
     assert same_bits(dbeta, want[2])
 
 
-@pytest.mark.parametrize("shape", [(3, 32768 * 64 + 8), (255, 72), (512, 64)])
+@pytest.mark.parametrize("shape", [(3, 32768 * 64 + 8), (255, 72), (512, 64), (3, 32768 * 128 + 8),
+                                   (3500, 1920), (3841, 1920), (3841, 1928), (3841, 1992)])
 def test_bias_gradient_at_the_edges_of_its_grid(flint, shape):
-    """More 64-column tiles than one layer of the grid holds; ragged tiles and chunks."""
+    """More tiles than one layer of the grid holds; ragged tiles of 64 and of 128 columns (these
+    from more than three 64-column tiles and chunks per SM on: 444 on 148) and ragged chunks."""
     rows, cols = shape
     rng = np.random.default_rng(cols)
     dy = crafted(rng, shape).astype(np.float16)
