@@ -162,7 +162,8 @@ def ulps32(a, b):
     return np.abs(a - b) / spacing
 
 
-@pytest.mark.parametrize("shape", [(8192, 768), (5, 8), (33, 100), (7, 257), (3, 2048), (9, 1536)])
+@pytest.mark.parametrize("shape", [(8192, 768), (5, 8), (33, 100), (7, 257), (3, 2048), (9, 1536),
+                                   (5, 1540), (9, 1600), (3, 1664), (3, 1668)])
 def test_layernorm_forward_statistics_and_output(flint, shape):
     rows, cols = shape
     rng = np.random.default_rng(cols)
@@ -257,11 +258,15 @@ def test_layernorm_parameter_sums_wherever_they_lie(flint, shape, accumulate_dx)
     flint.layernorm_backward(dx, dgamma, dbeta, to(dy), to(x), to(mean), to(rstd), to(gamma), rows, cols,
                              accumulate_dx, False, ws)
     torch.cuda.synchronize()
-    want = oracle.layernorm_backward(dy, x, mean, rstd, gamma)
+    want = oracle.layernorm_backward(dy, x, mean, rstd, gamma, with_partials=True)
     want_dx = (old + want[0]).astype(np.float32) if accumulate_dx else want[0]
     assert same_bits(dx, want_dx)
     assert same_bits(dgamma, want[1])
     assert same_bits(dbeta, want[2])
+    chunks = -(-rows // 256)
+    held = ws[: chunks * cols * 8].view(torch.float32).view(chunks, 2, cols).cpu()
+    assert same_bits(held[:, 0], want[3])
+    assert same_bits(held[:, 1], want[4])
 
 
 @pytest.mark.parametrize("shape", [(3, 32768 * 64 + 8), (255, 72), (512, 64), (3, 32768 * 128 + 8),
