@@ -144,13 +144,18 @@ __device__ __forceinline__ float load_fresh_float(const float* p) {
     return v;
 }
 
-__device__ __forceinline__ void mma_16x8x16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2,
+// 16 products per element, added by the tensor core; never onto an earlier sum. (It cuts sums
+// off where FP32 additions round them, and over a chain of MMAs the cuts add up. Relative error
+// of dot products of 3,072 values, signed and all positive: FP32 FMAs and a butterfly 1.7e-7
+// and 0.5e-7, MMA chains 2.7e-7 and 8.6e-7, one MMA at a time with FP32 additions 1.0e-7 and
+// 0.7e-7; of 768: 1.0e-7 and 0.5e-7, 1.2e-7 and 1.7e-7, 0.9e-7 and 0.7e-7.)
+__device__ __forceinline__ void mma_16x8x16(float (&d)[4], unsigned a0, unsigned a1, unsigned a2,
                                             unsigned a3, unsigned b0, unsigned b1) {
     asm volatile(
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-        "{%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+        "{%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
 }
 
 // Four int8 values as two FP16 pairs: the byte with its sign bit flipped is v + 128, under
@@ -202,13 +207,31 @@ __device__ __forceinline__ void multiply(float (&acc)[(RB + 1) / 2][NT][4], cons
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 unsigned b0, b1;
+                float first[4];
+                float second[4];
                 Step<W>::weights(raw[nt], 2 * piece, b0, b1);
-                mma_16x8x16(acc[m][nt], xa.x, xb.x, xa.y, xb.y, b0, b1);
+                mma_16x8x16(first, xa.x, xb.x, xa.y, xb.y, b0, b1);
                 Step<W>::weights(raw[nt], 2 * piece + 1, b0, b1);
-                mma_16x8x16(acc[m][nt], xa.z, xb.z, xa.w, xb.w, b0, b1);
+                mma_16x8x16(second, xa.z, xb.z, xa.w, xb.w, b0, b1);
+#pragma unroll
+                for (int i = 0; i < (RB == 1 ? 2 : 4); ++i) {
+                    acc[m][nt][i] += first[i] + second[i];
+                }
             }
         }
     }
+}
+
+template <int N>
+__device__ __forceinline__ float add_pairwise(float (&part)[N]) {
+#pragma unroll
+    for (int stride = 1; stride < N; stride *= 2) {
+#pragma unroll
+        for (int i = 0; i + stride < N; i += 2 * stride) {
+            part[i] += part[i + stride];
+        }
+    }
+    return part[0];
 }
 
 // LayerNorm of `rows` FP32 rows into FP16 rows of k + 8 values in shared memory (the 16 bytes
@@ -216,6 +239,13 @@ __device__ __forceinline__ void multiply(float (&acc)[(RB + 1) / 2][NT][4], cons
 // row in registers, QN float4s a lane. Each lane takes its own values' mean and centred
 // squares; one butterfly merges both (Chan, Golub and LeVeque's update for equal counts: k is
 // a multiple of 128, so every lane has k / 32 values).
+// Precision: a lane's few values are added pairwise, the merges of the squares keep their
+// rounding errors (TwoSum), and 1 / sqrt is rsqrtf() with a Newton-Raphson step behind it. A
+// row before its rounding to FP16 is then as close to the exact one as
+// flint_layernorm_forward's compensated sums bring it (relative error, emulated on rows of
+// normal values: 5.4e-8 against 5.9e-8 for 256 columns, 5.7e-8 against 6.0e-8 for 768; with outlier
+// channels 5.7e-8 against 5.8e-8); with plain merges and rsqrtf() alone it was 1.0e-7. That
+// function's own sums, or sums in 64 bits, made a step 9 to 36 % longer here, these 2 %.
 template <int QN>
 __device__ __forceinline__ void normalise_rows(__half* h, const float* x, const float* gain,
                                                const float* shift, int rows, int k) {
@@ -233,33 +263,42 @@ __device__ __forceinline__ void normalise_rows(__half* h, const float* x, const 
                                    __uint_as_float(raw.z), __uint_as_float(raw.w));
             }
         }
-        float4 sum = v[0];
-#pragma unroll
-        for (int i = 1; i < QN; ++i) {
-            sum = make_float4(sum.x + v[i].x, sum.y + v[i].y, sum.z + v[i].z, sum.w + v[i].w);
-        }
-        float mean = ((sum.x + sum.y) + (sum.z + sum.w)) * inverse;
-        float4 squares = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        // (Absent float4s are zeros: they change neither sum.)
+        float part[QN];
 #pragma unroll
         for (int i = 0; i < QN; ++i) {
+            part[i] = (v[i].x + v[i].y) + (v[i].z + v[i].w);
+        }
+        float mean = add_pairwise(part) * inverse;
+#pragma unroll
+        for (int i = 0; i < QN; ++i) {
+            part[i] = 0.0f;
             if (128 * i < k) {
                 const float4 d = make_float4(v[i].x - mean, v[i].y - mean, v[i].z - mean, v[i].w - mean);
-                squares = make_float4(fmaf(d.x, d.x, squares.x), fmaf(d.y, d.y, squares.y),
-                                      fmaf(d.z, d.z, squares.z), fmaf(d.w, d.w, squares.w));
+                part[i] = fmaf(d.x, d.x, d.y * d.y) + fmaf(d.z, d.z, d.w * d.w);
             }
         }
-        float centred = (squares.x + squares.y) + (squares.z + squares.w);
+        float centred = add_pairwise(part);
+        float lost = 0.0f;                                  // what the merges of `centred` left over
         float half_count = static_cast<float>(k) / 64.0f;   // half of what each side has
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
             const float other = __shfl_xor_sync(fb::kFullMask, mean, off);
             const float theirs = __shfl_xor_sync(fb::kFullMask, centred, off);
+            const float their_loss = __shfl_xor_sync(fb::kFullMask, lost, off);
             const float apart = other - mean;
             mean = 0.5f * (mean + other);
-            centred = (centred + theirs) + apart * apart * half_count;
+            const float both = __fadd_rn(centred, theirs);
+            const float added = __fsub_rn(both, centred);
+            const float error = __fadd_rn(__fsub_rn(centred, __fsub_rn(both, added)),
+                                          __fsub_rn(theirs, added));
+            centred = both;
+            lost = (lost + their_loss) + fmaf(apart * apart, half_count, error);
             half_count *= 2.0f;
         }
-        const float rstd = rsqrtf(centred * (1.0f / static_cast<float>(k)) + kEps);
+        const float variance = fmaf(centred + lost, 1.0f / static_cast<float>(k), kEps);
+        const float guess = rsqrtf(variance);
+        const float rstd = fmaf(0.5f * guess, fmaf(-(variance * guess), guess, 1.0f), guess);
 #pragma unroll
         for (int i = 0; i < QN; ++i) {
             const int q = lane + 32 * i;
@@ -299,10 +338,23 @@ __host__ __device__ constexpr int linear_bytes(bool norm, int rb, int nt, int ro
                   : (first > sums_bytes(rb, nt) ? first : sums_bytes(rb, nt));
 }
 
+// CTAs per SM that registers must leave room for. Kernels of a step are resident several deep,
+// so a few registers decide what fits beside what: with 42 instead of 40 for the small int8
+// projection four sequences took 189 us a step instead of 171, and one CTA per SM in place of
+// two for the widest FP16 one made a step of one sequence 1,536 wide 378 us instead of 349.
+constexpr int linear_blocks(bool norm, int rb, int steps) {
+    return rb == 8                       ? 1
+           : norm || steps > 3 || rb > 2 ? (rb == 4 && steps > 12 ? 1 : 2)
+           : rb == 2                     ? 4
+           : steps == 3                  ? 5
+                                         : 6;
+}
+
 // A CTA owns 8 NT features, its warps a share of k each; the warps' sums meet in shared
 // memory and are added in warp order. kSteps: the steps a warp's share can have.
 template <typename W, Act A, bool kNorm, int RB, int NT, int kSteps, int QN>
-__global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p) {
+__global__ void __launch_bounds__(kThreads, linear_blocks(kNorm, RB, kSteps))
+    fb_decode_linear(const LinearArgs p) {
     using S = Step<W>;
     constexpr int kColumns = 8 * NT;
     extern __shared__ __align__(16) unsigned char decode_smem[];
@@ -360,13 +412,11 @@ __global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p)
         x = rows;
         stride = p.k + 8;
     }
-    // Activations of a chunk of steps are all asked for before the first product needs one, and
-    // two sets of accumulators take turns, so that neither loads nor MMAs form one long chain.
+    // Activations of a chunk of steps are all asked for before the first product needs one.
     constexpr int MB = (RB + 1) / 2;
-    constexpr int kSets = MB == 1 ? 2 : 1;
     constexpr int kRoom = RB == 1 ? 12 : RB == 2 ? 6 : 2;          // steps' worth of registers
     constexpr int kChunk = kSteps * S::kPieces <= kRoom ? kSteps : (kRoom + S::kPieces - 1) / S::kPieces;
-    float acc[kSets][MB][NT][4] = {};
+    float acc[MB][NT][4] = {};
 #pragma unroll
     for (int from = 0; from < kSteps; from += kChunk) {
         if (from >= mine) {
@@ -393,7 +443,7 @@ __global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p)
 #pragma unroll
         for (int j = 0; j < kChunk; ++j) {
             if (from + j < kSteps && from + j < mine) {
-                multiply<W, RB, NT>(acc[j % kSets], raw[from + j < kSteps ? from + j : 0],
+                multiply<W, RB, NT>(acc, raw[from + j < kSteps ? from + j : 0],
                                     [&](int block, int piece) { return values[j][block][piece]; });
             }
         }
@@ -407,19 +457,19 @@ __global__ void __launch_bounds__(kThreads) fb_decode_linear(const LinearArgs p)
         for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
             for (int i = 0; i < (RB == 1 ? 2 : 4); ++i) {
-                const float v = acc[0][m][nt][i] + (kSets == 2 ? acc[kSets - 1][m][nt][i] : 0.0f);
-                sums[warp][16 * m + 8 * (i / 2) + g][8 * nt + 2 * t + i % 2] = v;
+                sums[warp][16 * m + 8 * (i / 2) + g][8 * nt + 2 * t + i % 2] = acc[m][nt][i];
             }
         }
     }
     __syncthreads();
     // kThreads is a multiple of kColumns: a thread keeps its feature from row to row.
     for (int row = threadIdx.x / kColumns; row < p.rows; row += kThreads / kColumns) {
-        float v = sums[0][row][threadIdx.x % kColumns];
+        float of_warp[kWarps];
 #pragma unroll
-        for (int other = 1; other < kWarps; ++other) {
-            v += sums[other][row][threadIdx.x % kColumns];
+        for (int other = 0; other < kWarps; ++other) {
+            of_warp[other] = sums[other][row][threadIdx.x % kColumns];
         }
+        float v = add_pairwise(of_warp);
         if (sizeof(W) == 1) {
             v *= scale;
         }
@@ -784,16 +834,24 @@ __global__ void __launch_bounds__(kAttentionThreads)
                 }
             }
         }
-        float even[4] = {};
-        float odd[4] = {};
-        mma_16x8x16(even, k[0].x, k[2].x, k[0].y, k[2].y, q0.x, q0.y);
-        mma_16x8x16(odd, k[1].x, k[3].x, k[1].y, k[3].y, q1.x, q1.y);
-        mma_16x8x16(even, k[0].z, k[2].z, k[0].w, k[2].w, q0.z, q0.w);
-        mma_16x8x16(odd, k[1].z, k[3].z, k[1].w, k[3].w, q1.z, q1.w);
+        float s0;
+        float s1;
+        {
+            float a[4];
+            float b[4];
+            mma_16x8x16(a, k[0].x, k[2].x, k[0].y, k[2].y, q0.x, q0.y);
+            mma_16x8x16(b, k[0].z, k[2].z, k[0].w, k[2].w, q0.z, q0.w);
+            s0 = a[0] + b[0];
+            s1 = a[2] + b[2];
+            mma_16x8x16(a, k[1].x, k[3].x, k[1].y, k[3].y, q1.x, q1.y);
+            mma_16x8x16(b, k[1].z, k[3].z, k[1].w, k[3].w, q1.z, q1.w);
+            s0 += a[0] + b[0];
+            s1 += a[2] + b[2];
+        }
         // Positions g and g + 8, in lanes 4g (column 0).
         const bool holds = lane % 4 == 0;
-        float s0 = holds && first + lane / 4 < newest ? (even[0] + odd[0]) * to_base2 : -INFINITY;
-        float s1 = holds && first + lane / 4 + 8 < newest ? (even[2] + odd[2]) * to_base2 : -INFINITY;
+        s0 = holds && first + lane / 4 < newest ? s0 * to_base2 : -INFINITY;
+        s1 = holds && first + lane / 4 + 8 < newest ? s1 * to_base2 : -INFINITY;
         float top = fmaxf(s0, s1);
         top = fmaxf(top, __shfl_xor_sync(fb::kFullMask, top, 4));
         top = fmaxf(top, __shfl_xor_sync(fb::kFullMask, top, 8));

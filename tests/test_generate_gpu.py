@@ -8,6 +8,11 @@ approximation), so the bound is the kernels' own error: relative L2 <= 5e-3 on a
 logits (FP16 activations under FP32 accumulation, as for the training forward pass).
 """
 
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 import torch
@@ -95,6 +100,69 @@ def test_decode_kernels_at_their_edges_match_the_full_model(flint, sequences, he
                 got = gen.logits().cpu()
                 assert rel_l2(got, want[:, t]) <= 5e-3, t
                 assert torch.equal(chosen, got.argmax(1)), t
+    finally:
+        model.close()
+
+
+def teacher_forced_logits(flint, int8):
+    """After a prompt and after each of six captured steps, of 8 sequences on six layers."""
+    cfg = dict(n_layer=6, n_head=4, n_embd=256, block_size=320, vocab_size=200, padded_vocab_size=208)
+    g = torch.Generator().manual_seed(9)
+    tokens = torch.randint(0, 200, (8, 296 + 6), generator=g)
+    model = model_for(flint, cfg, weights(cfg))
+    try:
+        with Generator(flint, model, 8, 320, int8) as gen:
+            gen.prefill(u16(tokens[:, :296]))
+            logits = [gen.logits().cpu()]
+            for t in range(296, 302):
+                gen.step(u16(tokens[:, t]), graph=True)
+                logits.append(gen.logits().cpu())
+    finally:
+        model.close()
+    return torch.stack(logits)
+
+
+PLAIN_ORDER = """
+import sys, numpy as np
+sys.path[:0] = sys.argv[2:]
+import flint_b200, test_generate_gpu as t
+np.savez(sys.argv[1], *[t.teacher_forced_logits(flint_b200.Flint(), q).numpy() for q in (False, True)])
+"""
+
+
+def test_kernels_that_start_early_leave_what_plain_stream_order_leaves(flint, tmp_path):
+    """A decode step's kernels are resident several deep and read ahead of their wait. In plain
+    stream order (another process, FLINT_B200_PDL=0) nothing can be read too early: same bits."""
+    root = Path(__file__).resolve().parent.parent
+    out = tmp_path / "plain.npz"
+    subprocess.run([sys.executable, "-c", PLAIN_ORDER, str(out), str(root / "tests"), str(root / "oracle"),
+                    str(root)], check=True, env={**os.environ, "FLINT_B200_PDL": "0"}, timeout=300)
+    plain = np.load(out)
+    for i, int8 in enumerate((False, True)):
+        assert np.array_equal(teacher_forced_logits(flint, int8).numpy(), plain[f"arr_{i}"])
+
+
+@pytest.mark.parametrize("sequences", [1, 12, 40])
+def test_logits_are_sums_in_fp32(flint, sequences):
+    """A final LayerNorm of gain 0 leaves its bias, exactly: the logits are then dot products of
+    known FP16 values, here 1,536 positive ones, whose FP32 sums show. Bound: 48 additions, each
+    off by 2.4e-8 rms of what has been added up so far (1e-7 together), and 32 products added
+    by the tensor core, cut at 2^-23 at worst (1.2e-7). A chain of 96 MMAs is off by over 1e-6."""
+    cfg = dict(n_layer=1, n_head=24, n_embd=1536, block_size=64, vocab_size=200, padded_vocab_size=208)
+    params = weights(cfg)
+    g = torch.Generator().manual_seed(10)
+    params["ln_f.weight"] = torch.zeros(1536)
+    params["ln_f.bias"] = torch.randn(1536, generator=g).abs().half().float()
+    params["wte.weight"] = (torch.randn(208, 1536, generator=g).abs() * 0.02).half().float()
+    want = params["wte.weight"].double() @ params["ln_f.bias"].double()
+    tokens = torch.randint(0, 200, (sequences, 9), generator=g)
+    model = model_for(flint, cfg, params)
+    try:
+        with Generator(flint, model, sequences, 64, False) as gen:
+            gen.prefill(u16(tokens[:, :8]))
+            assert rel_l2(gen.logits().cpu(), want[:200].expand(sequences, -1)) <= 2.5e-7
+            gen.step(u16(tokens[:, 8]))
+            assert rel_l2(gen.logits().cpu(), want[:200].expand(sequences, -1)) <= 2.5e-7
     finally:
         model.close()
 
