@@ -104,6 +104,32 @@ def test_decode_kernels_at_their_edges_match_the_full_model(flint, sequences, he
         model.close()
 
 
+@pytest.mark.parametrize("int8", [False, True], ids=["fp16", "int8"])
+@pytest.mark.parametrize("sequences, heads", [(12, 24), (24, 14), (33, 20), (64, 24)])
+def test_wide_models_at_every_count_of_rows_match_the_full_model(flint, sequences, heads, int8):
+    """Widths of 896 to 1,536 with 9 to 64 sequences: the linear kernels' longest shares of k, and
+    normalised rows up to what shared memory holds (64 of 1,536: the sums then take their place)."""
+    cfg = dict(n_layer=2, n_head=heads, n_embd=64 * heads, block_size=64, vocab_size=200, padded_vocab_size=208)
+    params = weights(cfg)
+    prompt, steps = 8, 4
+    g = torch.Generator().manual_seed(8)
+    tokens = torch.randint(0, 200, (sequences, prompt + steps), generator=g)
+    want = oracle.gpt2_decode_logits(cfg, params, tokens, int8=int8)
+    model = model_for(flint, cfg, params)
+    try:
+        with Generator(flint, model, sequences, 64, int8) as gen:
+            gen.prefill(u16(tokens[:, :prompt]))
+            assert rel_l2(gen.logits().cpu(), want[:, prompt - 1]) <= 5e-3
+            for t in range(prompt, prompt + steps):
+                chosen = gen.step(u16(tokens[:, t]), graph=t > prompt).cpu().to(torch.int64) & 0xFFFF
+                got = gen.logits().cpu()
+                assert rel_l2(got, want[:, t]) <= 5e-3, t
+                assert torch.equal(chosen, got.argmax(1)), t
+    finally:
+        model.close()
+    assert not flint.kernel_fault()
+
+
 def teacher_forced_logits(flint, int8):
     """After a prompt and after each of six captured steps, of 8 sequences on six layers."""
     cfg = dict(n_layer=6, n_head=4, n_embd=256, block_size=320, vocab_size=200, padded_vocab_size=208)
