@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         bool ok = true;
         // Waits for the ring's next tile and returns its address (0 after an abort).
         auto next_tile = [&]() -> uint32_t {
-            if (!sm100::mbar_wait(bar.slot_full(slot), phase, abort)) {
+            if (!sm100::mbar_wait_warp(bar.slot_full(slot), phase, abort)) {
                 ok = false;
                 return 0u;
             }
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             }
             const int b = ahead.round & 1;
             if (ahead.j == 0 && ahead.t == 0 &&
-                !sm100::mbar_wait(bar.q_full(b), (ahead.round >> 1) & 1, abort)) {
+                !sm100::mbar_wait_warp(bar.q_full(b), (ahead.round >> 1) & 1, abort)) {
                 ok = false;
                 return;
             }
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         issue_scores();
         uint32_t n = 0;
         for (FwdCursor at = enter(0); ok && valid(at); advance(at), ++n) {
-            if (!sm100::mbar_wait(bar.p_ready(n % 3), (n / 3) & 1, abort)) {
+            if (!sm100::mbar_wait_warp(bar.p_ready(n % 3), (n / 3) & 1, abort)) {
                 break;
             }
             const uint32_t v_tile = next_tile();
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             fb::F2 l = 0;         // this thread's share of the row sum, in two partial sums
             for (int j = 0; ok && j <= qb; ++j) {
                 const uint32_t n = 2 * (before + j) + tile;   // this step's number
-                if (!sm100::mbar_wait(bar.s_full(n % 3), (n / 3) & 1, abort)) {
+                if (!sm100::mbar_wait_warp(bar.s_full(n % 3), (n / 3) & 1, abort)) {
                     ok = false;
                     break;
                 }
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 if (j > 0 && __any_sync(0xffffffffu, moved)) {
                     // The previous key tile's P V must have finished (it cannot be more than
                     // one behind: the next one needs this step's probabilities).
-                    if (!sm100::mbar_wait(bar.pv_done(tile), (before + j - 1) & 1, abort)) {
+                    if (!sm100::mbar_wait_warp(bar.pv_done(tile), (before + j - 1) & 1, abort)) {
                         ok = false;
                         break;
                     }
@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 // last one be issued at all (afterwards a slow warp could find both complete
                 // and wait for a parity that no longer comes).
                 if (j == qb && qb > 0 &&
-                    !sm100::mbar_wait(bar.pv_done(tile), (before + qb - 1) & 1, abort)) {
+                    !sm100::mbar_wait_warp(bar.pv_done(tile), (before + qb - 1) & 1, abort)) {
                     ok = false;
                     break;
                 }
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                     sm100::mbar_arrive(bar.p_ready(n % 3));
                 }
             }
-            if (!ok || !sm100::mbar_wait(bar.pv_done(tile), (before + qb) & 1, abort)) {
+            if (!ok || !sm100::mbar_wait_warp(bar.pv_done(tile), (before + qb) & 1, abort)) {
                 ok = false;
                 break;
             }
@@ -891,13 +891,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
             int round = 0;
             for (int item = item_of(0); ok && item < items; item = item_of(++round)) {
                 const int steps = 2 * (p.blocks - item / bh_count);
-                ok = sm100::mbar_wait(bar.a_ready(), round & 1, abort);
+                ok = sm100::mbar_wait_warp(bar.a_ready(), round & 1, abort);
                 sm100::tc_fence_after_sync();
                 // S^T and dP^T of sub-step g into accumulator pair g & 1.
                 auto issue_scores = [&](int g) -> bool {
                     const uint32_t count = before + g;
                     const int stage = count % kBwdStages;
-                    if (!sm100::mbar_wait(bar.stage_full(stage), (count / kBwdStages) & 1, abort)) {
+                    if (!sm100::mbar_wait_warp(bar.stage_full(stage), (count / kBwdStages) & 1, abort)) {
                         return false;
                     }
                     sm100::tc_fence_after_sync();
@@ -926,7 +926,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
                         ok = false;
                         break;
                     }
-                    if (!sm100::mbar_wait(bar.operands_ready(b), (count >> 1) & 1, abort)) {
+                    if (!sm100::mbar_wait_warp(bar.operands_ready(b), (count >> 1) & 1, abort)) {
                         ok = false;
                         break;
                     }
@@ -965,7 +965,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         // K and V of an item become the A operands of its score MMAs. Called when every
         // score MMA of the item before has completed (its last scores_full was awaited).
         auto install = [&](int round) -> bool {
-            if (!sm100::mbar_wait(bar.resident(), round & 1, abort)) {
+            if (!sm100::mbar_wait_warp(bar.resident(), round & 1, abort)) {
                 return false;
             }
             tile_row_to_tmem(tmem_k + lane_base, k_tile, row, part);
@@ -991,10 +991,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
                 // stage_full covers the statistics; scores_full the two accumulators (and,
                 // the tensor pipe being in order, that the MMAs which read this pair's
                 // previous P^T and dS^T have finished).
-                if (!sm100::mbar_wait(bar.scores_full(b), (count >> 1) & 1, abort)) {
-                    ok = false;
-                    break;
-                }
+                // A lane that gives up goes along with its warp to the end of the sub-step (what it
+                // computes stays in tensor memory), where the lanes agree at no cost; agreeing
+                // right here, mbar_wait_warp(), made the two backward kernels 1.7 % slower.
+                bool there = sm100::mbar_wait(bar.scores_full(b), (count >> 1) & 1, abort);
                 sm100::tc_fence_after_sync();
                 const uint32_t my_scores = tmem_st(b) + lane_base + part * kPart;
                 const uint32_t my_weights = tmem_dpt(b) + lane_base + part * kPart;
@@ -1002,10 +1002,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
                 uint32_t dp_raw[kPart];
                 sm100::tmem_ld_32x16(my_scores, s_raw);
                 sm100::tmem_ld_32x16(my_weights, dp_raw);
-                if (!sm100::mbar_wait(bar.stage_full(stage), (count / kBwdStages) & 1, abort)) {
-                    ok = false;
-                    break;
-                }
+                there = sm100::mbar_wait(bar.stage_full(stage), (count / kBwdStages) & 1, abort) && there;
                 // My 16 queries' statistics: every lane reads the same addresses (broadcast).
                 const uint32_t stat = stats + stage * 2 * kStatBytes + part * kPart * 4;
                 float lse2[kPart];
@@ -1058,6 +1055,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
                 pack_pairs(packed, dsv);
                 sm100::tmem_st_32x8(my_weights, packed);
                 warp_arrive_after_stores(bar.operands_ready(b), lane);
+                ok = __all_sync(0xffffffffu, there);
             }
             before += steps;
             if (!ok) {
@@ -1069,7 +1067,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
                 ok = false;
                 break;
             }
-            if (!sm100::mbar_wait(bar.done(), round & 1, abort)) {
+            if (!sm100::mbar_wait_warp(bar.done(), round & 1, abort)) {
                 ok = false;
                 break;
             }
@@ -1208,12 +1206,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
             int round = 0;
             for (int item = item_of(0); ok && item < items; item = item_of(++round)) {
                 const int steps = 2 * (p.blocks - item / bh_count);
-                ok = sm100::mbar_wait(bar.a_ready(), round & 1, abort);
+                ok = sm100::mbar_wait_warp(bar.a_ready(), round & 1, abort);
                 sm100::tc_fence_after_sync();
                 auto issue_scores = [&](int g) -> bool {
                     const uint32_t count = before + g;
                     const int stage = count % kBwdStages;
-                    if (!sm100::mbar_wait(bar.stage_full(stage), (count / kBwdStages) & 1, abort)) {
+                    if (!sm100::mbar_wait_warp(bar.stage_full(stage), (count / kBwdStages) & 1, abort)) {
                         return false;
                     }
                     sm100::tc_fence_after_sync();
@@ -1242,7 +1240,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
                         ok = false;
                         break;
                     }
-                    if (!sm100::mbar_wait(bar.operands_ready(b), (count >> 1) & 1, abort)) {
+                    if (!sm100::mbar_wait_warp(bar.operands_ready(b), (count >> 1) & 1, abort)) {
                         ok = false;
                         break;
                     }
@@ -1274,7 +1272,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         const float scale2 = p.scale * kLog2e;
         // Q and dO of an item become the A operands of its score MMAs.
         auto install = [&](int round) -> bool {
-            if (!sm100::mbar_wait(bar.resident(), round & 1, abort)) {
+            if (!sm100::mbar_wait_warp(bar.resident(), round & 1, abort)) {
                 return false;
             }
             tile_row_to_tmem(tmem_q + lane_base, q_tile, row, part);
@@ -1302,10 +1300,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
             for (int g = 0; ok && g < steps; ++g) {
                 const int b = g & 1;
                 const uint32_t count = before + g;
-                if (!sm100::mbar_wait(bar.scores_full(b), (count >> 1) & 1, abort)) {
-                    ok = false;
-                    break;
-                }
+                // (As in dK/dV: the warp's lanes agree at the end of the sub-step.)
+                const bool there = sm100::mbar_wait(bar.scores_full(b), (count >> 1) & 1, abort);
                 sm100::tc_fence_after_sync();
                 const uint32_t my_weights = tmem_dp(b) + lane_base + part * kPart;
                 uint32_t s_raw[kPart];
@@ -1338,6 +1334,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
                 pack_pairs(packed, dsv);
                 sm100::tmem_st_32x8(my_weights, packed);
                 warp_arrive_after_stores(bar.operands_ready(b), lane);
+                ok = __all_sync(0xffffffffu, there);
             }
             before += steps;
             if (!ok) {
@@ -1347,7 +1344,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
                 ok = false;
                 break;
             }
-            if (!sm100::mbar_wait(bar.done(), round & 1, abort)) {
+            if (!sm100::mbar_wait_warp(bar.done(), round & 1, abort)) {
                 ok = false;
                 break;
             }
@@ -1582,7 +1579,7 @@ __global__ void __launch_bounds__(128, 1) fb_mma_clocks(int n, int a_in_tmem, in
             sm100::mma_commit(bar);
         }
         __syncwarp();
-        sm100::mbar_wait(bar, 0, &abort_flag);
+        sm100::mbar_wait_warp(bar, 0, &abort_flag);
         const long long completed = clock64();
         if (sm100::elect_one()) {
             g_mma_clocks[0] = issued - start;

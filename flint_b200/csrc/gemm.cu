@@ -777,32 +777,26 @@ __global__ void __launch_bounds__(kThreads, 1)
     } else if (warp == 1) {
         // ---- MMA issuer ----
         // The whole warp runs the loop, so that its state stays warp-uniform; one elected
-        // lane issues (with the loop inside `lane == 0`, every MMA paid moves into uniform
-        // registers: a k-block of a 64-column tile took 0.27 us instead of 0.24).
+        // lane waits and issues (with the loop inside `lane == 0`, every MMA paid moves into uniform
+        // registers: a k-block of a 64-column tile took 0.27 us instead of 0.24). If its wait
+        // gives up it stays in the loop, whose elections need every lane, and issues nothing more.
         {
             int stage = 0;
             uint32_t phase = 0;
             int acc = 0;
             uint32_t acc_phase = 0;
-            bool ok = true;
-            for (long long id = blockIdx.x; ok && id < p.tiles_total; id += gridDim.x) {
+            bool alive = true;   // the elected lane's: its waits have not given up
+            for (long long id = blockIdx.x; id < p.tiles_total; id += gridDim.x) {
                 const TileCoord t = decode_tile(p, id);
                 const bool split_k = kIsTn && !p.batched;
                 const int k0 = split_k ? static_cast<int>(t.z) * p.split_len : 0;
                 const int k1 = split_k ? min(p.k, k0 + p.split_len) : p.k;
-                if (!sm100::mbar_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort)) {
-                    ok = false;
-                    break;
+                if (sm100::elect_one()) {
+                    alive = alive && sm100::mbar_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort);
                 }
-                sm100::tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
                 uint32_t accumulate = 0;
                 for (int kk = k0; kk < k1; kk += kBK) {
-                    if (!sm100::mbar_wait(full_bar(stage), phase, abort)) {
-                        ok = false;
-                        break;
-                    }
-                    sm100::tc_fence_after_sync();
                     const uint32_t a_addr = smem_base + stage * R::kStage;
                     const uint32_t b_addr = a_addr + R::kStageA;
                     const uint64_t a_desc = kAMn ? sm100::smem_desc_sw128(a_addr, 8192, 1024)
@@ -810,16 +804,20 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const uint64_t b_desc = kBMn ? sm100::smem_desc_sw128(b_addr, 8192, 1024)
                                                  : sm100::smem_desc_sw128(b_addr, 16, 1024);
                     if (sm100::elect_one()) {
+                        alive = alive && sm100::mbar_wait(full_bar(stage), phase, abort);
+                        if (alive) {
+                            sm100::tc_fence_after_sync();
 #pragma unroll
-                        for (int ks = 0; ks < kBK / 16; ++ks) {
-                            if (ks == 0) {
-                                sm100::mma_f16_ss_at<-1>(d_tmem, a_desc, 0, b_desc, 0, kIdesc, accumulate);
-                            } else {
-                                sm100::mma_f16_ss_at<1>(d_tmem, a_desc, ks * (kAMn ? 128 : 2), b_desc,
-                                                        ks * (kBMn ? 128 : 2), kIdesc);
+                            for (int ks = 0; ks < kBK / 16; ++ks) {
+                                if (ks == 0) {
+                                    sm100::mma_f16_ss_at<-1>(d_tmem, a_desc, 0, b_desc, 0, kIdesc, accumulate);
+                                } else {
+                                    sm100::mma_f16_ss_at<1>(d_tmem, a_desc, ks * (kAMn ? 128 : 2), b_desc,
+                                                            ks * (kBMn ? 128 : 2), kIdesc);
+                                }
                             }
+                            sm100::mma_commit(empty_bar(stage));
                         }
-                        sm100::mma_commit(empty_bar(stage));
                     }
                     accumulate = 1;
                     if (++stage == R::kStages) {
@@ -827,10 +825,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         phase ^= 1u;
                     }
                 }
-                if (!ok) {
-                    break;
-                }
-                if (sm100::elect_one()) {
+                if (sm100::elect_one() && alive) {
                     sm100::mma_commit(acc_full_bar(acc));
                 }
                 acc ^= 1;
@@ -863,7 +858,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 load_aux<E>(aux, p, batch_offset, row - lane, col0 + column_half * 32,
                             min(32, p.n - (col0 + column_half * 32)), lane);
             }
-            if (!sm100::mbar_wait(acc_full_bar(acc), acc_phase, abort)) {
+            if (!sm100::mbar_wait_warp(acc_full_bar(acc), acc_phase, abort)) {
                 ok = false;
                 break;
             }
@@ -1117,25 +1112,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
             uint32_t phase = 0;
             int acc = 0;
             uint32_t acc_phase = 0;
-            bool ok = true;
-            for (long long id = pair; ok && id < p.tiles_total; id += pairs) {
+            bool alive = true;   // the elected lane's: its waits have not given up
+            for (long long id = pair; id < p.tiles_total; id += pairs) {
                 const TileCoord t = decode_pair_tile(p, id);
                 const bool split_k = kIsTn && !p.batched;
                 const int k0 = split_k ? static_cast<int>(t.z) * p.split_len : 0;
                 const int k1 = split_k ? min(p.k, k0 + p.split_len) : p.k;
-                if (!sm100::mbar_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort)) {
-                    ok = false;
-                    break;
+                if (sm100::elect_one()) {
+                    alive = alive && sm100::mbar_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort);
                 }
-                sm100::tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kPairBN);
                 uint32_t accumulate = 0;
                 for (int kk = k0; kk < k1; kk += kBK) {
-                    if (!sm100::mbar_wait(full_bar(stage), phase, abort)) {
-                        ok = false;
-                        break;
-                    }
-                    sm100::tc_fence_after_sync();
                     const uint32_t a_addr = smem_base + stage * kPairStage;
                     const uint32_t b_addr = a_addr + kPairStageA;
                     const uint64_t a_desc = kAMn ? sm100::smem_desc_sw128(a_addr, 8192, 1024)
@@ -1143,13 +1131,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
                     const uint64_t b_desc = kBMn ? sm100::smem_desc_sw128(b_addr, 8192, 1024)
                                                  : sm100::smem_desc_sw128(b_addr, 16, 1024);
                     if (sm100::elect_one()) {
+                        alive = alive && sm100::mbar_wait(full_bar(stage), phase, abort);
+                        if (alive) {
+                            sm100::tc_fence_after_sync();
 #pragma unroll
-                        for (int ks = 0; ks < kBK / 16; ++ks) {
-                            sm100::mma_f16_ss_pair(d_tmem, a_desc + ks * (kAMn ? 128 : 2),
-                                                   b_desc + ks * (kBMn ? 128 : 2), kIdesc,
-                                                   ks == 0 ? accumulate : 1u);
+                            for (int ks = 0; ks < kBK / 16; ++ks) {
+                                sm100::mma_f16_ss_pair(d_tmem, a_desc + ks * (kAMn ? 128 : 2),
+                                                       b_desc + ks * (kBMn ? 128 : 2), kIdesc,
+                                                       ks == 0 ? accumulate : 1u);
+                            }
+                            sm100::mma_commit_pair(empty_bar(stage), 3);
                         }
-                        sm100::mma_commit_pair(empty_bar(stage), 3);
                     }
                     accumulate = 1;
                     if (++stage == kPairStages) {
@@ -1157,10 +1149,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
                         phase ^= 1u;
                     }
                 }
-                if (!ok) {
-                    break;
-                }
-                if (sm100::elect_one()) {
+                if (sm100::elect_one() && alive) {
                     sm100::mma_commit_pair(acc_full_bar(acc), 3);
                 }
                 acc ^= 1;
@@ -1200,7 +1189,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
             }
             aux_requested = false;
             float bias_next = load_bias_lane<E>(p, col0 + column_part * 32, lane);
-            if (!sm100::mbar_wait(acc_full_bar(acc), acc_phase, abort)) {
+            if (!sm100::mbar_wait_warp(acc_full_bar(acc), acc_phase, abort)) {
                 ok = false;
                 break;
             }

@@ -81,22 +81,44 @@ __device__ __forceinline__ uint32_t shared_address(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+__device__ __forceinline__ bool staged_try(uint32_t bar, uint32_t parity) {
+    uint32_t done = 0;
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
 // Bounded mbarrier wait: false (and the flag set) after about a second of SM clocks.
 __device__ __forceinline__ bool staged_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
     const long long start = clock64();
     for (uint32_t spin = 0;; ++spin) {
-        uint32_t done = 0;
-        asm volatile(
-            "{\n.reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done != 0) {
+        if (staged_try(bar, parity)) {
             return true;
         }
         if ((spin & 63u) == 63u && (*abort != 0 || clock64() - start > 2000000000LL)) {
+            *abort = 1;
+            return false;
+        }
+    }
+}
+
+// The same for a whole warp, with one outcome for all its lanes (a lane that left alone would
+// leave the others waiting for it in the next __syncwarp).
+__device__ __forceinline__ bool staged_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort) {
+    const long long start = clock64();
+    bool done = false;
+    for (uint32_t spin = 0;; ++spin) {
+        done = done || staged_try(bar, parity);
+        if (__all_sync(fb::kFullMask, done)) {
+            return true;
+        }
+        if ((spin & 63u) == 63u &&
+            __any_sync(fb::kFullMask, *abort != 0 || clock64() - start > 2000000000LL)) {
             *abort = 1;
             return false;
         }
@@ -194,7 +216,7 @@ __global__ void __launch_bounds__(kAddThreads + 32)
         for (int k = 0; k < stages_total; ++k) {
             const int slot = k % S::kStages;
             if (k >= S::kStages &&
-                !staged_wait(empty_bar(slot), static_cast<uint32_t>(k / S::kStages - 1) & 1u,
+                !staged_wait_warp(empty_bar(slot), static_cast<uint32_t>(k / S::kStages - 1) & 1u,
                              abort)) {
                 ok = false;
                 break;
@@ -263,10 +285,9 @@ __global__ void __launch_bounds__(kAddThreads + 32)
         const int at_x = S::kMainStage + lane * (S::kXBytes / 4);
         for (int k = 0; k < stages_total; ++k) {
             const int slot = k % S::kStages;
-            if (!staged_wait(full_bar(slot), static_cast<uint32_t>(k / S::kStages) & 1u, abort)) {
-                ok = false;
-                break;
-            }
+            // (A lane that gives up goes on with the others, who would wait for it in __syncwarp;
+            // what it adds is thrown away.)
+            ok = staged_wait(full_bar(slot), static_cast<uint32_t>(k / S::kStages) & 1u, abort) && ok;
             const int here = min(S::kRows, chunk_rows - k * S::kRows);
             const uint32_t stage = staging + slot * S::kStage;
             // The first `pairs` of this lane's column pairs, whose rows are added in step.
@@ -333,7 +354,7 @@ __global__ void __launch_bounds__(kAddThreads + 32)
             }
         }
     }
-    if (!ok && lane == 0) {
+    if (!__all_sync(fb::kFullMask, ok) && lane == 0) {
         atomicExch(&g_reduction_error, 1);
     }
     __syncthreads();

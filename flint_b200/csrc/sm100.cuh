@@ -93,6 +93,30 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// The same for a whole warp (all 32 lanes, converged): one outcome for all its lanes. Lanes that
+// polled for themselves could disagree when time runs out just as the phase completes; those
+// that gave up would leave, and the others wait for them in the next warp-wide instruction
+// (elect.sync, __syncwarp, tcgen05.ld) for good.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort,
+                                               long long limit_cycles = 2000000000LL) {
+    bool done = mbar_try_wait(bar, parity);
+    if (__all_sync(0xffffffffu, done)) {
+        return true;
+    }
+    const long long start = clock64();
+    for (uint32_t spin = 0;; ++spin) {
+        done = done || mbar_try_wait(bar, parity);
+        if (__all_sync(0xffffffffu, done)) {
+            return true;
+        }
+        if ((spin & 63u) == 63u &&
+            __any_sync(0xffffffffu, *abort != 0 || clock64() - start > limit_cycles)) {
+            *abort = 1;
+            return false;
+        }
+    }
+}
+
 // ---- TMA ---------------------------------------------------------------------------
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
