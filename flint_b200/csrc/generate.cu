@@ -17,6 +17,7 @@
 //             Products run on mma.sync with the sequences as the 16 rows of A and eight
 //             output features as the columns of B, so up to 16 sequences cost one MMA per
 //             16 weights of a feature.
+//             (Many rows of a wide FP16 model take the prompt's GEMMs: tensor_core_step().)
 //             Positions live in device memory, so a step's launches do not change from
 //             token to token and are captured once into a CUDA graph.
 //
@@ -489,7 +490,8 @@ __global__ void __launch_bounds__(kThreads, linear_blocks(kNorm, RB, kSteps))
 //
 // The one kernel of a step whose weights are many (77 MB in FP16): two CTAs per SM stream
 // them, a warp per eight features, the next twelve steps' weights on their way while twelve
-// are used. Every lane remembers the largest logit it saw; a sequence's best candidates meet
+// are used (eight with more than 16 rows, whose sums need the registers: 64 rows of 768, FP16,
+// 872 -> 852 us a step). Every lane remembers the largest logit it saw; a sequence's best candidates meet
 // in a 64-bit maximum of (ordered logit, inverted index), and the last CTA writes the tokens,
 // advances the position and leaves the scratch as it found it.
 
@@ -518,7 +520,7 @@ __global__ void __launch_bounds__(kThreads, 2) fb_decode_head(const HeadArgs p) 
     using S = Step<W>;
     constexpr int MB = (RB + 1) / 2;
     constexpr int kHalves = RB == 1 ? 1 : 2;
-    constexpr int kAhead = 12 / S::kPieces;   // steps per batch of loads
+    constexpr int kAhead = (RB < 4 ? 12 : 8) / S::kPieces;   // steps per batch of loads
     extern __shared__ __align__(16) unsigned char decode_smem[];
     __shared__ unsigned long long chosen[kWarps][8 * RB];
     __shared__ bool last_cta;
@@ -1186,6 +1188,17 @@ flint_status run_prompt(flint_b200_generator& g, size_t count, cudaStream_t stre
     return FLINT_OK;
 }
 
+// Whether a step's linear layers run on the prompt's GEMMs (FP16 weights only: int8 ones would be
+// expanded on every step). The step's own kernels read every row in every CTA, which grows with
+// rows times width and passes what 128-row tensor-core tiles waste at about 33 rows of 1,280, 41
+// of 1,024 or 47 of 896; models up to 768 wide never get there. us per step of 12 layers, own
+// kernels -> GEMMs: 33 x 1,280 1,298 -> 1,074, 33 x 1,536 1,463 -> 1,274, 48 x 1,024 1,059 -> 1,015,
+// 64 x 896 1,170 -> 1,013, 64 x 1,536 2,127 -> 1,498; but 33 x 896 810 -> 848, 33 x 1,024 864 -> 908,
+// 40 x 1,024 941 -> 959, 64 x 768 852 -> 886, 32 x 1,536 1,209 -> 1,251.
+bool tensor_core_step(const flint_b200_generator& g) {
+    return !g.int8 && g.sequences > 32 && g.width > 768 && g.sequences * g.width >= 42000;
+}
+
 // The transformer over one new position per sequence.
 flint_status run_token(flint_b200_generator& g, cudaStream_t stream) {
     // Shared memory for as many positions as there can be, within what one CTA per SM may have,
@@ -1197,17 +1210,31 @@ flint_status run_token(flint_b200_generator& g, cudaStream_t stream) {
                                             (g.max_length + kBatchPositions - 1) / kBatchPositions);
     static std::atomic<bool> configured[64] = {};
     FB_CUDA(fb::allow_shared_memory(fb_decode_attention, attention_bytes(kMostStaged), configured));
+    const bool dense = tensor_core_step(g);
+    const size_t rows = g.sequences;
     for (size_t i = 0; i < g.layers; ++i) {
         const Layer& l = g.blocks[i];
-        FB_TRY(decode_linear<Act::kNone>(g, l.attn, g.qkv, g.x_a, l.ln1_w, l.ln1_b, nullptr, stream));
+        if (dense) {
+            FB_TRY(layernorm(g, l.ln1_w, l.ln1_b, g.x_a, rows, stream));
+            FB_TRY(linear<Act::kNone>(g, l.attn, g.qkv, g.h, nullptr, rows, stream));
+        } else {
+            FB_TRY(decode_linear<Act::kNone>(g, l.attn, g.qkv, g.x_a, l.ln1_w, l.ln1_b, nullptr, stream));
+        }
         FB_CUDA(fb::launch_dependent(
             fb_decode_attention, dim3(static_cast<unsigned>(pairs)), dim3(kAttentionThreads),
             static_cast<size_t>(attention_bytes(static_cast<int>(batches))),
             stream, g.attn, g.qkv, g.keys(i), g.values(i), g.position, static_cast<int>(g.heads),
             static_cast<int>(g.max_length), static_cast<int>(batches), attention_scale()));
-        FB_TRY(decode_linear<Act::kResidual>(g, l.proj, g.x_b, g.attn, nullptr, nullptr, g.x_a, stream));
-        FB_TRY(decode_linear<Act::kGelu>(g, l.fc, g.act, g.x_b, l.ln2_w, l.ln2_b, nullptr, stream));
-        FB_TRY(decode_linear<Act::kResidual>(g, l.fcproj, g.x_a, g.act, nullptr, nullptr, g.x_b, stream));
+        if (dense) {
+            FB_TRY(linear<Act::kResidual>(g, l.proj, g.x_b, g.attn, g.x_a, rows, stream));
+            FB_TRY(layernorm(g, l.ln2_w, l.ln2_b, g.x_b, rows, stream));
+            FB_TRY(linear<Act::kGelu>(g, l.fc, g.act, g.h, nullptr, rows, stream));
+            FB_TRY(linear<Act::kResidual>(g, l.fcproj, g.x_a, g.act, g.x_b, rows, stream));
+        } else {
+            FB_TRY(decode_linear<Act::kResidual>(g, l.proj, g.x_b, g.attn, nullptr, nullptr, g.x_a, stream));
+            FB_TRY(decode_linear<Act::kGelu>(g, l.fc, g.act, g.x_b, l.ln2_w, l.ln2_b, nullptr, stream));
+            FB_TRY(decode_linear<Act::kResidual>(g, l.fcproj, g.x_a, g.act, nullptr, nullptr, g.x_b, stream));
+        }
     }
     return FLINT_OK;
 }

@@ -105,7 +105,7 @@ def test_decode_kernels_at_their_edges_match_the_full_model(flint, sequences, he
 
 
 @pytest.mark.parametrize("int8", [False, True], ids=["fp16", "int8"])
-@pytest.mark.parametrize("sequences, heads", [(12, 24), (24, 14), (33, 20), (64, 24)])
+@pytest.mark.parametrize("sequences, heads", [(12, 24), (24, 14), (40, 14), (33, 20), (64, 24)])
 def test_wide_models_at_every_count_of_rows_match_the_full_model(flint, sequences, heads, int8):
     """Widths of 896 to 1,536 with 9 to 64 sequences: the linear kernels' longest shares of k, and
     normalised rows up to what shared memory holds (64 of 1,536: the sums then take their place)."""
