@@ -59,10 +59,19 @@ unsigned long long launch_count();
 // Launches `kernel` so that it may begin while the kernel before it in the stream
 // is still draining (programmatic dependent launch): its CTAs become resident as the
 // earlier kernel's CTAs retire, and its set-up (barrier initialisation, tensor-memory
-// allocation, index arithmetic) overlaps that tail. Every kernel launched this way
-// calls fb::dependency_wait() before its first access to global memory; the earlier
-// kernel allows the early start with fb::dependency_release(). FLINT_B200_PDL=0 in the
-// environment turns the attribute off (plain stream order). Counts the launch.
+// allocation, index arithmetic) overlaps that tail. FLINT_B200_PDL=0 in the environment turns
+// the attribute off (plain stream order). Counts the launch.
+//
+// What a kernel launched this way keeps to:
+//   - it calls fb::dependency_wait() before it reads or writes anything that an earlier kernel
+//     may have written or may still read, and reads such memory through fb::after_wait()
+//     pointers, volatile loads or bulk copies, never behind `const __restrict__` alone or __ldg;
+//   - it allows the next kernel's early start, fb::dependency_release(), only behind its own
+//     wait: when a kernel begins, all but the one right before it are then over.
+// The decode kernels (fb_decode_linear, fb_decode_head, fb_decode_attention) read weights, the
+// position and older cache rows before their wait. That is right only because the first kernel
+// of their chain is launched the ordinary way (fb_decode_embed of a step, fb_take_last_rows of a
+// prompt), so that whatever wrote those has finished before any of them begins.
 bool dependent_launch_enabled();
 
 template <typename... Params, typename... Args>

@@ -1405,6 +1405,7 @@ flint_status flint_b200_generator_prefill(flint_b200_generator* generator, const
     FB_TRY(flint_embedding_forward(g.x_a, tokens, g.wte, g.wpe, g.sequences, length, g.padded_vocab,
                                    g.width, stream));
     FB_TRY(run_prompt(g, length, stream));
+    // Launched the ordinary way: the kernel behind it reads weights before its wait.
     fb_take_last_rows<<<static_cast<unsigned>(g.sequences), 256, 0, stream>>>(
         g.last, g.x_a, static_cast<int>(length), static_cast<int>(g.width));
     FB_CUDA(fb::after_launch());

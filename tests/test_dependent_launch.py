@@ -75,3 +75,16 @@ def test_a_kernel_releases_the_next_one_behind_its_own_wait(parameters, body):
     # So that whatever a kernel depends on is over before the one after the next can begin.
     assert "dependency_release()" in body
     assert body.index("dependency_wait()") < body.index("dependency_release()")
+
+
+def test_kernels_that_read_before_their_wait_stand_behind_an_ordinary_launch():
+    """The decode kernels read weights, the position and older cache rows ahead of their wait: the
+    chain that they end has to begin with a launch that waits for everything before it."""
+    text = (SOURCES[0].parent / "generate.cu").read_text()
+    for function, first, then in (("enqueue_step", "fb_decode_embed", "run_token("),
+                                  ("flint_b200_generator_prefill", "fb_take_last_rows", "run_head(")):
+        body = text[re.search(rf"flint_status {function}\(", text).start():]
+        body = body[:body.index("\n}\n")]
+        assert f"{first}<<<" in body and body.index(f"{first}<<<") < body.index(then)
+        between = body[body.index(f"{first}<<<"):body.index(then)]
+        assert "launch_dependent" not in between
