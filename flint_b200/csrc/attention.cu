@@ -454,20 +454,20 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         const float scale2 = p.scale * kLog2e;
         const fb::F2 scale_pair = fb::f2_pack(scale2, scale2);
         uint32_t before = 0;   // key tiles of this CTA's earlier items
-        bool ok = true;
-        for (FwdCursor item = enter(0); ok && valid(item); item = enter(item.round + 1)) {
+        // No wait has given up. A thread whose wait did stays in the loops to their end, where it
+        // only stores nothing more: the other lanes meet it in warp-wide instructions, and the
+        // other warp of its rows at their barrier. (Its waits then end at once.)
+        bool there = true;
+        for (FwdCursor item = enter(0); valid(item); item = enter(item.round + 1)) {
             const int qb = item.qb;
             const int bh = head_of(item, tile);
             const bool stores = 2 * item.pair + tile < bh_count;
             const int q_index = qb * kTile + row;
             float m = -INFINITY;  // reference exponent of the row (base 2), shared by the pair
             fb::F2 l = 0;         // this thread's share of the row sum, in two partial sums
-            for (int j = 0; ok && j <= qb; ++j) {
+            for (int j = 0; j <= qb; ++j) {
                 const uint32_t n = 2 * (before + j) + tile;   // this step's number
-                if (!sm100::mbar_wait_warp(bar.s_full(n % 3), (n / 3) & 1, abort)) {
-                    ok = false;
-                    break;
-                }
+                there = sm100::mbar_wait(bar.s_full(n % 3), (n / 3) & 1, abort) && there;
                 const int parity = j & 1;
                 const uint32_t my_scores = tmem + 128u * (n % 3) + lane_base + half * 64;
                 sm100::tc_fence_after_sync();
@@ -515,10 +515,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 if (j > 0 && __any_sync(0xffffffffu, moved)) {
                     // The previous key tile's P V must have finished (it cannot be more than
                     // one behind: the next one needs this step's probabilities).
-                    if (!sm100::mbar_wait_warp(bar.pv_done(tile), (before + j - 1) & 1, abort)) {
-                        ok = false;
-                        break;
-                    }
+                    there = sm100::mbar_wait(bar.pv_done(tile), (before + j - 1) & 1, abort) && there;
                     sm100::tc_fence_after_sync();
                     const fb::F2 a2 = fb::f2_pack(alpha, alpha);
 #pragma unroll 1
@@ -569,20 +566,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 // last but one is awaited first, and here, before this warp's arrival lets the
                 // last one be issued at all (afterwards a slow warp could find both complete
                 // and wait for a parity that no longer comes).
-                if (j == qb && qb > 0 &&
-                    !sm100::mbar_wait_warp(bar.pv_done(tile), (before + qb - 1) & 1, abort)) {
-                    ok = false;
-                    break;
+                if (j == qb && qb > 0) {
+                    there = sm100::mbar_wait(bar.pv_done(tile), (before + qb - 1) & 1, abort) && there;
                 }
                 __syncwarp();
                 if (lane == 0) {
                     sm100::mbar_arrive(bar.p_ready(n % 3));
                 }
             }
-            if (!ok || !sm100::mbar_wait_warp(bar.pv_done(tile), (before + qb) & 1, abort)) {
-                ok = false;
-                break;
-            }
+            there = sm100::mbar_wait(bar.pv_done(tile), (before + qb) & 1, abort) && there;
             before += qb + 1;
             sm100::tc_fence_after_sync();
             uint32_t acc[32];
@@ -600,7 +592,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             quadrant_sync(pair_barrier);
             const float total = mine + pair_max[tile][parity][half ^ 1][row];
             quadrant_sync(pair_barrier);     // both have read before either writes a maximum there
-            if (stores && q_index < p.length) {
+            if (there && stores && q_index < p.length) {
                 const float inv = 1.0f / total;
                 const int head = bh % p.heads;
                 const int seq = bh / p.heads;

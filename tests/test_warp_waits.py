@@ -50,7 +50,7 @@ def test_lanes_of_a_warp_do_not_decide_for_themselves(source, name):
 
 
 @pytest.mark.parametrize("source, name, least", [("gemm.cu", "sm100::mbar_wait_warp", 2),
-                                                 ("attention.cu", "sm100::mbar_wait_warp", 14),
+                                                 ("attention.cu", "sm100::mbar_wait_warp", 11),
                                                  ("reductions.cu", "staged_wait_warp", 1)])
 def test_the_warps_waits_are_found(source, name, least):
     assert len(list(waits((CSRC / source).read_text(), name))) >= least
@@ -58,8 +58,18 @@ def test_the_warps_waits_are_found(source, name, least):
 
 def test_lanes_that_go_along_agree_before_the_next_step():
     text = (CSRC / "attention.cu").read_text()
-    loops = re.findall(r"bool there = .*?\n( *)ok = __all_sync\(0xffffffffu, there\);\n\1?\s*\}", text, re.S)
-    assert len(loops) == len(re.findall(r"\bbool there = ", text)) == 2
+    loops = re.findall(r"bool there = sm100.*?\n( *)ok = __all_sync\(0xffffffffu, there\);\n\1?\s*\}", text, re.S)
+    assert len(loops) == len(re.findall(r"\bbool there = sm100", text)) == 2
+
+
+def test_forward_softmax_warps_leave_their_loops_only_at_the_end():
+    """Two warps share the rows of a query tile and meet at a barrier without a limit."""
+    text = (CSRC / "attention.cu").read_text()
+    begin = text.index("bool there = true;")
+    loops = re.sub(r"//[^\n]*", "", text[begin:text.index("fb::dependency_release()", begin)])
+    assert loops.count("quadrant_sync(pair_barrier)") == 3
+    assert not re.search(r"\b(break|continue|return)\b", loops)
+    assert "if (there && stores" in loops
 
 
 @pytest.mark.parametrize("source, function", [("sm100.cuh", "mbar_wait_warp"), ("reductions.cu", "staged_wait_warp")])
