@@ -33,7 +33,11 @@ constexpr size_t kMaxRows8 = size_t{0x7fffffff} * 8;
 // ---- LayerNorm forward -----------------------------------------------------------
 
 // Rows of up to 128 * kQuads values with cols % 4 == 0: the warp holds the row
-// in registers, lane l owning float4 groups l, l + 32, ...
+// in registers, lane l owning float4 groups l, l + 32, ... kQuads is 2, 6, 12 or 13: up to 1,664
+// columns the registers still pay (4,096 x 1,664 9.9 us, 16,384 x 1,664 33.0; the streaming kernel
+// takes 12.8 and 43.6 for 1,668 columns), and 13 is apart from 12 so that 1,536 columns do
+// not pay for 1,600. (The backward kernel re-reads rows of over 1,536 columns: it would hold dy
+// and x, and with both in registers 4,096 x 1,600 took 87 us instead of 55.)
 // kPlain (the model on the fused attention kernels only; the public entry point never uses it):
 // the two row sums take ordinary FP32 adds in four interleaved streams and a butterfly,
 // deterministic and within a few 2^-24 of the compensated result, at a seventh of the
