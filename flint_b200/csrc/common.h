@@ -92,6 +92,30 @@ cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
     return e != cudaSuccess ? e : last;
 }
 
+// The same in clusters of `cluster` CTAs along x (up to 8).
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent_cluster(void (*kernel)(Params...), dim3 grid, dim3 block,
+                                     unsigned cluster, size_t smem, cudaStream_t stream,
+                                     Args&&... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = cluster;
+    attributes[0].val.clusterDim.y = 1;
+    attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = dependent_launch_enabled() ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+    const cudaError_t last = after_launch();
+    return e != cudaSuccess ? e : last;
+}
+
 // Raises a kernel's dynamic shared-memory limit once per device (the attribute belongs
 // to the device's copy of the function); `done` is the caller's static per-kernel table.
 // Host threads may race on a first call: the slots are atomics and the attribute call is

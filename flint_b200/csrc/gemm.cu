@@ -14,7 +14,9 @@
 // Tensor memory holds two accumulators, so the epilogue of tile i overlaps the
 // main loop of tile i+1. Every k-block is 64 wide for every layout, so all
 // variants of a shape add their products in the same order and the batched
-// forms reproduce the plain ones bit for bit.
+// forms reproduce the plain ones bit for bit. (Small outputs with a long k take their
+// sums in two or four parts, by a rule on the shape alone.) Large problems run on
+// CTA pairs (fb_gemm_pair), those of a single round on fb_gemm_once.
 //
 // Operand layouts map onto UMMA "major-ness" instead of register transposes:
 // NT reads both operands K-major, NN reads w (k x n) MN-major, TN reads both x
@@ -933,6 +935,539 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
 }
 
+// ---- one tile per CTA, k over a cluster -------------------------------------------------------
+//
+// For problems whose tiles all run at once. Nothing overlaps such a launch's last epilogue, and
+// a tile's k loop is the launch's time: 0.235 us per 64 of k for 64 columns, 0.265 / 0.305 /
+// 0.345 for 128 / 192 / 256, i.e. 58 to 76 bytes per clock into one SM, whatever the ring's
+// depth from three stages on and however many blocks an issue round takes; so this kernel
+//   - divides k over the 1, 2 or 4 CTAs of a cluster that share a tile. Each forms a partial
+//     tile and sends CTA r rows [128 r / c, 128 (r + 1) / c) of it, FP32, through distributed
+//     shared memory; CTA r adds them in cluster order, whoever came first, so a tile's bits
+//     do not depend on timing. (st.async into a box of its own, counted by an mbarrier, was
+//     0.4 us faster than staging and bulk copies; either moves about 20 bytes per clock.)
+//     NN 256 x 768 x 3,072: 13.7 -> 7.9 us, 64 x 1,600 x 6,400: 25.1 -> 10.9,
+//     1,000 x 768 x 3,072: 14.7 -> 11.5;
+//   - has sixteen epilogue warps, four per scheduler: with eight, a tile's last chunks of 32
+//     columns cost 1.4 us each in a biased or element-wise epilogue, mostly latency
+//     (bias+GELU 1,000 x 3,072 x 768: 12.4 -> 10.1 us, with 192 columns a tile);
+//   - stores its rows straight from registers (see store_row): NN 256 x 768 x 768, 64 columns,
+//     5.64 -> 5.54 us, in clusters of two 5.65 -> 5.25.
+// The accumulator is not double-buffered. Where the shape's sums are taken in parts (see
+// sum_parts) but a cluster is not wanted, one CTA forms the same partial sums in as many
+// accumulators.
+
+constexpr int kOnceWarps = 16;   // warp 0 loads and warp 1 issues MMAs before their share of the epilogue
+constexpr int kOnceThreads = 32 * kOnceWarps;
+constexpr int kOnceMostStages = 8;
+
+// Shared memory: the ring, whose memory is later the staging of sums and outputs, then what the
+// other CTAs of the cluster send, then the barriers.
+template <int BN>
+struct OnceRing {
+    static constexpr int kStageA = kBM * kBK * 2;
+    static constexpr int kStageB = BN * kBK * 2;
+    static constexpr int kStage = kStageA + kStageB;
+    // 32 x 32 chunks of 4 KB: those of the CTA's own rows, and those that a CTA sends or gets.
+    static constexpr int own(int cluster) { return BN / 32 * 4 / cluster; }
+    static constexpr int received(int cluster) { return own(cluster) * (cluster - 1); }
+    static constexpr int stages(int cluster) {
+        const int fit = (216 * 1024 - received(cluster) * 4096) / kStage;
+        return fit < kOnceMostStages ? fit : kOnceMostStages;
+    }
+    static constexpr int bytes(int cluster) {
+        return stages(cluster) * kStage + received(cluster) * 4096 + 1024 + 256;
+    }
+};
+
+// 16 bytes to another CTA of the cluster, whose mbarrier counts them as they arrive.
+__device__ __forceinline__ void send_to_cta(uint32_t cluster_dst, const uint32_t* v,
+                                            uint32_t cluster_bar) {
+    asm volatile(
+        "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+        ::"r"(cluster_dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(cluster_bar)
+        : "memory");
+}
+
+// ---- output rows straight from registers ----
+//
+// A lane's 32 columns of its row are 64 bytes (FP16) or 128 (FP32): whole sectors, so they
+// need no trip through shared memory. Where nothing overlaps the epilogue that trip's fence,
+// copy and wait cost more than the scattered rows do.
+
+template <int W>
+__device__ __forceinline__ void store_words(void* at, const uint32_t* w) {
+    if constexpr (W == 8) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(at), "r"(w[0]),
+                     "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                     : "memory");
+    } else {
+        *reinterpret_cast<uint4*>(at) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// `bytes_valid` of the row's 64 or 128 bytes are inside the matrix (a multiple of 16).
+template <int kWords>
+__device__ __forceinline__ void store_row(void* at, const uint32_t (&w)[kWords], int bytes_valid,
+                                          bool wide) {
+    unsigned char* out = static_cast<unsigned char*>(at);
+    if (wide) {
+#pragma unroll
+        for (int i = 0; i < kWords; i += 8) {
+            if (i * 4 < bytes_valid) {
+                store_words<8>(out + i * 4, w + i);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kWords; i += 4) {
+            if (i * 4 < bytes_valid) {
+                store_words<4>(out + i * 4, w + i);
+            }
+        }
+    }
+}
+
+// The second operand of a lane's row segment: the residual, the old value or the saved
+// pre-activation (see Aux), in row order.
+template <Epilogue E>
+__device__ __forceinline__ void load_row_aux(Aux<E>& aux, const GemmParams& p, size_t at, int valid) {
+    if constexpr (E == Epilogue::kBiasResidual || E == Epilogue::kTnStore) {
+        const float* old = E == Epilogue::kBiasResidual ? static_cast<const float*>(p.aux_in) + at
+                                                        : static_cast<const float*>(p.y) + at;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            aux.q[i] = i * 4 < valid ? *reinterpret_cast<const uint4*>(old + i * 4)
+                                     : make_uint4(0u, 0u, 0u, 0u);
+        }
+    } else if constexpr (E == Epilogue::kDGelu) {
+        const __half* pre = static_cast<const __half*>(p.aux_in) + at;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            aux.q[i] = i * 8 < valid ? *reinterpret_cast<const uint4*>(pre + i * 8)
+                                     : make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+}
+
+// The epilogue of a lane's row segment: 32 sums from column `col` on, `at` its first element.
+// The arithmetic is store_chunk's.
+template <Epilogue E>
+__device__ __forceinline__ void finish_row(const GemmParams& p, bool wide, size_t at, float (&acc)[32], int valid,
+                                           bool inside, const Aux<E>& aux, float bias_lane) {
+    if constexpr (E == Epilogue::kBias || E == Epilogue::kBiasGelu || E == Epilogue::kBiasResidual) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            acc[j] = __fadd_rn(acc[j], __shfl_sync(0xffffffffu, bias_lane, j));
+        }
+    }
+    if (!inside) {
+        return;
+    }
+    if constexpr (E == Epilogue::kScale) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            acc[j] = __fmul_rn(acc[j], p.scale);
+        }
+    }
+    if constexpr (E == Epilogue::kBiasResidual || E == Epilogue::kTnStore) {
+        if (E == Epilogue::kBiasResidual || p.accumulate) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                acc[4 * i] = __fadd_rn(__uint_as_float(aux.q[i].x), acc[4 * i]);
+                acc[4 * i + 1] = __fadd_rn(__uint_as_float(aux.q[i].y), acc[4 * i + 1]);
+                acc[4 * i + 2] = __fadd_rn(__uint_as_float(aux.q[i].z), acc[4 * i + 2]);
+                acc[4 * i + 3] = __fadd_rn(__uint_as_float(aux.q[i].w), acc[4 * i + 3]);
+            }
+        }
+        uint32_t words[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            words[j] = __float_as_uint(acc[j]);
+        }
+        store_row(static_cast<float*>(p.y) + at, words, valid * 4, wide);
+    } else {
+        if constexpr (E == Epilogue::kDGelu) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const unsigned w[4] = {aux.q[c].x, aux.q[c].y, aux.q[c].z, aux.q[c].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float lo = half_bits_to_float(static_cast<unsigned short>(w[j]));
+                    const float hi = half_bits_to_float(static_cast<unsigned short>(w[j] >> 16));
+                    float g0, g1;
+                    fb::f2_unpack(gelu_tanh_grad2(fb::f2_pack(lo, hi)), g0, g1);
+                    acc[c * 8 + 2 * j] = __fmul_rn(acc[c * 8 + 2 * j], g0);
+                    acc[c * 8 + 2 * j + 1] = __fmul_rn(acc[c * 8 + 2 * j + 1], g1);
+                }
+            }
+        }
+        uint32_t words[16];
+        auto pack = [&]() {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const __half2 h = __floats2half2_rn(acc[2 * j], acc[2 * j + 1]);
+                words[j] = *reinterpret_cast<const unsigned*>(&h);
+            }
+        };
+        pack();
+        if constexpr (E == Epilogue::kBiasGelu) {
+            store_row(static_cast<__half*>(p.aux_out) + at, words, valid * 2, wide);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                fb::f2_unpack(gelu_tanh2(fb::f2_pack(acc[2 * j], acc[2 * j + 1])), acc[2 * j],
+                              acc[2 * j + 1]);
+            }
+            pack();
+        }
+        store_row(static_cast<__half*>(p.y) + at, words, valid * 2, wide);
+    }
+}
+
+struct OnceParams {
+    GemmParams gemm;
+    int cluster;    // CTAs that share a tile and divide its k
+    int parts;      // accumulators of one CTA, each for a part of k
+    int stages;     // of the operand ring
+    int wide_out;   // every row segment of the output is 32-byte aligned
+};
+
+// kParted: k is taken in parts, by a cluster or one after another.
+template <Layout L, Epilogue E, int BN, bool kParted>
+__global__ void __launch_bounds__(kOnceThreads, 1)
+    fb_gemm_once(const __grid_constant__ OnceParams once) {
+    const GemmParams& p = once.gemm;
+    using R = OnceRing<BN>;
+    constexpr bool kAMn = L == Layout::kTN;
+    constexpr bool kBMn = L != Layout::kNT;
+    constexpr uint32_t kIdesc = sm100::instr_desc_f16(kBM, BN, kAMn, kBMn);
+    constexpr int kChunks = BN / 32;   // per 32 rows
+
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t smem_base = (sm100::smem_u32(smem_raw) + 1023u) & ~1023u;
+    const int cluster = kParted ? once.cluster : 1;
+    const int rank = cluster > 1 ? static_cast<int>(sm100::cluster_cta_rank()) : 0;
+    const int quadrants = 4 / cluster;          // of 32 rows that this CTA finishes
+    const int total = quadrants * kChunks;      // their chunks
+    const int stages = once.stages;
+    const int parts = kParted ? once.parts : 1;   // of this CTA's blocks of k, each with an accumulator of its own
+    const uint32_t tmem_columns = parts * BN <= 64 ? 64 : parts * BN <= 128 ? 128 : parts * BN <= 256 ? 256 : 512;
+    const uint32_t inbox = smem_base + static_cast<uint32_t>(stages) * R::kStage;
+    const uint32_t bars = inbox + static_cast<uint32_t>(total * (cluster - 1)) * 4096u;
+    auto full_bar = [&](int s) { return bars + 8u * s; };
+    auto empty_bar = [&](int s) { return bars + 8u * (kOnceMostStages + s); };
+    const uint32_t acc_full_bar = bars + 16u * kOnceMostStages;
+    const uint32_t inbox_bar = acc_full_bar + 8u;
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+
+    const int warp = threadIdx.x / 32;
+    const int lane = threadIdx.x % 32;
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < stages; ++s) {
+            sm100::mbar_init(full_bar(s), 1);
+            sm100::mbar_init(empty_bar(s), 1);
+        }
+        sm100::mbar_init(acc_full_bar, 1);
+        sm100::mbar_init(inbox_bar, 1);
+        sm100::mbar_fence_init();
+        sm100::tma_prefetch_descriptor(&p.map_a);
+        sm100::tma_prefetch_descriptor(&p.map_b);
+    }
+    if (warp == 1) {
+        sm100::tmem_alloc(sm100::smem_u32(&tmem_base_slot), tmem_columns);
+    }
+    sm100::tc_fence_before_sync();
+    __syncthreads();
+    if (cluster > 1) {
+        // Every CTA's barriers exist before another one signals them.
+        if (threadIdx.x == 0) {
+            sm100::mbar_expect_tx(inbox_bar, static_cast<uint32_t>(total * (cluster - 1)) * 4096u);
+        }
+        sm100::cluster_sync_all();
+    }
+    sm100::tc_fence_after_sync();
+    const uint32_t tmem_base = tmem_base_slot;
+    volatile int* abort = &abort_flag;
+
+    const TileCoord t = decode_tile(p, blockIdx.x / cluster);
+    // This CTA's share of the blocks of k.
+    const int all_blocks = (p.k + kBK - 1) / kBK;
+    const int block0 = all_blocks * rank / cluster;
+    const int blocks = all_blocks * (rank + 1) / cluster - block0;
+    const int k0 = block0 * kBK;
+
+    // Everything above ran while the previous kernel in the stream may still have been
+    // finishing; global memory is touched only from here on.
+    fb::dependency_wait();
+    if (threadIdx.x == 0) {
+        fb::dependency_release();
+    }
+
+    if (warp == 0) {
+        // ---- TMA producer ----
+        if (lane == 0) {
+            int stage = 0;
+            uint32_t phase = 0;
+            const int batch = p.batched ? static_cast<int>(t.z) : 0;
+            const int row_a = t.tm * kBM;
+            const int row_b = t.tn * BN;
+            for (int i = 0; i < blocks; ++i) {
+                const int kk = k0 + i * kBK;
+                if (!sm100::mbar_wait(empty_bar(stage), phase ^ 1u, abort)) {
+                    break;
+                }
+                const uint32_t a_dst = smem_base + stage * R::kStage;
+                const uint32_t b_dst = a_dst + R::kStageA;
+                const uint32_t bar = full_bar(stage);
+                sm100::mbar_expect_tx(bar, R::kStage);
+                if constexpr (!kAMn) {
+                    if (p.batched) {
+                        sm100::tma_load_3d(a_dst, &p.map_a, bar, kk, row_a, batch);
+                    } else {
+                        sm100::tma_load_2d(a_dst, &p.map_a, bar, kk, row_a);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < kBM / 64; ++j) {
+                        if (p.batched) {
+                            sm100::tma_load_3d(a_dst + j * 8192, &p.map_a, bar, row_a + 64 * j, kk,
+                                               batch);
+                        } else {
+                            sm100::tma_load_2d(a_dst + j * 8192, &p.map_a, bar, row_a + 64 * j, kk);
+                        }
+                    }
+                }
+                if constexpr (!kBMn) {
+                    if (p.batched) {
+                        sm100::tma_load_3d(b_dst, &p.map_b, bar, kk, row_b, batch);
+                    } else {
+                        sm100::tma_load_2d(b_dst, &p.map_b, bar, kk, row_b);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < BN / 64; ++j) {
+                        if (p.batched) {
+                            sm100::tma_load_3d(b_dst + j * 8192, &p.map_b, bar, row_b + 64 * j, kk,
+                                               batch);
+                        } else {
+                            sm100::tma_load_2d(b_dst + j * 8192, &p.map_b, bar, row_b + 64 * j, kk);
+                        }
+                    }
+                }
+                if (++stage == stages) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---- MMA issuer: warp-uniform, one elected lane issues (see fb_gemm_tc) ----
+        int stage = 0;
+        uint32_t phase = 0;
+        bool alive = true;   // the elected lane's: its waits have not given up
+        uint32_t accumulate = 0;
+        uint32_t d_tmem = tmem_base;
+        int part = 0;
+        int part_end = blocks / parts;   // (parts > 1 only with the whole of k: cluster == 1)
+        for (int i = 0; i < blocks; ++i) {
+            if (i == part_end) {
+                ++part;
+                part_end = blocks * (part + 1) / parts;
+                d_tmem += BN;
+                accumulate = 0;
+            }
+            const uint32_t a_addr = smem_base + stage * R::kStage;
+            const uint32_t b_addr = a_addr + R::kStageA;
+            const uint64_t a_desc = kAMn ? sm100::smem_desc_sw128(a_addr, 8192, 1024)
+                                         : sm100::smem_desc_sw128(a_addr, 16, 1024);
+            const uint64_t b_desc = kBMn ? sm100::smem_desc_sw128(b_addr, 8192, 1024)
+                                         : sm100::smem_desc_sw128(b_addr, 16, 1024);
+            if (sm100::elect_one()) {
+                alive = alive && sm100::mbar_wait(full_bar(stage), phase, abort);
+                if (alive) {
+                    sm100::tc_fence_after_sync();
+                    sm100::mma_f16_ss_at<-1>(d_tmem, a_desc, 0, b_desc, 0, kIdesc, accumulate);
+#pragma unroll
+                    for (int ks = 1; ks < kBK / 16; ++ks) {
+                        sm100::mma_f16_ss_at<1>(d_tmem, a_desc, ks * (kAMn ? 128 : 2), b_desc,
+                                                ks * (kBMn ? 128 : 2), kIdesc);
+                    }
+                    sm100::mma_commit(empty_bar(stage));
+                    if (i + 1 == blocks) {
+                        sm100::mma_commit(acc_full_bar);
+                    }
+                }
+            }
+            accumulate = 1;
+            if (++stage == stages) {
+                stage = 0;
+                phase ^= 1u;
+            }
+        }
+    }
+    __syncwarp();
+    // ---- epilogue, by every warp ----
+    {
+        const int quadrant = warp % 4;   // the TMEM lanes this warp may read
+        const int part = warp / 4;       // which of every four chunks of the quadrant's rows
+        const int row_tile = t.tm * kBM;
+        const int col0 = t.tn * BN;
+        const size_t batch_offset =
+            p.batched ? static_cast<size_t>(t.z) * p.m * static_cast<size_t>(p.n) : 0;
+        const bool coalesced = chunk_path_ok<E>(p);
+        // The chunks this warp finishes: chunk `work` of the CTA's rows, then every sixteenth.
+        // With one CTA to a tile a warp has its own quadrant's, so that they come straight from
+        // tensor memory; from shared memory any warp may take any.
+        auto chunk_at = [&](int work, int& row, int& column) {
+            if (cluster == 1) {
+                row = quadrant;
+                column = work / 4;       // work = 4 * column + quadrant's place
+            } else {
+                row = rank * quadrants + work / kChunks;
+                column = work % kChunks;
+            }
+        };
+        const int first = warp;
+        Aux<E> aux;
+        float bias_lane = 0.0f;
+        // A chunk's second operands, asked for ahead of its sums.
+        auto request = [&](int work) {
+            int row, column;
+            chunk_at(work, row, column);
+            const int col = col0 + column * 32;
+            const size_t mine = static_cast<size_t>(row_tile) + row * 32 + lane;
+            if (p.n - col > 0) {
+                if (aux_slots<E>() > 1 && coalesced && mine < static_cast<size_t>(p.m) &&
+                    (E != Epilogue::kTnStore || p.accumulate)) {
+                    load_row_aux<E>(aux, p, batch_offset + mine * p.n + col, min(32, p.n - col));
+                }
+                bias_lane = load_bias_lane<E>(p, col, lane);
+            }
+        };
+        if (first < total) {
+            request(first);
+        }
+        bool there = sm100::mbar_wait_warp(acc_full_bar, 0, abort);
+        sm100::tc_fence_after_sync();
+        const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quadrant * 32) << 16);
+        if (cluster > 1) {
+            // All 128 rows' chunks go to their owners; this CTA's own to the ring's memory. (The
+            // MMAs have read their operands, and no more are on the way.)
+            const int owner = quadrant / quadrants;
+            const int place = quadrant % quadrants * kChunks;   // of the quadrant, among its owner's
+            if (there) {
+#pragma unroll 1
+                for (int c = part; c < kChunks; c += 4) {
+                    uint32_t raw[32];
+                    sm100::tmem_ld_32x32(t_addr + c * 32, raw);
+                    sm100::tmem_ld_wait();
+                    const uint32_t offset = static_cast<uint32_t>(place + c) * 4096u + lane * 16u;
+                    if (owner == rank) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            st_shared_v4(smem_base + offset + j * 512u,
+                                         make_uint4(raw[4 * j], raw[4 * j + 1], raw[4 * j + 2], raw[4 * j + 3]));
+                        }
+                    } else {
+                        const uint32_t slot = static_cast<uint32_t>((rank - (rank > owner ? 1 : 0)) * total) * 4096u;
+                        const uint32_t to = sm100::map_to_cta(inbox + slot + offset, static_cast<uint32_t>(owner));
+                        const uint32_t bar = sm100::map_to_cta(inbox_bar, static_cast<uint32_t>(owner));
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            send_to_cta(to + j * 512u, raw + 4 * j, bar);
+                        }
+                    }
+                }
+            }
+            // The CTA's own chunks are there for any warp to read; so are, then, the others'.
+            __syncthreads();
+            there = sm100::mbar_wait_warp(inbox_bar, 0, abort) && there;
+        }
+        if (there) {
+#pragma unroll 1
+            for (int work = first; work < total; work += kOnceWarps) {
+                int row32, column;
+                chunk_at(work, row32, column);
+                const int col = col0 + column * 32;
+                const int valid = min(32, p.n - col);
+                if (work != first) {
+                    request(work);
+                }
+                float v[32];
+                if constexpr (!kParted) {
+                    uint32_t raw[32];
+                    sm100::tmem_ld_32x32(t_addr + column * 32, raw);
+                    sm100::tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        v[j] = __uint_as_float(raw[j]);
+                    }
+                } else {
+                    // The partial sums in the order of k.
+                    const int sums = cluster == 1 ? parts : cluster;
+#pragma unroll 1
+                    for (int r = 0; r < sums; ++r) {
+                        uint32_t raw[32];
+                        if (cluster == 1) {
+                            sm100::tmem_ld_32x32(t_addr + r * BN + column * 32, raw);
+                            sm100::tmem_ld_wait();
+                        } else {
+                            const int place = r == rank ? work : (r - (r > rank ? 1 : 0)) * total + work;
+                            const uint32_t from =
+                                (r == rank ? smem_base : inbox) + static_cast<uint32_t>(place) * 4096u + lane * 16u;
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                const uint4 q = ld_shared_v4(from + j * 512u);
+                                raw[4 * j] = q.x;
+                                raw[4 * j + 1] = q.y;
+                                raw[4 * j + 2] = q.z;
+                                raw[4 * j + 3] = q.w;
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            const float sum = __uint_as_float(raw[j]);
+                            v[j] = r == 0 ? sum : __fadd_rn(v[j], sum);
+                        }
+                    }
+                }
+                const size_t row = static_cast<size_t>(row_tile) + row32 * 32 + lane;
+                if (valid > 0) {
+                    const bool inside = row < static_cast<size_t>(p.m);
+                    if (coalesced) {
+                        finish_row<E>(p, once.wide_out != 0, batch_offset + row * p.n + col, v, valid, inside, aux, bias_lane);
+                    } else if (inside) {
+                        store_segment<E>(p, batch_offset, t.z, row, col, v, valid);
+                    }
+                }
+            }
+        }
+    }
+
+    // ---- teardown: no CTA leaves while another may still write to its shared memory ----
+    __syncthreads();
+    if (cluster > 1) {
+        sm100::cluster_sync_all();
+    }
+    if (abort_flag != 0) {
+        if (threadIdx.x == 0) {
+            atomicExch(&g_gemm_error, 1);
+        }
+        // Let any copy still in flight land before shared memory is released.
+        const long long start = clock64();
+        while (clock64() - start < 2000000LL) {
+        }
+        __syncthreads();
+    }
+    if (warp == 1) {
+        sm100::tc_fence_after_sync();
+        sm100::tmem_dealloc(tmem_base, tmem_columns);
+    }
+}
+
 // ---- the CTA-pair kernel: 256 x 256 tiles --------------------------------------------------
 //
 // Two CTAs of a cluster work on one 256 x 256 output tile with
@@ -948,8 +1483,6 @@ constexpr int kPairBN = 256;
 constexpr int kPairStageA = kBM * kBK * 2;          // 16 KB
 constexpr int kPairStageB = 128 * kBK * 2;          // 16 KB: half of the 256 B rows
 constexpr int kPairStage = kPairStageA + kPairStageB;
-constexpr int kPairStages = kRingBytes / kPairStage;  // 6
-constexpr int kPairSmemBytes = kPairStages * kPairStage + kEpilogueWarps * 4096 + 1024 + 256;
 constexpr int kPairGroupM = 4;  // rows of 256-row tiles handed out together
 
 __device__ __forceinline__ TileCoord decode_pair_tile(const GemmParams& p, long long id) {
@@ -967,20 +1500,26 @@ __device__ __forceinline__ TileCoord decode_pair_tile(const GemmParams& p, long 
     return c;
 }
 
-// Epilogue warps per CTA of the pair kernel: two per TMEM lane quadrant, 4 KB of
-// staging each. (Four per quadrant were measured for the element-wise FP16
-// epilogues and were slower: 96 registers per thread spill.)
-template <Epilogue E>
-__host__ __device__ constexpr int pair_epilogue_warps() {
-    return 8;
+// Epilogue warps per CTA of the pair kernel, with 4 KB of staging each: two per TMEM lane
+// quadrant, and four for bias+GELU over a short k. Those warps mostly wait (with eight, 28 % of the
+// issue slots and 30 % of the special-function unit are in use), and at k = 768 a tile's epilogue
+// outlasts its k loop: 8,192 x 3,072 x 768 44.0 -> 41.9 us, 16,384 rows 82.5 -> 78.9, for a stage
+// of the ring. At k = 1,600 the loop is the longer one: 4,096 x 6,400 68.9 -> 71.6. (Four for dGELU
+// 51.4 -> 59 us, which then has no registers to ask for its pre-activations a chunk ahead; for
+// bias+residual 42 -> 45.)
+constexpr int kManyWarps = 16;
+constexpr size_t kManyWarpsMostK = 1024;
+__host__ __device__ constexpr int pair_stages(int epilogue_warps) { return epilogue_warps == 8 ? 6 : 5; }
+__host__ __device__ constexpr int pair_smem_bytes(int epilogue_warps) {
+    return pair_stages(epilogue_warps) * kPairStage + epilogue_warps * 4096 + 1024 + 256;
 }
 
-template <Layout L, Epilogue E>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilogue_warps<E>(), 1)
+template <Layout L, Epilogue E, int kEpi>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * kEpi, 1)
     fb_gemm_pair(const __grid_constant__ GemmParams p) {
-    constexpr int kEpi = pair_epilogue_warps<E>();
+    constexpr int kStages = pair_stages(kEpi);
     constexpr int kColumnStep = 32 * (kEpi / 4);            // between a warp's chunks
-    constexpr uint32_t kSlotBytes = kEpilogueWarps * 4096 / kEpi;
+    constexpr uint32_t kSlotBytes = 4096;
     constexpr bool kAMn = L == Layout::kTN;
     constexpr bool kBMn = L != Layout::kNT;
     constexpr bool kIsTn = L == Layout::kTN;
@@ -989,12 +1528,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
 
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem_base = (sm100::smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t staging = smem_base + kPairStages * kPairStage;
-    const uint32_t bars = staging + kEpilogueWarps * 4096;
+    const uint32_t staging = smem_base + kStages * kPairStage;
+    const uint32_t bars = staging + kEpi * 4096;
     auto full_bar = [&](int s) { return bars + 8u * s; };
-    auto empty_bar = [&](int s) { return bars + 8u * (kPairStages + s); };
-    auto acc_full_bar = [&](int a) { return bars + 8u * (2 * kPairStages + a); };
-    auto acc_empty_bar = [&](int a) { return bars + 8u * (2 * kPairStages + 2 + a); };
+    auto empty_bar = [&](int s) { return bars + 8u * (kStages + s); };
+    auto acc_full_bar = [&](int a) { return bars + 8u * (2 * kStages + a); };
+    auto acc_empty_bar = [&](int a) { return bars + 8u * (2 * kStages + 2 + a); };
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
@@ -1007,7 +1546,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
-        for (int s = 0; s < kPairStages; ++s) {
+        for (int s = 0; s < kStages; ++s) {
             sm100::mbar_init(full_bar(s), 1);
             sm100::mbar_init(empty_bar(s), 1);
         }
@@ -1098,7 +1637,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
                             }
                         }
                     }
-                    if (++stage == kPairStages) {
+                    if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1u;
                     }
@@ -1144,7 +1683,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
                         }
                     }
                     accumulate = 1;
-                    if (++stage == kPairStages) {
+                    if (++stage == kStages) {
                         stage = 0;
                         phase ^= 1u;
                     }
@@ -1204,7 +1743,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
             // The epilogues with second operands already hold a chunk of those ahead; a
             // second accumulator set in flight as well would not fit in registers.
             constexpr bool kPipelined =
-                !(E == Epilogue::kBiasResidual || E == Epilogue::kTnStore ||
+                !(E == Epilogue::kBiasResidual || kEpi == kManyWarps || E == Epilogue::kTnStore ||
                   E == Epilogue::kTnPartial || E == Epilogue::kDGelu);
             uint32_t raw[2][32];
             auto chunk_column = [&](int i) { return column_part * 32 + i * kColumnStep; };
@@ -1212,7 +1751,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * pair_epilo
             if (kPipelined && chunk_valid(0) > 0) {
                 sm100::tmem_ld_32x32(t_addr + chunk_column(0), raw[0]);
             }
-#pragma unroll
+#pragma unroll (kEpi == kManyWarps ? 1 : 64)
             for (int i = 0; i < kChunks; ++i) {
                 const bool last = i + 1 == kChunks;
                 const int c = chunk_column(i);
@@ -1499,22 +2038,32 @@ bool pair_disabled() {
     return cached == 1;
 }
 
-// ---- which tile a problem gets ---------------------------------------------------------------
+// ---- which kernel and tile a problem gets ----------------------------------------------------
 //
 // The pair kernel's 256 x 256 tiles move the fewest bytes per FLOP and win wherever they fill
 // the GPU more than twice. Below that a problem is a few rounds of tiles at most, and its
 // time is what one SM spends: the k loop of a tile, which costs about the same per 64 of k
-// for every width up to 128 (0.24-0.26 us; 0.28 for a pair, 0.34 for 128 x 256), and the
-// epilogue, which grows with the tile's columns. So small problems take the narrowest tile
-// that still fits one round. Measured in a chain of launches, pair -> chosen: bias+residual
-// 1,000 x 768 x 768 12.3 -> 6.2 us, x 3,072 22.6 -> 14.8; NN 1,000 x 768 x 3,072 18.2 -> 14.3,
-// 2,048 x 768 x 3,072 18.4 -> 16.5; bias 1,000 x 2,304 x 768 9.3 -> 7.4; TN 3,072 x 768 x 1,000
-// 12.4 -> 9.8; bias+GELU 500 x 3,072 x 768 11.6 -> 9.5. The estimate below reproduces the
-// measured times of 64 to 8,192 rows (widths 768 to 3,072) to about 15 %.
+// for every width up to 128, and the epilogue, which grows with the tile's columns. So small
+// problems take the narrowest tile that still fits one round, on fb_gemm_once, and divide long
+// k loops over clusters. The estimates below reproduce the measured times of 64 to 8,192 rows (widths
+// 256 to 1,600; 1,900 timings of fb_gemm_once) to about 15 %; against the best of all tiles, the choice
+// lost 5 % or less nearly everywhere.
 
-enum class Tile { k64, k128, k256, kPair };
+enum class Tile { k64, k128, k256, kPair, kOnce64, kOnce128, kOnce192 };
 
-int tile_columns(Tile t) { return t == Tile::k64 ? 64 : t == Tile::k128 ? 128 : 256; }
+struct Plan {
+    Tile tile;
+    int cluster;   // CTAs over which fb_gemm_once divides k
+    int parts;     // or its accumulators
+    int splits;    // TN: pieces of k with partial sums in the workspace
+};
+
+int tile_columns(Tile t) {
+    constexpr int kColumns[] = {64, 128, 256, 256, 64, 128, 192};
+    return kColumns[static_cast<int>(t)];
+}
+
+constexpr Tile kOnceTiles[] = {Tile::kOnce64, Tile::kOnce128, Tile::kOnce192};
 
 // Microseconds that all tiles have alike, and per 32-column chunk of an epilogue warp: when
 // it is the last thing a launch does, and when it runs beside the next tile's k loop (the
@@ -1558,18 +2107,72 @@ long long tile_count(Tile t, size_t m, size_t n) {
     return static_cast<long long>((m + rows - 1) / rows) * static_cast<long long>((n + columns - 1) / columns);
 }
 
-// Whether a shape can use a tile at all: no tile whose second half would be empty.
+// Whether a shape can use a tile at all: no tile whose last 64 (of 256: 128) columns would be empty.
 bool tile_fits(Tile t, size_t m, size_t n) {
     switch (t) {
     case Tile::k64:
+    case Tile::kOnce64:
         return true;
     case Tile::k128:
+    case Tile::kOnce128:
         return n > 64;
-    case Tile::k256:
-        return n > 128;
-    default:
+    case Tile::kPair:
         return !pair_disabled() && m > 128 && n > 128;
+    default:
+        return n > 128;
     }
+}
+
+// fb_gemm_once: microseconds, or 0 where the CTAs would not run at once (a batch of products taken
+// in parts has no other kernel, and may run in rounds) or the tile cannot be used. Of clusters of
+// four, 33 fit this GPU's 148 SMs: a processing cluster of SMs holds whole ones only.
+double once_time(Tile t, Layout l, Epilogue e, size_t m, size_t n, size_t k, long long batches,
+                 int cluster, int parts, int sms) {
+    const int i = static_cast<int>(t) - static_cast<int>(Tile::kOnce64);
+    const size_t blocks = (k + kBK - 1) / kBK;
+    const long long ctas = tile_count(t, m, n) * batches * cluster;
+    const bool at_once = ctas <= (cluster == 4 ? sms * 8 / 9 : sms);
+    if (!tile_fits(t, m, n) || parts * tile_columns(t) > 512 || (!at_once && parts == 1)) {
+        return 0.0;
+    }
+    constexpr double kBlock[2][3] = {{0.235, 0.265, 0.305}, {0.285, 0.335, 0.37}};
+    // Everything but the k loop, with up to half of the SMs and with more of them at work.
+    const int busy = ctas > sms / 2;
+    constexpr double kNone[3][2] = {{2.3, 3.0}, {2.9, 3.8}, {3.3, 4.6}}, kBias[3][2] = {{2.6, 3.0}, {3.1, 3.9}, {3.9, 4.6}},
+                     kGelu[3][2] = {{3.3, 3.8}, {4.1, 5.0}, {5.4, 6.2}}, kDGelu[3][2] = {{3.4, 3.8}, {4.6, 5.1}, {6.9, 7.7}},
+                     kResidual[3][2] = {{3.3, 3.9}, {4.5, 5.4}, {6.7, 8.9}}, kTn[3][2] = {{2.6, 3.2}, {3.3, 4.2}, {4.6, 5.4}};
+    const double(*rest)[2] = kNone;
+    double more = 0.0;   // than a plain epilogue takes in a cluster, where no warp finishes two chunks
+    switch (e) {
+    case Epilogue::kBias:
+        rest = kBias;
+        more = 0.1;
+        break;
+    case Epilogue::kBiasGelu:
+        rest = kGelu;
+        more = 0.5;
+        break;
+    case Epilogue::kDGelu:
+        rest = kDGelu;
+        more = 0.7;
+        break;
+    case Epilogue::kBiasResidual:
+        rest = kResidual;
+        more = 0.3;
+        break;
+    case Epilogue::kTnStore:
+    case Epilogue::kTnPartial:
+        rest = kTn;
+        more = 0.2;
+        break;
+    default:
+        break;
+    }
+    // The same in clusters of two and four, the exchange of partial sums included.
+    constexpr double kCluster[2][3][2] = {{{4.0, 5.0}, {4.8, 6.1}, {5.7, 7.0}}, {{4.4, 5.5}, {5.2, 6.5}, {6.3, 7.8}}};
+    const double one = (cluster > 1 ? kCluster[cluster / 4][i][busy] + more : rest[i][busy]) +
+                       kBlock[l == Layout::kTN][i] * static_cast<double>((blocks + cluster - 1) / cluster);
+    return one * static_cast<double>((ctas + sms - 1) / sms);
 }
 
 // How often TN may split k with tile `t`: into pieces of at least 1,024, and not at all where
@@ -1584,59 +2187,105 @@ int most_splits(Tile t, size_t m, size_t n, size_t k, int sms) {
     return static_cast<int>(std::min<size_t>(16, std::max<size_t>(1, k / 1024)));
 }
 
-// The tile for `batches` problems of one shape; *splits (TN, or null) is how often k is split,
-// whose partial sums cost a second launch that reads and adds them.
-Tile pick_tile(Layout l, Epilogue e, size_t m, size_t n, size_t k, long long batches, int sms,
-               int* splits) {
-    constexpr Tile kTiles[] = {Tile::kPair, Tile::k256, Tile::k128, Tile::k64};
-    Tile chosen = Tile::k64;
+// In how many parts an output's sum over k is taken, each part's sum in order and then the parts'
+// sums in order. A function of the shape alone, so that every form of a product (NT, NN, TN without a
+// workspace, biased, batched) rounds the same sums: what suits the plain NT product. Products a head
+// wide are left whole, because those come in batches that fill the GPU by themselves.
+int sum_parts(size_t m, size_t n, size_t k, int sms) {
+    if (n < 256 || k < 512) {
+        return 1;
+    }
     double best = 0.0;
-    for (Tile t : kTiles) {
+    for (Tile t : {Tile::kPair, Tile::k256, Tile::k128, Tile::k64}) {
+        if (tile_fits(t, m, n)) {
+            const double time = tile_time(t, Layout::kNT, Epilogue::kNone, tile_count(t, m, n), k, sms);
+            best = best == 0.0 ? time : std::min(best, time);
+        }
+    }
+    int parts = 1;
+    for (int cluster : {1, 2, 4}) {
+        for (Tile t : kOnceTiles) {
+            const double time = once_time(t, Layout::kNT, Epilogue::kNone, m, n, k, 1, cluster, 1, sms);
+            if (time != 0.0 && time < (parts < cluster ? 0.95 : 1.0) * best) {
+                best = time;
+                parts = cluster;
+            }
+        }
+    }
+    return parts;
+}
+
+// The kernel for `batches` problems of one shape. With `may_split` (TN) k may also be split with
+// partial sums in a workspace, which cost a second launch that reads and adds them.
+Plan pick_plan(Layout l, Epilogue e, size_t m, size_t n, size_t k, long long batches, int sms,
+               bool may_split) {
+    Plan plan = {Tile::k64, 1, 1, 1};
+    double best = 0.0;
+    // A wider tile, or fewer splits, are given up for a gain of a twentieth, no less.
+    auto consider = [&](double time, const Plan& p) {
+        if (time != 0.0 && (best == 0.0 || time < 0.95 * best)) {
+            best = time;
+            plan = p;
+        }
+    };
+    const int parts = sum_parts(m, n, k, sms);
+    if (parts > 1) {
+        for (Tile t : kOnceTiles) {
+            consider(once_time(t, l, e, m, n, k, batches, parts, 1, sms), Plan{t, parts, 1, 1});
+        }
+        if (best == 0.0) {   // a batch of them
+            for (Tile t : {Tile::kOnce128, Tile::kOnce64}) {
+                consider(once_time(t, l, e, m, n, k, batches, 1, parts, sms), Plan{t, 1, parts, 1});
+            }
+        }
+    }
+    for (Tile t : {Tile::kPair, Tile::k256, Tile::k128, Tile::k64}) {
         if (!tile_fits(t, m, n)) {
             continue;
         }
-        const int most = splits != nullptr ? most_splits(t, m, n, k, sms) : 1;
-        for (int s = 1; s <= most; ++s) {
+        const int most = may_split ? most_splits(t, m, n, k, sms) : 1;
+        for (int s = parts > 1 ? 2 : 1; s <= most; ++s) {
             double time = tile_time(t, l, e, tile_count(t, m, n) * batches * s, (k + s - 1) / s, sms);
             if (s > 1) {
                 time += 1.0 + static_cast<double>(s + 1) * static_cast<double>(m) * static_cast<double>(n) * 4.0 / 16e6;
             }
-            // A wider tile, or fewer splits, are given up for a gain of a twentieth, no less.
-            if (best == 0.0 || time < 0.95 * best) {
-                best = time;
-                chosen = t;
-                if (splits != nullptr) {
-                    *splits = s;
-                }
-            }
+            consider(time, Plan{t, 1, 1, s});
         }
         if (t == Tile::kPair && tile_count(t, m, n) * batches > static_cast<long long>(sms)) {
-            break;  // more than two rounds of pairs
+            return plan;  // more than two rounds of pairs
         }
     }
-    return chosen;
+    if (parts == 1) {
+        for (Tile t : kOnceTiles) {
+            const double time = once_time(t, l, e, m, n, k, batches, 1, 1, sms);
+            if (time != 0.0 && time < best) {
+                best = time;
+                plan = Plan{t, 1, 1, 1};
+            }
+        }
+    }
+    return plan;
+}
+
+// Tensor maps of both operands, B in boxes of `columns` rows (or 64-column panels of it).
+template <Layout L>
+cudaError_t make_operand_maps(GemmParams& p, const void* x, const void* w, int columns) {
+    const bool batched = p.batched != 0;
+    const cudaError_t e =
+        L == Layout::kTN ? make_map(&p.map_a, x, p.m, p.k, p.batches, batched, kBK)
+                         : make_map(&p.map_a, x, p.k, p.m, p.batches, batched, kBM);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    return L != Layout::kNT ? make_map(&p.map_b, w, p.n, p.k, p.batches, batched, kBK)
+                            : make_map(&p.map_b, w, p.k, p.n, p.batches, batched, columns);
 }
 
 template <Layout L, Epilogue E, int BN>
 cudaError_t launch_tc(GemmParams& p, const void* x, const void* w, int sms, cudaStream_t stream) {
     using R = Ring<BN>;
-    constexpr bool kAMn = L == Layout::kTN;
-    constexpr bool kBMn = L != Layout::kNT;
     const bool batched = p.batched != 0;
-    cudaError_t e;
-    if (kAMn) {
-        e = make_map(&p.map_a, x, p.m, p.k, p.batches, batched, kBK);
-    } else {
-        e = make_map(&p.map_a, x, p.k, p.m, p.batches, batched, kBM);
-    }
-    if (e != cudaSuccess) {
-        return e;
-    }
-    if (kBMn) {
-        e = make_map(&p.map_b, w, p.n, p.k, p.batches, batched, kBK);
-    } else {
-        e = make_map(&p.map_b, w, p.k, p.n, p.batches, batched, BN);
-    }
+    cudaError_t e = make_operand_maps<L>(p, x, w, BN);
     if (e != cudaSuccess) {
         return e;
     }
@@ -1661,23 +2310,8 @@ cudaError_t launch_tc(GemmParams& p, const void* x, const void* w, int sms, cuda
 
 template <Layout L, Epilogue E>
 cudaError_t launch_pair(GemmParams& p, const void* x, const void* w, int sms, cudaStream_t stream) {
-    constexpr bool kAMn = L == Layout::kTN;
-    constexpr bool kBMn = L != Layout::kNT;
     const bool batched = p.batched != 0;
-    cudaError_t e;
-    if (kAMn) {
-        e = make_map(&p.map_a, x, p.m, p.k, p.batches, batched, kBK);
-    } else {
-        e = make_map(&p.map_a, x, p.k, p.m, p.batches, batched, kBM);
-    }
-    if (e != cudaSuccess) {
-        return e;
-    }
-    if (kBMn) {
-        e = make_map(&p.map_b, w, p.n, p.k, p.batches, batched, kBK);
-    } else {
-        e = make_map(&p.map_b, w, p.k, p.n, p.batches, batched, 128);
-    }
+    cudaError_t e = make_operand_maps<L>(p, x, w, 128);
     if (e != cudaSuccess) {
         return e;
     }
@@ -1690,15 +2324,57 @@ cudaError_t launch_pair(GemmParams& p, const void* x, const void* w, int sms, cu
     const long long z = L == Layout::kTN && !batched ? p.splits : p.batches;
     p.tiles_total = static_cast<long long>(p.tiles_m) * p.tiles_n * z;
 
-    static std::atomic<bool> configured[64] = {};
-    auto kernel = fb_gemm_pair<L, E>;
-    e = fb::allow_shared_memory(kernel, kPairSmemBytes, configured);
+    const long long pairs = std::min<long long>(p.tiles_total, sms / 2);
+    auto launch = [&](auto kernel, int epilogue_warps, std::atomic<bool> (&configured)[64]) {
+        const cudaError_t error = fb::allow_shared_memory(kernel, pair_smem_bytes(epilogue_warps), configured);
+        if (error != cudaSuccess) {
+            return error;
+        }
+        return fb::launch_dependent(kernel, dim3(static_cast<unsigned>(2 * pairs)), dim3(64 + 32 * epilogue_warps),
+                                    pair_smem_bytes(epilogue_warps), stream, p);
+    };
+    static std::atomic<bool> configured[2][64] = {};
+    if constexpr (E == Epilogue::kBiasGelu) {
+        if (static_cast<size_t>(p.k) <= kManyWarpsMostK) {
+            return launch(fb_gemm_pair<L, E, kManyWarps>, kManyWarps, configured[1]);
+        }
+    }
+    return launch(fb_gemm_pair<L, E, kEpilogueWarps>, kEpilogueWarps, configured[0]);
+}
+
+template <Layout L, Epilogue E, int BN>
+cudaError_t launch_once(GemmParams& p, const void* x, const void* w, const Plan& plan,
+                        cudaStream_t stream) {
+    const int cluster = plan.cluster;
+    using R = OnceRing<BN>;
+    cudaError_t e = make_operand_maps<L>(p, x, w, BN);
     if (e != cudaSuccess) {
         return e;
     }
-    const long long pairs = std::min<long long>(p.tiles_total, sms / 2);
-    return fb::launch_dependent(kernel, dim3(static_cast<unsigned>(2 * pairs)),
-                                dim3(64 + 32 * pair_epilogue_warps<E>()), kPairSmemBytes, stream, p);
+    constexpr bool kFloatOut = E == Epilogue::kBiasResidual || E == Epilogue::kTnStore;
+    auto wide = [](const void* at) { return reinterpret_cast<uintptr_t>(at) % 32 == 0; };
+    OnceParams once;
+    once.wide_out = p.n % (kFloatOut ? 8 : 16) == 0 && wide(p.y) && wide(p.aux_out);
+    once.cluster = cluster;
+    once.parts = plan.parts;
+    p.tiles_m = (p.m + kBM - 1) / kBM;
+    p.tiles_n = (p.n + BN - 1) / BN;
+    p.tiles_total = static_cast<long long>(p.tiles_m) * p.tiles_n * p.batches;
+
+    once.stages = R::stages(cluster);
+    once.gemm = p;
+    auto launch = [&](auto kernel, std::atomic<bool> (&configured)[64]) {
+        const cudaError_t error = fb::allow_shared_memory(kernel, 220 * 1024, configured);
+        if (error != cudaSuccess) {
+            return error;
+        }
+        return fb::launch_dependent_cluster(kernel, dim3(static_cast<unsigned>(p.tiles_total * cluster)),
+                                            dim3(kOnceThreads), static_cast<unsigned>(cluster),
+                                            R::bytes(cluster), stream, once);
+    };
+    static std::atomic<bool> configured[2][64] = {};
+    return cluster * plan.parts > 1 ? launch(fb_gemm_once<L, E, BN, true>, configured[1])
+                                    : launch(fb_gemm_once<L, E, BN, false>, configured[0]);
 }
 
 template <Layout L, Epilogue E>
@@ -1716,14 +2392,21 @@ cudaError_t launch_any(GemmParams& p, const void* x, const void* w, cudaStream_t
                                                      static_cast<const __half*>(w));
         return fb::after_launch();
     }
-    Tile tile;
-    if (L == Layout::kTN && p.batched == 0) {
-        int splits = 1;   // as gemm_tn has set them already
-        tile = pick_tile(L, E, p.m, p.n, p.k, 1, sms, &splits);
-    } else {
-        tile = pick_tile(L, E, p.m, p.n, p.k, p.batches, sms, nullptr);
+    // (With k split already, the plan for these splits is the one that gemm_tn has followed.)
+    const Plan plan = pick_plan(L, E, p.m, p.n, p.k, p.batches, sms, L == Layout::kTN && p.batched == 0);
+    if constexpr (E != Epilogue::kTnPartial) {
+        switch (plan.tile) {
+        case Tile::kOnce192:
+            return launch_once<L, E, 192>(p, x, w, plan, stream);
+        case Tile::kOnce128:
+            return launch_once<L, E, 128>(p, x, w, plan, stream);
+        case Tile::kOnce64:
+            return launch_once<L, E, 64>(p, x, w, plan, stream);
+        default:
+            break;
+        }
     }
-    switch (tile) {
+    switch (plan.tile) {
     case Tile::kPair:
         return launch_pair<L, E>(p, x, w, sms, stream);
     case Tile::k256:
@@ -1756,8 +2439,7 @@ GemmParams base_params(void* y, size_t m, size_t n, size_t k, size_t batches, bo
 
 TnSplit tn_split(size_t m, size_t n, size_t k, int sms) {
     // (kTnPartial's and kTnStore's chunks cost the same, so both see one choice.)
-    int want = 1;
-    pick_tile(Layout::kTN, Epilogue::kTnStore, m, n, k, 1, sms, &want);
+    const int want = pick_plan(Layout::kTN, Epilogue::kTnStore, m, n, k, 1, sms, true).splits;
     const size_t per = (k + want - 1) / want;
     TnSplit r;
     r.len = static_cast<int>((per + kBK - 1) / kBK * kBK);

@@ -435,3 +435,82 @@ def test_small_problems_agree_between_layouts_and_epilogues(flint, m, n, k):
     assert torch.equal(nn, nt) and torch.equal(pre, nt) and torch.equal(biased, nt)
     assert torch.equal(added.half(), nt)
     assert batched is None or (torch.equal(batched[0], nt) and torch.equal(batched[1], nt))
+
+
+# Sums over k in two or four parts: by a cluster whose CTAs exchange their partial tiles, or (a batch that
+# does not fit at once) in as many accumulators of one CTA. Edges: rows that end inside the 32 of a
+# cluster's CTA, columns that end inside a tile or a chunk, rows of 16- but not 32-byte multiples, k whose
+# blocks of 64 do not divide evenly, and the shapes just past the last that are divided.
+@pytest.mark.parametrize("m, n, k", [(1, 256, 512), (64, 768, 3072), (129, 264, 1032), (33, 1600, 6400),
+                                     (250, 776, 1032), (512, 768, 2304), (1000, 768, 3072), (2000, 768, 2312),
+                                     (200, 520, 520), (100, 256, 504), (100, 248, 1024)])
+def test_sums_in_parts_agree_between_layouts_epilogues_and_batches(flint, m, n, k):
+    x, w = inputs((m, k), (n, k), m + n)
+    xd, wd = x.to(DEV), w.to(DEV)
+    zero = torch.full((n,), -0.0, device=DEV)
+    nt, nn, biased, pre, act, again = (torch.full((m, n), 7.0, dtype=torch.half, device=DEV) for _ in range(6))
+    flint.gemm_nt(nt, xd, wd, m, n, k)
+    flint.gemm_nt(again, xd, wd, m, n, k)
+    flint.gemm_nn(nn, xd, wd.t().contiguous(), m, n, k)
+    flint.gemm_nt_bias(biased, xd, wd, zero, m, n, k)
+    flint.gemm_nt_bias_gelu(act, pre, xd, wd, zero, m, n, k)
+    added = torch.full((m, n), 7.0, device=DEV)
+    flint.gemm_nt_bias_residual(added, xd, wd, zero, torch.zeros(m, n, device=DEV), m, n, k)
+    no_fault(flint)
+    want = oracle.gemm_nt(x, w)
+    assert rel_error(added, want) <= 1e-5 and rel_error(nt, want) <= 2e-3
+    assert rel_error(act, oracle.gelu_tanh(want)) <= 2e-3
+    assert torch.equal(again, nt)
+    assert torch.equal(nn, nt) and torch.equal(pre, nt) and torch.equal(biased, nt)
+    assert torch.equal(added.half(), nt)
+    if m <= 1024:
+        for batches in (1, 12):
+            batched = torch.full((batches, m, n), 7.0, dtype=torch.half, device=DEV)
+            flint.gemm_nt_batched(batched, xd.expand(batches, m, k).contiguous(), wd.expand(batches, n, k).contiguous(),
+                                  batches, m, n, k)
+            assert all(torch.equal(one, nt) for one in batched), batches
+    if m % 8 == 0:
+        space = torch.empty(max(flint.gemm_tn_workspace(m, n, k), 16), dtype=torch.uint8, device=DEV)
+        xt, wt = xd.t().contiguous(), wd.t().contiguous()
+        tn, old = torch.full((m, n), 7.0, device=DEV), torch.randn(m, n, device=DEV)
+        flint.gemm_tn(tn, xt, wt, m, n, k, workspace=space)
+        both = old.clone()
+        flint.gemm_tn(both, xt, wt, m, n, k, True, workspace=space)
+        assert rel_error(tn, want) <= 1e-5
+        assert torch.equal(both, old + tn)
+        if flint.gemm_tn_workspace(m, n, k) == 0:
+            assert torch.equal(tn, added)
+    no_fault(flint)
+
+
+# Rows stored straight from registers: 16-byte pieces, 32-byte pieces, and two bytes at a time.
+@pytest.mark.parametrize("m, n, offset", [(70, 72, 0), (70, 80, 0), (70, 80, 16), (70, 77, 0), (129, 200, 0)])
+def test_small_problem_rows_at_every_alignment(flint, m, n, offset):
+    k = 64
+    x, w = inputs((m, k), (n, k), m + n)
+    xd, wd = x.to(DEV), w.to(DEV)
+    bias = torch.randn(n, device=DEV)
+    want = oracle.gemm_nt(x, w)
+
+    def output(dtype):
+        space = torch.full((m * n * dtype.itemsize + 64,), 0x55, dtype=torch.uint8, device=DEV)
+        body = space[offset:offset + m * n * dtype.itemsize]
+        return space, body.view(dtype).view(m, n)
+
+    def untouched(space, dtype):
+        return bool((space[:offset] == 0x55).all() and (space[offset + m * n * dtype.itemsize:] == 0x55).all())
+
+    space, y = output(torch.half)
+    flint.gemm_nt(y, xd, wd, m, n, k)
+    assert rel_error(y, want) <= 2e-3 and untouched(space, torch.half)
+    (space, y), (pre_space, pre) = output(torch.half), output(torch.half)
+    flint.gemm_nt_bias_gelu(y, pre, xd, wd, bias, m, n, k)
+    biased = want + bias.cpu().double()
+    assert rel_error(pre, biased) <= 2e-3 and rel_error(y, oracle.gelu_tanh(biased)) <= 2e-3
+    assert untouched(space, torch.half) and untouched(pre_space, torch.half)
+    if n % 2 == 0:
+        space, y = output(torch.float)
+        residual = torch.randn(m, n, device=DEV)
+        flint.gemm_nt_bias_residual(y, xd, wd, bias, residual, m, n, k)
+        assert rel_error(y, residual.cpu().double() + biased) <= 1e-5 and untouched(space, torch.float)
+    no_fault(flint)
