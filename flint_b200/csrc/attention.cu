@@ -2,9 +2,9 @@
 // (extension; the reference materialises scores and probabilities instead,
 // src/api/gpt2.cpp:495-530 and :559-618, and lists flash attention as planned).
 //
-// Three kernels, all warp-specialised like the GEMM (warp 0 = TMA producer,
+// Two kernels, both warp-specialised like the GEMM (warp 0 = TMA producer,
 // warp 1 = tcgen05.mma issuer, the rest compute on accumulators read from
-// tensor memory), all persistent (one CTA per SM over a work-ordered item list):
+// tensor memory), both persistent (one CTA per SM over a work-ordered item list):
 //   forward   items of (head, two adjacent 128-query tiles) sharing the K and V
 //             tiles that stream through a ring: S = Q K^T into TMEM, base-2
 //             softmax in registers, P written back over S as FP16 pairs and read
@@ -18,8 +18,9 @@
 //             dK += dS^T Q accumulated in TMEM
 //   dQ        items of (head, 128 queries) over 64-key sub-steps:
 //             dQ += dS K accumulated in TMEM
-// dQ has its own kernel so that no gradient needs atomics: every output element
-// is produced by one CTA in a fixed order, so results are deterministic.
+// dK/dV and dQ are items of one launch. dQ recomputes the scores so that no gradient needs
+// atomics: every output element is produced by one CTA in a fixed order, so results are
+// deterministic.
 //
 // Q, K, V, O and their gradients are addressed through strided 4-D tensor maps
 // (column, row, head, sequence), so the same kernels read the heads layout
@@ -55,11 +56,14 @@ struct AttnParams {
     CUtensorMap map_q, map_k, map_v, map_do;          // 128-row boxes
     CUtensorMap map_q64, map_k64, map_v64, map_do64;  // 64-row boxes (backward sub-steps)
     // Outputs and row statistics are addressed directly.
-    void* out0;            // forward: O; dkv: dK; dq: dQ
-    void* out1;            // dkv: dV
+    void* out0;            // forward: O; backward: dK
+    void* out1;            // backward: dV
     long long out_row, out_head, out_seq;  // element strides of out0/out1
     float* lse;            // [seqs * heads, length]
     const float* delta;    // [seqs * heads, length]
+    void* dq;              // backward
+    long long dq_row, dq_head, dq_seq;
+    int dkv_ctas;          // backward: CTAs that work on dK and dV
     int length, heads, seqs, blocks;
     float scale;           // applied to the raw scores
 };
@@ -150,6 +154,11 @@ __device__ __forceinline__ void quadrant_sync(int quadrant) {
     asm volatile("bar.sync %0, 64;" ::"r"(quadrant + 1) : "memory");
 }
 
+// The four warps of a quadrant: both column halves of both tiles (barriers 9..12).
+__device__ __forceinline__ void item_sync(int quadrant) {
+    asm volatile("bar.sync %0, 128;" ::"r"(quadrant + 9) : "memory");
+}
+
 // Descriptors for the three ways a tile is read.
 // K-major tile [128 rows][64 cols] (rows = M or N index): 16-column step = 32 bytes.
 __device__ __forceinline__ uint64_t desc_kmajor(uint32_t tile, int kstep) {
@@ -203,6 +212,14 @@ __device__ __forceinline__ void finish(int abort_value, uint32_t tmem_base, uint
 // only then does the thread wait for the previous P V, read O back, rescale and rewrite it.
 // The tensor pipe runs one thread's MMAs in issue order, which is what lets S(n + 3)
 // overwrite the columns that P(n) occupies: it is issued after the P V that reads them.
+// Few heads do not make enough such items for the GPU, and the longest one is the launch's
+// time. There (by_keys) an item is one query tile of one head, and its two tiles share out the
+// key tiles: tile t takes key tiles t, t + 2, ..., with its own reference exponents, row sums and
+// accumulator, and at the item's end tile 1's go to tile 0 through shared memory. That halves the
+// longest item for one merge of 128 x 64 values. Where the number of key tiles is odd, tile 1
+// takes one more, all masked, whose K and V are read from outside the tensor, as zeros.
+// Measured, pairs -> keys: 4 heads x 512 positions 10.1 -> 7.4 us, 12 x 1,000 16.1 -> 10.5, 24 x 1,024
+// 16.8 -> 12.1, 48 x 256 7.6 -> 6.5; 48 x 600, whose 240 items make two rounds, 11.8 -> 12.3.
 // Every K and V tile passes through one ring in the order the MMAs use them: K(0), K(1),
 // K(2), then V(n), K(n + 3) alternately. The query tiles are double-buffered by item.
 // Tensor memory: score buffers at 0, 128, 256; O of tile 0 at 384, of tile 1 at 448.
@@ -227,9 +244,11 @@ struct FwdBarriers {
 struct FwdCursor {
     int round, j, t;
     int qb;      // the item's query tile (it has qb + 1 key tiles); -1 past the last item
-    int pair;    // which pair of heads
+    int pair;    // which pair of heads, or (by_keys) which head
+    int last;    // the largest j
 };
 
+template <bool by_keys>
 __global__ void __launch_bounds__(kFwdThreads, 1)
     fb_attention_forward(const __grid_constant__ AttnParams p) {
     extern __shared__ unsigned char smem_raw[];
@@ -240,11 +259,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     __shared__ float pair_max[2][2][2][kTile];  // [query tile][iteration parity][column half][row]
+    __shared__ float merge_max[kTile], merge_sum[kTile];   // by_keys: tile 1's, per row
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0);
     const int lane = threadIdx.x % 32;
     const int bh_count = p.heads * p.seqs;
-    const int head_pairs = (bh_count + 1) / 2;
+    const int head_pairs = by_keys ? bh_count : (bh_count + 1) / 2;   // or heads
     const int items = p.blocks * head_pairs;
     const int first_item = static_cast<int>(blockIdx.x);
     const int stride = static_cast<int>(gridDim.x);
@@ -257,20 +277,25 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
     // done here, once per item, not in the roles' inner loops).
     auto enter = [&](int round) {
         const int item = item_of(round);
-        FwdCursor c{round, 0, 0, -1, 0};
+        FwdCursor c{round, 0, 0, -1, 0, 0};
         if (item < items) {
             c.qb = p.blocks - 1 - item / head_pairs;
             c.pair = item % head_pairs;
+            c.last = by_keys ? c.qb / 2 : c.qb;
         }
         return c;
     };
     auto valid = [](const FwdCursor& c) { return c.qb >= 0; };
     // The (sequence, head) a tile of the item works on. With an odd number of heads in all,
     // the last item's second tile repeats the first one's head and stores nothing.
-    auto head_of = [&](const FwdCursor& c, int t) { return min(2 * c.pair + t, bh_count - 1); };
+    auto head_of = [&](const FwdCursor& c, int t) {
+        return by_keys ? c.pair : min(2 * c.pair + t, bh_count - 1);
+    };
+    // The key tile of a step; beyond the query tile only where tile 1 has one step too many.
+    auto key_tile = [&](const FwdCursor& c) { return by_keys ? 2 * c.j + c.t : c.j; };
     auto advance = [&](FwdCursor& c) {
         c.t ^= 1;
-        if (c.t == 0 && ++c.j > c.qb) {
+        if (c.t == 0 && ++c.j > c.last) {
             c = enter(c.round + 1);
         }
     };
@@ -315,8 +340,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 }
                 const int bh = head_of(c, c.t);
                 sm100::mbar_expect_tx(bar.slot_full(slot), kTileBytes);
-                tma_load_4d(ring + slot * kTileBytes, map, bar.slot_full(slot), 0, c.j * kTile,
-                            bh % p.heads, bh / p.heads);
+                const int tile = key_tile(c);
+                tma_load_4d(ring + slot * kTileBytes, map, bar.slot_full(slot), 0,
+                            (tile > c.qb ? p.blocks : tile) * kTile, bh % p.heads, bh / p.heads);
                 if (++slot == kFwdSlots) {
                     slot = 0;
                     phase ^= 1u;
@@ -338,8 +364,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                             !sm100::mbar_wait(bar.q_empty(b), ((keys.round >> 1) - 1) & 1, abort)) {
                             break;
                         }
-                        sm100::mbar_expect_tx(bar.q_full(b), 2 * kTileBytes);
-                        for (int t = 0; t < 2; ++t) {
+                        const int tiles = by_keys ? 1 : 2;
+                        sm100::mbar_expect_tx(bar.q_full(b), tiles * kTileBytes);
+                        for (int t = 0; t < tiles; ++t) {
                             const int bh = head_of(keys, t);
                             tma_load_4d(q_tiles + (2 * b + t) * kTileBytes, &p.map_q, bar.q_full(b), 0,
                                         keys.qb * kTile, bh % p.heads, bh / p.heads);
@@ -390,10 +417,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             if (k_tile == 0) {
                 return;
             }
-            const uint64_t q_desc = desc_kmajor(q_tiles + (2 * b + ahead.t) * kTileBytes, 0);
+            const uint64_t q_desc =
+                desc_kmajor(q_tiles + (2 * b + (by_keys ? 0 : ahead.t)) * kTileBytes, 0);
             const uint64_t k_desc = desc_kmajor(k_tile, 0);
             const uint32_t s_at = tmem + 128u * (issued % 3);
-            const bool last_of_item = ahead.t == 1 && ahead.j == ahead.qb;
+            const bool last_of_item = ahead.t == 1 && ahead.j == ahead.last;
             if (sm100::elect_one()) {
                 sm100::mma_f16_ss_at<0>(s_at, q_desc, 0, k_desc, 0, kIdescS);
                 sm100::mma_f16_ss_at<1>(s_at, q_desc, 2, k_desc, 2, kIdescS);
@@ -460,12 +488,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
         bool there = true;
         for (FwdCursor item = enter(0); valid(item); item = enter(item.round + 1)) {
             const int qb = item.qb;
+            const int last = item.last;
             const int bh = head_of(item, tile);
-            const bool stores = 2 * item.pair + tile < bh_count;
+            const bool stores = by_keys ? tile == 0 : 2 * item.pair + tile < bh_count;
             const int q_index = qb * kTile + row;
             float m = -INFINITY;  // reference exponent of the row (base 2), shared by the pair
             fb::F2 l = 0;         // this thread's share of the row sum, in two partial sums
-            for (int j = 0; j <= qb; ++j) {
+            for (int j = 0; j <= last; ++j) {
                 const uint32_t n = 2 * (before + j) + tile;   // this step's number
                 there = sm100::mbar_wait(bar.s_full(n % 3), (n / 3) & 1, abort) && there;
                 const int parity = j & 1;
@@ -475,11 +504,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 sm100::tmem_ld_32x32(my_scores, reinterpret_cast<uint32_t(&)[32]>(raw[0]));
                 sm100::tmem_ld_32x32(my_scores + 32, reinterpret_cast<uint32_t(&)[32]>(raw[32]));
                 sm100::tmem_ld_wait();
-                if (j == qb) {
-                    // The diagonal tile: keys after the query count as minus infinity.
+                const int keys = by_keys ? 2 * j + tile : j;
+                if (keys >= qb) {
+                    // The diagonal tile (or the one too many): keys after the query count as
+                    // minus infinity.
+                    const int visible = row - (keys - qb) * kTile;
 #pragma unroll
                     for (int i = 0; i < 64; ++i) {
-                        raw[i] = (half * 64 + i <= row) ? raw[i] : 0xff800000u;
+                        raw[i] = (half * 64 + i <= visible) ? raw[i] : 0xff800000u;
                     }
                 }
                 float top[4];
@@ -566,16 +598,16 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 // last but one is awaited first, and here, before this warp's arrival lets the
                 // last one be issued at all (afterwards a slow warp could find both complete
                 // and wait for a parity that no longer comes).
-                if (j == qb && qb > 0) {
-                    there = sm100::mbar_wait(bar.pv_done(tile), (before + qb - 1) & 1, abort) && there;
+                if (j == last && last > 0) {
+                    there = sm100::mbar_wait(bar.pv_done(tile), (before + last - 1) & 1, abort) && there;
                 }
                 __syncwarp();
                 if (lane == 0) {
                     sm100::mbar_arrive(bar.p_ready(n % 3));
                 }
             }
-            there = sm100::mbar_wait(bar.pv_done(tile), (before + qb) & 1, abort) && there;
-            before += qb + 1;
+            there = sm100::mbar_wait(bar.pv_done(tile), (before + last) & 1, abort) && there;
+            before += last + 1;
             sm100::tc_fence_after_sync();
             uint32_t acc[32];
             sm100::tmem_ld_32x32(my_output, acc);
@@ -587,11 +619,51 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             float l_lo, l_hi;
             fb::f2_unpack(l, l_lo, l_hi);
             const float mine = l_lo + l_hi;
-            const int parity = (qb + 1) & 1;   // not the slot the last key tile used
+            const int parity = (last + 1) & 1;   // not the slot the last key tile used
             pair_max[tile][parity][half][row] = mine;
             quadrant_sync(pair_barrier);
-            const float total = mine + pair_max[tile][parity][half ^ 1][row];
+            float total = mine + pair_max[tile][parity][half ^ 1][row];
             quadrant_sync(pair_barrier);     // both have read before either writes a maximum there
+            if (by_keys) {
+                // Tile 1's half of the keys joins tile 0's: its values go where the second query
+                // tiles of a pair of heads would be. (The next item's cannot come before tile 0 has
+                // read these: their products wait for tile 0's next probabilities.)
+                const uint32_t merge = q_tiles + (2 * half + 1) * kTileBytes + row * 16;
+                if (tile == 1) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(merge + i * 2048),
+                                     "r"(acc[4 * i]), "r"(acc[4 * i + 1]), "r"(acc[4 * i + 2]),
+                                     "r"(acc[4 * i + 3])
+                                     : "memory");
+                    }
+                    if (half == 0) {
+                        merge_max[row] = m;
+                        merge_sum[row] = total;
+                    }
+                }
+                item_sync(quadrant);
+                if (tile == 0 && qb > 0) {   // (with one key tile, tile 1 saw none)
+                    const float other = merge_max[row];
+                    const float top = fmaxf(m, other);
+                    const float mine_by = fast_exp2(m - top), other_by = fast_exp2(other - top);
+                    total = total * mine_by + merge_sum[row] * other_by;
+                    m = top;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        float v[4];
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                                     : "r"(merge + i * 2048)
+                                     : "memory");
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            acc[4 * i + c] = __float_as_uint(
+                                __uint_as_float(acc[4 * i + c]) * mine_by + v[c] * other_by);
+                        }
+                    }
+                }
+            }
             if (there && stores && q_index < p.length) {
                 const float inv = 1.0f / total;
                 const int head = bh % p.heads;
@@ -692,6 +764,7 @@ constexpr int kBwdUsed = 1024 + 2 * kTileBytes + kBwdStages * 2 * kSubBytes +
 // (which happens when CTAs become resident one SM at a time, behind an earlier kernel,
 // and leaves other SMs idle while the pair takes turns).
 constexpr int kBwdSmem = kBwdUsed > 120 * 1024 ? kBwdUsed : 120 * 1024;
+constexpr double kDkvShare = 0.575;  // of the CTAs, for dK and dV
 constexpr uint32_t kIdescSub = sm100::instr_desc_f16(128, 64, false, false);  // A Bsub^T
 
 struct BwdBarriers {
@@ -760,6 +833,15 @@ __device__ __forceinline__ uint64_t desc_advance(uint64_t desc, uint32_t bytes) 
     return desc + (bytes >> 4);
 }
 
+// What the two gradients' roles share: the CTA's memory, barriers and tensor memory.
+struct BwdShared {
+    uint32_t base;      // resident pair, ring, statistics
+    BwdBarriers bar;
+    uint32_t tmem;
+    volatile int* abort;
+    int warp;           // warp-uniform
+};
+
 // ---- backward: dK and dV ------------------------------------------------------------------------
 //
 // Persistent CTAs, one per SM, each taking (head, 128 keys) items round-robin from a
@@ -776,25 +858,19 @@ __device__ __forceinline__ uint64_t desc_advance(uint64_t desc, uint32_t bytes) 
 // Tensor memory: S^T at 0/64, dP^T at 128/192 (P^T and dS^T overwrite 4 x 8 columns of
 // each), dV 256, dK 320, K 384, V 416.
 
-__global__ void __launch_bounds__(kBwdThreads, 1)
-    fb_attention_dkv(const __grid_constant__ AttnParams p) {
-    extern __shared__ unsigned char smem_raw[];
-    const uint32_t base = (sm100::smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t k_tile = base;
-    const uint32_t v_tile = base + kTileBytes;
-    const uint32_t ring = base + 2 * kTileBytes;                   // stage: Q_h then dO_h
+__device__ __forceinline__ void dkv_items(const AttnParams& p, const BwdShared& shared,
+                                           int first_item, int stride) {
+    const uint32_t k_tile = shared.base;
+    const uint32_t v_tile = shared.base + kTileBytes;
+    const uint32_t ring = shared.base + 2 * kTileBytes;            // stage: Q_h then dO_h
     const uint32_t stats = ring + kBwdStages * 2 * kSubBytes;      // stage: lse[64] then delta[64]
-    const BwdBarriers bar{stats + kBwdStages * 2 * kStatBytes};
-    __shared__ uint32_t tmem_slot;
-    __shared__ int abort_flag;
-
-    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0);
+    const BwdBarriers bar = shared.bar;
+    volatile int* abort = shared.abort;
+    const int warp = shared.warp;
     const int lane = threadIdx.x % 32;
     const int bh_count = p.heads * p.seqs;
     const int items = bh_count * p.blocks;
-    const int first_item = static_cast<int>(blockIdx.x);
-    const int stride = static_cast<int>(gridDim.x);
-    // Items are dealt in rounds of gridDim.x, alternately in ascending and descending CTA
+    // Items are dealt in rounds of `stride`, alternately in ascending and descending CTA
     // order (the list is sorted by work, so this evens the CTAs' totals out); a result
     // >= items ends the list, and only the last round can be short.
     auto item_of = [&](int round) {
@@ -802,23 +878,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         return round * stride + slot;
     };
 
-    if (threadIdx.x == 0) {
-        abort_flag = 0;
-        init_bwd_barriers(bar);
-    }
-    if (warp == 1) {
-        sm100::tmem_alloc(sm100::smem_u32(&tmem_slot), 512);
-    }
-    sm100::tc_fence_before_sync();
-    __syncthreads();
-    sm100::tc_fence_after_sync();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = shared.tmem;
     auto tmem_st = [&](int b) { return tmem + 64u * b; };
     auto tmem_dpt = [&](int b) { return tmem + 128u + 64u * b; };
     const uint32_t tmem_dv = tmem + 256, tmem_dk = tmem + 320;
     const uint32_t tmem_k = tmem + 384, tmem_v = tmem + 416;
-    volatile int* abort = &abort_flag;
-    fb::dependency_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -1092,12 +1156,6 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
             sm100::tc_fence_before_sync();
         }
     }
-    // A persistent CTA lets the next kernel in only when its own work is done: a
-    // dependent that became resident earlier was measured to slow this kernel down.
-    if (threadIdx.x == 0) {
-        fb::dependency_release();
-    }
-    finish(abort_flag, tmem, 512, warp);
 }
 
 // ---- backward: dQ ---------------------------------------------------------------------------------
@@ -1108,25 +1166,18 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 // dQ += dS K accumulated in TMEM. Items overlap as in the dK/dV kernel.
 // Tensor memory: S at 0/64, dP at 128/192, dQ 256, Q 320, dO 352.
 
-__global__ void __launch_bounds__(kBwdThreads, 1)
-    fb_attention_dq(const __grid_constant__ AttnParams p) {
-    extern __shared__ unsigned char smem_raw[];
-    const uint32_t base = (sm100::smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t q_tile = base;
-    const uint32_t do_tile = base + kTileBytes;
-    const uint32_t ring = base + 2 * kTileBytes;                   // stage: K_g then V_g
-    const uint32_t stats = ring + kBwdStages * 2 * kSubBytes;      // unused here
-    const BwdBarriers bar{stats + kBwdStages * 2 * kStatBytes};
-    __shared__ uint32_t tmem_slot;
-    __shared__ int abort_flag;
-
-    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0);
+__device__ __forceinline__ void dq_items(const AttnParams& p, const BwdShared& shared,
+                                           int first_item, int stride) {
+    const uint32_t q_tile = shared.base;
+    const uint32_t do_tile = shared.base + kTileBytes;
+    const uint32_t ring = shared.base + 2 * kTileBytes;            // stage: K_g then V_g
+    const BwdBarriers bar = shared.bar;
+    volatile int* abort = shared.abort;
+    const int warp = shared.warp;
     const int lane = threadIdx.x % 32;
     const int bh_count = p.heads * p.seqs;
     const int items = bh_count * p.blocks;
-    const int first_item = static_cast<int>(blockIdx.x);
-    const int stride = static_cast<int>(gridDim.x);
-    // Items are dealt in rounds of gridDim.x, alternately in ascending and descending CTA
+    // Items are dealt in rounds of `stride`, alternately in ascending and descending CTA
     // order (the list is sorted by work, so this evens the CTAs' totals out); a result
     // >= items ends the list, and only the last round can be short.
     auto item_of = [&](int round) {
@@ -1134,23 +1185,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
         return round * stride + slot;
     };
 
-    if (threadIdx.x == 0) {
-        abort_flag = 0;
-        init_bwd_barriers(bar);
-    }
-    if (warp == 1) {
-        sm100::tmem_alloc(sm100::smem_u32(&tmem_slot), 512);
-    }
-    sm100::tc_fence_before_sync();
-    __syncthreads();
-    sm100::tc_fence_after_sync();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = shared.tmem;
     auto tmem_s = [&](int b) { return tmem + 64u * b; };
     auto tmem_dp = [&](int b) { return tmem + 128u + 64u * b; };
     const uint32_t tmem_dq = tmem + 256;
     const uint32_t tmem_q = tmem + 320, tmem_do = tmem + 352;
-    volatile int* abort = &abort_flag;
-    fb::dependency_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -1345,8 +1384,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
             sm100::tmem_ld_32x16(tmem_dq + lane_base + part * kPart, raw);
             sm100::tmem_ld_wait();
             if (row_valid) {
-                __half* out = static_cast<__half*>(p.out0) + seq * p.out_seq + head * p.out_head +
-                              static_cast<long long>(q_index) * p.out_row + part * kPart;
+                __half* out = static_cast<__half*>(p.dq) + seq * p.dq_seq + head * p.dq_head +
+                              static_cast<long long>(q_index) * p.dq_row + part * kPart;
 #pragma unroll
                 for (int c = 0; c < kPart / 8; ++c) {
                     float a[8];
@@ -1360,12 +1399,53 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
             sm100::tc_fence_before_sync();
         }
     }
+}
+
+// ---- backward: one launch ------------------------------------------------------------------------
+//
+// The first `dkv_ctas` CTAs work through the dK/dV items, the others through dQ's. Neither gradient
+// needs the other, so side by side they have one tail and one start-up instead of two; and few
+// heads, whose items do not fill the GPU (12 heads of 1,000 positions: 96 of each kind, the longest
+// with 16 sub-steps in a row), leave it idle half as long. Both have as many sub-steps; dK/dV's take
+// longer (four products against three, row statistics), which sets the CTAs' shares: 0.57 and
+// 0.58 of them were best for 24 to 192 heads, 0.55 and 0.60 2 to 5 % slower.
+// Two launches -> one, the delta kernel included: 4 heads x 64 positions 10.1 -> 6.3 us, 12 x 1,000
+// 27.3 -> 17.2, 96 x 256 18.9 -> 16.2, 96 x 1,024 88.0 -> 84.0, 192 x 1,024 163.4 -> 158.6.
+
+__global__ void __launch_bounds__(kBwdThreads, 1)
+    fb_attention_backward(const __grid_constant__ AttnParams p) {
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t base = (sm100::smem_u32(smem_raw) + 1023u) & ~1023u;
+    const BwdBarriers bar{base + kBwdUsed - 1024 - 256};
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0);
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        init_bwd_barriers(bar);
+    }
+    if (warp == 1) {
+        sm100::tmem_alloc(sm100::smem_u32(&tmem_slot), 512);
+    }
+    sm100::tc_fence_before_sync();
+    __syncthreads();
+    sm100::tc_fence_after_sync();
+    const BwdShared shared{base, bar, tmem_slot, &abort_flag, warp};
+    fb::dependency_wait();
+
+    const int cta = static_cast<int>(blockIdx.x);
+    if (cta < p.dkv_ctas) {
+        dkv_items(p, shared, cta, p.dkv_ctas);
+    } else {
+        dq_items(p, shared, cta - p.dkv_ctas, static_cast<int>(gridDim.x) - p.dkv_ctas);
+    }
     // A persistent CTA lets the next kernel in only when its own work is done: a
     // dependent that became resident earlier was measured to slow this kernel down.
     if (threadIdx.x == 0) {
         fb::dependency_release();
     }
-    finish(abort_flag, tmem, 512, warp);
+    finish(abort_flag, shared.tmem, 512, warp);
 }
 
 // ---- host side ---------------------------------------------------------------------------------
@@ -1443,17 +1523,26 @@ cudaError_t attention_forward(const AttentionView& o, float* lse, const Attentio
     p.out_head = o.head_stride;
     p.out_seq = o.sequence_stride;
     p.lse = lse;
-    static std::atomic<bool> configured[64] = {};
-    e = fb::allow_shared_memory(fb_attention_forward, kFwdSmem, configured);
+    int sms = 148;
+    sm_count(&sms);
+    // The launch's time in steps: the longest item, or all of them shared out. Items by keys have
+    // half the steps, rounded up, and a merge worth about one.
+    const long long heads = static_cast<long long>(shape.sequences * shape.heads);
+    const double pair_steps = std::max(2.0 * p.blocks, (heads + 1) / 2 * p.blocks * (p.blocks + 1.0) / sms);
+    const long long half = (p.blocks + 1) / 2;
+    const long long all = 2 * (half * half + half - (p.blocks % 2) * half);   // a head's steps: 2 (qb / 2 + 1) each
+    const long long rounds = (heads * p.blocks + sms - 1) / sms;
+    const double key_steps = std::max(2.0 * half, (rounds > 1 ? 1.25 : 1.0) * heads * all / sms) + rounds;
+    const bool by_keys = key_steps < 0.9 * pair_steps;
+    const long long items = (by_keys ? heads : (heads + 1) / 2) * p.blocks;
+    const unsigned grid = static_cast<unsigned>(std::min<long long>(items, sms));
+    const auto kernel = by_keys ? fb_attention_forward<true> : fb_attention_forward<false>;
+    static std::atomic<bool> configured[2][64] = {};
+    e = fb::allow_shared_memory(kernel, kFwdSmem, configured[by_keys]);
     if (e != cudaSuccess) {
         return e;
     }
-    int sms = 148;
-    sm_count(&sms);
-    const long long items = static_cast<long long>((shape.sequences * shape.heads + 1) / 2) * p.blocks;
-    const unsigned grid = static_cast<unsigned>(std::min<long long>(items, sms));
-    return fb::launch_dependent(fb_attention_forward, dim3(grid), dim3(kFwdThreads), kFwdSmem, stream,
-                                p);
+    return fb::launch_dependent(kernel, dim3(grid), dim3(kFwdThreads), kFwdSmem, stream, p);
 }
 
 cudaError_t attention_backward(const AttentionView& dq, const AttentionView& dk,
@@ -1490,38 +1579,29 @@ cudaError_t attention_backward(const AttentionView& dq, const AttentionView& dk,
     }
     p.lse = const_cast<float*>(lse);
     p.delta = delta;
-    // One persistent CTA per SM (fewer when there are fewer items).
-    const unsigned items = static_cast<unsigned>(shape.sequences * shape.heads * p.blocks);
-    const unsigned bwd_grid = std::min(items, static_cast<unsigned>(sms));
-
-    static std::atomic<bool> dkv_configured[64] = {};
-    e = fb::allow_shared_memory(fb_attention_dkv, kBwdSmem, dkv_configured);
-    if (e != cudaSuccess) {
-        return e;
-    }
     // dK and dV must share strides (they do in both supported layouts).
     p.out0 = const_cast<void*>(dk.base);
     p.out1 = const_cast<void*>(dv.base);
     p.out_row = dk.row_stride;
     p.out_head = dk.head_stride;
     p.out_seq = dk.sequence_stride;
-    e = fb::launch_dependent(fb_attention_dkv, dim3(bwd_grid), dim3(kBwdThreads), kBwdSmem, stream,
-                             p);
+    p.dq = const_cast<void*>(dq.base);
+    p.dq_row = dq.row_stride;
+    p.dq_head = dq.head_stride;
+    p.dq_seq = dq.sequence_stride;
+    // One persistent CTA per SM (fewer when there are fewer items), but one for each gradient at least.
+    const int items = static_cast<int>(shape.sequences * shape.heads * p.blocks);
+    const int ctas = std::max(2, static_cast<int>(std::min<long long>(2LL * items, sms)));
+    p.dkv_ctas = 2LL * items <= sms ? items : std::max(1, std::min(items, static_cast<int>(ctas * kDkvShare + 0.5)));
+    const int dq_ctas = std::min(items, std::max(1, ctas - p.dkv_ctas));
+
+    static std::atomic<bool> configured[64] = {};
+    e = fb::allow_shared_memory(fb_attention_backward, kBwdSmem, configured);
     if (e != cudaSuccess) {
         return e;
     }
-    static std::atomic<bool> dq_configured[64] = {};
-    e = fb::allow_shared_memory(fb_attention_dq, kBwdSmem, dq_configured);
-    if (e != cudaSuccess) {
-        return e;
-    }
-    p.out0 = const_cast<void*>(dq.base);
-    p.out1 = nullptr;
-    p.out_row = dq.row_stride;
-    p.out_head = dq.head_stride;
-    p.out_seq = dq.sequence_stride;
-    return fb::launch_dependent(fb_attention_dq, dim3(bwd_grid), dim3(kBwdThreads), kBwdSmem, stream,
-                                p);
+    return fb::launch_dependent(fb_attention_backward, dim3(static_cast<unsigned>(p.dkv_ctas + dq_ctas)),
+                                dim3(kBwdThreads), kBwdSmem, stream, p);
 }
 
 // ---- diagnostic: MMA rate on an idle SM ----------------------------------------------------------

@@ -49,6 +49,28 @@ def test_attention_forward_and_backward(flint, batches, length):
     assert rel_error(dv, want_dv) <= 5e-3
 
 
+# Few heads, whose forward items are one head and share its key tiles between two accumulators: one
+# to eight key tiles, odd numbers of them (the second accumulator then meets a wholly masked one), a last
+# tile of one row group, and items that are not merged (one key tile). Large scores move the maxima
+# of the two halves far apart, either way round.
+@pytest.mark.parametrize("batches, length", [(1, 128), (2, 136), (3, 384), (9, 392), (12, 640), (5, 1000), (20, 1024)])
+@pytest.mark.parametrize("size", [1.0, 12.0])
+def test_attention_of_few_heads(flint, batches, length, size):
+    g = torch.Generator().manual_seed(length + batches)
+    q, k, v, d_o = (torch.randn(batches, length, 64, generator=g).half() for _ in range(4))
+    tiles = torch.arange(length) // 128
+    k[:, tiles % 2 == 1] *= size
+    k[:, tiles % 4 == 2] *= size
+    o = torch.full((batches, length, 64), 7.0, dtype=torch.half, device=DEV)
+    lse = torch.zeros(batches, length, device=DEV)
+    flint.attention_forward(o, lse, q.to(DEV), k.to(DEV), v.to(DEV), batches, length, 64, 0.125)
+    torch.cuda.synchronize()
+    assert not flint.kernel_fault()
+    want_o, want_lse, *_ = oracle.attention(q, k, v, 0.125, d_o)
+    assert rel_error(o, want_o) <= 2e-3
+    assert np.allclose(lse.cpu().numpy(), want_lse, rtol=1e-4, atol=1e-4)
+
+
 def test_attention_is_deterministic_and_row_zero_copies_v(flint):
     batches, length = 12, 1024
     g = torch.Generator().manual_seed(1)
