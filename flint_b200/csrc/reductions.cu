@@ -142,12 +142,36 @@ struct ColumnMaps {
 // The FP16-times-xhat kernel (LayerNorm's dgamma) also sums the FP16 values themselves
 // (dbeta) from the same staged rows, with the operations the FP16 kernel would use, and
 // writes those partial sums to `second` (unless kAlso is false).
+// The barriers and statistics of a CTA that adds a tile of a chunk.
+template <Source kSource, int kPairs>
+struct PartialsShared {
+    float mean[kSource == Source::kHalfTimesXhat ? kChunkRows : 1];
+    float rstd[kSource == Source::kHalfTimesXhat ? kChunkRows : 1];
+    alignas(8) unsigned long long barriers[2 * Staging<kSource, kPairs>::kStages];
+    int abort_flag;
+
+    // By one thread, before the CTA waits for earlier kernels.
+    __device__ void init() {
+        using S = Staging<kSource, kPairs>;
+        const uint32_t bar0 = shared_address(barriers);
+        abort_flag = 0;
+        for (int i = 0; i < S::kStages; ++i) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8u * i) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0 + 8u * (S::kStages + i)),
+                         "r"(kLaneRows)
+                         : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+};
+
+// Tile `tile` of chunk `chunk`, by kAddThreads + 32 threads. (The pointers are after_wait() ones.)
 template <Source kSource, bool kPlain, bool kAlso, int kPairs>
-__global__ void __launch_bounds__(kAddThreads + 32)
-    fb_column_partials(const __grid_constant__ ColumnMaps maps, float* __restrict__ partial,
-                       float* __restrict__ second, const void* __restrict__ src, const float4* __restrict__ x,
-                       const float* __restrict__ mean, const float* __restrict__ rstd, size_t rows,
-                       int pieces) {
+__device__ __forceinline__ void add_tile(const ColumnMaps& maps, float* partial, float* second, const void* src,
+                                         const float4* x, const float* mean, const float* rstd, size_t rows,
+                                         int pieces, size_t chunk, unsigned tile,
+                                         PartialsShared<kSource, kPairs>& shared, unsigned char* staging_raw) {
     using S = Staging<kSource, kPairs>;
     constexpr int kTilePieces = S::kTilePieces;
     constexpr int kTileColumns = S::kTileColumns;
@@ -155,53 +179,25 @@ __global__ void __launch_bounds__(kAddThreads + 32)
     static_assert(S::kStages * S::kStage >= 2 * kLaneRows * kTileColumns * 4 &&
                       kTileColumns <= kAddThreads,
                   "the merge buffers must fit in the ring, and a thread merge a column");
-    extern __shared__ unsigned char staging_raw[];
-    __shared__ float sh_mean[kSource == Source::kHalfTimesXhat ? kChunkRows : 1];
-    __shared__ float sh_rstd[kSource == Source::kHalfTimesXhat ? kChunkRows : 1];
-    __shared__ alignas(8) unsigned long long barriers[2 * S::kStages];
-    __shared__ int abort_flag;
     const int lane = threadIdx.x % 32;
     const int ly = threadIdx.x / 32;     // 0-7: the row stream; 8: fetching
-    const int first_piece = (blockIdx.z * kTilesY + blockIdx.y) * kTilePieces;
-    if (first_piece >= pieces) {
-        return;
-    }
+    const int first_piece = static_cast<int>(tile) * kTilePieces;
     const int width = min(kTilePieces, pieces - first_piece);  // pieces this tile holds
-    const size_t first = size_t{blockIdx.x} * kChunkRows;
+    const size_t first = chunk * kChunkRows;
     const int chunk_rows = static_cast<int>(rows - first < kChunkRows ? rows - first : kChunkRows);
     const int stages_total = (chunk_rows + S::kRows - 1) / S::kRows;
     const uint32_t staging = (shared_address(staging_raw) + 127u) & ~127u;
-    const uint32_t bar0 = shared_address(barriers);
+    const uint32_t bar0 = shared_address(shared.barriers);
     auto full_bar = [&](int slot) { return bar0 + 8u * slot; };
     auto empty_bar = [&](int slot) { return bar0 + 8u * (S::kStages + slot); };
-
-    if (threadIdx.x == 0) {
-        abort_flag = 0;
-        for (int i = 0; i < S::kStages; ++i) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full_bar(i)) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty_bar(i)),
-                         "r"(kLaneRows)
-                         : "memory");
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    fb::dependency_wait();
-    if (threadIdx.x == 0) {
-        fb::dependency_release();
-    }
-    src = fb::after_wait(src);
-    x = fb::after_wait(x);
-    mean = fb::after_wait(mean);
-    rstd = fb::after_wait(rstd);
     if constexpr (kSource == Source::kHalfTimesXhat) {
         for (int t = threadIdx.x; t < chunk_rows; t += kAddThreads + 32) {
-            sh_mean[t] = mean[first + t];
-            sh_rstd[t] = rstd[first + t];
+            shared.mean[t] = mean[first + t];
+            shared.rstd[t] = rstd[first + t];
         }
     }
     __syncthreads();
-    volatile int* abort = &abort_flag;
+    volatile int* abort = &shared.abort_flag;
     bool ok = true;
     int issued = 0;  // fetching warp: stages whose copies have been started
     fb::Comp2 sums[kPairs];
@@ -319,8 +315,8 @@ __global__ void __launch_bounds__(kAddThreads + 32)
                                          : "=l"(xs)
                                          : "r"(stage + row * (kTilePieces * S::kXBytes) + at_x +
                                                i * (kPairPieces * S::kXBytes)));
-                            const float m = sh_mean[k * S::kRows + row];
-                            const float rs = sh_rstd[k * S::kRows + row];
+                            const float m = shared.mean[k * S::kRows + row];
+                            const float rs = shared.rstd[k * S::kRows + row];
                             const fb::F2 xhat =
                                 fb::f2_mul(fb::f2_sub(xs, fb::f2_pack(m, m)), fb::f2_pack(rs, rs));
                             if constexpr (kPlain) {
@@ -358,7 +354,7 @@ __global__ void __launch_bounds__(kAddThreads + 32)
         atomicExch(&g_reduction_error, 1);
     }
     __syncthreads();
-    if (abort_flag != 0) {
+    if (shared.abort_flag != 0) {
         // A wait gave up (the flag was written before the barrier above, so every thread
         // sees the same value). The error word is set; this CTA writes no sums. Before it
         // leaves, the fetching warp waits, again with a limit, for the copies it started
@@ -405,10 +401,37 @@ __global__ void __launch_bounds__(kAddThreads + 32)
                            sh_e[other * kTileColumns + column]);
         }
         // Chunk c occupies rows 2c (sums) and 2c+1 (errors) of a [2*chunks, cols] FP32 matrix.
-        float* out = (set == 0 ? partial : second) + size_t{blockIdx.x} * pieces * 16 + first_piece * 8 + column;
+        float* out = (set == 0 ? partial : second) + chunk * pieces * 16 + first_piece * 8 + column;
         out[0] = total.s;
         out[size_t(pieces) * 8] = total.e;
     }
+}
+
+template <Source kSource, bool kPlain, bool kAlso, int kPairs>
+__global__ void __launch_bounds__(kAddThreads + 32)
+    fb_column_partials(const __grid_constant__ ColumnMaps maps, float* __restrict__ partial,
+                       float* __restrict__ second, const void* __restrict__ src, const float4* __restrict__ x,
+                       const float* __restrict__ mean, const float* __restrict__ rstd, size_t rows,
+                       int pieces) {
+    extern __shared__ unsigned char staging_raw[];
+    __shared__ PartialsShared<kSource, kPairs> shared;
+    const unsigned tile = blockIdx.z * kTilesY + blockIdx.y;
+    if (tile * static_cast<unsigned>(Staging<kSource, kPairs>::kTilePieces) >= static_cast<unsigned>(pieces)) {
+        return;
+    }
+    if (threadIdx.x == 0) {
+        shared.init();
+    }
+    fb::dependency_wait();
+    if (threadIdx.x == 0) {
+        fb::dependency_release();
+    }
+    src = fb::after_wait(src);
+    x = fb::after_wait(x);
+    mean = fb::after_wait(mean);
+    rstd = fb::after_wait(rstd);
+    add_tile<kSource, kPlain, kAlso, kPairs>(maps, partial, second, src, x, mean, rstd, rows, pieces, blockIdx.x,
+                                             tile, shared, staging_raw);
 }
 
 // Second pass: a warp per 4 columns.
@@ -590,24 +613,11 @@ constexpr int kWarpsPerBlock = 8;
 // A warp per row, lane l owning the 8-column pieces l, l+32, ... kPieces > 0:
 // the lane keeps its pieces of dy and x in registers (rows up to 256*kPieces
 // wide) and the row is read once; kPieces == 0 re-reads the row for the
-// second pass.
+// second pass. (The pointers are after_wait() ones.)
 template <int kPieces>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock)
-    fb_layernorm_backward_dx(float4* __restrict__ dx, const uint4* __restrict__ dy,
-                             const float4* __restrict__ x, const float* __restrict__ mean,
-                             const float* __restrict__ rstd, const float4* __restrict__ gamma,
-                             size_t rows, int pieces, bool accumulate, uint4* __restrict__ dx_half) {
-    fb::dependency_wait();
-    fb::dependency_release();
-    dy = fb::after_wait(dy);
-    x = fb::after_wait(x);
-    mean = fb::after_wait(mean);
-    rstd = fb::after_wait(rstd);
-    gamma = fb::after_wait(gamma);
-    const size_t row = size_t{blockIdx.x} * kWarpsPerBlock + threadIdx.x / 32;
-    if (row >= rows) {
-        return;
-    }
+__device__ __forceinline__ void layernorm_dx_row(float4* dx, const uint4* dy, const float4* x, const float* mean,
+                                                 const float* rstd, const float4* gamma, size_t row, int pieces,
+                                                 bool accumulate, uint4* dx_half) {
     const int lane = threadIdx.x % 32;
     const uint4* dyr = dy + row * pieces;
     const float4* xr = x + row * pieces * 2;
@@ -711,6 +721,125 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
             }
         }
     }
+}
+
+template <int kPieces>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+    fb_layernorm_backward_dx(float4* __restrict__ dx, const uint4* __restrict__ dy,
+                             const float4* __restrict__ x, const float* __restrict__ mean,
+                             const float* __restrict__ rstd, const float4* __restrict__ gamma,
+                             size_t first, size_t rows, int pieces, bool accumulate,
+                             uint4* __restrict__ dx_half) {
+    fb::dependency_wait();
+    fb::dependency_release();
+    dy = fb::after_wait(dy);
+    x = fb::after_wait(x);
+    mean = fb::after_wait(mean);
+    rstd = fb::after_wait(rstd);
+    gamma = fb::after_wait(gamma);
+    const size_t row = first + size_t{blockIdx.x} * kWarpsPerBlock + threadIdx.x / 32;
+    if (row < rows) {
+        layernorm_dx_row<kPieces>(dx, dy, x, mean, rstd, gamma, row, pieces, accumulate, dx_half);
+    }
+}
+
+// The parameter gradients' partial sums and dx side by side: the former are chains of additions
+// on 64-column tiles, the latter moves bytes, and both read dy and x, which then come from
+// memory once. CTA 2 i (i < sums) adds tile i / chunks of chunk i % chunks, the others take eight
+// rows of dx each, up to `dx_rows`.
+// Two launches -> one (all of the backward): 8,192 x 768 26.2 -> 24.0 us, 16,384 x 768 46.7 -> 41.7,
+// 1,000 x 768 13.3 -> 10.2, 8,192 x 256 16.6 -> 12.5; in the training step (plain sums) 25 -> 22.9.
+template <bool kPlain, int kPieces>
+__global__ void __launch_bounds__(kAddThreads + 32)
+    fb_layernorm_backward_both(const __grid_constant__ ColumnMaps maps, float* __restrict__ partial,
+                               float* __restrict__ second, float4* __restrict__ dx,
+                               const uint4* __restrict__ dy, const float4* __restrict__ x,
+                               const float* __restrict__ mean, const float* __restrict__ rstd,
+                               const float4* __restrict__ gamma, size_t rows, int pieces, unsigned chunks,
+                               unsigned sums, size_t dx_rows, bool accumulate, uint4* __restrict__ dx_half) {
+    extern __shared__ unsigned char staging_raw[];
+    __shared__ PartialsShared<Source::kHalfTimesXhat, 1> shared;
+    const unsigned block = blockIdx.x;
+    const bool adds = block / 2 < sums && block % 2 == 0;
+    if (adds && threadIdx.x == 0) {
+        shared.init();
+    }
+    fb::dependency_wait();
+    if (threadIdx.x == 0) {
+        fb::dependency_release();
+    }
+    dy = fb::after_wait(dy);
+    x = fb::after_wait(x);
+    mean = fb::after_wait(mean);
+    rstd = fb::after_wait(rstd);
+    gamma = fb::after_wait(gamma);
+    if (adds) {
+        add_tile<Source::kHalfTimesXhat, kPlain, true, 1>(maps, partial, second, dy, x, mean, rstd, rows, pieces,
+                                                          block / 2 % chunks, block / 2 / chunks, shared,
+                                                          staging_raw);
+        return;
+    }
+    const size_t index = block / 2 < sums ? block / 2 : block - sums;
+    const size_t row = index * kWarpsPerBlock + threadIdx.x / 32;
+    if (threadIdx.x < 32 * kWarpsPerBlock && row < dx_rows) {
+        layernorm_dx_row<kPieces>(dx, dy, x, mean, rstd, gamma, row, pieces, accumulate, dx_half);
+    }
+}
+
+template <bool kPlain, int kPieces>
+cudaError_t launch_both(void* dx, const void* dy, const void* x, const void* mean, const void* rstd,
+                        const void* gamma, size_t rows, size_t cols, bool accumulate, void* partial,
+                        void* second, size_t dx_rows, void* dx_half, cudaStream_t stream) {
+    using S = Staging<Source::kHalfTimesXhat, 1>;
+    const unsigned chunks = static_cast<unsigned>((rows + kChunkRows - 1) / kChunkRows);
+    const int pieces = static_cast<int>(cols / 8);
+    const unsigned sums = chunks * static_cast<unsigned>((pieces + S::kTilePieces - 1) / S::kTilePieces);
+    const unsigned row_blocks = static_cast<unsigned>((dx_rows + kWarpsPerBlock - 1) / kWarpsPerBlock);
+    ColumnMaps maps;
+    maps.use = 1;
+    cudaError_t e = fb::encode_rows_map(&maps.main, dy, rows, cols, S::kMainBytes / 8, S::kTilePieces * 8, S::kRows);
+    if (e == cudaSuccess) {
+        e = fb::encode_rows_map(&maps.x, x, rows, cols, 4, S::kTilePieces * 8, S::kRows);
+    }
+    static std::atomic<bool> configured[64] = {};
+    const auto kernel = fb_layernorm_backward_both<kPlain, kPieces>;
+    if (e == cudaSuccess) {
+        e = fb::allow_shared_memory(kernel, S::kBytes, configured);
+    }
+    if (e != cudaSuccess) {
+        return e;
+    }
+    // (Whichever kind there are more of, the last of them follow one another.)
+    const unsigned blocks = std::max(2 * sums, sums + row_blocks);
+    return fb::launch_dependent(kernel, dim3(blocks), dim3(kAddThreads + 32), S::kBytes, stream, maps,
+                                static_cast<float*>(partial), static_cast<float*>(second),
+                                static_cast<float4*>(dx), static_cast<const uint4*>(dy),
+                                static_cast<const float4*>(x), static_cast<const float*>(mean),
+                                static_cast<const float*>(rstd), static_cast<const float4*>(gamma), rows, pieces,
+                                chunks, sums, dx_rows, accumulate, static_cast<uint4*>(dx_half));
+}
+
+template <bool kPlain>
+cudaError_t launch_both(void* dx, const void* dy, const void* x, const void* mean, const void* rstd,
+                        const void* gamma, size_t rows, size_t cols, bool accumulate, void* partial,
+                        void* second, size_t dx_rows, void* dx_half, cudaStream_t stream) {
+    const auto launch = cols <= 256 ? launch_both<kPlain, 1> : launch_both<kPlain, 3>;
+    return launch(dx, dy, x, mean, rstd, gamma, rows, cols, accumulate, partial, second, dx_rows, dx_half, stream);
+}
+
+cudaError_t launch_dx(void* dx, const void* dy, const void* x, const void* mean, const void* rstd,
+                      const void* gamma, size_t first, size_t rows, size_t cols, bool accumulate, void* dx_half,
+                      cudaStream_t stream) {
+    const auto kernel = cols <= 256    ? fb_layernorm_backward_dx<1>
+                        : cols <= 768  ? fb_layernorm_backward_dx<3>
+                        : cols <= 1536 ? fb_layernorm_backward_dx<6>
+                                       : fb_layernorm_backward_dx<0>;
+    const unsigned blocks = static_cast<unsigned>((rows - first + kWarpsPerBlock - 1) / kWarpsPerBlock);
+    return fb::launch_dependent(kernel, dim3(blocks), dim3(32 * kWarpsPerBlock), 0, stream,
+                                static_cast<float4*>(dx), static_cast<const uint4*>(dy),
+                                static_cast<const float4*>(x), static_cast<const float*>(mean),
+                                static_cast<const float*>(rstd), static_cast<const float4*>(gamma), first, rows,
+                                static_cast<int>(cols / 8), accumulate, static_cast<uint4*>(dx_half));
 }
 
 // ---- embedding backward: bucket the rows by token -----------------------------------
@@ -1488,71 +1617,60 @@ cudaError_t launch_layernorm_backward(void* dx, void* dgamma, void* dbeta, const
                                       bool accumulate_dx, bool accumulate_params, void* workspace,
                                       cudaStream_t stream, void* dx_half, bool plain,
                                       ColumnFinishList* later) {
-    // One pass over dy serves both parameter gradients: dgamma's partial sums fill the
-    // workspace, dbeta's follow them (plain: the caller provides twice the public workspace
-    // size), or else lie where dx will be written afterwards. Where dx holds something that
-    // is added to, or has less room (a single row), dbeta takes a pass of its own, before
-    // dgamma's partial sums reuse the workspace (stream order).
+    // dgamma's partial sums fill the workspace. dbeta's follow them (plain: the caller provides
+    // twice the public workspace size), or else lie at the end of dx, whose last rows are then
+    // written after the second pass. Where dx holds something that is added to, or has less room
+    // (a single row), dbeta takes a pass of its own, before dgamma's partial sums reuse the workspace
+    // (stream order), and dx comes last.
     const size_t partial_bytes = column_sum_workspace(rows, cols);
-    void* second = static_cast<unsigned char*>(workspace) + partial_bytes;
-    const bool apart = !plain && (accumulate_dx || rows * cols * 4 < partial_bytes);
+    const bool apart = rows >= (size_t{1} << 31) || (!plain && (accumulate_dx || rows * cols * 4 < partial_bytes));
     cudaError_t e = cudaSuccess;
     if (apart) {
-        e = launch_bias_gradient(dbeta, dy, rows, cols, accumulate_params, workspace, stream, false);
-        second = nullptr;
-    } else if (!plain) {
-        second = dx;
+        e = launch_bias_gradient(dbeta, dy, rows, cols, accumulate_params, workspace, stream, plain);
+        if (e == cudaSuccess) {
+            e = plain ? launch_partials<Source::kHalfTimesXhat, true, false>(workspace, dy, x, mean, rstd, rows,
+                                                                             cols, stream)
+                      : launch_partials<Source::kHalfTimesXhat, false, false>(workspace, dy, x, mean, rstd,
+                                                                              rows, cols, stream);
+        }
+        if (e == cudaSuccess) {
+            e = launch_finish(dgamma, workspace, rows, cols, accumulate_params, stream);
+        }
+        return e == cudaSuccess ? launch_dx(dx, dy, x, mean, rstd, gamma, 0, rows, cols, accumulate_dx, dx_half, stream)
+                                : e;
     }
-    if (e == cudaSuccess) {
-        e = plain ? launch_partials<Source::kHalfTimesXhat, true>(workspace, dy, x, mean, rstd, rows,
-                                                                  cols, stream, second)
-            : apart ? launch_partials<Source::kHalfTimesXhat, false, false>(
-                          workspace, dy, x, mean, rstd, rows, cols, stream)
-                    : launch_partials<Source::kHalfTimesXhat>(workspace, dy, x, mean, rstd, rows, cols,
-                                                              stream, second);
+    // The rows of dx that are free: all, or those before the partial sums at its end.
+    const size_t lent = plain ? 0 : (partial_bytes + cols * 4 - 1) / (cols * 4);
+    const size_t dx_rows = rows - lent;
+    void* second = plain ? static_cast<unsigned char*>(workspace) + partial_bytes
+                         : static_cast<unsigned char*>(dx) + dx_rows * cols * 4;
+    // (Beyond 768 columns dx's warps hold so many registers that one CTA of a common launch is left to an
+    // SM: 8,192 x 1,024 33.7 us apart, 47.8 together, 4,096 x 1,280 26.0 and 31.8.)
+    const bool together = cols <= 768;
+    if (together) {
+        e = plain ? launch_both<true>(dx, dy, x, mean, rstd, gamma, rows, cols, accumulate_dx, workspace, second,
+                                      dx_rows, dx_half, stream)
+                  : launch_both<false>(dx, dy, x, mean, rstd, gamma, rows, cols, false, workspace, second, dx_rows,
+                                       dx_half, stream);
+    } else {
+        e = plain ? launch_partials<Source::kHalfTimesXhat, true>(workspace, dy, x, mean, rstd, rows, cols, stream,
+                                                                  second)
+                  : launch_partials<Source::kHalfTimesXhat>(workspace, dy, x, mean, rstd, rows, cols, stream, second);
     }
     if (e != cudaSuccess) {
         return e;
     }
-    if (!plain) {
-        later = nullptr;   // (dx is written below: the sums in it do not keep)
-    }
     ColumnFinishList here;
-    ColumnFinishList* list = later != nullptr ? later : &here;
-    if (!list->add(dgamma, workspace, cols, accumulate_params) ||
-        (second != nullptr && !list->add(dbeta, second, cols, accumulate_params))) {
+    ColumnFinishList* list = plain && later != nullptr ? later : &here;
+    if (!list->add(dgamma, workspace, cols, accumulate_params) || !list->add(dbeta, second, cols, accumulate_params)) {
         return cudaErrorInvalidValue;
     }
-    if (later == nullptr) {
+    if (list == &here) {
         e = launch_column_finishes(here, rows, stream);
-        if (e != cudaSuccess) {
-            return e;
-        }
     }
-    const int pieces = static_cast<int>(cols / 8);
-    const unsigned blocks = static_cast<unsigned>((rows + kWarpsPerBlock - 1) / kWarpsPerBlock);
-    auto* dxq = static_cast<float4*>(dx);
-    const auto* dyq = static_cast<const uint4*>(dy);
-    const auto* xq = static_cast<const float4*>(x);
-    const auto* mf = static_cast<const float*>(mean);
-    const auto* rf = static_cast<const float*>(rstd);
-    const auto* gq = static_cast<const float4*>(gamma);
-    if (pieces <= 32) {
-        e = fb::launch_dependent(fb_layernorm_backward_dx<1>, dim3(blocks), dim3(32 * kWarpsPerBlock), 0,
-                                 stream, dxq, dyq, xq, mf, rf, gq, rows, pieces, accumulate_dx,
-                                 static_cast<uint4*>(dx_half));
-    } else if (pieces <= 96) {
-        e = fb::launch_dependent(fb_layernorm_backward_dx<3>, dim3(blocks), dim3(32 * kWarpsPerBlock), 0,
-                                 stream, dxq, dyq, xq, mf, rf, gq, rows, pieces, accumulate_dx,
-                                 static_cast<uint4*>(dx_half));
-    } else if (pieces <= 192) {
-        e = fb::launch_dependent(fb_layernorm_backward_dx<6>, dim3(blocks), dim3(32 * kWarpsPerBlock), 0,
-                                 stream, dxq, dyq, xq, mf, rf, gq, rows, pieces, accumulate_dx,
-                                 static_cast<uint4*>(dx_half));
-    } else {
-        e = fb::launch_dependent(fb_layernorm_backward_dx<0>, dim3(blocks), dim3(32 * kWarpsPerBlock), 0,
-                                 stream, dxq, dyq, xq, mf, rf, gq, rows, pieces, accumulate_dx,
-                                 static_cast<uint4*>(dx_half));
+    const size_t done = together ? dx_rows : 0;
+    if (e == cudaSuccess && done < rows) {
+        e = launch_dx(dx, dy, x, mean, rstd, gamma, done, rows, cols, accumulate_dx, dx_half, stream);
     }
     return e;
 }

@@ -269,6 +269,13 @@ def test_layernorm_parameter_sums_wherever_they_lie(flint, shape, accumulate_dx)
     assert same_bits(held[:, 1], want[4])
 
 
+# The sums' CTAs and the rows' run in one launch, and the last rows of dx, two per 256, hold sums first: no,
+# one or most rows left for that launch, more tiles of sums than blocks of rows, every way to hold a row.
+@pytest.mark.parametrize("shape", [(3, 1544), (9, 256), (256, 264), (258, 768), (1025, 72)])
+def test_layernorm_rows_beside_and_behind_the_sums(flint, shape):
+    test_layernorm_parameter_sums_wherever_they_lie(flint, shape, False)
+
+
 @pytest.mark.parametrize("shape", [(3, 32768 * 64 + 8), (255, 72), (512, 64), (3, 32768 * 128 + 8),
                                    (3500, 1920), (3841, 1920), (3841, 1928), (3841, 1992)])
 def test_bias_gradient_at_the_edges_of_its_grid(flint, shape):
