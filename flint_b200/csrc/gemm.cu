@@ -56,7 +56,7 @@ struct GemmParams {
     CUtensorMap map_a;
     CUtensorMap map_b;
     CUtensorMap map_y;    // FP16 outputs leave through TMA stores
-    CUtensorMap map_pre;  // bias+GELU: the pre-activation output
+    CUtensorMap map_pre;  // bias+GELU: the pre-activation output; residual boxes: the residual
     int tma_out;          // the two maps above are valid
     void* y;
     void* aux_out;        // bias+GELU: the pre-activation output
@@ -1509,15 +1509,32 @@ __device__ __forceinline__ TileCoord decode_pair_tile(const GemmParams& p, long 
 // bias+residual 42 -> 45.)
 constexpr int kManyWarps = 16;
 constexpr size_t kManyWarpsMostK = 1024;
-__host__ __device__ constexpr int pair_stages(int epilogue_warps) { return epilogue_warps == 8 ? 6 : 5; }
-__host__ __device__ constexpr int pair_smem_bytes(int epilogue_warps) {
-    return pair_stages(epilogue_warps) * kPairStage + epilogue_warps * 4096 + 1024 + 256;
+
+// Residual boxes (kBoxes): with rows of 16-byte multiples and a short k the FP32 residual comes, and
+// the FP32 output leaves, by tensor copies of boxes of 128 rows x 32 columns through a ring in shared
+// memory, loaded ahead by a warp of their own; the epilogue adds to a box in place. (A warp that
+// fetches its own second operands a chunk ahead has 4 KB on their way, an SM 32 KB, which at a loaded
+// memory's latency is 2.5 TB/s.) 768 x 768: 16,384 rows 36.1 -> 29.4 us, 8,192 24.0 -> 20.7, 4,096 13.7 -> 11.4. With a long k
+// the two stages that the boxes cost the operand ring count for more: 8,192 x 768 x 3,072 41.7 -> 46.4.
+constexpr int kBoxBytes = kBM * 32 * 4;
+constexpr int kBoxSlots = 6;
+constexpr size_t kBoxesMostK = 1024;
+
+__host__ __device__ constexpr int pair_threads(int epilogue_warps, bool boxes) {
+    return 64 + 32 * epilogue_warps + (boxes ? 32 : 0);
+}
+__host__ __device__ constexpr int pair_stages(int epilogue_warps, bool boxes) {
+    return boxes ? 4 : epilogue_warps == 8 ? 6 : 5;
+}
+__host__ __device__ constexpr int pair_smem_bytes(int epilogue_warps, bool boxes) {
+    return pair_stages(epilogue_warps, boxes) * kPairStage +
+           (boxes ? kBoxSlots * kBoxBytes : epilogue_warps * 4096) + 1024 + 256;
 }
 
-template <Layout L, Epilogue E, int kEpi>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * kEpi, 1)
+template <Layout L, Epilogue E, int kEpi, bool kBoxes = false>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(kEpi, kBoxes), 1)
     fb_gemm_pair(const __grid_constant__ GemmParams p) {
-    constexpr int kStages = pair_stages(kEpi);
+    constexpr int kStages = pair_stages(kEpi, kBoxes);
     constexpr int kColumnStep = 32 * (kEpi / 4);            // between a warp's chunks
     constexpr uint32_t kSlotBytes = 4096;
     constexpr bool kAMn = L == Layout::kTN;
@@ -1529,11 +1546,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * kEpi, 1)
     extern __shared__ unsigned char smem_raw[];
     const uint32_t smem_base = (sm100::smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t staging = smem_base + kStages * kPairStage;
-    const uint32_t bars = staging + kEpi * 4096;
+    const uint32_t bars = staging + (kBoxes ? kBoxSlots * kBoxBytes : kEpi * 4096);
     auto full_bar = [&](int s) { return bars + 8u * s; };
     auto empty_bar = [&](int s) { return bars + 8u * (kStages + s); };
     auto acc_full_bar = [&](int a) { return bars + 8u * (2 * kStages + a); };
     auto acc_empty_bar = [&](int a) { return bars + 8u * (2 * kStages + 2 + a); };
+    auto box_full_bar = [&](int s) { return bars + 8u * (2 * kStages + 4 + s); };
+    auto box_empty_bar = [&](int s) { return bars + 8u * (2 * kStages + 4 + kBoxSlots + s); };
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
@@ -1553,6 +1572,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * kEpi, 1)
         for (int a = 0; a < 2; ++a) {
             sm100::mbar_init(acc_full_bar(a), 1);
             sm100::mbar_init(acc_empty_bar(a), 2 * kEpi);
+        }
+        if (kBoxes) {
+            for (int s = 0; s < kBoxSlots; ++s) {
+                sm100::mbar_init(box_full_bar(s), 1);
+                sm100::mbar_init(box_empty_bar(s), 4);   // a warp per quadrant
+            }
         }
         sm100::mbar_fence_init();
         sm100::tma_prefetch_descriptor(&p.map_a);
@@ -1696,6 +1721,121 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * kEpi, 1)
                     acc_phase ^= 1u;
                 }
             }
+        }
+    } else if (kBoxes && warp == 2 + kEpi) {
+        // ---- residual producer (both CTAs): a tile's eight boxes in column order ----
+        if (lane == 0) {
+            uint32_t sequence = 0;
+            bool ok = true;
+            for (long long id = pair; ok && id < p.tiles_total; id += pairs) {
+                const TileCoord t = decode_pair_tile(p, id);
+                const int row = t.tm * 256 + static_cast<int>(rank) * 128;
+                for (int box = 0; box < kPairBN / 32; ++box, ++sequence) {
+                    const int slot = sequence % kBoxSlots;
+                    if (!sm100::mbar_wait(box_empty_bar(slot), ((sequence / kBoxSlots) & 1u) ^ 1u, abort)) {
+                        ok = false;
+                        break;
+                    }
+                    sm100::mbar_expect_tx(box_full_bar(slot), kBoxBytes);
+                    sm100::tma_load_2d(staging + slot * kBoxBytes, &p.map_pre, box_full_bar(slot),
+                                       t.tn * kPairBN + box * 32, row);
+                }
+            }
+        }
+    } else if (kBoxes) {
+        // ---- epilogue warps (both CTAs): a quadrant's 32 rows of every other box ----
+        const int quadrant = warp % 4;
+        const int column_part = (warp - 2) / 4;
+        const int row_in_box = quadrant * 32 + lane;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        uint32_t boxes = 0;          // of earlier tiles
+        int held = -1;               // the slot whose store may still be read
+        bool ok = true;
+        for (long long id = pair; ok && id < p.tiles_total; id += pairs, boxes += kPairBN / 32) {
+            const TileCoord t = decode_pair_tile(p, id);
+            const int row = t.tm * 256 + static_cast<int>(rank) * 128 + quadrant * 32;
+            const int col0 = t.tn * kPairBN;
+            float bias_next = load_bias_lane<E>(p, col0 + column_part * 32, lane);
+            if (!sm100::mbar_wait_warp(acc_full_bar(acc), acc_phase, abort)) {
+                ok = false;
+                break;
+            }
+            sm100::tc_fence_after_sync();
+            const uint32_t t_addr = tmem_base + static_cast<uint32_t>(acc * kPairBN) +
+                                    (static_cast<uint32_t>(quadrant * 32) << 16);
+            const uint32_t leader_empty = sm100::map_to_cta(acc_empty_bar(acc), 0);
+#pragma unroll 1
+            for (int box = column_part; box < kPairBN / 32; box += 2) {
+                const bool last = box + 2 >= kPairBN / 32;
+                const int col = col0 + box * 32;
+                const float bias_lane = bias_next;
+                if (!last) {
+                    bias_next = load_bias_lane<E>(p, col + 64, lane);
+                }
+                const uint32_t sequence = boxes + box;
+                const int slot = sequence % kBoxSlots;
+                uint32_t raw[32];
+                sm100::tmem_ld_32x32(t_addr + box * 32, raw);
+                if (!sm100::mbar_wait_warp(box_full_bar(slot), (sequence / kBoxSlots) & 1u, abort)) {
+                    sm100::tmem_ld_wait();
+                    ok = false;
+                    break;
+                }
+                sm100::tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; j += 8) {
+                    asm volatile(""
+                                 : "+r"(raw[j]), "+r"(raw[j + 1]), "+r"(raw[j + 2]), "+r"(raw[j + 3]),
+                                   "+r"(raw[j + 4]), "+r"(raw[j + 5]), "+r"(raw[j + 6]), "+r"(raw[j + 7]));
+                }
+                if (last) {
+                    // This warp's reads of the accumulator are complete: hand it back.
+                    sm100::tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) {
+                        sm100::mbar_arrive_cluster(leader_empty);
+                    }
+                }
+                // 16-byte piece c of row r lies at c ^ (r & 7) (the tensor map's 128-byte swizzle).
+                const uint32_t at = staging + slot * kBoxBytes + row_in_box * 128;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const uint32_t piece = at + ((c ^ (row_in_box & 7)) << 4);
+                    const uint4 old = ld_shared_v4(piece);
+                    const uint32_t was[4] = {old.x, old.y, old.z, old.w};
+                    uint32_t now[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float sum = __fadd_rn(__uint_as_float(raw[4 * c + j]),
+                                                    __shfl_sync(0xffffffffu, bias_lane, 4 * c + j));
+                        now[j] = __float_as_uint(__fadd_rn(__uint_as_float(was[j]), sum));
+                    }
+                    st_shared_v4(piece, make_uint4(now[0], now[1], now[2], now[3]));
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    if (col < p.n) {
+                        store_chunk_async(&p.map_y, staging + slot * kBoxBytes + quadrant * 4096, col, row);
+                    }
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    // The box before this one has been read by its store: its slot is free.
+                    asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    if (held >= 0) {
+                        sm100::mbar_arrive(box_empty_bar(held));
+                    }
+                }
+                held = slot;
+            }
+            acc ^= 1;
+            if (acc == 0) {
+                acc_phase ^= 1u;
+            }
+        }
+        // Asynchronous output stores must have landed before the kernel is over.
+        if (lane == 0) {
+            store_wait_all();
         }
     } else {
         // ---- epilogue warps (both CTAs) ----
@@ -2072,7 +2212,7 @@ constexpr double kTileFixed = 2.7;
 struct ChunkTime {
     double last, steady_pair, steady_single;
 };
-constexpr ChunkTime chunk_time(Epilogue e) {
+constexpr ChunkTime chunk_time(Epilogue e, size_t k) {
     switch (e) {
     case Epilogue::kNone:
     case Epilogue::kScale:
@@ -2083,7 +2223,7 @@ constexpr ChunkTime chunk_time(Epilogue e) {
     case Epilogue::kTnPartial:
         return {1.1, 1.3, 1.5};
     case Epilogue::kBiasResidual:
-        return {1.4, 2.3, 2.6};
+        return {1.4, k <= kBoxesMostK ? 2.2 : 2.3, 3.9};
     case Epilogue::kDGelu:
         return {1.5, 1.7, 2.7};
     default:
@@ -2097,7 +2237,7 @@ double tile_time(Tile t, Layout l, Epilogue e, long long tiles, size_t k, int sm
     const long long slots = t == Tile::kPair ? std::max(1, sms / 2) : sms;
     const double more = static_cast<double>((tiles + slots - 1) / slots - 1);
     const int chunks = tile_columns(t) / 64;   // per epilogue warp
-    const ChunkTime c = chunk_time(e);
+    const ChunkTime c = chunk_time(e, k);
     return kTileFixed + loop + chunks * c.last + more * std::max(1.2 * loop, chunks * (t == Tile::kPair ? c.steady_pair : c.steady_single));
 }
 
@@ -2171,7 +2311,8 @@ double once_time(Tile t, Layout l, Epilogue e, size_t m, size_t n, size_t k, lon
     // The same in clusters of two and four, the exchange of partial sums included.
     constexpr double kCluster[2][3][2] = {{{4.0, 5.0}, {4.8, 6.1}, {5.7, 7.0}}, {{4.4, 5.5}, {5.2, 6.5}, {6.3, 7.8}}};
     const double one = (cluster > 1 ? kCluster[cluster / 4][i][busy] + more : rest[i][busy]) +
-                       kBlock[l == Layout::kTN][i] * static_cast<double>((blocks + cluster - 1) / cluster);
+                       (l == Layout::kTN && cluster > 1 && i == 2 ? 0.42 : kBlock[l == Layout::kTN][i]) *
+                           static_cast<double>((blocks + cluster - 1) / cluster);
     return one * static_cast<double>((ctas + sms - 1) / sms);
 }
 
@@ -2221,9 +2362,10 @@ Plan pick_plan(Layout l, Epilogue e, size_t m, size_t n, size_t k, long long bat
                bool may_split) {
     Plan plan = {Tile::k64, 1, 1, 1};
     double best = 0.0;
-    // A wider tile, or fewer splits, are given up for a gain of a twentieth, no less.
+    // A wider tile, or fewer splits, are given up for a gain of a twentieth, no less; a cluster for
+    // splits in memory more easily (TN 2,304 x 768 x 8,192: 30.1 us in splits, 33.4 over clusters).
     auto consider = [&](double time, const Plan& p) {
-        if (time != 0.0 && (best == 0.0 || time < 0.95 * best)) {
+        if (time != 0.0 && (best == 0.0 || time < (plan.cluster > 1 ? 0.98 : 0.95) * best)) {
             best = time;
             plan = p;
         }
@@ -2265,6 +2407,26 @@ Plan pick_plan(Layout l, Epilogue e, size_t m, size_t n, size_t k, long long bat
         }
     }
     return plan;
+}
+
+// Tensor maps of the FP32 residual, loaded in boxes of 128 rows, and of the FP32 output, stored in
+// boxes of 32.
+cudaError_t make_box_maps(GemmParams& p) {
+    EncodeTiled encode = nullptr;
+    const cudaError_t e = encode_fn(&encode);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(p.n), static_cast<cuuint64_t>(p.m)};
+    const cuuint64_t strides[1] = {dims[0] * 4};
+    const cuuint32_t elem[2] = {1, 1};
+    auto make = [&](CUtensorMap* map, const void* base, cuuint32_t rows) {
+        const cuuint32_t box[2] = {32, rows};
+        return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box,
+                      elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    return make(&p.map_pre, p.aux_in, kBM) && make(&p.map_y, p.y, 32) ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 // Tensor maps of both operands, B in boxes of `columns` rows (or 64-column panels of it).
@@ -2325,21 +2487,30 @@ cudaError_t launch_pair(GemmParams& p, const void* x, const void* w, int sms, cu
     p.tiles_total = static_cast<long long>(p.tiles_m) * p.tiles_n * z;
 
     const long long pairs = std::min<long long>(p.tiles_total, sms / 2);
-    auto launch = [&](auto kernel, int epilogue_warps, std::atomic<bool> (&configured)[64]) {
-        const cudaError_t error = fb::allow_shared_memory(kernel, pair_smem_bytes(epilogue_warps), configured);
+    auto launch = [&](auto kernel, int epilogue_warps, bool boxes, std::atomic<bool> (&configured)[64]) {
+        const int smem = pair_smem_bytes(epilogue_warps, boxes);
+        const cudaError_t error = fb::allow_shared_memory(kernel, smem, configured);
         if (error != cudaSuccess) {
             return error;
         }
-        return fb::launch_dependent(kernel, dim3(static_cast<unsigned>(2 * pairs)), dim3(64 + 32 * epilogue_warps),
-                                    pair_smem_bytes(epilogue_warps), stream, p);
+        return fb::launch_dependent(kernel, dim3(static_cast<unsigned>(2 * pairs)),
+                                    dim3(static_cast<unsigned>(pair_threads(epilogue_warps, boxes))),
+                                    static_cast<size_t>(smem), stream, p);
     };
     static std::atomic<bool> configured[2][64] = {};
-    if constexpr (E == Epilogue::kBiasGelu) {
-        if (static_cast<size_t>(p.k) <= kManyWarpsMostK) {
-            return launch(fb_gemm_pair<L, E, kManyWarps>, kManyWarps, configured[1]);
+    if constexpr (E == Epilogue::kBiasResidual) {
+        if (p.n % 4 == 0 && static_cast<size_t>(p.k) <= kBoxesMostK) {
+            e = make_box_maps(p);
+            return e != cudaSuccess ? e
+                                    : launch(fb_gemm_pair<L, E, kEpilogueWarps, true>, kEpilogueWarps, true, configured[1]);
         }
     }
-    return launch(fb_gemm_pair<L, E, kEpilogueWarps>, kEpilogueWarps, configured[0]);
+    if constexpr (E == Epilogue::kBiasGelu) {
+        if (static_cast<size_t>(p.k) <= kManyWarpsMostK) {
+            return launch(fb_gemm_pair<L, E, kManyWarps>, kManyWarps, false, configured[1]);
+        }
+    }
+    return launch(fb_gemm_pair<L, E, kEpilogueWarps>, kEpilogueWarps, false, configured[0]);
 }
 
 template <Layout L, Epilogue E, int BN>

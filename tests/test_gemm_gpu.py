@@ -514,3 +514,19 @@ def test_small_problem_rows_at_every_alignment(flint, m, n, offset):
         flint.gemm_nt_bias_residual(y, xd, wd, bias, residual, m, n, k)
         assert rel_error(y, residual.cpu().double() + biased) <= 1e-5 and untouched(space, torch.float)
     no_fault(flint)
+
+
+# Residual and output by boxes of 128 rows x 32 columns (more than two rounds of 256 x 256 tiles): the last box of a
+# row of tiles wholly outside, partly outside, and rows that end inside a box of 32.
+@pytest.mark.parametrize("m, n, k", [(5000, 2312, 72), (4200, 3076, 64), (8191, 1540, 200)])
+def test_residual_boxes_at_ragged_edges(flint, m, n, k):
+    x, w = inputs((m, k), (n, k), m + n)
+    g = torch.Generator().manual_seed(m)
+    bias, residual = torch.randn(n, generator=g), torch.randn(m, n, generator=g)
+    space = torch.full((m * n + 64,), 7.0, device=DEV)
+    y = space[32:-32].view(m, n)
+    flint.gemm_nt_bias_residual(y, x.to(DEV), w.to(DEV), bias.to(DEV), residual.to(DEV), m, n, k)
+    no_fault(flint)
+    want = residual.double() + oracle.gemm_nt(x, w, bias)
+    assert rel_error(y, want) <= 1e-5
+    assert bool((space[:32] == 7).all()) and bool((space[-32:] == 7).all())
