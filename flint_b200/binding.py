@@ -210,12 +210,26 @@ def pointer(value):
     return value.data_ptr()
 
 
+_raw_stream = None  # torch's current stream as a number, once CUDA is up
+
+
+def _current_stream():
+    """torch's current stream's handle, by way of a stream object (which brings CUDA up); later calls ask
+    for the number alone where this torch can give it."""
+    global _raw_stream
+    import torch
+
+    handle = torch.cuda.current_stream().cuda_stream
+    raw, device = (getattr(torch._C, name, None) for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+    if raw is not None and device is not None:
+        _raw_stream = lambda: raw(device())
+    return handle
+
+
 def stream_handle(stream):
     """A cudaStream_t value from a torch stream, an int handle, or None (torch's current)."""
     if stream is None:
-        import torch
-
-        return torch.cuda.current_stream().cuda_stream
+        return _current_stream() if _raw_stream is None else _raw_stream()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
@@ -241,6 +255,25 @@ def _bind(lib, functions: dict) -> None:
         function.argtypes = [_C_TYPES[c_type] for c_type, _ in params]
 
 
+def _caller(function, params):
+    """A Python function of the C function's parameters that converts and passes them: tensors
+    become addresses, bools ints; the stream comes last. Written out for the one signature, because
+    deciding each argument's treatment on every call took longer than the launch."""
+    names = [f"a{i}" for i in range(len(params))]
+    passed = []
+    for (c_type, _), name in zip(params, names):
+        if c_type == "flint_stream":
+            passed.append(f"stream_handle({name})")
+        elif _C_TYPES[c_type] is ctypes.c_void_p:
+            passed.append(f"{name} if {name} is None or isinstance({name}, int) else {name}.data_ptr()")
+        elif c_type == "int":
+            passed.append(f"int({name})")
+        else:
+            passed.append(name)
+    scope = {"function": function, "stream_handle": stream_handle}
+    return eval(f"lambda {', '.join(names)}: function({', '.join(passed)})", scope)
+
+
 class Flint:
     """The loaded library. Methods mirror the C functions without the flint_ prefix."""
 
@@ -254,6 +287,7 @@ class Flint:
         self.lib = ctypes.CDLL(str(self.path), mode=ctypes.RTLD_GLOBAL)
         self.functions = declared_functions()
         _bind(self.lib, self.functions)
+        self._callers = {}
         self._train = None
 
     @property
@@ -295,22 +329,16 @@ class Flint:
     def call(self, name: str, *args, stream=None):
         """Calls a status-returning function: tensors become addresses, bools ints, and
         the stream argument (always last in the C signature) is filled in."""
-        _, params = self.functions[name]
-        converted = []
-        values = list(args)
-        for c_type, param in params:
-            if c_type == "flint_stream":
-                converted.append(stream_handle(stream))
-                continue
-            value = values.pop(0)
-            if _C_TYPES[c_type] is ctypes.c_void_p:
-                value = pointer(value)
-            elif c_type == "int":
-                value = int(value)
-            converted.append(value)
-        if values:
-            raise TypeError(f"{name}: {len(values)} arguments too many")
-        self.check(getattr(self.lib, name)(*converted))
+        caller = self._callers.get(name)
+        if caller is None:
+            params = self.functions[name][1]
+            caller = _caller(getattr(self.lib, name), params)
+            if all(c_type != "flint_stream" for c_type, _ in params):
+                caller = (lambda inner: lambda *values: inner(*values[:-1]))(caller)
+            self._callers[name] = caller
+        status = caller(*args, stream)
+        if status != OK:
+            self.check(status)
 
     def _size_query(self, name: str, *dims) -> int:
         size = ctypes.c_size_t()

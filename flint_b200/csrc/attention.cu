@@ -53,8 +53,7 @@ constexpr float kLn2 = 0.6931471805599453f;
 __device__ int g_attention_error = 0;
 
 struct AttnParams {
-    CUtensorMap map_q, map_k, map_v, map_do;          // 128-row boxes
-    CUtensorMap map_q64, map_k64, map_v64, map_do64;  // 64-row boxes (backward sub-steps)
+    CUtensorMap map_q, map_k, map_v, map_do;   // boxes of 128 rows (forward) or 64 (backward)
     // Outputs and row statistics are addressed directly.
     void* out0;            // forward: O; backward: dK
     void* out1;            // backward: dV
@@ -901,8 +900,11 @@ __device__ __forceinline__ void dkv_items(const AttnParams& p, const BwdShared& 
                     break;
                 }
                 sm100::mbar_expect_tx(bar.resident(), 2 * kTileBytes);
-                tma_load_4d(k_tile, &p.map_k, bar.resident(), 0, kb * kTile, head, seq);
-                tma_load_4d(v_tile, &p.map_v, bar.resident(), 0, kb * kTile, head, seq);
+                for (int half = 0; half < 2; ++half) {
+                    const int row = kb * kTile + half * kSub;
+                    tma_load_4d(k_tile + half * kSubBytes, &p.map_k, bar.resident(), 0, row, head, seq);
+                    tma_load_4d(v_tile + half * kSubBytes, &p.map_v, bar.resident(), 0, row, head, seq);
+                }
                 for (int h = 0; h < steps; ++h) {
                     if (!sm100::mbar_wait(bar.stage_empty(stage), phase ^ 1u, abort)) {
                         ok = false;
@@ -917,8 +919,8 @@ __device__ __forceinline__ void dkv_items(const AttnParams& p, const BwdShared& 
                     const uint32_t stat_bytes =
                         present > 0 ? static_cast<uint32_t>(present) * 4u : 0u;
                     sm100::mbar_expect_tx(bar.stage_full(stage), 2 * kSubBytes + 2 * stat_bytes);
-                    tma_load_4d(dst, &p.map_q64, bar.stage_full(stage), 0, q0, head, seq);
-                    tma_load_4d(dst + kSubBytes, &p.map_do64, bar.stage_full(stage), 0, q0, head,
+                    tma_load_4d(dst, &p.map_q, bar.stage_full(stage), 0, q0, head, seq);
+                    tma_load_4d(dst + kSubBytes, &p.map_do, bar.stage_full(stage), 0, q0, head,
                                 seq);
                     if (stat_bytes != 0) {
                         const size_t at = static_cast<size_t>(bh) * p.length + q0;
@@ -1208,8 +1210,11 @@ __device__ __forceinline__ void dq_items(const AttnParams& p, const BwdShared& s
                     break;
                 }
                 sm100::mbar_expect_tx(bar.resident(), 2 * kTileBytes);
-                tma_load_4d(q_tile, &p.map_q, bar.resident(), 0, qb * kTile, head, seq);
-                tma_load_4d(do_tile, &p.map_do, bar.resident(), 0, qb * kTile, head, seq);
+                for (int half = 0; half < 2; ++half) {
+                    const int row = qb * kTile + half * kSub;
+                    tma_load_4d(q_tile + half * kSubBytes, &p.map_q, bar.resident(), 0, row, head, seq);
+                    tma_load_4d(do_tile + half * kSubBytes, &p.map_do, bar.resident(), 0, row, head, seq);
+                }
                 for (int g = 0; g < steps; ++g) {
                     if (!sm100::mbar_wait(bar.stage_empty(stage), phase ^ 1u, abort)) {
                         ok = false;
@@ -1217,8 +1222,8 @@ __device__ __forceinline__ void dq_items(const AttnParams& p, const BwdShared& s
                     }
                     const uint32_t dst = ring + stage * 2 * kSubBytes;
                     sm100::mbar_expect_tx(bar.stage_full(stage), 2 * kSubBytes);
-                    tma_load_4d(dst, &p.map_k64, bar.stage_full(stage), 0, g * kSub, head, seq);
-                    tma_load_4d(dst + kSubBytes, &p.map_v64, bar.stage_full(stage), 0, g * kSub,
+                    tma_load_4d(dst, &p.map_k, bar.stage_full(stage), 0, g * kSub, head, seq);
+                    tma_load_4d(dst + kSubBytes, &p.map_v, bar.stage_full(stage), 0, g * kSub,
                                 head, seq);
                     if (++stage == kBwdStages) {
                         stage = 0;
@@ -1476,7 +1481,7 @@ cudaError_t encode_fn(EncodeTiled* out) {
 
 // (column 0..63, row 0..length-1, head, sequence) view of an FP16 tensor.
 cudaError_t make_map(CUtensorMap* map, const AttentionView& v, const AttentionShape& s,
-                     int box_rows = kTile) {
+                     int box_rows) {
     EncodeTiled encode = nullptr;
     const cudaError_t e = encode_fn(&encode);
     if (e != cudaSuccess) {
@@ -1512,9 +1517,9 @@ cudaError_t attention_forward(const AttentionView& o, float* lse, const Attentio
                               const AttentionView& k, const AttentionView& v,
                               const AttentionShape& shape, float scale, cudaStream_t stream) {
     AttnParams p = base_params(shape, scale);
-    cudaError_t e = make_map(&p.map_q, q, shape);
-    if (e == cudaSuccess) e = make_map(&p.map_k, k, shape);
-    if (e == cudaSuccess) e = make_map(&p.map_v, v, shape);
+    cudaError_t e = make_map(&p.map_q, q, shape, kTile);
+    if (e == cudaSuccess) e = make_map(&p.map_k, k, shape, kTile);
+    if (e == cudaSuccess) e = make_map(&p.map_v, v, shape, kTile);
     if (e != cudaSuccess) {
         return e;
     }
@@ -1552,14 +1557,11 @@ cudaError_t attention_backward(const AttentionView& dq, const AttentionView& dk,
                                const AttentionView& v, const AttentionShape& shape, float scale,
                                cudaStream_t stream) {
     AttnParams p = base_params(shape, scale);
-    cudaError_t e = make_map(&p.map_q, q, shape);
-    if (e == cudaSuccess) e = make_map(&p.map_k, k, shape);
-    if (e == cudaSuccess) e = make_map(&p.map_v, v, shape);
-    if (e == cudaSuccess) e = make_map(&p.map_do, d_o, shape);
-    if (e == cudaSuccess) e = make_map(&p.map_q64, q, shape, kSub);
-    if (e == cudaSuccess) e = make_map(&p.map_k64, k, shape, kSub);
-    if (e == cudaSuccess) e = make_map(&p.map_v64, v, shape, kSub);
-    if (e == cudaSuccess) e = make_map(&p.map_do64, d_o, shape, kSub);
+    // One map per tensor: the 128-row tiles are two boxes of a sub-step's 64.
+    cudaError_t e = make_map(&p.map_q, q, shape, kSub);
+    if (e == cudaSuccess) e = make_map(&p.map_k, k, shape, kSub);
+    if (e == cudaSuccess) e = make_map(&p.map_v, v, shape, kSub);
+    if (e == cudaSuccess) e = make_map(&p.map_do, d_o, shape, kSub);
     if (e != cudaSuccess) {
         return e;
     }

@@ -2549,7 +2549,8 @@ cudaError_t launch_once(GemmParams& p, const void* x, const void* w, const Plan&
 }
 
 template <Layout L, Epilogue E>
-cudaError_t launch_any(GemmParams& p, const void* x, const void* w, cudaStream_t stream) {
+cudaError_t launch_any(GemmParams& p, const void* x, const void* w, cudaStream_t stream,
+                       const Plan* given = nullptr) {
     int sms = 0;
     cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) {
@@ -2563,8 +2564,7 @@ cudaError_t launch_any(GemmParams& p, const void* x, const void* w, cudaStream_t
                                                      static_cast<const __half*>(w));
         return fb::after_launch();
     }
-    // (With k split already, the plan for these splits is the one that gemm_tn has followed.)
-    const Plan plan = pick_plan(L, E, p.m, p.n, p.k, p.batches, sms, L == Layout::kTN && p.batched == 0);
+    const Plan plan = given != nullptr ? *given : pick_plan(L, E, p.m, p.n, p.k, p.batches, sms, false);
     if constexpr (E != Epilogue::kTnPartial) {
         switch (plan.tile) {
         case Tile::kOnce192:
@@ -2608,14 +2608,21 @@ GemmParams base_params(void* y, size_t m, size_t n, size_t k, size_t batches, bo
 
 // ---- internal launchers (declared in gemm.h) --------------------------------------------
 
+namespace {
+// (kTnPartial's and kTnStore's chunks cost the same, so both see one plan.)
+Plan tn_plan(size_t m, size_t n, size_t k, int sms, TnSplit* split) {
+    const Plan plan = pick_plan(Layout::kTN, Epilogue::kTnStore, m, n, k, 1, sms, true);
+    const size_t per = (k + plan.splits - 1) / plan.splits;
+    split->len = static_cast<int>((per + kBK - 1) / kBK * kBK);
+    split->count = static_cast<int>((k + split->len - 1) / split->len);
+    return plan;
+}
+}  // namespace
+
 TnSplit tn_split(size_t m, size_t n, size_t k, int sms) {
-    // (kTnPartial's and kTnStore's chunks cost the same, so both see one choice.)
-    const int want = pick_plan(Layout::kTN, Epilogue::kTnStore, m, n, k, 1, sms, true).splits;
-    const size_t per = (k + want - 1) / want;
-    TnSplit r;
-    r.len = static_cast<int>((per + kBK - 1) / kBK * kBK);
-    r.count = static_cast<int>((k + r.len - 1) / r.len);
-    return r;
+    TnSplit split;
+    tn_plan(m, n, k, sms, &split);
+    return split;
 }
 
 cudaError_t gemm_nt(Epilogue e, void* y, void* pre, const void* x, const void* w,
@@ -2658,14 +2665,18 @@ cudaError_t gemm_tn(void* y, const void* x, const void* w, size_t m, size_t n, s
     }
     GemmParams p = base_params(y, m, n, k, 1, false);
     p.accumulate = accumulate ? 1 : 0;
-    const TnSplit s = use_simt() ? TnSplit{1, p.split_len} : tn_split(m, n, k, sms);
+    TnSplit s{1, p.split_len};
+    Plan plan{Tile::k64, 1, 1, 1};
+    if (!use_simt()) {
+        plan = tn_plan(m, n, k, sms, &s);
+    }
     if (s.count == 1) {
-        return launch_any<Layout::kTN, Epilogue::kTnStore>(p, x, w, stream);
+        return launch_any<Layout::kTN, Epilogue::kTnStore>(p, x, w, stream, &plan);
     }
     p.splits = s.count;
     p.split_len = s.len;
     p.partials = static_cast<float*>(workspace);
-    e = launch_any<Layout::kTN, Epilogue::kTnPartial>(p, x, w, stream);
+    e = launch_any<Layout::kTN, Epilogue::kTnPartial>(p, x, w, stream, &plan);
     if (e != cudaSuccess) {
         return e;
     }
