@@ -1130,6 +1130,7 @@ struct OnceParams {
     int parts;      // accumulators of one CTA, each for a part of k
     int stages;     // of the operand ring
     int wide_out;   // every row segment of the output is 32-byte aligned
+    int steady_b;   // B was written before the kernel before this one began: see fetch below
 };
 
 // kParted: k is taken in parts, by a cluster or one after another.
@@ -1199,8 +1200,38 @@ __global__ void __launch_bounds__(kOnceThreads, 1)
     const int blocks = all_blocks * (rank + 1) / cluster - block0;
     const int k0 = block0 * kBK;
 
+    const int batch = p.batched ? static_cast<int>(t.z) : 0;
+    const int row_a = t.tm * kBM;
+    const int row_b = t.tn * BN;
+    auto fetch_b = [&](uint32_t b_dst, uint32_t bar, int kk) {
+        if constexpr (!kBMn) {
+            if (p.batched) {
+                sm100::tma_load_3d(b_dst, &p.map_b, bar, kk, row_b, batch);
+            } else {
+                sm100::tma_load_2d(b_dst, &p.map_b, bar, kk, row_b);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < BN / 64; ++j) {
+                if (p.batched) {
+                    sm100::tma_load_3d(b_dst + j * 8192, &p.map_b, bar, row_b + 64 * j, kk, batch);
+                } else {
+                    sm100::tma_load_2d(b_dst + j * 8192, &p.map_b, bar, row_b + 64 * j, kk);
+                }
+            }
+        }
+    };
+    // Weights that no running kernel writes fill the ring's half of the first stages already.
+    const int early = once.steady_b != 0 ? min(stages, blocks) : 0;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < early; ++i) {
+            sm100::mbar_expect_tx(full_bar(i), R::kStage);
+            fetch_b(smem_base + i * R::kStage + R::kStageA, full_bar(i), k0 + i * kBK);
+        }
+    }
+
     // Everything above ran while the previous kernel in the stream may still have been
-    // finishing; global memory is touched only from here on.
+    // finishing; what that kernel may have written is touched only from here on.
     fb::dependency_wait();
     if (threadIdx.x == 0) {
         fb::dependency_release();
@@ -1211,18 +1242,17 @@ __global__ void __launch_bounds__(kOnceThreads, 1)
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0;
-            const int batch = p.batched ? static_cast<int>(t.z) : 0;
-            const int row_a = t.tm * kBM;
-            const int row_b = t.tn * BN;
             for (int i = 0; i < blocks; ++i) {
                 const int kk = k0 + i * kBK;
                 if (!sm100::mbar_wait(empty_bar(stage), phase ^ 1u, abort)) {
                     break;
                 }
                 const uint32_t a_dst = smem_base + stage * R::kStage;
-                const uint32_t b_dst = a_dst + R::kStageA;
                 const uint32_t bar = full_bar(stage);
-                sm100::mbar_expect_tx(bar, R::kStage);
+                if (i >= early) {
+                    sm100::mbar_expect_tx(bar, R::kStage);
+                    fetch_b(a_dst + R::kStageA, bar, kk);
+                }
                 if constexpr (!kAMn) {
                     if (p.batched) {
                         sm100::tma_load_3d(a_dst, &p.map_a, bar, kk, row_a, batch);
@@ -1237,23 +1267,6 @@ __global__ void __launch_bounds__(kOnceThreads, 1)
                                                batch);
                         } else {
                             sm100::tma_load_2d(a_dst + j * 8192, &p.map_a, bar, row_a + 64 * j, kk);
-                        }
-                    }
-                }
-                if constexpr (!kBMn) {
-                    if (p.batched) {
-                        sm100::tma_load_3d(b_dst, &p.map_b, bar, kk, row_b, batch);
-                    } else {
-                        sm100::tma_load_2d(b_dst, &p.map_b, bar, kk, row_b);
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < BN / 64; ++j) {
-                        if (p.batched) {
-                            sm100::tma_load_3d(b_dst + j * 8192, &p.map_b, bar, row_b + 64 * j, kk,
-                                               batch);
-                        } else {
-                            sm100::tma_load_2d(b_dst + j * 8192, &p.map_b, bar, row_b + 64 * j, kk);
                         }
                     }
                 }
@@ -2514,7 +2527,7 @@ cudaError_t launch_pair(GemmParams& p, const void* x, const void* w, int sms, cu
 }
 
 template <Layout L, Epilogue E, int BN>
-cudaError_t launch_once(GemmParams& p, const void* x, const void* w, const Plan& plan,
+cudaError_t launch_once(GemmParams& p, const void* x, const void* w, const Plan& plan, bool steady_w,
                         cudaStream_t stream) {
     const int cluster = plan.cluster;
     using R = OnceRing<BN>;
@@ -2525,6 +2538,7 @@ cudaError_t launch_once(GemmParams& p, const void* x, const void* w, const Plan&
     constexpr bool kFloatOut = E == Epilogue::kBiasResidual || E == Epilogue::kTnStore;
     auto wide = [](const void* at) { return reinterpret_cast<uintptr_t>(at) % 32 == 0; };
     OnceParams once;
+    once.steady_b = steady_w ? 1 : 0;
     once.wide_out = p.n % (kFloatOut ? 8 : 16) == 0 && wide(p.y) && wide(p.aux_out);
     once.cluster = cluster;
     once.parts = plan.parts;
@@ -2550,7 +2564,7 @@ cudaError_t launch_once(GemmParams& p, const void* x, const void* w, const Plan&
 
 template <Layout L, Epilogue E>
 cudaError_t launch_any(GemmParams& p, const void* x, const void* w, cudaStream_t stream,
-                       const Plan* given = nullptr) {
+                       const Plan* given = nullptr, bool steady_w = false) {
     int sms = 0;
     cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) {
@@ -2568,11 +2582,11 @@ cudaError_t launch_any(GemmParams& p, const void* x, const void* w, cudaStream_t
     if constexpr (E != Epilogue::kTnPartial) {
         switch (plan.tile) {
         case Tile::kOnce192:
-            return launch_once<L, E, 192>(p, x, w, plan, stream);
+            return launch_once<L, E, 192>(p, x, w, plan, steady_w, stream);
         case Tile::kOnce128:
-            return launch_once<L, E, 128>(p, x, w, plan, stream);
+            return launch_once<L, E, 128>(p, x, w, plan, steady_w, stream);
         case Tile::kOnce64:
-            return launch_once<L, E, 64>(p, x, w, plan, stream);
+            return launch_once<L, E, 64>(p, x, w, plan, steady_w, stream);
         default:
             break;
         }
@@ -2627,7 +2641,7 @@ TnSplit tn_split(size_t m, size_t n, size_t k, int sms) {
 
 cudaError_t gemm_nt(Epilogue e, void* y, void* pre, const void* x, const void* w,
                     const void* bias, const void* residual, size_t m, size_t n, size_t k,
-                    cudaStream_t stream) {
+                    cudaStream_t stream, bool steady_w) {
     GemmParams p = base_params(y, m, n, k, 1, false);
     p.bias = static_cast<const float*>(bias);
     p.aux_out = pre;
@@ -2636,11 +2650,11 @@ cudaError_t gemm_nt(Epilogue e, void* y, void* pre, const void* x, const void* w
     case Epilogue::kNone:
         return launch_any<Layout::kNT, Epilogue::kNone>(p, x, w, stream);
     case Epilogue::kBias:
-        return launch_any<Layout::kNT, Epilogue::kBias>(p, x, w, stream);
+        return launch_any<Layout::kNT, Epilogue::kBias>(p, x, w, stream, nullptr, steady_w);
     case Epilogue::kBiasGelu:
-        return launch_any<Layout::kNT, Epilogue::kBiasGelu>(p, x, w, stream);
+        return launch_any<Layout::kNT, Epilogue::kBiasGelu>(p, x, w, stream, nullptr, steady_w);
     case Epilogue::kBiasResidual:
-        return launch_any<Layout::kNT, Epilogue::kBiasResidual>(p, x, w, stream);
+        return launch_any<Layout::kNT, Epilogue::kBiasResidual>(p, x, w, stream, nullptr, steady_w);
     default:
         return cudaErrorInvalidValue;
     }

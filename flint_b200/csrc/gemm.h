@@ -31,9 +31,12 @@ struct TnSplit {
 
 TnSplit tn_split(size_t m, size_t n, size_t k, int sms);
 
+// steady_w: nothing that may still run when the kernel before this launch begins writes w (it
+// was written at least two kernels earlier in the stream, each of which keeps to what common.h asks
+// of a dependent launch, or is an ordinary one); its first tiles may then be fetched early.
 cudaError_t gemm_nt(Epilogue e, void* y, void* pre, const void* x, const void* w,
                     const void* bias, const void* residual, size_t m, size_t n, size_t k,
-                    cudaStream_t stream);
+                    cudaStream_t stream, bool steady_w = false);
 
 cudaError_t gemm_nn(Epilogue e, void* y, const void* x, const void* w, const void* pre, size_t m,
                     size_t n, size_t k, cudaStream_t stream);

@@ -82,6 +82,28 @@ def test_prefill_and_teacher_forced_steps_match_the_full_model(flint, sequences,
 
 
 @pytest.mark.parametrize("int8", [False, True], ids=["fp16", "int8"])
+@pytest.mark.parametrize("layers, sequences, heads, prompt", [(1, 1, 2, 8), (1, 20, 4, 24), (3, 64, 2, 8), (2, 5, 14, 136)])
+def test_prompt_logits_come_from_the_last_rows_alone(flint, layers, sequences, heads, prompt, int8):
+    """Behind the last block's attention a prompt goes on with one row per sequence, on the decode
+    kernels: 1 to 64 rows, a model whose first block is its last, and the cache that a step then reads."""
+    cfg = dict(n_layer=layers, n_head=heads, n_embd=64 * heads, block_size=160, vocab_size=200, padded_vocab_size=208)
+    params = weights(cfg)
+    g = torch.Generator().manual_seed(7)
+    tokens = torch.randint(0, 200, (sequences, prompt + 1), generator=g)
+    want = oracle.gpt2_decode_logits(cfg, params, tokens, int8=int8)
+    model = model_for(flint, cfg, params)
+    try:
+        with Generator(flint, model, sequences, 160, int8) as gen:
+            gen.prefill(u16(tokens[:, :prompt]))
+            assert rel_l2(gen.logits().cpu(), want[:, prompt - 1]) <= 5e-3
+            gen.step(u16(tokens[:, prompt]))
+            assert rel_l2(gen.logits().cpu(), want[:, prompt]) <= 5e-3
+    finally:
+        model.close()
+    assert not flint.kernel_fault()
+
+
+@pytest.mark.parametrize("int8", [False, True], ids=["fp16", "int8"])
 @pytest.mark.parametrize("sequences, heads, prompt", [(1, 2, 600), (20, 4, 8), (40, 4, 584), (2, 24, 24)])
 def test_decode_kernels_at_their_edges_match_the_full_model(flint, sequences, heads, prompt, int8):
     """More positions than attention stages in shared memory; 17 to 32 and 33 to 64 rows of the
