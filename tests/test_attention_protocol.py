@@ -358,12 +358,12 @@ def test_the_checker_notices_a_wait_that_comes_too_late():
 
 # ---- the dK/dV kernel -------------------------------------------------------------------------
 #
-# fb_attention_dkv: the producer fetches an item's K and V tiles (one shared-memory pair,
+# fb_attention_backward, dkv_items: the producer fetches an item's K and V tiles (one shared-memory pair,
 # refilled once the compute warps have copied the item before into tensor memory) and streams
 # 64-query stages through a ring of four; the MMA warp issues the scores of sub-step h + 1
 # before it waits for sub-step h's probabilities (two accumulator pairs), then the gradient
 # MMAs; sixteen compute warps turn scores into probabilities in place, install the next item's
-# K and V after their last sub-step and write the item's gradients out. fb_attention_dq has the
+# K and V after their last sub-step and write the item's gradients out. dq_items has the
 # same protocol with the roles of queries and keys exchanged.
 
 STAGES = 4         # kBwdStages
