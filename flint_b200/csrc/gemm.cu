@@ -1519,9 +1519,11 @@ __device__ __forceinline__ TileCoord decode_pair_tile(const GemmParams& p, long 
 // outlasts its k loop: 8,192 x 3,072 x 768 44.0 -> 41.9 us, 16,384 rows 82.5 -> 78.9, for a stage
 // of the ring. At k = 1,600 the loop is the longer one: 4,096 x 6,400 68.9 -> 71.6. (Four for dGELU
 // 51.4 -> 59 us, which then has no registers to ask for its pre-activations a chunk ahead; for
-// bias+residual 42 -> 45.)
+// bias+residual 42 -> 45.) The scaled batched product of k = 64, attention's scores, is epilogue
+// alone: 24 x 1,024 x 1,024 15.8 -> 14.0 us, 48 x 512 x 512 10.2 -> 9.2.
 constexpr int kManyWarps = 16;
 constexpr size_t kManyWarpsMostK = 1024;
+constexpr size_t kManyWarpsMostScaledK = 128;
 
 // Residual boxes (kBoxes): with rows of 16-byte multiples and a short k the FP32 residual comes, and
 // the FP32 output leaves, by tensor copies of boxes of 128 rows x 32 columns through a ring in shared
@@ -2518,8 +2520,8 @@ cudaError_t launch_pair(GemmParams& p, const void* x, const void* w, int sms, cu
                                     : launch(fb_gemm_pair<L, E, kEpilogueWarps, true>, kEpilogueWarps, true, configured[1]);
         }
     }
-    if constexpr (E == Epilogue::kBiasGelu) {
-        if (static_cast<size_t>(p.k) <= kManyWarpsMostK) {
+    if constexpr (E == Epilogue::kBiasGelu || E == Epilogue::kScale) {
+        if (static_cast<size_t>(p.k) <= (E == Epilogue::kScale ? kManyWarpsMostScaledK : kManyWarpsMostK)) {
             return launch(fb_gemm_pair<L, E, kManyWarps>, kManyWarps, false, configured[1]);
         }
     }
