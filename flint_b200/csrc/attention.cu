@@ -566,7 +566,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                         sm100::tmem_st_32x16(my_output + c * 16, acc);
                     }
                 }
-                const fb::F2 shift = fb::f2_pack(-m, -m);
+                // (While every key so far scored minus infinity, m is that: -inf - -inf would be NaN.)
+                const float reference = m == -INFINITY ? 0.0f : m;
+                const fb::F2 shift = fb::f2_pack(-reference, -reference);
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     uint32_t packed[16];
@@ -645,7 +647,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 if (tile == 0 && qb > 0) {   // (with one key tile, tile 1 saw none)
                     const float other = merge_max[row];
                     const float top = fmaxf(m, other);
-                    const float mine_by = fast_exp2(m - top), other_by = fast_exp2(other - top);
+                    // A half whose keys all scored minus infinity weighs nothing.
+                    const float reference = top == -INFINITY ? 0.0f : top;
+                    const float mine_by = fast_exp2(m - reference), other_by = fast_exp2(other - reference);
                     total = total * mine_by + merge_sum[row] * other_by;
                     m = top;
 #pragma unroll
@@ -662,6 +666,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                         }
                     }
                 }
+            }
+            if (m == -INFINITY) {
+                total *= 0.0f;   // no key counts: 0 / 0 (the polynomial's least power of two is not 0)
             }
             if (there && stores && q_index < p.length) {
                 const float inv = 1.0f / total;

@@ -71,6 +71,35 @@ def test_attention_of_few_heads(flint, batches, length, size):
     assert np.allclose(lse.cpu().numpy(), want_lse, rtol=1e-4, atol=1e-4)
 
 
+# Keys whose score is minus infinity (an infinity in K) weigh nothing, wherever they lie: one key, which is the
+# only one that a row sees in an odd key tile; the key tiles that one of two accumulators gets, first and
+# only ones among them; the first keys of all, before which a row sees none (0 / 0: NaN, as from softmax).
+# Few heads, whose key tiles are shared between two accumulators, and many, whose are not.
+@pytest.mark.parametrize("batches, length", [(2, 136), (3, 520), (12, 1000), (192, 264)])
+@pytest.mark.parametrize("keys", [range(128, 129), range(128, 256), range(0, 64), range(0, 128), range(0, 130),
+                                  range(64, 200), range(0, 1000, 2), range(256, 1024)], ids=str)
+def test_attention_gives_keys_of_minus_infinity_no_weight(flint, batches, length, keys):
+    g = torch.Generator().manual_seed(length + batches)
+    q, k, v = (torch.randn(batches, length, 64, generator=g).half() for _ in range(3))
+    q[:, :, 5] = q[:, :, 5].abs() + 0.5
+    k[:, [j for j in keys if j < length], 5] = float("-inf")
+    q[-1, 7, 0] = float("nan")      # a row of its own
+    o = torch.full((batches, length, 64), 7.0, dtype=torch.half, device=DEV)
+    lse = torch.zeros(batches, length, device=DEV)
+    flint.attention_forward(o, lse, q.to(DEV), k.to(DEV), v.to(DEV), batches, length, 64, 0.125)
+    torch.cuda.synchronize()
+    assert not flint.kernel_fault()
+    want_o, want_lse = (torch.from_numpy(t) for t in oracle.attention(q, k, v, 0.125))
+    o, lse = o.cpu(), lse.cpu()
+    sees_none = torch.isneginf(want_lse)
+    assert torch.equal(torch.isnan(o), torch.isnan(want_o))
+    assert torch.equal(torch.isnan(lse), torch.isnan(want_lse)) and torch.equal(torch.isneginf(lse), sees_none)
+    counted = ~torch.isnan(want_o[:, :, 0])
+    assert bool(counted.any()) and torch.equal(sees_none | torch.isnan(want_lse), ~counted)
+    assert rel_error(o[counted], want_o[counted]) <= 2e-3
+    assert np.allclose(lse[counted].numpy(), want_lse[counted].numpy(), rtol=1e-4, atol=1e-4)
+
+
 def test_attention_is_deterministic_and_row_zero_copies_v(flint):
     batches, length = 12, 1024
     g = torch.Generator().manual_seed(1)
