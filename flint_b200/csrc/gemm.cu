@@ -65,6 +65,7 @@ struct GemmParams {
     float* partials;      // split TN: [split][m][n] FP32
     int m, n, k;
     int batches;          // 1 for the plain forms
+    int parts;            // of a sum over k, each in order, then added in order (kernels for parts only)
     int splits;           // TN only
     int split_len;        // k per split, a multiple of 64
     int tiles_m, tiles_n;
@@ -656,7 +657,102 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, long long 
     return c;
 }
 
-template <Layout L, Epilogue E, int BN>
+// The blocks of 64 of k that part `part` of `parts` (2 or 4) takes begin here, and end where the next
+// part's begin. (A division here was 0.1 us per part between two issues of products.)
+__device__ __forceinline__ int part_begin(int blocks, int part, int parts) {
+    return blocks * part >> (parts / 2);
+}
+
+// A tile's epilogue where its sums over k are taken in parts (p.parts): each part has an accumulator to
+// itself, in turn, and a warp keeps the running sums of all its chunks in registers, so that the next
+// part's products (of this tile or the next) are on their way meanwhile. `columns` of tensor memory
+// per accumulator, the warp's first chunk at `at` in the first of them; `full` names an accumulator's
+// barrier and `hand_back` returns it. False if a wait gave up.
+// A part costs 0.2 us between the products of two accumulators, which four accumulators instead of two
+// do not change. Batches on these kernels with whole sums -> on fb_gemm_once in parts, which does not
+// overlap its epilogues -> here: 96 x 512 x 256 x 1,024 33.3 -> 63 -> 35 us, 24 x 768 x 768 x 2,048 49.8 -> 82 -> 51,
+// 48 x 512 x 512 x 1,536 38.1 -> 70 -> 40; of one round, 12 x 256 x 256 x 1,024 7.0 -> 8.1 -> 7.6.
+template <Epilogue E, int kChunks, int kStep, typename Full, typename HandBack>
+__device__ __forceinline__ bool finish_parts(const GemmParams& p, uint32_t at, int columns, int& acc,
+                                             uint32_t& acc_phase, Full full, HandBack hand_back,
+                                             volatile int* abort, uint32_t stage, size_t batch_offset,
+                                             long long z, size_t row, int col, int lane) {
+    float sums[kChunks][32];
+#pragma unroll
+    for (int i = 0; i < kChunks; ++i) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            sums[i][j] = -0.0f;   // what a sum begins with: -0 + x is x
+        }
+    }
+    auto add_chunk = [&](int i) {
+#pragma unroll
+        for (int h = 0; h < 32; h += 16) {
+            uint32_t raw[16];
+            sm100::tmem_ld_32x16(at + static_cast<uint32_t>(acc * columns + i * kStep + h), raw);
+            sm100::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; j += 8) {   // (nothing that reads them moves above the wait)
+                asm volatile(""
+                             : "+r"(raw[j]), "+r"(raw[j + 1]), "+r"(raw[j + 2]), "+r"(raw[j + 3]),
+                               "+r"(raw[j + 4]), "+r"(raw[j + 5]), "+r"(raw[j + 6]), "+r"(raw[j + 7]));
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                sums[i][h + j] = __fadd_rn(sums[i][h + j], __uint_as_float(raw[j]));
+            }
+        }
+    };
+    auto done_with_accumulator = [&]() {
+        sm100::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+            hand_back(acc);
+        }
+        acc ^= 1;
+        if (acc == 0) {
+            acc_phase ^= 1u;
+        }
+    };
+#pragma unroll 1
+    for (int part = 1; part < p.parts; ++part) {
+        if (!sm100::mbar_wait_warp(full(acc), acc_phase, abort)) {
+            return false;
+        }
+        sm100::tc_fence_after_sync();
+#pragma unroll
+        for (int i = 0; i < kChunks; ++i) {
+            add_chunk(i);
+        }
+        done_with_accumulator();
+    }
+    if (!sm100::mbar_wait_warp(full(acc), acc_phase, abort)) {
+        return false;
+    }
+    sm100::tc_fence_after_sync();
+    const bool coalesced = chunk_path_ok<E>(p);
+#pragma unroll
+    for (int i = 0; i < kChunks; ++i) {
+        add_chunk(i);
+        if (i + 1 == kChunks) {
+            done_with_accumulator();
+        }
+        const int valid = min(32, p.n - (col + i * kStep));  // warp-uniform
+        if (valid <= 0) {
+            continue;
+        }
+        if (coalesced) {
+            store_chunk<E>(p, stage, batch_offset, z, row - lane, col + i * kStep, sums[i], valid, lane,
+                           Aux<E>{}, 0.0f);
+        } else if (row < static_cast<size_t>(p.m)) {
+            store_segment<E>(p, batch_offset, z, row, col + i * kStep, sums[i], valid);
+        }
+    }
+    return true;
+}
+
+// kParted: sums over k in p.parts parts (batches of products whose shape takes them so).
+template <Layout L, Epilogue E, int BN, bool kParted = false>
 __global__ void __launch_bounds__(kThreads, 1)
     fb_gemm_tc(const __grid_constant__ GemmParams p) {
     using R = Ring<BN>;
@@ -793,46 +889,51 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const bool split_k = kIsTn && !p.batched;
                 const int k0 = split_k ? static_cast<int>(t.z) * p.split_len : 0;
                 const int k1 = split_k ? min(p.k, k0 + p.split_len) : p.k;
-                if (sm100::elect_one()) {
-                    alive = alive && sm100::mbar_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort);
-                }
-                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-                uint32_t accumulate = 0;
-                for (int kk = k0; kk < k1; kk += kBK) {
-                    const uint32_t a_addr = smem_base + stage * R::kStage;
-                    const uint32_t b_addr = a_addr + R::kStageA;
-                    const uint64_t a_desc = kAMn ? sm100::smem_desc_sw128(a_addr, 8192, 1024)
-                                                 : sm100::smem_desc_sw128(a_addr, 16, 1024);
-                    const uint64_t b_desc = kBMn ? sm100::smem_desc_sw128(b_addr, 8192, 1024)
-                                                 : sm100::smem_desc_sw128(b_addr, 16, 1024);
+                for (int part = 0; part < (kParted ? p.parts : 1); ++part) {
+                    const int blocks = (p.k + kBK - 1) / kBK;
+                    const int from = kParted ? part_begin(blocks, part, p.parts) * kBK : k0;
+                    const int to = kParted ? part_begin(blocks, part + 1, p.parts) * kBK : k1;
                     if (sm100::elect_one()) {
-                        alive = alive && sm100::mbar_wait(full_bar(stage), phase, abort);
-                        if (alive) {
-                            sm100::tc_fence_after_sync();
+                        alive = alive && sm100::mbar_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort);
+                    }
+                    const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
+                    uint32_t accumulate = 0;
+                    for (int kk = from; kk < to; kk += kBK) {
+                        const uint32_t a_addr = smem_base + stage * R::kStage;
+                        const uint32_t b_addr = a_addr + R::kStageA;
+                        const uint64_t a_desc = kAMn ? sm100::smem_desc_sw128(a_addr, 8192, 1024)
+                                                     : sm100::smem_desc_sw128(a_addr, 16, 1024);
+                        const uint64_t b_desc = kBMn ? sm100::smem_desc_sw128(b_addr, 8192, 1024)
+                                                     : sm100::smem_desc_sw128(b_addr, 16, 1024);
+                        if (sm100::elect_one()) {
+                            alive = alive && sm100::mbar_wait(full_bar(stage), phase, abort);
+                            if (alive) {
+                                sm100::tc_fence_after_sync();
 #pragma unroll
-                            for (int ks = 0; ks < kBK / 16; ++ks) {
-                                if (ks == 0) {
-                                    sm100::mma_f16_ss_at<-1>(d_tmem, a_desc, 0, b_desc, 0, kIdesc, accumulate);
-                                } else {
-                                    sm100::mma_f16_ss_at<1>(d_tmem, a_desc, ks * (kAMn ? 128 : 2), b_desc,
-                                                            ks * (kBMn ? 128 : 2), kIdesc);
+                                for (int ks = 0; ks < kBK / 16; ++ks) {
+                                    if (ks == 0) {
+                                        sm100::mma_f16_ss_at<-1>(d_tmem, a_desc, 0, b_desc, 0, kIdesc, accumulate);
+                                    } else {
+                                        sm100::mma_f16_ss_at<1>(d_tmem, a_desc, ks * (kAMn ? 128 : 2), b_desc,
+                                                                ks * (kBMn ? 128 : 2), kIdesc);
+                                    }
                                 }
+                                sm100::mma_commit(empty_bar(stage));
                             }
-                            sm100::mma_commit(empty_bar(stage));
+                        }
+                        accumulate = 1;
+                        if (++stage == R::kStages) {
+                            stage = 0;
+                            phase ^= 1u;
                         }
                     }
-                    accumulate = 1;
-                    if (++stage == R::kStages) {
-                        stage = 0;
-                        phase ^= 1u;
+                    if (sm100::elect_one() && alive) {
+                        sm100::mma_commit(acc_full_bar(acc));
                     }
-                }
-                if (sm100::elect_one() && alive) {
-                    sm100::mma_commit(acc_full_bar(acc));
-                }
-                acc ^= 1;
-                if (acc == 0) {
-                    acc_phase ^= 1u;
+                    acc ^= 1;
+                    if (acc == 0) {
+                        acc_phase ^= 1u;
+                    }
                 }
             }
         }
@@ -853,6 +954,13 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int col0 = t.tn * BN;
             const size_t batch_offset =
                 p.batched ? static_cast<size_t>(t.z) * p.m * static_cast<size_t>(p.n) : 0;
+            if constexpr (kParted) {
+                ok = finish_parts<E, BN / 64, 64>(
+                    p, tmem_base + (static_cast<uint32_t>(quadrant * 32) << 16) + column_half * 32, BN, acc, acc_phase,
+                    acc_full_bar, [&](int a) { sm100::mbar_arrive(acc_empty_bar(a)); }, abort, stage, batch_offset, t.z,
+                    row, col0 + column_half * 32, lane);
+                continue;
+            }
             // The first chunk's second operands are requested before the accumulator is
             // awaited, each later chunk's while the one before it is processed.
             Aux<E> aux;
@@ -953,9 +1061,9 @@ __global__ void __launch_bounds__(kThreads, 1)
 //     (bias+GELU 1,000 x 3,072 x 768: 12.4 -> 10.1 us, with 192 columns a tile);
 //   - stores its rows straight from registers (see store_row): NN 256 x 768 x 768, 64 columns,
 //     5.64 -> 5.54 us, in clusters of two 5.65 -> 5.25.
-// The accumulator is not double-buffered. Where the shape's sums are taken in parts (see
-// sum_parts) but a cluster is not wanted, one CTA forms the same partial sums in as many
-// accumulators.
+// The accumulator is not double-buffered. A batch of products whose shape takes its sums in parts
+// (see sum_parts) but which does not fit the GPU at once runs on the persistent kernels, which
+// then form the same partial sums in one accumulator after the other (see finish_parts).
 
 constexpr int kOnceWarps = 16;   // warp 0 loads and warp 1 issues MMAs before their share of the epilogue
 constexpr int kOnceThreads = 32 * kOnceWarps;
@@ -1127,13 +1235,12 @@ __device__ __forceinline__ void finish_row(const GemmParams& p, bool wide, size_
 struct OnceParams {
     GemmParams gemm;
     int cluster;    // CTAs that share a tile and divide its k
-    int parts;      // accumulators of one CTA, each for a part of k
     int stages;     // of the operand ring
     int wide_out;   // every row segment of the output is 32-byte aligned
     int steady_b;   // B was written before the kernel before this one began: see fetch below
 };
 
-// kParted: k is taken in parts, by a cluster or one after another.
+// kParted: k is divided over a cluster.
 template <Layout L, Epilogue E, int BN, bool kParted>
 __global__ void __launch_bounds__(kOnceThreads, 1)
     fb_gemm_once(const __grid_constant__ OnceParams once) {
@@ -1151,8 +1258,7 @@ __global__ void __launch_bounds__(kOnceThreads, 1)
     const int quadrants = 4 / cluster;          // of 32 rows that this CTA finishes
     const int total = quadrants * kChunks;      // their chunks
     const int stages = once.stages;
-    const int parts = kParted ? once.parts : 1;   // of this CTA's blocks of k, each with an accumulator of its own
-    const uint32_t tmem_columns = parts * BN <= 64 ? 64 : parts * BN <= 128 ? 128 : parts * BN <= 256 ? 256 : 512;
+    constexpr uint32_t kTmemCols = BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
     const uint32_t inbox = smem_base + static_cast<uint32_t>(stages) * R::kStage;
     const uint32_t bars = inbox + static_cast<uint32_t>(total * (cluster - 1)) * 4096u;
     auto full_bar = [&](int s) { return bars + 8u * s; };
@@ -1178,7 +1284,7 @@ __global__ void __launch_bounds__(kOnceThreads, 1)
         sm100::tma_prefetch_descriptor(&p.map_b);
     }
     if (warp == 1) {
-        sm100::tmem_alloc(sm100::smem_u32(&tmem_base_slot), tmem_columns);
+        sm100::tmem_alloc(sm100::smem_u32(&tmem_base_slot), kTmemCols);
     }
     sm100::tc_fence_before_sync();
     __syncthreads();
@@ -1282,16 +1388,7 @@ __global__ void __launch_bounds__(kOnceThreads, 1)
         uint32_t phase = 0;
         bool alive = true;   // the elected lane's: its waits have not given up
         uint32_t accumulate = 0;
-        uint32_t d_tmem = tmem_base;
-        int part = 0;
-        int part_end = blocks / parts;   // (parts > 1 only with the whole of k: cluster == 1)
         for (int i = 0; i < blocks; ++i) {
-            if (i == part_end) {
-                ++part;
-                part_end = blocks * (part + 1) / parts;
-                d_tmem += BN;
-                accumulate = 0;
-            }
             const uint32_t a_addr = smem_base + stage * R::kStage;
             const uint32_t b_addr = a_addr + R::kStageA;
             const uint64_t a_desc = kAMn ? sm100::smem_desc_sw128(a_addr, 8192, 1024)
@@ -1302,10 +1399,10 @@ __global__ void __launch_bounds__(kOnceThreads, 1)
                 alive = alive && sm100::mbar_wait(full_bar(stage), phase, abort);
                 if (alive) {
                     sm100::tc_fence_after_sync();
-                    sm100::mma_f16_ss_at<-1>(d_tmem, a_desc, 0, b_desc, 0, kIdesc, accumulate);
+                    sm100::mma_f16_ss_at<-1>(tmem_base, a_desc, 0, b_desc, 0, kIdesc, accumulate);
 #pragma unroll
                     for (int ks = 1; ks < kBK / 16; ++ks) {
-                        sm100::mma_f16_ss_at<1>(d_tmem, a_desc, ks * (kAMn ? 128 : 2), b_desc,
+                        sm100::mma_f16_ss_at<1>(tmem_base, a_desc, ks * (kAMn ? 128 : 2), b_desc,
                                                 ks * (kBMn ? 128 : 2), kIdesc);
                     }
                     sm100::mma_commit(empty_bar(stage));
@@ -1420,25 +1517,19 @@ __global__ void __launch_bounds__(kOnceThreads, 1)
                     }
                 } else {
                     // The partial sums in the order of k.
-                    const int sums = cluster == 1 ? parts : cluster;
 #pragma unroll 1
-                    for (int r = 0; r < sums; ++r) {
+                    for (int r = 0; r < cluster; ++r) {
                         uint32_t raw[32];
-                        if (cluster == 1) {
-                            sm100::tmem_ld_32x32(t_addr + r * BN + column * 32, raw);
-                            sm100::tmem_ld_wait();
-                        } else {
-                            const int place = r == rank ? work : (r - (r > rank ? 1 : 0)) * total + work;
-                            const uint32_t from =
-                                (r == rank ? smem_base : inbox) + static_cast<uint32_t>(place) * 4096u + lane * 16u;
+                        const int place = r == rank ? work : (r - (r > rank ? 1 : 0)) * total + work;
+                        const uint32_t from =
+                            (r == rank ? smem_base : inbox) + static_cast<uint32_t>(place) * 4096u + lane * 16u;
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                const uint4 q = ld_shared_v4(from + j * 512u);
-                                raw[4 * j] = q.x;
-                                raw[4 * j + 1] = q.y;
-                                raw[4 * j + 2] = q.z;
-                                raw[4 * j + 3] = q.w;
-                            }
+                        for (int j = 0; j < 8; ++j) {
+                            const uint4 q = ld_shared_v4(from + j * 512u);
+                            raw[4 * j] = q.x;
+                            raw[4 * j + 1] = q.y;
+                            raw[4 * j + 2] = q.z;
+                            raw[4 * j + 3] = q.w;
                         }
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
@@ -1477,7 +1568,7 @@ __global__ void __launch_bounds__(kOnceThreads, 1)
     }
     if (warp == 1) {
         sm100::tc_fence_after_sync();
-        sm100::tmem_dealloc(tmem_base, tmem_columns);
+        sm100::tmem_dealloc(tmem_base, kTmemCols);
     }
 }
 
@@ -1546,7 +1637,7 @@ __host__ __device__ constexpr int pair_smem_bytes(int epilogue_warps, bool boxes
            (boxes ? kBoxSlots * kBoxBytes : epilogue_warps * 4096) + 1024 + 256;
 }
 
-template <Layout L, Epilogue E, int kEpi, bool kBoxes = false>
+template <Layout L, Epilogue E, int kEpi, bool kBoxes = false, bool kParted = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(kEpi, kBoxes), 1)
     fb_gemm_pair(const __grid_constant__ GemmParams p) {
     constexpr int kStages = pair_stages(kEpi, kBoxes);
@@ -1697,43 +1788,48 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(kEpi, k
                 const bool split_k = kIsTn && !p.batched;
                 const int k0 = split_k ? static_cast<int>(t.z) * p.split_len : 0;
                 const int k1 = split_k ? min(p.k, k0 + p.split_len) : p.k;
-                if (sm100::elect_one()) {
-                    alive = alive && sm100::mbar_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort);
-                }
-                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kPairBN);
-                uint32_t accumulate = 0;
-                for (int kk = k0; kk < k1; kk += kBK) {
-                    const uint32_t a_addr = smem_base + stage * kPairStage;
-                    const uint32_t b_addr = a_addr + kPairStageA;
-                    const uint64_t a_desc = kAMn ? sm100::smem_desc_sw128(a_addr, 8192, 1024)
-                                                 : sm100::smem_desc_sw128(a_addr, 16, 1024);
-                    const uint64_t b_desc = kBMn ? sm100::smem_desc_sw128(b_addr, 8192, 1024)
-                                                 : sm100::smem_desc_sw128(b_addr, 16, 1024);
+                for (int part = 0; part < (kParted ? p.parts : 1); ++part) {
+                    const int blocks = (p.k + kBK - 1) / kBK;
+                    const int from = kParted ? part_begin(blocks, part, p.parts) * kBK : k0;
+                    const int to = kParted ? part_begin(blocks, part + 1, p.parts) * kBK : k1;
                     if (sm100::elect_one()) {
-                        alive = alive && sm100::mbar_wait(full_bar(stage), phase, abort);
-                        if (alive) {
-                            sm100::tc_fence_after_sync();
+                        alive = alive && sm100::mbar_wait(acc_empty_bar(acc), acc_phase ^ 1u, abort);
+                    }
+                    const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * kPairBN);
+                    uint32_t accumulate = 0;
+                    for (int kk = from; kk < to; kk += kBK) {
+                        const uint32_t a_addr = smem_base + stage * kPairStage;
+                        const uint32_t b_addr = a_addr + kPairStageA;
+                        const uint64_t a_desc = kAMn ? sm100::smem_desc_sw128(a_addr, 8192, 1024)
+                                                     : sm100::smem_desc_sw128(a_addr, 16, 1024);
+                        const uint64_t b_desc = kBMn ? sm100::smem_desc_sw128(b_addr, 8192, 1024)
+                                                     : sm100::smem_desc_sw128(b_addr, 16, 1024);
+                        if (sm100::elect_one()) {
+                            alive = alive && sm100::mbar_wait(full_bar(stage), phase, abort);
+                            if (alive) {
+                                sm100::tc_fence_after_sync();
 #pragma unroll
-                            for (int ks = 0; ks < kBK / 16; ++ks) {
-                                sm100::mma_f16_ss_pair(d_tmem, a_desc + ks * (kAMn ? 128 : 2),
-                                                       b_desc + ks * (kBMn ? 128 : 2), kIdesc,
-                                                       ks == 0 ? accumulate : 1u);
+                                for (int ks = 0; ks < kBK / 16; ++ks) {
+                                    sm100::mma_f16_ss_pair(d_tmem, a_desc + ks * (kAMn ? 128 : 2),
+                                                           b_desc + ks * (kBMn ? 128 : 2), kIdesc,
+                                                           ks == 0 ? accumulate : 1u);
+                                }
+                                sm100::mma_commit_pair(empty_bar(stage), 3);
                             }
-                            sm100::mma_commit_pair(empty_bar(stage), 3);
+                        }
+                        accumulate = 1;
+                        if (++stage == kStages) {
+                            stage = 0;
+                            phase ^= 1u;
                         }
                     }
-                    accumulate = 1;
-                    if (++stage == kStages) {
-                        stage = 0;
-                        phase ^= 1u;
+                    if (sm100::elect_one() && alive) {
+                        sm100::mma_commit_pair(acc_full_bar(acc), 3);
                     }
-                }
-                if (sm100::elect_one() && alive) {
-                    sm100::mma_commit_pair(acc_full_bar(acc), 3);
-                }
-                acc ^= 1;
-                if (acc == 0) {
-                    acc_phase ^= 1u;
+                    acc ^= 1;
+                    if (acc == 0) {
+                        acc_phase ^= 1u;
+                    }
                 }
             }
         }
@@ -1877,6 +1973,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(kEpi, k
             const int col0 = t.tn * kPairBN;
             const size_t batch_offset =
                 p.batched ? static_cast<size_t>(t.z) * p.m * static_cast<size_t>(p.n) : 0;
+            if constexpr (kParted) {
+                ok = finish_parts<E, kPairBN / kColumnStep, kColumnStep>(
+                    p, tmem_base + (static_cast<uint32_t>(quadrant * 32) << 16) + column_part * 32, kPairBN, acc,
+                    acc_phase, acc_full_bar,
+                    [&](int a) { sm100::mbar_arrive_cluster(sm100::map_to_cta(acc_empty_bar(a), 0)); }, abort, stage,
+                    batch_offset, t.z, row, col0 + column_part * 32, lane);
+                continue;
+            }
             if (prefetch && !aux_requested && p.n - (col0 + column_part * 32) > 0) {
                 load_aux<E>(aux, p, batch_offset, row - lane, col0 + column_part * 32,
                             min(32, p.n - (col0 + column_part * 32)), lane);
@@ -2220,7 +2324,7 @@ enum class Tile { k64, k128, k256, kPair, kOnce64, kOnce128, kOnce192 };
 struct Plan {
     Tile tile;
     int cluster;   // CTAs over which fb_gemm_once divides k
-    int parts;     // or its accumulators
+    int parts;     // of a sum over k, on the persistent kernels
     int splits;    // TN: pieces of k with partial sums in the workspace
 };
 
@@ -2289,16 +2393,14 @@ bool tile_fits(Tile t, size_t m, size_t n) {
     }
 }
 
-// fb_gemm_once: microseconds, or 0 where the CTAs would not run at once (a batch of products taken
-// in parts has no other kernel, and may run in rounds) or the tile cannot be used. Of clusters of
-// four, 33 fit this GPU's 148 SMs: a processing cluster of SMs holds whole ones only.
+// fb_gemm_once: microseconds, or 0 where the CTAs would not run at once or the tile cannot be used. Of
+// clusters of four, 33 fit this GPU's 148 SMs: a processing cluster of SMs holds whole ones only.
 double once_time(Tile t, Layout l, Epilogue e, size_t m, size_t n, size_t k, long long batches,
-                 int cluster, int parts, int sms) {
+                 int cluster, int sms) {
     const int i = static_cast<int>(t) - static_cast<int>(Tile::kOnce64);
     const size_t blocks = (k + kBK - 1) / kBK;
     const long long ctas = tile_count(t, m, n) * batches * cluster;
-    const bool at_once = ctas <= (cluster == 4 ? sms * 8 / 9 : sms);
-    if (!tile_fits(t, m, n) || parts * tile_columns(t) > 512 || (!at_once && parts == 1)) {
+    if (!tile_fits(t, m, n) || ctas > (cluster == 4 ? sms * 8 / 9 : sms)) {
         return 0.0;
     }
     constexpr double kBlock[2][3] = {{0.235, 0.265, 0.305}, {0.285, 0.335, 0.37}};
@@ -2336,10 +2438,9 @@ double once_time(Tile t, Layout l, Epilogue e, size_t m, size_t n, size_t k, lon
     }
     // The same in clusters of two and four, the exchange of partial sums included.
     constexpr double kCluster[2][3][2] = {{{4.0, 5.0}, {4.8, 6.1}, {5.7, 7.0}}, {{4.4, 5.5}, {5.2, 6.5}, {6.3, 7.8}}};
-    const double one = (cluster > 1 ? kCluster[cluster / 4][i][busy] + more : rest[i][busy]) +
-                       (l == Layout::kTN && cluster > 1 && i == 2 ? 0.42 : kBlock[l == Layout::kTN][i]) *
-                           static_cast<double>((blocks + cluster - 1) / cluster);
-    return one * static_cast<double>((ctas + sms - 1) / sms);
+    return (cluster > 1 ? kCluster[cluster / 4][i][busy] + more : rest[i][busy]) +
+           (l == Layout::kTN && cluster > 1 && i == 2 ? 0.42 : kBlock[l == Layout::kTN][i]) *
+               static_cast<double>((blocks + cluster - 1) / cluster);
 }
 
 // How often TN may split k with tile `t`: into pieces of at least 1,024, and not at all where
@@ -2372,7 +2473,7 @@ int sum_parts(size_t m, size_t n, size_t k, int sms) {
     int parts = 1;
     for (int cluster : {1, 2, 4}) {
         for (Tile t : kOnceTiles) {
-            const double time = once_time(t, Layout::kNT, Epilogue::kNone, m, n, k, 1, cluster, 1, sms);
+            const double time = once_time(t, Layout::kNT, Epilogue::kNone, m, n, k, 1, cluster, sms);
             if (time != 0.0 && time < (parts < cluster ? 0.95 : 1.0) * best) {
                 best = time;
                 parts = cluster;
@@ -2399,12 +2500,7 @@ Plan pick_plan(Layout l, Epilogue e, size_t m, size_t n, size_t k, long long bat
     const int parts = sum_parts(m, n, k, sms);
     if (parts > 1) {
         for (Tile t : kOnceTiles) {
-            consider(once_time(t, l, e, m, n, k, batches, parts, 1, sms), Plan{t, parts, 1, 1});
-        }
-        if (best == 0.0) {   // a batch of them
-            for (Tile t : {Tile::kOnce128, Tile::kOnce64}) {
-                consider(once_time(t, l, e, m, n, k, batches, 1, parts, sms), Plan{t, 1, parts, 1});
-            }
+            consider(once_time(t, l, e, m, n, k, batches, parts, sms), Plan{t, parts, 1, 1});
         }
     }
     for (Tile t : {Tile::kPair, Tile::k256, Tile::k128, Tile::k64}) {
@@ -2412,12 +2508,13 @@ Plan pick_plan(Layout l, Epilogue e, size_t m, size_t n, size_t k, long long bat
             continue;
         }
         const int most = may_split ? most_splits(t, m, n, k, sms) : 1;
-        for (int s = parts > 1 ? 2 : 1; s <= most; ++s) {
+        // (One product that is taken in parts runs on clusters: sum_parts has seen that they fit.)
+        for (int s = parts > 1 && batches == 1 ? 2 : 1; s <= most; ++s) {
             double time = tile_time(t, l, e, tile_count(t, m, n) * batches * s, (k + s - 1) / s, sms);
             if (s > 1) {
                 time += 1.0 + static_cast<double>(s + 1) * static_cast<double>(m) * static_cast<double>(n) * 4.0 / 16e6;
             }
-            consider(time, Plan{t, 1, 1, s});
+            consider(time, Plan{t, 1, batches > 1 ? parts : 1, s});
         }
         if (t == Tile::kPair && tile_count(t, m, n) * batches > static_cast<long long>(sms)) {
             return plan;  // more than two rounds of pairs
@@ -2425,7 +2522,7 @@ Plan pick_plan(Layout l, Epilogue e, size_t m, size_t n, size_t k, long long bat
     }
     if (parts == 1) {
         for (Tile t : kOnceTiles) {
-            const double time = once_time(t, l, e, m, n, k, batches, 1, 1, sms);
+            const double time = once_time(t, l, e, m, n, k, batches, 1, sms);
             if (time != 0.0 && time < best) {
                 best = time;
                 plan = Plan{t, 1, 1, 1};
@@ -2469,6 +2566,12 @@ cudaError_t make_operand_maps(GemmParams& p, const void* x, const void* w, int c
                             : make_map(&p.map_b, w, p.k, p.n, p.batches, batched, columns);
 }
 
+// The forms that gemm_batched launches.
+template <Layout L, Epilogue E>
+constexpr bool batched_form() {
+    return E == (L == Layout::kNT ? Epilogue::kScale : Epilogue::kNone);
+}
+
 template <Layout L, Epilogue E, int BN>
 cudaError_t launch_tc(GemmParams& p, const void* x, const void* w, int sms, cudaStream_t stream) {
     using R = Ring<BN>;
@@ -2486,14 +2589,21 @@ cudaError_t launch_tc(GemmParams& p, const void* x, const void* w, int sms, cuda
     const long long z = L == Layout::kTN && !batched ? p.splits : p.batches;
     p.tiles_total = static_cast<long long>(p.tiles_m) * p.tiles_n * z;
 
-    static std::atomic<bool> configured[64] = {};
-    auto kernel = fb_gemm_tc<L, E, BN>;
-    e = fb::allow_shared_memory(kernel, R::kSmemBytes, configured);
-    if (e != cudaSuccess) {
-        return e;
+    auto launch = [&](auto kernel, std::atomic<bool> (&configured)[64]) {
+        const cudaError_t error = fb::allow_shared_memory(kernel, R::kSmemBytes, configured);
+        if (error != cudaSuccess) {
+            return error;
+        }
+        const unsigned grid = static_cast<unsigned>(std::min<long long>(p.tiles_total, sms));
+        return fb::launch_dependent(kernel, dim3(grid), dim3(kThreads), R::kSmemBytes, stream, p);
+    };
+    static std::atomic<bool> configured[2][64] = {};
+    if constexpr (batched_form<L, E>()) {
+        if (p.parts > 1) {
+            return launch(fb_gemm_tc<L, E, BN, true>, configured[1]);
+        }
     }
-    const unsigned grid = static_cast<unsigned>(std::min<long long>(p.tiles_total, sms));
-    return fb::launch_dependent(kernel, dim3(grid), dim3(kThreads), R::kSmemBytes, stream, p);
+    return launch(fb_gemm_tc<L, E, BN>, configured[0]);
 }
 
 template <Layout L, Epilogue E>
@@ -2523,7 +2633,12 @@ cudaError_t launch_pair(GemmParams& p, const void* x, const void* w, int sms, cu
                                     dim3(static_cast<unsigned>(pair_threads(epilogue_warps, boxes))),
                                     static_cast<size_t>(smem), stream, p);
     };
-    static std::atomic<bool> configured[2][64] = {};
+    static std::atomic<bool> configured[3][64] = {};
+    if constexpr (batched_form<L, E>()) {
+        if (p.parts > 1) {
+            return launch(fb_gemm_pair<L, E, kEpilogueWarps, false, true>, kEpilogueWarps, false, configured[2]);
+        }
+    }
     if constexpr (E == Epilogue::kBiasResidual) {
         if (p.n % 4 == 0 && static_cast<size_t>(p.k) <= kBoxesMostK) {
             e = make_box_maps(p);
@@ -2554,7 +2669,6 @@ cudaError_t launch_once(GemmParams& p, const void* x, const void* w, const Plan&
     once.steady_b = steady_w ? 1 : 0;
     once.wide_out = p.n % (kFloatOut ? 8 : 16) == 0 && wide(p.y) && wide(p.aux_out);
     once.cluster = cluster;
-    once.parts = plan.parts;
     p.tiles_m = (p.m + kBM - 1) / kBM;
     p.tiles_n = (p.n + BN - 1) / BN;
     p.tiles_total = static_cast<long long>(p.tiles_m) * p.tiles_n * p.batches;
@@ -2571,7 +2685,7 @@ cudaError_t launch_once(GemmParams& p, const void* x, const void* w, const Plan&
                                             R::bytes(cluster), stream, once);
     };
     static std::atomic<bool> configured[2][64] = {};
-    return cluster * plan.parts > 1 ? launch(fb_gemm_once<L, E, BN, true>, configured[1])
+    return cluster > 1 ? launch(fb_gemm_once<L, E, BN, true>, configured[1])
                                     : launch(fb_gemm_once<L, E, BN, false>, configured[0]);
 }
 
@@ -2604,6 +2718,7 @@ cudaError_t launch_any(GemmParams& p, const void* x, const void* w, cudaStream_t
             break;
         }
     }
+    p.parts = plan.parts;
     switch (plan.tile) {
     case Tile::kPair:
         return launch_pair<L, E>(p, x, w, sms, stream);
@@ -2625,6 +2740,7 @@ GemmParams base_params(void* y, size_t m, size_t n, size_t k, size_t batches, bo
     p.k = static_cast<int>(k);
     p.batches = static_cast<int>(batches);
     p.batched = batched ? 1 : 0;
+    p.parts = 1;
     p.splits = 1;
     p.split_len = static_cast<int>((k + kBK - 1) / kBK * kBK);
     p.scale = 1.0f;

@@ -483,6 +483,53 @@ def test_sums_in_parts_agree_between_layouts_epilogues_and_batches(flint, m, n, 
     no_fault(flint)
 
 
+def guarded(batches, m, n):
+    space = torch.full((batches * m * n + 64,), 7.0, dtype=torch.half, device=DEV)
+    return space, space[32:-32].view(batches, m, n)
+
+
+# Batches that fill the GPU more than once and take their sums over k in two or four parts: on tiles of 64, 128 and
+# 256 columns and on CTA pairs. Rows and columns that end inside a tile, whole chunks outside, NT's rows
+# of odd length (stored a value at a time), k whose blocks do not divide evenly.
+@pytest.mark.parametrize("batches, m, n, k", [(14, 104, 264, 1032), (14, 104, 261, 1032), (40, 200, 264, 1032),
+                                              (40, 200, 261, 1032), (24, 72, 1032, 1032), (24, 72, 1031, 1032),
+                                              (24, 392, 488, 1544), (24, 392, 485, 2056)])
+def test_many_products_in_parts_equal_the_plain_ones(flint, batches, m, n, k):
+    g = torch.Generator(device=DEV).manual_seed(m + n)
+    x = torch.randn(batches, m, k, generator=g, device=DEV).half()
+    w = torch.randn(batches, n, k, generator=g, device=DEV).half()
+    xt, wt = x.transpose(1, 2).contiguous(), w.transpose(1, 2).contiguous()
+    one = torch.empty(m, n, dtype=torch.half, device=DEV)
+    spaces, outs = zip(*(guarded(batches, m, n) for _ in range(3 if n % 8 == 0 else 1)))
+    flint.gemm_nt_batched(outs[0], x, w, batches, m, n, k)
+    if n % 8 == 0:
+        flint.gemm_nn_batched(outs[1], x, wt, batches, m, n, k)
+        flint.gemm_tn_batched(outs[2], xt, wt, batches, m, n, k)
+    for j in range(batches):
+        flint.gemm_nt(one, x[j], w[j], m, n, k)
+        assert all(torch.equal(out[j], one) for out in outs), j
+    no_fault(flint)
+    for j in (0, batches - 1):
+        assert rel_error(outs[0][j], oracle.gemm_nt(x[j].cpu(), w[j].cpu())) <= 2e-3
+    assert all(bool((s[:32] == 7).all()) and bool((s[-32:] == 7).all()) for s in spaces)
+
+
+# Scores of more than two rounds of CTA pairs at lengths that are no multiple of a tile (sixteen epilogue warps up
+# to k = 128, eight beyond): edges inside a tile, chunks wholly outside, rows of odd length.
+@pytest.mark.parametrize("batches, m, n, k", [(24, 1000, 1000, 64), (30, 904, 904, 72), (30, 904, 903, 72),
+                                              (24, 1000, 1000, 136)])
+def test_ragged_scaled_batches_on_cta_pairs(flint, batches, m, n, k):
+    g = torch.Generator().manual_seed(m + n + k)
+    x = torch.randn(batches, m, k, generator=g).half()
+    w = torch.randn(batches, n, k, generator=g).half()
+    space, y = guarded(batches, m, n)
+    flint.gemm_nt_batched(y, x.to(DEV), w.to(DEV), batches, m, n, k, 0.125)
+    no_fault(flint)
+    for j in range(batches):
+        assert rel_error(y[j], oracle.gemm_nt(x[j], w[j]) * 0.125) <= 2e-3, j
+    assert bool((space[:32] == 7).all()) and bool((space[-32:] == 7).all())
+
+
 # Rows stored straight from registers: 16-byte pieces, 32-byte pieces, and two bytes at a time.
 @pytest.mark.parametrize("m, n, offset", [(70, 72, 0), (70, 80, 0), (70, 80, 16), (70, 77, 0), (129, 200, 0)])
 def test_small_problem_rows_at_every_alignment(flint, m, n, offset):
