@@ -256,22 +256,25 @@ def _bind(lib, functions: dict) -> None:
 
 
 def _caller(function, params):
-    """A Python function of the C function's parameters that converts and passes them: tensors
-    become addresses, bools ints; the stream comes last. Written out for the one signature, because
-    deciding each argument's treatment on every call took longer than the launch."""
-    names = [f"a{i}" for i in range(len(params))]
-    passed = []
-    for (c_type, _), name in zip(params, names):
-        if c_type == "flint_stream":
-            passed.append(f"stream_handle({name})")
-        elif _C_TYPES[c_type] is ctypes.c_void_p:
+    """A Python function of the C function's parameters but the stream, and then the stream (which it
+    ignores where there is none), that converts and passes them: tensors become addresses, bools
+    ints. Written out for the one signature, because deciding each argument's treatment on every call
+    took longer than the launch."""
+    names, passed = [], []
+    for c_type, _ in params:
+        if c_type == "flint_stream":     # wherever it stands in the C signature
+            passed.append("stream_handle(stream)")
+            continue
+        name = f"a{len(names)}"
+        names.append(name)
+        if _C_TYPES[c_type] is ctypes.c_void_p:
             passed.append(f"{name} if {name} is None or isinstance({name}, int) else {name}.data_ptr()")
         elif c_type == "int":
             passed.append(f"int({name})")
         else:
             passed.append(name)
     scope = {"function": function, "stream_handle": stream_handle}
-    return eval(f"lambda {', '.join(names)}: function({', '.join(passed)})", scope)
+    return eval(f"lambda {', '.join([*names, 'stream'])}: function({', '.join(passed)})", scope)
 
 
 class Flint:
@@ -328,13 +331,10 @@ class Flint:
 
     def call(self, name: str, *args, stream=None):
         """Calls a status-returning function: tensors become addresses, bools ints, and
-        the stream argument (always last in the C signature) is filled in."""
+        the stream argument is filled in where the C signature has it."""
         caller = self._callers.get(name)
         if caller is None:
-            params = self.functions[name][1]
-            caller = _caller(getattr(self.lib, name), params)
-            if all(c_type != "flint_stream" for c_type, _ in params):
-                caller = (lambda inner: lambda *values: inner(*values[:-1]))(caller)
+            caller = _caller(getattr(self.lib, name), self.functions[name][1])
             self._callers[name] = caller
         status = caller(*args, stream)
         if status != OK:

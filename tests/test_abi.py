@@ -115,6 +115,23 @@ def test_validation_runs_before_any_cuda_call(flint):
     flint.causal_softmax_forward(None, None, 0, 8, stream=s)
 
 
+@pytest.mark.parametrize("name", sorted(n for n, (ret, _) in binding.declared_functions().items()
+                                        if ret == "flint_status"))
+def test_call_puts_the_stream_where_the_signature_has_it(name):
+    """Flint.call takes the arguments but the stream in C order: three functions have it before
+    their last parameter, and some have none."""
+    params = binding.declared_functions()[name][1]
+    seen = []
+    flint = flint_b200.Flint.__new__(flint_b200.Flint)
+    flint.functions, flint._callers = binding.declared_functions(), {}
+    flint.lib = type("Library", (), {name: staticmethod(lambda *values: seen.append(values) or 0)})()
+    want = [-7 if c_type == "flint_stream" else 100 + i for i, (c_type, _) in enumerate(params)]
+    flint.call(name, *(value for value in want if value != -7), stream=-7)
+    assert seen == [tuple(want)]
+    with pytest.raises(TypeError):
+        flint.call(name, *want, 1, stream=-7)
+
+
 def test_workspace_formulas(flint):
     assert flint.bias_gradient_workspace(8192, 768) == 32 * 768 * 8
     assert flint.bias_gradient_workspace(257, 8) == 2 * 8 * 8
