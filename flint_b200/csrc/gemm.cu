@@ -2406,9 +2406,9 @@ double once_time(Tile t, Layout l, Epilogue e, size_t m, size_t n, size_t k, lon
     constexpr double kBlock[2][3] = {{0.235, 0.265, 0.305}, {0.285, 0.335, 0.37}};
     // Everything but the k loop, with up to half of the SMs and with more of them at work.
     const int busy = ctas > sms / 2;
-    constexpr double kNone[3][2] = {{2.3, 3.0}, {2.9, 3.8}, {3.3, 4.6}}, kBias[3][2] = {{2.6, 3.0}, {3.1, 3.9}, {3.9, 4.6}},
-                     kGelu[3][2] = {{3.3, 3.8}, {4.1, 5.0}, {5.4, 6.2}}, kDGelu[3][2] = {{3.4, 3.8}, {4.6, 5.1}, {6.9, 7.7}},
-                     kResidual[3][2] = {{3.3, 3.9}, {4.5, 5.4}, {6.7, 8.9}}, kTn[3][2] = {{2.6, 3.2}, {3.3, 4.2}, {4.6, 5.4}};
+    constexpr double kNone[3][2] = {{2.3, 3.0}, {2.9, 3.8}, {3.9, 4.6}}, kBias[3][2] = {{2.6, 3.0}, {3.1, 3.9}, {3.9, 4.6}},
+                     kGelu[3][2] = {{3.3, 3.8}, {4.1, 5.3}, {5.4, 6.2}}, kDGelu[3][2] = {{3.4, 3.8}, {4.6, 5.1}, {6.9, 7.7}},
+                     kResidual[3][2] = {{3.3, 4.0}, {4.5, 5.4}, {6.7, 8.9}}, kTn[3][2] = {{3.5, 4.1}, {3.9, 4.2}, {4.6, 5.4}};
     const double(*rest)[2] = kNone;
     double more = 0.0;   // than a plain epilogue takes in a cluster, where no warp finishes two chunks
     switch (e) {
@@ -2430,17 +2430,34 @@ double once_time(Tile t, Layout l, Epilogue e, size_t m, size_t n, size_t k, lon
         break;
     case Epilogue::kTnStore:
     case Epilogue::kTnPartial:
-        rest = kTn;
-        more = 0.2;
+        rest = kTn;   // (clusters of two at 0.2 more gave up splits in memory: 1,024 x 1,024 x 3,072 13.7 -> 14.9 us)
+        more = cluster == 2 && busy != 0 ? 1.2 : 0.2;
         break;
     default:
         break;
     }
     // The same in clusters of two and four, the exchange of partial sums included.
     constexpr double kCluster[2][3][2] = {{{4.0, 5.0}, {4.8, 6.1}, {5.7, 7.0}}, {{4.4, 5.5}, {5.2, 6.5}, {6.3, 7.8}}};
+    const double block = l == Layout::kTN && cluster > 1 && i == 2 ? 0.42 : kBlock[l == Layout::kTN][i];
     return (cluster > 1 ? kCluster[cluster / 4][i][busy] + more : rest[i][busy]) +
-           (l == Layout::kTN && cluster > 1 && i == 2 ? 0.42 : kBlock[l == Layout::kTN][i]) *
-               static_cast<double>((blocks + cluster - 1) / cluster);
+           block * static_cast<double>((blocks + cluster - 1) / cluster);
+}
+
+// What whole sums on fb_gemm_once's 64-column tile take beyond that: past the ring's first rounds its loads
+// are slower where most SMs load, or rows are many, and always for TN. (Without this fb_gemm_tc's tile
+// was given up for a loss: 2,048 x 512 x 2,048 10.6 -> 11.1 us, with the residual 10.9 -> 11.8, TN 2,048 x 512 x 768
+// 6.7 -> 7.2. sum_parts does without: bits change with it.)
+double late_blocks(Tile t, Layout l, size_t m, size_t n, size_t k, long long batches, int sms) {
+    const double blocks = static_cast<double>((k + kBK - 1) / kBK);
+    const long long ctas = tile_count(t, m, n) * batches;
+    if (t != Tile::kOnce64) {
+        return 0.0;
+    }
+    if (l == Layout::kTN) {
+        return std::max(0.0, 0.08 * (blocks - 8.0));
+    }
+    const bool many = ctas > sms / 2 && (m > 2 * kBM || (m > kBM && ctas * 4 > sms * 3));
+    return many ? std::max(0.0, 0.04 * (blocks - 10.0)) : 0.0;
 }
 
 // How often TN may split k with tile `t`: into pieces of at least 1,024, and not at all where
@@ -2522,7 +2539,10 @@ Plan pick_plan(Layout l, Epilogue e, size_t m, size_t n, size_t k, long long bat
     }
     if (parts == 1) {
         for (Tile t : kOnceTiles) {
-            const double time = once_time(t, l, e, m, n, k, batches, 1, sms);
+            double time = once_time(t, l, e, m, n, k, batches, 1, sms);
+            if (time != 0.0) {
+                time += late_blocks(t, l, m, n, k, batches, sms);
+            }
             if (time != 0.0 && time < best) {
                 best = time;
                 plan = Plan{t, 1, 1, 1};
