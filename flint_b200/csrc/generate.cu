@@ -1243,15 +1243,6 @@ flint_status run_prompt(flint_b200_generator& g, size_t count, cudaStream_t stre
     return FLINT_OK;
 }
 
-// The rest of the last block for one row per sequence: the residual stream in g.last, the attention
-// output in g.h; the block's output in g.last. (For all rows of a 4 x 256 prompt it took 32 us.)
-flint_status run_last_rows(flint_b200_generator& g, cudaStream_t stream) {
-    const Layer& l = g.blocks.back();
-    FB_TRY(decode_linear<Act::kResidual>(g, l.proj, g.x_b, g.h, nullptr, nullptr, g.last, stream));
-    FB_TRY(decode_linear<Act::kGelu>(g, l.fc, g.act, g.x_b, l.ln2_w, l.ln2_b, nullptr, stream));
-    return decode_linear<Act::kResidual>(g, l.fcproj, g.last, g.act, nullptr, nullptr, g.x_b, stream);
-}
-
 // Whether a step's linear layers run on the prompt's GEMMs (FP16 weights only: int8 ones would be
 // expanded on every step). The step's own kernels read every row in every CTA, which grows with
 // rows times width and passes what 128-row tensor-core tiles waste at about 33 rows of 1,280, 41
@@ -1261,6 +1252,24 @@ flint_status run_last_rows(flint_b200_generator& g, cudaStream_t stream) {
 // 40 x 1,024 941 -> 959, 64 x 768 852 -> 886, 32 x 1,536 1,209 -> 1,251.
 bool tensor_core_step(const flint_b200_generator& g) {
     return !g.int8 && g.sequences > 32 && g.width > 768 && g.sequences * g.width >= 42000;
+}
+
+// The rest of the last block for one row per sequence, on what a step would use: the residual stream in
+// g.last, the attention output in g.h; the block's output in g.last. (For all rows of a 4 x 256
+// prompt it took 32 us. FP16, 64 sequences of 8 tokens at 1,536 columns, one layer: 164 us with all 512
+// rows on the GEMMs, 173 with the last 64 on the decode kernels, 131 with those on the GEMMs.)
+flint_status run_last_rows(flint_b200_generator& g, cudaStream_t stream) {
+    const Layer& l = g.blocks.back();
+    if (tensor_core_step(g)) {
+        const size_t rows = g.sequences;
+        FB_TRY(linear<Act::kResidual>(g, l.proj, l.proj.half, g.x_b, g.h, g.last, rows, stream));
+        FB_TRY(layernorm(g, l.ln2_w, l.ln2_b, g.x_b, rows, stream));
+        FB_TRY(linear<Act::kGelu>(g, l.fc, l.fc.half, g.act, g.h, nullptr, rows, stream));
+        return linear<Act::kResidual>(g, l.fcproj, l.fcproj.half, g.last, g.act, g.x_b, rows, stream);
+    }
+    FB_TRY(decode_linear<Act::kResidual>(g, l.proj, g.x_b, g.h, nullptr, nullptr, g.last, stream));
+    FB_TRY(decode_linear<Act::kGelu>(g, l.fc, g.act, g.x_b, l.ln2_w, l.ln2_b, nullptr, stream));
+    return decode_linear<Act::kResidual>(g, l.fcproj, g.last, g.act, nullptr, nullptr, g.x_b, stream);
 }
 
 // The transformer over one new position per sequence.

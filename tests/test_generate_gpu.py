@@ -104,6 +104,31 @@ def test_prompt_logits_come_from_the_last_rows_alone(flint, layers, sequences, h
 
 
 @pytest.mark.parametrize("int8", [False, True], ids=["fp16", "int8"])
+@pytest.mark.parametrize("layers, sequences, heads", [(1, 64, 24), (2, 33, 20), (1, 33, 16), (1, 64, 12)])
+def test_a_prompts_last_rows_run_on_what_a_step_runs_on(flint, layers, sequences, heads, int8):
+    """Of many sequences of a wide FP16 model a step's linear layers run on the tensor-core GEMMs, with a LayerNorm
+    launch of its own before MLP up; so do the prompt's last rows. The two last cases stay just below that."""
+    cfg = dict(n_layer=layers, n_head=heads, n_embd=64 * heads, block_size=64, vocab_size=200, padded_vocab_size=208)
+    params = weights(cfg)
+    g = torch.Generator().manual_seed(11)
+    tokens = torch.randint(0, 200, (sequences, 8), generator=g)
+    want = oracle.gpt2_decode_logits(cfg, params, tokens, int8=int8)
+    model = model_for(flint, cfg, params)
+    launches = []
+    try:
+        for count in (1, sequences):
+            with Generator(flint, model, count, 64, int8) as gen:
+                before = flint.launch_count()
+                gen.prefill(u16(tokens[:count]))
+                launches.append(flint.launch_count() - before)
+                assert rel_l2(gen.logits().cpu(), want[:count, 7]) <= 5e-3
+    finally:
+        model.close()
+    assert launches[1] - launches[0] == (not int8 and sequences * 64 * heads >= 42000 and heads > 12)
+    assert not flint.kernel_fault()
+
+
+@pytest.mark.parametrize("int8", [False, True], ids=["fp16", "int8"])
 @pytest.mark.parametrize("sequences, heads, prompt", [(1, 2, 600), (20, 4, 8), (40, 4, 584), (2, 24, 24)])
 def test_decode_kernels_at_their_edges_match_the_full_model(flint, sequences, heads, prompt, int8):
     """More positions than attention stages in shared memory; 17 to 32 and 33 to 64 rows of the
