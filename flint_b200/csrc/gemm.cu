@@ -1605,16 +1605,21 @@ __device__ __forceinline__ TileCoord decode_pair_tile(const GemmParams& p, long 
 }
 
 // Epilogue warps per CTA of the pair kernel, with 4 KB of staging each: two per TMEM lane
-// quadrant, and four for bias+GELU over a short k. Those warps mostly wait (with eight, 28 % of the
-// issue slots and 30 % of the special-function unit are in use), and at k = 768 a tile's epilogue
-// outlasts its k loop: 8,192 x 3,072 x 768 44.0 -> 41.9 us, 16,384 rows 82.5 -> 78.9, for a stage
-// of the ring. At k = 1,600 the loop is the longer one: 4,096 x 6,400 68.9 -> 71.6. (Four for dGELU
-// 51.4 -> 59 us, which then has no registers to ask for its pre-activations a chunk ahead; for
-// bias+residual 42 -> 45.) The scaled batched product of k = 64, attention's scores, is epilogue
-// alone: 24 x 1,024 x 1,024 15.8 -> 14.0 us, 48 x 512 x 512 10.2 -> 9.2.
+// quadrant, and four for bias+GELU over a short k in more than one round. Those warps mostly wait (with
+// eight, 28 % of the issue slots and 30 % of the special-function unit are in use), and at k = 768 a tile's
+// epilogue outlasts its k loop: 8,192 x 3,072 x 768 44.8 -> 42.5 us, 16,384 rows 94.2 -> 85.0, for a stage
+// of the ring. With a longer k the loop counts for more: 8,192 x 4,096 and 16,384 x 3,072 gain 2 % at k = 896
+// and lose 5 and 7 % at 1,024. In a single round there is nothing to gain (1,000 x 4,104 x 768 12.5 -> 13.1).
+// (Four for dGELU 51.4 -> 59 us, which then has no registers to ask for its pre-activations a chunk ahead;
+// for bias+residual 42 -> 45.) The scaled batched product of k = 64, attention's scores, is epilogue alone:
+// 24 x 1,024 x 1,024 15.0 -> 13.2 us, 48 x 512 x 512 9.9 -> 8.7.
+// Rows that are no multiples of 32 bytes share sectors, and where the outputs outgrow two thirds of the L2,
+// sixteen warps lose by it: scores of 48 x 904 x 904 24.3 -> 23.2 us but 48 x 1,000 x 1,000 x 128 28.9 -> 32.0, 96 x 904 x 904 44.8 -> 51.5
+// (96 x 992 x 992 44.3 -> 40.2); bias+GELU 8,192 x 2,312 x 512 34.3 -> 31.0 but 8,192 x 4,104 x 768 63.0 -> 65.5.
 constexpr int kManyWarps = 16;
-constexpr size_t kManyWarpsMostK = 1024;
+constexpr size_t kManyWarpsMostK = 960;
 constexpr size_t kManyWarpsMostScaledK = 128;
+constexpr size_t kManyWarpsMostRaggedBytes = size_t{84} << 20;
 
 // Residual boxes (kBoxes): with rows of 16-byte multiples and a short k the FP32 residual comes, and
 // the FP32 output leaves, by tensor copies of boxes of 128 rows x 32 columns through a ring in shared
@@ -2667,7 +2672,10 @@ cudaError_t launch_pair(GemmParams& p, const void* x, const void* w, int sms, cu
         }
     }
     if constexpr (E == Epilogue::kBiasGelu || E == Epilogue::kScale) {
-        if (static_cast<size_t>(p.k) <= (E == Epilogue::kScale ? kManyWarpsMostScaledK : kManyWarpsMostK)) {
+        constexpr bool kScores = E == Epilogue::kScale;
+        const size_t bytes = static_cast<size_t>(p.batches) * p.m * p.n * (kScores ? 2 : 4);   // of all outputs
+        if (static_cast<size_t>(p.k) <= (kScores ? kManyWarpsMostScaledK : kManyWarpsMostK) &&
+            (p.n % 16 == 0 || bytes <= kManyWarpsMostRaggedBytes) && (kScores || p.tiles_total > pairs)) {
             return launch(fb_gemm_pair<L, E, kManyWarps>, kManyWarps, false, configured[1]);
         }
     }
