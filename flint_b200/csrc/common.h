@@ -72,6 +72,11 @@ unsigned long long launch_count();
 // position and older cache rows before their wait. That is right only because the first kernel
 // of their chain is launched the ordinary way (fb_decode_embed of a step, fb_take_last_rows of a
 // prompt), so that whatever wrote those has finished before any of them begins.
+// fb_gemm_once fetches its first weight tiles before its wait where the caller says that the weights
+// are steady (gemm_nt's steady_w): that is right where at least one whole kernel lies between what wrote
+// them and the GEMM, because the GEMM begins only when all but the kernel right before it are over. A
+// prompt's expansion of int8 weights (dense_weights) therefore comes before the block's LayerNorm, not after.
+// tests/test_dependent_launch.py holds both orders.
 bool dependent_launch_enabled();
 
 template <typename... Params, typename... Args>

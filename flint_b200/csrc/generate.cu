@@ -1227,6 +1227,7 @@ flint_status run_prompt(flint_b200_generator& g, size_t count, cudaStream_t stre
     for (size_t i = 0; i < g.layers; ++i) {
         const Layer& l = g.blocks[i];
         DenseLayer dense;
+        // (Ahead of the LayerNorm: the GEMM behind it fetches weights before its wait, see common.h.)
         FB_TRY(dense_weights(g, i, &dense, stream));
         FB_TRY(layernorm(g, l.ln1_w, l.ln1_b, g.x_a, rows, stream));
         FB_TRY(linear<Act::kNone>(g, l.attn, dense.attn, g.qkv, g.h, nullptr, rows, stream));

@@ -88,3 +88,46 @@ def test_kernels_that_read_before_their_wait_stand_behind_an_ordinary_launch():
         assert f"{first}<<<" in body and body.index(f"{first}<<<") < body.index(then)
         between = body[body.index(f"{first}<<<"):body.index(then)]
         assert "launch_dependent" not in between
+
+
+def function_body(text, name):
+    body = text[re.search(rf"\n\S[^\n;]*\b{name}\(", text).start():]
+    return body[:body.index("\n}\n")]
+
+
+def launches_in_order(body):
+    """The launching calls of a function of generate.cu, in source order."""
+    return re.findall(r"\b(dense_weights|layernorm|decode_linear|linear<Act::\w+>|fb_cache_store|attention_forward|"
+                      r"fb_decode_attention|flint_embedding_forward|run_prompt)\(", body.replace("fb_cache_store,", "fb_cache_store("))
+
+
+def steady_weights_have_a_kernel_between(text):
+    """linear() tells its GEMM that the weights are steady, so that it fetches some before its wait. What may have
+    written them just before is dense_weights' expansion, or, ahead of a prompt, anything."""
+    prompt = launches_in_order(function_body(text, "run_prompt"))
+    expansion = prompt.index("dense_weights")
+    first_gemm = next(i for i, name in enumerate(prompt) if name.startswith("linear<"))
+    prefill = launches_in_order(function_body(text, "flint_b200_generator_prefill"))
+    return (prompt.count("dense_weights") == 1 and first_gemm - expansion >= 2
+            and prefill.index("flint_embedding_forward") < prefill.index("run_prompt"))
+
+
+def test_weights_fetched_before_the_wait_were_written_a_kernel_earlier():
+    text = re.sub(r"//[^\n]*", "", (SOURCES[0].parent / "generate.cu").read_text())
+    assert steady_weights_have_a_kernel_between(text)
+    # Only linear() says so, and it is called behind an expansion (above) or an ordinary launch
+    # (test_kernels_that_read_before_their_wait_stand_behind_an_ordinary_launch).
+    assert text.count("stream, true));") == 3 == function_body(text, "linear").count("stream, true));")
+    gemm = re.sub(r"//[^\n]*", "", (SOURCES[0].parent / "gemm.cu").read_text())
+    once = gemm[gemm.index("fb_gemm_once(const"):]
+    ahead = once[:once.index("dependency_wait()")]
+    assert re.findall(r"\bearly = ([^;]*);", ahead) == ["once.steady_b != 0 ? min(stages, blocks) : 0"]
+    assert re.findall(r"&p\.map_\w", ahead.split("auto fetch_b")[1].split("};")[1]) == []
+
+
+def test_the_check_notices_an_expansion_right_before_its_gemm():
+    text = (SOURCES[0].parent / "generate.cu").read_text()
+    expansion = re.search(r"\n *FB_TRY\(dense_weights\([^\n]*", text).group(0)
+    norm = re.search(r"\n *FB_TRY\(layernorm\(g, l\.ln1_w[^\n]*", text).group(0)
+    assert expansion + norm in text
+    assert not steady_weights_have_a_kernel_between(text.replace(expansion + norm, norm + expansion))
