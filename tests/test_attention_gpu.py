@@ -71,6 +71,33 @@ def test_attention_of_few_heads(flint, batches, length, size):
     assert np.allclose(lse.cpu().numpy(), want_lse, rtol=1e-4, atol=1e-4)
 
 
+# As above, but with more items than SMs: a CTA's second item, of two to seven key tiles, goes through the
+# memory that its first one's halves were merged in. Cold and warm loads must give the same bits.
+@pytest.mark.parametrize("batches, length", [(24, 1024), (30, 1000), (34, 1024)])
+def test_attention_of_few_heads_in_a_second_round(flint, batches, length):
+    g = torch.Generator().manual_seed(length + batches)
+    q, k, v = (torch.randn(batches, length, 64, generator=g).half() for _ in range(3))
+    k[:, torch.arange(length) // 128 % 2 == 1] *= 4
+    want_o, want_lse = oracle.attention(q, k, v, 0.125)
+    qd, kd, vd = (t.to(DEV) for t in (q, k, v))
+    flush = torch.empty(256 << 20, dtype=torch.uint8, device=DEV)
+    first = None
+    for trial in range(6):
+        o = torch.full((batches, length, 64), float(trial), dtype=torch.half, device=DEV)
+        lse = torch.full((batches, length), float(trial), device=DEV)
+        if trial % 2 == 0:
+            flush.fill_(trial)
+        flint.attention_forward(o, lse, qd, kd, vd, batches, length, 64, 0.125)
+        torch.cuda.synchronize()
+        assert not flint.kernel_fault()
+        if first is None:
+            first = (o, lse)
+            assert rel_error(o, want_o) <= 2e-3
+            assert np.allclose(lse.cpu().numpy(), want_lse, rtol=1e-4, atol=1e-4)
+        assert torch.equal(o.view(torch.int16), first[0].view(torch.int16))
+        assert torch.equal(lse.view(torch.int32), first[1].view(torch.int32))
+
+
 # Keys whose score is minus infinity (an infinity in K) weigh nothing, wherever they lie: one key, which is the
 # only one that a row sees in an odd key tile; the key tiles that one of two accumulators gets, first and
 # only ones among them; the first keys of all, before which a row sees none (0 / 0: NaN, as from softmax).

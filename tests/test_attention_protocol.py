@@ -15,7 +15,9 @@ against the data it must see:
 * S(n + 3) executing before P V(n) has read the buffer, P V(n) before all eight warps wrote P;
 * a softmax warp reading scores that are not there yet or already overwritten, rescaling or
   reading O before the P V it needs has finished;
-* a ring slot or a query buffer reloaded before its readers are done; a deadlock.
+* a ring slot or a query buffer reloaded before its readers are done; a deadlock;
+* by_keys (few heads; two accumulators share a query tile's keys): the second accumulator's values
+  handed over before they are there, or written over while the first one's warps still read.
 
 Two tests put two earlier forms of the forward kernel's final waits into the model and require
 the checker to find their faults, which is what pins the model's power to find that class of bug.
@@ -54,10 +56,11 @@ class Barrier:
 
 
 class Cursor:
-    """FwdCursor with enter()/advance(): item `round` of this CTA, key tile j, query tile t."""
+    """FwdCursor with enter()/advance(): item `round` of this CTA, key tile j, query tile t. by_keys: one
+    query tile, of whose key tiles t takes t, t + 2, ... (one too many where their number is odd)."""
 
-    def __init__(self, items, round_=0):
-        self.items, self.round, self.j, self.t = items, round_, 0, 0
+    def __init__(self, items, round_=0, by_keys=False):
+        self.items, self.round, self.j, self.t, self.by_keys = items, round_, 0, 0, by_keys
 
     @property
     def valid(self):
@@ -67,11 +70,15 @@ class Cursor:
     def qb(self):
         return self.items[self.round]
 
+    @property
+    def last(self):
+        return self.qb // 2 if self.by_keys else self.qb
+
     def advance(self):
         self.t ^= 1
         if self.t == 0:
             self.j += 1
-            if self.j > self.qb:
+            if self.j > self.last:
                 self.round, self.j = self.round + 1, 0
 
     def key(self):
@@ -79,12 +86,14 @@ class Cursor:
 
 
 class Model:
-    def __init__(self, items, seed, variant="kernel"):
+    def __init__(self, items, seed, variant="kernel", by_keys=False):
         self.items = items                      # query tile index (qb) of each item
+        self.by_keys = by_keys
         self.rng = random.Random(seed)
         # "kernel": what the kernel does. Two earlier forms, kept to show that the checker finds
         # their faults: "single" waits only for the last P V; "after_arrival" waits for the last
-        # but one as well, but after the warp's last arrival.
+        # but one as well, but after the warp's last arrival. "no_item_sync": a by_keys item whose
+        # halves are merged without waiting for one another.
         self.variant = variant
         self.bar = {}
         for b in range(2):
@@ -98,6 +107,10 @@ class Model:
             self.bar["slot_full", s] = Barrier(f"slot_full{s}", 1)
             self.bar["slot_empty", s] = Barrier(f"slot_empty{s}", 1)
         self.pair_sync = {}                     # (tile, quadrant, count) -> arrivals
+        self.item_sync = {}                     # (quadrant, round) -> arrivals
+        self.handed = {}                        # (quadrant, half) -> round of tile 1's values there
+        self.handed_stats = {}                  # quadrant -> round of tile 1's maxima and sums there
+        self.taken = {}                         # (quadrant, half) -> rounds read by tile 0
         # Data state.
         self.slot_content = [None] * SLOTS      # tile id now readable in the slot
         self.slot_readers_done = [True] * SLOTS
@@ -108,11 +121,14 @@ class Model:
         self.tma = []                           # pending loads: (kind, payload)
         self.pipe = []                          # MMA groups and commits, in issue order
         self.steps = []                         # step number -> (round, j, t)
-        c = Cursor(items)
+        c = self.cursor()
         while c.valid:
             self.steps.append(c.key())
             c.advance()
         self.step_of = {key: n for n, key in enumerate(self.steps)}
+
+    def cursor(self):
+        return Cursor(self.items, by_keys=self.by_keys)
 
     # ---- waits -----------------------------------------------------------------------------
     def wait(self, kind, index, parity, phase):
@@ -127,7 +143,7 @@ class Model:
     # ---- roles -----------------------------------------------------------------------------
     def producer(self):
         slot, phase = 0, 0
-        keys, values = Cursor(self.items), Cursor(self.items)
+        keys, values = self.cursor(), self.cursor()
         loads = {"k": 0, "v": 0}
         ahead = 0
         uses = [0] * SLOTS
@@ -165,7 +181,7 @@ class Model:
     def mma_warp(self):
         slot, phase = 0, 0
         uses = [0] * SLOTS
-        ahead = Cursor(self.items)
+        ahead = self.cursor()
         issued = 0
 
         def next_tile(expect):
@@ -193,7 +209,7 @@ class Model:
             self.pipe.append(("scores", issued, slot, b, ahead.round))
             self.pipe.append(("commit", ("s_full", issued % 3)))
             self.pipe.append(("commit", ("slot_empty", slot)))
-            if ahead.t == 1 and ahead.j == ahead.qb:
+            if ahead.t == 1 and ahead.j == ahead.last:
                 self.pipe.append(("commit", ("q_empty", b)))
             step_ring()
             issued += 1
@@ -201,7 +217,7 @@ class Model:
 
         for _ in range(3):
             yield from issue_scores()
-        at = Cursor(self.items)
+        at = self.cursor()
         n = 0
         while at.valid:
             yield from self.wait("p_ready", n % 3, (n // 3) & 1, n // 3)
@@ -218,7 +234,8 @@ class Model:
     def softmax_warp(self, tile, quadrant, half):
         before = 0
         for round_, qb in enumerate(self.items):
-            for j in range(qb + 1):
+            last_j = qb // 2 if self.by_keys else qb
+            for j in range(last_j + 1):
                 n = 2 * (before + j) + tile
                 need(self.steps[n] == (round_, j, tile), "step numbering out of line")
                 yield from self.wait("s_full", n % 3, (n // 3) & 1, n // 3)
@@ -238,20 +255,45 @@ class Model:
                 yield
                 need((n + 3) not in self.s_started, f"P of step {n} written over newer scores")
                 self.p_written[n] = self.p_written.get(n, 0) + 1
-                if self.variant == "kernel" and j == qb and qb > 0:
+                if self.variant in ("kernel", "no_item_sync") and j == last_j and last_j > 0:
                     # Before the arrival that lets the item's last P V be issued at all.
-                    yield from self.wait("pv_done", tile, (before + qb - 1) & 1, before + qb - 1)
+                    yield from self.wait("pv_done", tile, (before + last_j - 1) & 1, before + last_j - 1)
                 self.bar["p_ready", n % 3].arrive()
                 yield
-            if self.variant == "after_arrival" and qb > 0:
-                yield from self.wait("pv_done", tile, (before + qb - 1) & 1, before + qb - 1)
-            yield from self.wait("pv_done", tile, (before + qb) & 1, before + qb)
-            last = 2 * (before + qb) + tile
+            if self.variant == "after_arrival" and last_j > 0:
+                yield from self.wait("pv_done", tile, (before + last_j - 1) & 1, before + last_j - 1)
+            yield from self.wait("pv_done", tile, (before + last_j) & 1, before + last_j)
+            last = 2 * (before + last_j) + tile
             need(last in self.pv_done, f"O of item {round_} read before its last P V (step {last})")
-            need((last + 2) not in self.pv_started or qb + 1 == 0,
+            need((last + 2) not in self.pv_started or last_j + 1 == 0,
                  "O read after the next item's first P V started")
-            before += qb + 1
+            before += last_j + 1
             yield
+            if self.by_keys:
+                yield from self.merge(round_, qb, tile, quadrant, half)
+
+    def merge(self, round_, qb, tile, quadrant, half):
+        """Tile 1's accumulator, maxima and sums go to tile 0 through shared memory, which the next
+        item's go through again."""
+        if tile == 1:
+            before = [r for r in range(round_) if self.items[r] > 0]      # the items that were merged
+            for reader in (half,) if half else (0, 1):       # half 0 writes the statistics of both
+                need(not before or before[-1] in self.taken.get((quadrant, reader), set()),
+                     f"tile 1's values of item {round_} written over earlier ones that are still read")
+            self.handed[quadrant, half] = round_
+            if half == 0:
+                self.handed_stats[quadrant] = round_
+        if self.variant != "no_item_sync":
+            key = (quadrant, round_)
+            self.item_sync[key] = self.item_sync.get(key, 0) + 1
+            while self.item_sync[key] < 4:
+                yield
+        if tile == 0 and qb > 0:
+            for _ in range(2):      # the read takes its time
+                need(self.handed.get((quadrant, half)) == round_ and self.handed_stats.get(quadrant) == round_,
+                     f"item {round_} merged with values of another item, or with none")
+                yield
+            self.taken.setdefault((quadrant, half), set()).add(round_)
 
     # ---- engines ---------------------------------------------------------------------------
     def run_tma(self):
@@ -353,6 +395,36 @@ def test_the_checker_notices_a_wait_that_comes_too_late():
         except Violation as violation:
             found += 1
             assert "deadlock" in str(violation)
+    assert found > 0
+
+
+@pytest.mark.parametrize("items", ITEM_LISTS + [[7, 0, 7, 0], [1, 1, 1], [6, 5, 4, 3]], ids=str)
+def test_forward_protocol_by_keys_holds_under_random_schedules(items):
+    for seed in range(40):
+        Model(items, seed, by_keys=True).run()
+
+
+@pytest.mark.parametrize("items", [[7], [1], [7, 7], [2, 1, 0]], ids=str)
+def test_the_checker_notices_halves_merged_without_a_barrier(items):
+    found = 0
+    for seed in range(200):
+        try:
+            Model(items, seed, variant="no_item_sync", by_keys=True).run()
+        except Violation as violation:
+            found += 1
+            assert "merged with" in str(violation) or "still read" in str(violation)
+    assert found > 0
+
+
+@pytest.mark.parametrize("variant, message", [("single", "aliased wait"), ("after_arrival", "deadlock")])
+def test_the_checker_finds_the_earlier_faults_by_keys_too(variant, message):
+    found = 0
+    for seed in range(200):
+        try:
+            Model([15, 9, 3], seed, variant=variant, by_keys=True).run()
+        except Violation as violation:
+            found += 1
+            assert message in str(violation) or "O of item" in str(violation)
     assert found > 0
 
 
