@@ -98,6 +98,11 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // probabilities then stay below 2^8, well inside FP16.
 constexpr float kLazyShift = 8.0f;
 
+// The reference exponent of a row for which no key has counted so far: the least finite value, so that
+// keys of minus infinity (an infinity in K, or a mask) give probabilities of 2^-inf where -inf - -inf would be
+// NaN, and the first key that counts moves it.
+constexpr float kNoKey = -3.402823466e38f;
+
 // 2^x for two values at once on the FMA pipe, for the share of the forward kernel's
 // exponentials that the special-function unit has no time for: x = n + f with n the
 // nearest integer (taken from the low mantissa bits of x + 1.5 * 2^23), 2^f by a
@@ -491,7 +496,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
             const int bh = head_of(item, tile);
             const bool stores = by_keys ? tile == 0 : 2 * item.pair + tile < bh_count;
             const int q_index = qb * kTile + row;
-            float m = -INFINITY;  // reference exponent of the row (base 2), shared by the pair
+            float m = kNoKey;     // reference exponent of the row (base 2), shared by the pair
             fb::F2 l = 0;         // this thread's share of the row sum, in two partial sums
             for (int j = 0; j <= last; ++j) {
                 const uint32_t n = 2 * (before + j) + tile;   // this step's number
@@ -536,7 +541,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 pair_max[tile][parity][half][row] = local;
                 quadrant_sync(pair_barrier);
                 const float mx = fmaxf(m, fmaxf(local, pair_max[tile][parity][half ^ 1][row]));
-                const bool moved = mx - m > kLazyShift;   // always on the first tile (m = -inf)
+                const bool moved = mx - m > kLazyShift;   // always on the first tile with a key that counts
                 float alpha = 1.0f;
                 if (moved) {
                     alpha = fast_exp2(m - mx);
@@ -566,9 +571,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                         sm100::tmem_st_32x16(my_output + c * 16, acc);
                     }
                 }
-                // (While every key so far scored minus infinity, m is that: -inf - -inf would be NaN.)
-                const float reference = m == -INFINITY ? 0.0f : m;
-                const fb::F2 shift = fb::f2_pack(-reference, -reference);
+                const fb::F2 shift = fb::f2_pack(-m, -m);
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     uint32_t packed[16];
@@ -647,9 +650,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                 if (tile == 0 && qb > 0) {   // (with one key tile, tile 1 saw none)
                     const float other = merge_max[row];
                     const float top = fmaxf(m, other);
-                    // A half whose keys all scored minus infinity weighs nothing.
-                    const float reference = top == -INFINITY ? 0.0f : top;
-                    const float mine_by = fast_exp2(m - reference), other_by = fast_exp2(other - reference);
+                    const float mine_by = fast_exp2(m - top), other_by = fast_exp2(other - top);
                     total = total * mine_by + merge_sum[row] * other_by;
                     m = top;
 #pragma unroll
@@ -667,8 +668,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1)
                     }
                 }
             }
-            if (m == -INFINITY) {
-                total *= 0.0f;   // no key counts: 0 / 0 (the polynomial's least power of two is not 0)
+            if (m == kNoKey) {
+                total *= 0.0f;   // 0 / 0 (the polynomial's least power of two is not 0)
             }
             if (there && stores && q_index < p.length) {
                 const float inv = 1.0f / total;
