@@ -15,7 +15,7 @@
 // main loop of tile i+1. Every k-block is 64 wide for every layout, so all
 // variants of a shape add their products in the same order and the batched
 // forms reproduce the plain ones bit for bit. (Small outputs with a long k take their
-// sums in two or four parts, by a rule on the shape alone.) Large problems run on
+// sums in two or four parts, by a rule on the shape alone, the number of rows included.) Large problems run on
 // CTA pairs (fb_gemm_pair), those of a single round on fb_gemm_once.
 //
 // Operand layouts map onto UMMA "major-ness" instead of register transposes:
@@ -65,7 +65,6 @@ struct GemmParams {
     float* partials;      // split TN: [split][m][n] FP32
     int m, n, k;
     int batches;          // 1 for the plain forms
-    int parts;            // of a sum over k, each in order, then added in order (kernels for parts only)
     int splits;           // TN only
     int split_len;        // k per split, a multiple of 64
     int tiles_m, tiles_n;
@@ -73,6 +72,9 @@ struct GemmParams {
     float scale;
     int accumulate;
     int batched;
+    // Parts of a sum over k, each in order, then added in order (kernels for parts only). Last, where it moves no other
+    // member: behind `batches` it did, and single rounds on fb_gemm_tc took 0.1 us more (NN 4,096 x 512 x 512 5.54 -> 5.70).
+    int parts;
 };
 
 // ---- epilogue math ----------------------------------------------------------------
@@ -1609,7 +1611,7 @@ __device__ __forceinline__ TileCoord decode_pair_tile(const GemmParams& p, long 
 // eight, 28 % of the issue slots and 30 % of the special-function unit are in use), and at k = 768 a tile's
 // epilogue outlasts its k loop: 8,192 x 3,072 x 768 44.8 -> 42.5 us, 16,384 rows 94.2 -> 85.0, for a stage
 // of the ring. With a longer k the loop counts for more: 8,192 x 4,096 and 16,384 x 3,072 gain 2 % at k = 896
-// and lose 5 and 7 % at 1,024. In a single round there is nothing to gain (1,000 x 4,104 x 768 12.5 -> 13.1).
+// and lose 5 and 7 % at 1,024 (2,048 x 3,072 gains 4 %, 8,192 x 1,024 loses 11). In a single round there is nothing to gain (1,000 x 4,104 x 768 12.5 -> 13.1).
 // (Four for dGELU 51.4 -> 59 us, which then has no registers to ask for its pre-activations a chunk ahead;
 // for bias+residual 42 -> 45.) The scaled batched product of k = 64, attention's scores, is epilogue alone:
 // 24 x 1,024 x 1,024 15.0 -> 13.2 us, 48 x 512 x 512 9.9 -> 8.7.
