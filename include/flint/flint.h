@@ -67,7 +67,10 @@ FLINT_API flint_status flint_copy(void* dst, const void* src, size_t bytes, flin
  * Shared limits (ref: flint.h:59-62): all pointers 16-byte aligned, m and n at
  * most 8,388,480, k at most 65,536, outputs disjoint from inputs, and m == 0
  * or n == 0 succeeds without touching anything. Outputs that are FP16 round
- * once, to nearest even, from the FP32 value (overflow gives inf). */
+ * once, to nearest even, from the FP32 value (overflow gives inf). A sum over k
+ * is taken in order, or in two or four parts whose sums are then added in order:
+ * by a rule on m, n, k and the GPU's SM count that all forms of a product share,
+ * so that their bits agree; a row's bits can differ between two values of m. */
 
 /* y[m,n] = x[m,k] * w[n,k]^T, FP16 out. k a positive multiple of 8.
  * ref: flint.h:53-64 */
