@@ -1611,13 +1611,14 @@ __device__ __forceinline__ TileCoord decode_pair_tile(const GemmParams& p, long 
 // eight, 28 % of the issue slots and 30 % of the special-function unit are in use), and at k = 768 a tile's
 // epilogue outlasts its k loop: 8,192 x 3,072 x 768 44.8 -> 42.5 us, 16,384 rows 94.2 -> 85.0, for a stage
 // of the ring. With a longer k the loop counts for more: 8,192 x 4,096 and 16,384 x 3,072 gain 2 % at k = 896
-// and lose 5 and 7 % at 1,024 (2,048 x 3,072 gains 4 %, 8,192 x 1,024 loses 11). In a single round there is nothing to gain (1,000 x 4,104 x 768 12.5 -> 13.1).
+// and lose 5 and 7 % at 1,024 (2,048 x 3,072 gains 4 %, 8,192 x 1,024 loses 11). In a single round there is
+// nothing to gain (1,000 x 4,104 x 768 12.5 -> 13.1).
 // (Four for dGELU 51.4 -> 59 us, which then has no registers to ask for its pre-activations a chunk ahead;
 // for bias+residual 42 -> 45.) The scaled batched product of k = 64, attention's scores, is epilogue alone:
 // 24 x 1,024 x 1,024 15.0 -> 13.2 us, 48 x 512 x 512 9.9 -> 8.7.
 // Rows that are no multiples of 32 bytes share sectors, and where the outputs outgrow two thirds of the L2,
-// sixteen warps lose by it: scores of 48 x 904 x 904 24.3 -> 23.2 us but 48 x 1,000 x 1,000 x 128 28.9 -> 32.0, 96 x 904 x 904 44.8 -> 51.5
-// (96 x 992 x 992 44.3 -> 40.2); bias+GELU 8,192 x 2,312 x 512 34.3 -> 31.0 but 8,192 x 4,104 x 768 63.0 -> 65.5.
+// sixteen warps lose by it: scores of 48 x 904 x 904 24.3 -> 23.2 us but 48 x 1,000 x 1,000 x 128 28.9 -> 32.0,
+// 96 x 904 x 904 44.8 -> 51.5 (96 x 992 x 992 44.3 -> 40.2); bias+GELU 8,192 x 2,312 x 512 34.3 -> 31.0 but 8,192 x 4,104 x 768 63.0 -> 65.5.
 constexpr int kManyWarps = 16;
 constexpr size_t kManyWarpsMostK = 960;
 constexpr size_t kManyWarpsMostScaledK = 128;
